@@ -42,7 +42,7 @@ SHAPES = {
 def listed():
     return [
         # the smallest calls: a tiny float32 model answers four prompts of very different lengths; launches and host work count
-        case("tiny chat, float32", "qwen2", "tiny-b", 3, "float32", "turn", batch=4, context=257, spread=1.0, steps=24, page=32),
+        case("tiny chat float32", "qwen2", "tiny-b", 3, "float32", "turn", batch=4, context=257, spread=1.0, steps=24, page=32),
         # one user, long context: every weight is read for one token
         case("decode 1 x 4096", "qwen2", "7b", 8, "bfloat16", "decode", batch=1, context=4096),
         # the headline: eight users with about 4,096 tokens each
@@ -56,7 +56,7 @@ def listed():
         # the 32B long-prompt workload: the last portion of an 8,192-token prompt
         case("portion 2048 at 6144", "qwen2", "32b", 2, "bfloat16", "mixed", batch=1, context=6144, tokens=2048),
         # the 32-bit path at full width: three ragged prompts
-        case("prompts 3 x 250, float32", "qwen2", "7b", 2, "float32", "prompt", batch=3, context=250, spread=0.5),
+        case("prompts 3 x 250 float32", "qwen2", "7b", 2, "float32", "prompt", batch=3, context=250, spread=0.5),
         # the other designs at the sizes of their comparison: first tokens, and turns in which decoding has the larger part
         case("koronex prompt 2048", "koronex", "4k", 8, "bfloat16", "prompt", batch=1, context=2048),
         case("koronex turn 8 x 300", "koronex", "2k", 8, "bfloat16", "turn", batch=8, context=300, spread=0.6, steps=24),
