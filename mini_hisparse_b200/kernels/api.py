@@ -326,6 +326,34 @@ def gemm_simt(a, w, out, bias=None, nsplit=1, split_stride=0):
         c_int(nsplit), c_longlong(split_stride), _stream()), "gemm_simt")
 
 
+def gemm_f32_takes(a, w) -> bool:
+    """The float32 kernels of csrc/gemm_f32.cu take these operands (K in steps of 8, rows on 16 bytes)."""
+    return (a.dtype == torch.float32 and w.dtype == torch.float32 and a.shape[1] % 8 == 0 and a.stride(1) == 1
+            and w.stride(1) == 1 and a.stride(0) % 4 == 0 and w.stride(0) % 4 == 0 and a.data_ptr() % 16 == 0
+            and w.data_ptr() % 16 == 0)
+
+
+def gemm_f32(a, w, out, bn=0, nsplit=1, split_stride=0, parts=None, status=None):
+    """out[M, N] = a[M, K] @ w[N, K]^T in float32.  ``bn`` 0 (up to 8 rows): the weights stream through the CUDA cores.
+    64, 128 or 192: tiles of that many rows of ``a`` on the tensor cores, every number as three bfloat16 parts;
+    ``parts`` is scratch for 3 M K bfloat16, and with ``nsplit`` > 1 part z of K goes to out + z * split_stride.
+    ``w`` must not be written by the kernel launched before this one (weights)."""
+    lib = build.load("gemm_f32")
+    M, K = a.shape
+    N = w.shape[0]
+    if w.shape[1] != K:
+        raise KernelError(f"gemm: a is [{M},{K}] but w is {list(w.shape)}")
+    if a.stride(1) != 1 or w.stride(1) != 1 or out.stride(-1) != 1:
+        raise KernelError("gemm: the last dimension must be contiguous")
+    if a.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32:
+        raise KernelError("gemm_f32: operands and output are float32")
+    if bn and (parts is None or parts.dtype != torch.bfloat16 or parts.numel() < 3 * M * K):
+        raise KernelError("gemm_f32: the scratch for the rows' parts is too small")
+    _check(lib, lib.mhb_gemm_f32(_ptr(a), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), c_longlong(a.stride(0)),
+                                 c_longlong(w.stride(0)), c_longlong(out.stride(-2)), c_int(bn), c_int(nsplit),
+                                 c_longlong(split_stride), _ptr(parts), _ptr(status), _stream()), "gemm_f32")
+
+
 STREAM_K_PARTIAL_FLOATS = 2 * 160 * 128 * 256     # workspace of the persistent product: two tiles per CTA
 STREAM_K_FLAGS = 4 << 16                            # a counter for each quarter of each tile
 

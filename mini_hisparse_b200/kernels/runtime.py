@@ -1,6 +1,7 @@
 """The runtime of each compute dtype: which kernel a part's matrix product runs on.
 
-float32: the CUDA-core product (true 32-bit: FFMA, no tensor core, no reduced-precision mode).
+float32: every operand enters with all of its 24 bits and every sum is float32.  Up to 8 tokens the weights stream through
+the CUDA cores; with more, the tensor cores multiply exact sums of three bfloat16 parts (csrc/gemm_f32.cu).
 bfloat16: the tcgen05 tensor-core product; with up to 64 tokens the weights stream through the
 128-row operand and the K range is split over enough CTAs to fill the GPU (the consumer sums
 the partial matrices in order); with more, a persistent kernel gives every SM the same share
@@ -19,8 +20,55 @@ MIN_KB_PER_SPLIT = 4
 
 
 class Float32Runtime(Runtime):
+    def __init__(self, device, dtype=torch.float32):
+        super().__init__(device, dtype)
+        self.sm_count = torch.cuda.get_device_properties(self.device).multi_processor_count
+        self.status = None      # set by the runner: kernels report bounded waits that ran out
+
     def kernel_modules(self):
-        return ("elementwise", "gemm_simt", "sampling")
+        return ("elementwise", "gemm_simt", "gemm_f32", "sampling")
+
+    F32_BLOCK = 32          # elements of K in a block of the tensor-core product
+    # a CTA's time per block in us, measured at 7B-shape sizes, by its tokens: with tiles of 64 two CTAs share an SM
+    F32_BLOCK_US = {64: 1.3, 128: 1.0, 192: 1.3}
+
+    def _tile(self, M: int, N: int, Kd: int, allow_split: bool) -> tuple[int, int]:
+        """(tokens a CTA, K splits) of the product with more than 8 tokens: the pair whose rounds of CTAs, each as long as
+        its blocks and 6 blocks' time for its start and end, are done first, counting 8 bytes at 5 TB/s for every number
+        of a further partial matrix.  Measured (us): 750 x 3584 x 4608 147 with (192, 1) against 209 (128, 1) and 210
+        (64, 2); 64 x 18944 x 3584 87 with (64, 10) against 573 (64, 1); 400 x 3584 x 4608 110 with (128, 1), 136 (192, 1)."""
+        blocks = -(-Kd // self.F32_BLOCK)
+        best, best_us = (64, 1), None
+        for bn, us in self.F32_BLOCK_US.items():
+            if bn > 64 and M <= bn - 64:
+                break
+            tiles = -(-M // bn) * -(-N // 128)
+            slots = self.sm_count * (2 if bn == 64 else 1)
+            for n in range(1, (min(12, max(1, blocks // 8)) if allow_split else 1) + 1):
+                per = -(-blocks // n)
+                if (n - 1) * per >= blocks:
+                    continue
+                t = -(-tiles * n // slots) * (per + 6) * us + (n - 1) * M * N * 8 / 5e6
+                if best_us is None or t < best_us:
+                    best, best_us = (bn, n), t
+        return best
+
+    def linear(self, x, weight, ws: Workspace, name: str, out_dtype=None, bias=None, allow_split: bool = True) -> Product:
+        """K in steps of 8 and aligned rows: the kernels of gemm_f32 (CUDA cores up to 8 tokens, three bfloat16 parts on
+        the tensor cores beyond); any other shape, and a product with a bias: the general CUDA-core kernel."""
+        M, N, Kd = x.shape[0], weight.shape[0], x.shape[1]
+        if bias is not None or (out_dtype or self.dtype) != torch.float32 or not K.gemm_f32_takes(x, weight):
+            return super().linear(x, weight, ws, name, out_dtype, bias, allow_split)
+        if M <= 8:
+            out = ws.get(name, (M, N), torch.float32)
+            K.gemm_f32(x, weight, out)
+            return Product(out)
+        bn, nsplit = self._tile(M, N, Kd, allow_split)
+        parts = ws.get(name + "_parts", (3, M, Kd), torch.bfloat16)
+        out = ws.get(name, (nsplit, M, N) if nsplit > 1 else (M, N), torch.float32)
+        K.gemm_f32(x, weight, out, bn=bn, nsplit=nsplit, split_stride=out.stride(0) if nsplit > 1 else 0, parts=parts,
+                   status=self.status)
+        return Product(out, nsplit)
 
 
 class BFloat16Runtime(Runtime):

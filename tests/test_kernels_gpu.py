@@ -141,6 +141,53 @@ def test_gemm_is_true_float32():
     assert abs(float(out[0, 0]) - exact) < 1e-4
 
 
+@pytest.mark.parametrize("M,N,K_,bn,nsplit", [
+    (1, 5, 8, 0, 1), (2, 2400, 136, 0, 1), (3, 97, 1000, 0, 1), (4, 2369, 2056, 0, 1), (8, 130, 4104, 0, 1), (7, 2400, 520, 0, 1),
+    (9, 130, 8, 64, 1), (64, 128, 32, 64, 1), (65, 127, 40, 64, 2), (33, 300, 1000, 64, 5), (128, 129, 96, 128, 1),
+    (130, 128, 520, 128, 3), (97, 40, 2056, 128, 2), (192, 256, 64, 192, 1), (193, 130, 488, 192, 4), (400, 33, 3592, 192, 1),
+])
+@pytest.mark.parametrize("kind", ["signed", "positive", "special"])
+def test_gemm_f32(M, N, K_, bn, nsplit, kind):
+    """The float32 products at the edges of their tiles.  Bound, element by element, in units of S = sum |a||w|: the kernel
+    adds at most 14 tensor-core steps of 2^-23 S inside a block of 32, one rounding of 2^-24 per block, three parts' products
+    below 2^-24 that are left out; the CUDA-core kernel at most K / 128 + 9 roundings a lane and the sums across lanes and
+    splits.  "special": infinities and NaN come out where a chain of multiplications and additions puts them."""
+    a, w = rnd(M, K_, seed=1), rnd(N, K_, seed=2)
+    if kind == "positive":
+        a, w = a.abs(), w.abs()
+    if kind == "special":
+        a[M // 2, K_ // 2] = math.inf
+        a[0, 0] = math.nan
+        w[N - 1, K_ // 2] = -math.inf
+        a[M - 1, K_ - 1] = 3.4e38          # its first 8 bits round to infinity
+        w[:, K_ - 1] = 2.0 ** -20          # ... and none of its products overflows, which 64 bits would not show
+    out = torch.full((nsplit, M, N), math.nan, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    parts = torch.empty(3 * M * K_, dtype=torch.bfloat16, device=DEV) if bn else None
+    K().gemm_f32(a, w, out, bn=bn, nsplit=nsplit, split_stride=out.stride(0), parts=parts, status=status)
+    got, ref = out.double().sum(0), a.double() @ w.double().T
+    assert int(status) == 0
+    if kind == "special":
+        ref = ref.float().double()
+        assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got[got.isinf()], ref[ref.isinf()])
+    room = (14 * 2.0 ** -23 + (K_ / 32 + 20) * 2.0 ** -24) * (a.abs().double() @ w.abs().double().T)
+    fine = ref.isfinite()
+    assert ((got - ref).abs() <= room)[fine].all()
+
+
+def test_gemm_f32_takes():
+    """What the float32 kernels do not take is refused by the entry point and known beforehand."""
+    a, w = rnd(20, 64, seed=1), rnd(30, 64, seed=2)
+    assert K().gemm_f32_takes(a, w)
+    assert not K().gemm_f32_takes(a[:, :60], w[:, :60])           # K in steps of 8
+    assert not K().gemm_f32_takes(a[:, 1:57], w[:, :56])          # rows off 16 bytes
+    assert not K().gemm_f32_takes(a.bfloat16(), w)
+    out = torch.empty(20, 30, device=DEV)
+    for bad in (dict(), dict(bn=64), dict(bn=100, parts=torch.empty(3 * 20 * 64, dtype=torch.bfloat16, device=DEV))):
+        with pytest.raises(Exception, match="gemm_f32"):
+            K().gemm_f32(a, w, out, **bad)
+
+
 @pytest.mark.parametrize("M,N,K_,swap,bn,nsplit", [
     (128, 128, 64, False, 128, 1), (200, 300, 136, False, 128, 1), (333, 1000, 3584, False, 256, 1),
     (70, 520, 200, False, 128, 2), (8, 256, 512, True, 16, 1), (1, 777, 96, True, 16, 1),
@@ -504,6 +551,21 @@ def run_attention(nq, nkv, d, P_, seg_specs, dtype, window=None, fixed_nsplit=No
         for qq, kk, vv, (h, n) in zip(qs, ks, vs, seg_specs)
     ]).reshape(T, nq * d)
     return out.float().cpu(), ref, plan
+
+
+@pytest.mark.parametrize("nq,nkv,d,P_,dtype", [
+    (3, 1, 16, 16, torch.float32), (7, 7, 20, 5, torch.float32), (4, 2, 23, 3, torch.float32), (28, 4, 128, 16, torch.float32),
+    (18, 1, 256, 1, torch.float32), (5, 5, 184, 64, torch.float32), (4, 2, 24, 16, torch.bfloat16), (4, 2, 20, 7, torch.bfloat16),
+    (6, 1, 256, 16, torch.bfloat16)])
+def test_attention_simt_staging(nq, nkv, d, P_, dtype):
+    """The CUDA-core kernel's ways to stage a tile: 16-byte pieces or single elements (widths that are no whole number of
+    pieces), two buffers or one (wide rows), with no key, one, a tile's edge and many tiles, and splits of 64 keys."""
+    specs = [(0, 1), (30, 1), (31, 1), (32, 2), (63, 1), (200, 17), (330, 1)]
+    out, ref, plan = run_attention(nq, nkv, d, P_, specs, dtype)
+    assert plan.part_rows > 3
+    torch.testing.assert_close(out, ref, **tol(dtype, 4))
+    out, ref, _ = run_attention(nq, nkv, d, P_, specs, dtype, window=33, fixed_nsplit=3)
+    torch.testing.assert_close(out, ref, **tol(dtype, 4))
 
 
 @pytest.mark.parametrize("nq,nkv,d,P_", [(4, 2, 32, 16), (3, 1, 32, 32), (28, 4, 128, 16), (20, 1, 96, 8),
