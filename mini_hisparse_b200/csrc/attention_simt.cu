@@ -41,6 +41,7 @@
 //   vheads     nkv instead of 1: a query head's weights are applied to the values of EVERY KV head, and the
 //              output row is [nkv][dv] wide (for a mixer that mixes the heads' weights afterwards)
 #include "common.cuh"
+#include "mma_helpers.cuh"
 
 using namespace mhb;
 
@@ -81,6 +82,9 @@ struct AttnArgs {
     int vhead;                 // >= 0 (with vheads 1): the values of this KV head, whatever the query head's own
     size_t page_extra;         // elements of a page behind its keys and values
     const float* slopes;       // [nq] distance biases, or null
+    // how tiles are staged (launch_attention)
+    int vec, buffers, k_stride;
+    unsigned k_rcp, v_rcp;     // ceil(2^20 / 16-byte pieces of a key row, of a value row)
 };
 
 __device__ __forceinline__ float gate_of(const AttnArgs& a, int t, int col) {
@@ -91,14 +95,29 @@ __device__ __forceinline__ float gate_of(const AttnArgs& a, int t, int col) {
     return 1.f / (1.f + expf(-g));
 }
 
+// Four elements of a tile as float32 (the address is a multiple of four elements)
+__device__ __forceinline__ float4 tile4(const float* p) { return *(const float4*)p; }
+__device__ __forceinline__ float4 tile4(const __nv_bfloat16* p) {
+    const uint2 u = *(const uint2*)p;
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                       __uint_as_float(u.y & 0xffff0000u));
+}
+
+// What set the pace of a decoded token here was latency, tile after tile: a page looked up and a key loaded for each of a
+// warp's eight keys in turn, then the dot product's reads of shared memory one element at a time.  So tiles are double
+// buffered and arrive by 16-byte cp.async (a.vec: widths and pages allow it) while the tile before is attended to, their
+// pages are looked up a tile earlier, by one lane a key, and scores read four elements at once, for all of a warp's rows.
+// A decode step of 4 requests with up to 281 cached positions (3 heads of 32, float32) took 44 us a layer here before; the
+// whole step, with the products of gemm_f32.cu, went from 292 to 139 us.  Splits may now be as short as 64 keys.
 template <typename CT, int DPL>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_simt_kernel(const AttnArgs a) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) uint8_t smem_raw[];
     const int d = a.d, dv = a.dv * a.vheads;      // dv: the width of an output row
-    float* q_s = smem;                       // [R_TILE][d]
-    float* k_s = q_s + R_TILE * d;           // [KT][d + 1]
-    float* v_s = k_s + KT * (d + 1);         // [KT][dv]
+    const int k_stride = a.k_stride, dq = (d + 3) & ~3;
+    float* q_s = (float*)smem_raw;                           // [R_TILE][dq]
+    CT* tiles = (CT*)(q_s + R_TILE * dq);                    // [a.buffers] of [KT][k_stride] keys, [KT][dv] values
+    const int tile_elems = KT * (k_stride + dv);
     __shared__ int row_pos[R_TILE];
 
     pdl_launch_dependents();
@@ -120,7 +139,87 @@ attention_simt_kernel(const AttnArgs a) {
     const size_t page_elems = kv_elems + a.page_extra;
     const CT* q = (const CT*)a.q;
     const CT* cache = (const CT*)a.cache;
+    const int* table = a.block_table + (size_t)seg * a.width;
 
+    // keys beyond the window (see "prefix" at the top): positions below `beyond` have left the window of the
+    // item's last row, which is the one that sees the most of them
+    int pre_end = 0;
+    if (a.pre_kind && a.window > 0 && split <= 0 && nrows > 0) {
+        const int beyond = a.positions[tok0 + ntok - 1] - a.window + 1;
+        if (beyond > 0) pre_end = a.pre_kind == 1 ? min(a.pre_n, beyond) : beyond / a.pre_n;
+    }
+    // the tiles: those of the prefix, then those of the item's own keys
+    const int pre_tiles = (pre_end + KT - 1) / KT, tiles_all = pre_tiles + max(0, kv_end - kv_begin + KT - 1) / KT;
+    constexpr int PER_WARP = KT / WARPS;
+    // lane j < PER_WARP: the page of this warp's key j in tile u (-1: none)
+    auto look_up = [&](int u) {
+        int page = -1;
+        if (lane < PER_WARP && u < tiles_all) {
+            const bool own = u >= pre_tiles;
+            const int kp = (own ? kv_begin + (u - pre_tiles) * KT : u * KT) + warp * PER_WARP + lane;
+            if (kp < (own ? kv_end : pre_end)) {
+                page = table[!own && a.pre_kind == 2 ? (kp * a.pre_n + a.pre_n - 1) / a.P : kp / a.P];
+                if (page >= a.num_pages) page = -1;
+            }
+        }
+        return page;
+    };
+    // this warp's keys and values of tile u into a buffer; lanes run along the elements of eight keys
+    auto fetch = [&](int u, int page_of_lane, CT* dst) {
+        const bool own = u >= pre_tiles, pooled = !own && a.pre_kind == 2;
+        const int k0 = (own ? kv_begin + (u - pre_tiles) * KT : u * KT) + warp * PER_WARP;
+        // element offsets of lane j's key row and value row (of the first KV head it takes values from)
+        long long k_at = 0, v_at = 0;
+        const int vh0 = a.vheads > 1 ? 0 : (a.vhead >= 0 ? a.vhead : kvh);
+        const size_t v_head = pooled ? (size_t)a.pool_slots * dv1 : (size_t)a.P * v_ld;     // to the next KV head's values
+        if (lane < PER_WARP && page_of_lane >= 0) {
+            const int kp = k0 + lane, pg = pooled ? (kp * a.pre_n + a.pre_n - 1) / a.P : kp / a.P;
+            const size_t pbase = (size_t)page_of_lane * page_elems;
+            if (pooled) {
+                const int slot = kp - (int)(((long long)pg * a.P) / a.pre_n);
+                k_at = (long long)(pbase + kv_elems + ((size_t)kvh * a.pool_slots + slot) * d);
+                v_at = (long long)(pbase + kv_elems + (size_t)a.nkv * a.pool_slots * d + vh0 * v_head + (size_t)slot * dv1);
+            } else {
+                const int slot = kp - pg * a.P;
+                k_at = (long long)(pbase + ((size_t)kvh * a.P + slot) * k_ld + map * d);
+                v_at = (long long)(pbase + v_plane + vh0 * v_head + (size_t)slot * v_ld);
+            }
+        }
+        CT* ks = dst + warp * PER_WARP * k_stride;
+        CT* vs = dst + KT * k_stride + warp * PER_WARP * dv;
+        if (a.vec) {
+            constexpr int E = 16 / sizeof(CT);
+            const int kc = d / E, vc = dv1 / E;
+            for (int i0 = 0; i0 < PER_WARP * kc; i0 += 32) {
+                const int i = i0 + lane, j = min((int)(((unsigned)i * a.k_rcp) >> 20), PER_WARP - 1);
+                const int page = __shfl_sync(0xffffffffu, page_of_lane, j);
+                const long long at = __shfl_sync(0xffffffffu, k_at, j);
+                const int e = (i - j * kc) * E;
+                if (i < PER_WARP * kc) cp_async16((uint32_t)__cvta_generic_to_shared(ks + j * k_stride + e), cache + (page >= 0 ? at + e : 0), page >= 0 ? 16 : 0);
+            }
+            for (int c = 0; c < a.vheads; ++c) {
+                for (int i0 = 0; i0 < PER_WARP * vc; i0 += 32) {
+                    const int i = i0 + lane, j = min((int)(((unsigned)i * a.v_rcp) >> 20), PER_WARP - 1);
+                    const int page = __shfl_sync(0xffffffffu, page_of_lane, j);
+                    const long long at = __shfl_sync(0xffffffffu, v_at, j) + (long long)(c * v_head);
+                    const int e = (i - j * vc) * E;
+                    if (i < PER_WARP * vc) cp_async16((uint32_t)__cvta_generic_to_shared(vs + j * dv + c * dv1 + e), cache + (page >= 0 ? at + e : 0), page >= 0 ? 16 : 0);
+                }
+            }
+        } else {
+            for (int j = 0; j < PER_WARP; ++j) {
+                const bool in = __shfl_sync(0xffffffffu, page_of_lane, j) >= 0;
+                const long long kat = __shfl_sync(0xffffffffu, k_at, j), vat = __shfl_sync(0xffffffffu, v_at, j);
+                for (int e = lane; e < d; e += 32) ks[j * k_stride + e] = in ? cache[kat + e] : from_float<CT>(0.f);
+                for (int c = 0; c < a.vheads; ++c)
+                    for (int e = lane; e < dv1; e += 32)
+                        vs[j * dv + c * dv1 + e] = in ? cache[vat + (long long)(c * v_head) + e] : from_float<CT>(0.f);
+            }
+        }
+        cp_async_commit();
+    };
+
+    int page = look_up(0);
     // stage the queries (float32) and the rows' positions
     for (int idx = threadIdx.x; idx < R_TILE * d; idx += blockDim.x) {
         const int r = idx / d, e = idx - r * d;
@@ -129,14 +228,19 @@ attention_simt_kernel(const AttnArgs a) {
             const int t = tok0 + r / nheads, h = (kvh * groups + head0 + r % nheads) * kparts + map;
             v = to_float(q[((size_t)t * a.nq + h) * d + e]);
         }
-        q_s[idx] = v;
+        q_s[r * dq + e] = v;
     }
     if (threadIdx.x < R_TILE) {
         const int r = threadIdx.x;
         row_pos[r] = r < nrows ? a.positions[tok0 + r / nheads] : -1;
     }
-    __syncthreads();
+    const bool twice = a.buffers == 2;
+    if (tiles_all > 0 && twice) {
+        fetch(0, page, tiles);
+        page = look_up(1);
+    }
 
+    // l: this lane's share of the sum; the lanes' shares are added at the end
     float m[ROWS_PER_WARP], l[ROWS_PER_WARP], acc[ROWS_PER_WARP][DPL], slope[ROWS_PER_WARP];
 #pragma unroll
     for (int rs = 0; rs < ROWS_PER_WARP; ++rs) {
@@ -148,98 +252,109 @@ attention_simt_kernel(const AttnArgs a) {
         slope[rs] = a.slopes && r < nrows ? a.slopes[(kvh * groups + head0 + r % nheads) * kparts + map] : 0.f;
         if (a.sink && split <= 0 && r < nrows) {      // a single time per token: here or in split 0
             m[rs] = a.sink[(kvh * groups + head0 + r % nheads) * kparts + map];
-            l[rs] = 1.f;
+            l[rs] = lane == 0 ? 1.f : 0.f;
         }
     }
+    // rows of this warp: rs * WARPS + warp < nrows
+    const int my_rows = nrows > warp ? (nrows - warp + WARPS - 1) / WARPS : 0;
 
-    const int* table = a.block_table + (size_t)seg * a.width;
-    // keys beyond the window (see "prefix" at the top): positions below `beyond` have left the window of the
-    // item's last row, which is the one that sees the most of them
-    int pre_end = 0;
-    if (a.pre_kind && a.window > 0 && split <= 0 && nrows > 0) {
-        const int beyond = a.positions[tok0 + ntok - 1] - a.window + 1;
-        if (beyond > 0) pre_end = a.pre_kind == 1 ? min(a.pre_n, beyond) : beyond / a.pre_n;
-    }
-    for (int phase = pre_end > 0 ? 0 : 1; phase < 2; ++phase) {
-    const int begin = phase ? kv_begin : 0, end = phase ? kv_end : pre_end;
-    const bool pooled = !phase && a.pre_kind == 2;
-    for (int t0 = begin; t0 < end; t0 += KT) {
-        // load KT keys and values: warp w takes keys w*8 .. w*8+7, lanes run along d
-        for (int j = warp * (KT / WARPS); j < (warp + 1) * (KT / WARPS); ++j) {
-            const int kp = t0 + j;
-            int page = -1, slot = 0;
-            if (kp < end) {
-                const int pg = pooled ? (kp * a.pre_n + a.pre_n - 1) / a.P : kp / a.P;
-                slot = pooled ? kp - (int)(((long long)pg * a.P) / a.pre_n) : kp - pg * a.P;
-                page = table[pg];
-                if (page >= a.num_pages) page = -1;
-            }
-            if (page >= 0) {
-                const size_t pbase = (size_t)page * page_elems;
-                if (pooled) {
-                    const size_t off = pbase + kv_elems + ((size_t)kvh * a.pool_slots + slot) * d;
-                    for (int e = lane; e < d; e += 32) k_s[j * (d + 1) + e] = to_float(cache[off + e]);
-                    for (int c = 0; c < a.vheads; ++c) {
-                        const int vh = a.vheads > 1 ? c : (a.vhead >= 0 ? a.vhead : kvh);
-                        const size_t voff = pbase + kv_elems + (size_t)a.nkv * a.pool_slots * d +
-                                            ((size_t)vh * a.pool_slots + slot) * dv1;
-                        for (int e = lane; e < dv1; e += 32) v_s[j * dv + c * dv1 + e] = to_float(cache[voff + e]);
-                    }
-                } else {
-                    const size_t off = pbase + ((size_t)kvh * a.P + slot) * k_ld + map * d;
-                    for (int e = lane; e < d; e += 32) k_s[j * (d + 1) + e] = to_float(cache[off + e]);
-                    for (int c = 0; c < a.vheads; ++c) {
-                        const int vh = a.vheads > 1 ? c : (a.vhead >= 0 ? a.vhead : kvh);
-                        const size_t voff = pbase + v_plane + ((size_t)vh * a.P + slot) * v_ld;
-                        for (int e = lane; e < dv1; e += 32) v_s[j * dv + c * dv1 + e] = to_float(cache[voff + e]);
-                    }
-                }
+    for (int u = 0; u < tiles_all; ++u) {
+        CT* buf = tiles + (twice ? (u & 1) * tile_elems : 0);
+        if (twice) {
+            // the other buffer was read before the last barrier of the loop
+            if (u + 1 < tiles_all) {
+                fetch(u + 1, page, tiles + ((u + 1) & 1) * tile_elems);
+                page = look_up(u + 2);
+                cp_async_wait<1>();
             } else {
-                for (int e = lane; e < d; e += 32) k_s[j * (d + 1) + e] = 0.f;
-                for (int e = lane; e < dv; e += 32) v_s[j * dv + e] = 0.f;
+                cp_async_wait<0>();
             }
+        } else {
+            fetch(u, page, buf);
+            page = look_up(u + 1);
+            cp_async_wait<0>();
         }
         __syncthreads();
-        const int kp = t0 + lane;  // this lane's key
+        const CT* k_s = buf;
+        const CT* v_s = buf + KT * k_stride;
+        const bool own = u >= pre_tiles, pooled = !own && a.pre_kind == 2;
+        const int end = own ? kv_end : pre_end;
+        const int kp = (own ? kv_begin + (u - pre_tiles) * KT : u * KT) + lane;  // this lane's key
+        float s[ROWS_PER_WARP];
+#pragma unroll
+        for (int rs = 0; rs < ROWS_PER_WARP; ++rs) s[rs] = 0.f;
+        const CT* kr = k_s + lane * k_stride;
+        if (a.vec) {
+#pragma unroll 4
+            for (int e = 0; e < d; e += 4) {
+                const float4 k4 = tile4(kr + e);
+#pragma unroll
+                for (int rs = 0; rs < ROWS_PER_WARP; ++rs) {
+                    if (rs >= my_rows) break;
+                    const float4 q4 = *(const float4*)(q_s + (rs * WARPS + warp) * dq + e);
+                    s[rs] = fmaf(q4.x, k4.x, s[rs]);
+                    s[rs] = fmaf(q4.y, k4.y, s[rs]);
+                    s[rs] = fmaf(q4.z, k4.z, s[rs]);
+                    s[rs] = fmaf(q4.w, k4.w, s[rs]);
+                }
+            }
+        } else {
+            for (int e = 0; e < d; ++e) {
+                const float k1 = to_float(kr[e]);
+#pragma unroll
+                for (int rs = 0; rs < ROWS_PER_WARP; ++rs) {
+                    if (rs >= my_rows) break;
+                    s[rs] = fmaf(q_s[(rs * WARPS + warp) * dq + e], k1, s[rs]);
+                }
+            }
+        }
+        float p[ROWS_PER_WARP];
 #pragma unroll
         for (int rs = 0; rs < ROWS_PER_WARP; ++rs) {
-            const int r = rs * WARPS + warp;
-            if (r >= nrows) continue;  // uniform within the warp
-            const int qp = row_pos[r];
-            const float* qr = q_s + r * d;
-            const float* kr = k_s + lane * (d + 1);
-            float s = 0.f;
-            for (int e = 0; e < d; ++e) s = fmaf(qr[e], kr[e], s);
-            s *= a.scale;
-            if (a.softcap > 0.f) s = a.softcap * tanhf(s / a.softcap);
-            if (a.slopes) s = fmaf(-slope[rs], (float)(qp - kp), s);
+            p[rs] = 0.f;
+            if (rs >= my_rows) break;  // uniform within the warp
+            const int qp = row_pos[rs * WARPS + warp];
+            float x = s[rs] * a.scale;
+            if (a.softcap > 0.f) x = a.softcap * tanhf(x / a.softcap);
+            if (a.slopes) x = fmaf(-slope[rs], (float)(qp - kp), x);
             bool valid;
-            if (phase) valid = kp < end && kp <= qp && (a.window <= 0 || kp > qp - a.window);
+            if (own) valid = kp < end && kp <= qp && (a.window <= 0 || kp > qp - a.window);
             else if (pooled) valid = kp < end && qp - a.window + 1 > 0 && kp < (qp - a.window + 1) / a.pre_n;
             else valid = kp < end && kp <= qp - a.window;
-            if (!valid) s = -INFINITY;
-            const float m_new = fmaxf(m[rs], warp_max(s));
-            float p = 0.f, alpha = 1.f;
+            if (!valid) x = -INFINITY;
+            const float m_new = fmaxf(m[rs], warp_max(x));
+            float alpha = 1.f;
             if (m_new > -INFINITY) {
-                p = valid ? expf(s - m_new) : 0.f;
+                p[rs] = valid ? expf(x - m_new) : 0.f;
                 alpha = m[rs] > -INFINITY ? expf(m[rs] - m_new) : 0.f;
             }
-            l[rs] = l[rs] * alpha + warp_sum(p);
+            l[rs] = l[rs] * alpha + p[rs];
             m[rs] = m_new;
 #pragma unroll
             for (int i = 0; i < DPL; ++i) acc[rs][i] *= alpha;
+        }
+        if (my_rows > 0) {
+#pragma unroll 4
             for (int j = 0; j < KT; ++j) {
-                const float pj = __shfl_sync(0xffffffffu, p, j);
+                float v[DPL];
 #pragma unroll
                 for (int i = 0; i < DPL; ++i) {
                     const int e = lane + 32 * i;
-                    if (e < dv) acc[rs][i] = fmaf(pj, v_s[j * dv + e], acc[rs][i]);
+                    v[i] = e < dv ? to_float(v_s[j * dv + e]) : 0.f;
+                }
+#pragma unroll
+                for (int rs = 0; rs < ROWS_PER_WARP; ++rs) {
+                    if (rs >= my_rows) break;
+                    const float pj = __shfl_sync(0xffffffffu, p[rs], j);
+#pragma unroll
+                    for (int i = 0; i < DPL; ++i) acc[rs][i] = fmaf(pj, v[i], acc[rs][i]);
                 }
             }
         }
         __syncthreads();
     }
-    }
+#pragma unroll
+    for (int rs = 0; rs < ROWS_PER_WARP; ++rs) l[rs] = warp_sum(l[rs]);
 
 #pragma unroll
     for (int rs = 0; rs < ROWS_PER_WARP; ++rs) {
@@ -318,16 +433,36 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_acc,
 }
 
 template <typename CT>
-int launch_attention(const AttnArgs& a, int max_items, cudaStream_t stream) {
+int launch_attention(const AttnArgs& args, int max_items, cudaStream_t stream) {
+    AttnArgs a = args;
     const int dvt = a.dv * a.vheads;
     int dpl = (dvt + 31) / 32;
     if (dpl > 8) dpl = dpl <= 12 ? 12 : 16;      // wide values: accumulators for 384 or 512 elements per row
-    const size_t smem = sizeof(float) * ((size_t)R_TILE * a.d + (size_t)KT * (a.d + 1) + (size_t)KT * dvt);
+    // 16-byte pieces: every row that a tile is made of starts on 16 bytes and is a whole number of them (a row with the
+    // values of several KV heads is made of each one's)
+    constexpr int E = 16 / sizeof(CT);
+    a.vec = a.d % E == 0 && a.dv % E == 0 && a.page_extra % E == 0 && ((uintptr_t)a.cache & 15) == 0 && a.d / E <= 128 && a.dv / E <= 128;
+    auto bytes = [&](int vec, int buffers) {
+        return sizeof(float) * (size_t)R_TILE * ((a.d + 3) & ~3) + buffers * sizeof(CT) * (size_t)KT * (a.d + (vec ? E : 1) + dvt);
+    };
+    // keys E elements apart beyond their width: eight lanes' 16-byte reads of eight keys meet all banks.  Two buffers
+    // while three CTAs still fit an SM, one for wide rows.
+    const size_t limit = 227 * 1024 - 256;
+    if (a.vec && bytes(1, 1) > limit) a.vec = 0;
+    a.buffers = a.vec && bytes(1, 2) <= 75 * 1024 ? 2 : 1;
+    a.k_stride = a.d + (a.vec ? E : 1);
+    if (a.vec) {
+        a.k_rcp = (unsigned)(((1 << 20) + a.d / E - 1) / (a.d / E));
+        a.v_rcp = (unsigned)(((1 << 20) + a.dv / E - 1) / (a.dv / E));
+    } else {
+        a.k_rcp = a.v_rcp = 0;
+    }
+    const size_t smem = bytes(a.vec, a.buffers);
     dim3 grid(max_items, a.nkv * a.kparts);
 #define MHB_ATTN_CASE(N)                                                                        \
     case N: {                                                                                   \
         auto kern = attention_simt_kernel<CT, N>;                                               \
-        if (smem > 48 * 1024) {                                                                 \
+        if (smem > 47 * 1024) {      /* 48 KB without being asked, the static part included */  \
             cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, \
                                                  (int)smem);                                    \
             if (e != cudaSuccess) return fail("attention: shared memory %zu: %s", smem,        \

@@ -15,6 +15,7 @@ ROW_TILE = 16          # query rows (tokens x heads of one group) per CTA of the
 KEY_TILE = 64          # split boundaries are multiples of the kernels' key tile
 ITEM_INTS = 8
 MIN_KEYS_PER_SPLIT = 256
+MIN_KEYS_PER_SIMT_SPLIT = 64
 SPLIT_MAX_TOKENS = 16  # only short segments (decode tokens, tiny portions) are split along the keys
 MAX_SPLITS = 64
 MAX_BIG_SPLITS = 8       # key splits of a long portion's tile (tcgen05 kernel only)
@@ -32,6 +33,12 @@ class AttentionShape:
     kv_heads: int
     window: int | None = None
     tile_rows: int = ROW_TILE
+
+    @property
+    def min_keys(self) -> int:
+        """The shortest key split.  The tensor-core kernels walk 256 keys in the time a split costs to start and to merge;
+        the CUDA-core kernel (ROW_TILE rows for every portion) takes that long for two of its 32-key tiles."""
+        return MIN_KEYS_PER_SIMT_SPLIT if self.tile_rows == ROW_TILE else MIN_KEYS_PER_SPLIT
 
 
 @dataclass
@@ -93,7 +100,7 @@ def plan_attention(need: AttentionShape, segments, T: int, sm_count: int = 148,
     # SM, so that a long history beside short ones is cut into more parts and no CTA runs alone at
     # the end
     small_keys = sum(t[4] - t[3] for t in small_tiles) * len(small_chunks) * need.kv_heads
-    target = max(MIN_KEYS_PER_SPLIT, -(-small_keys // (2 * sm_count)))
+    target = max(need.min_keys, -(-small_keys // (2 * sm_count)))
     target = -(-target // KEY_TILE) * KEY_TILE
     items = []
     tok_part_row = np.zeros(T, np.int32)
@@ -104,7 +111,7 @@ def plan_attention(need: AttentionShape, segments, T: int, sm_count: int = 148,
         if fixed_nsplit is not None:
             nsplit = fixed_nsplit
         else:
-            fit = max(1, (kv_end - kv_begin) // MIN_KEYS_PER_SPLIT)
+            fit = max(1, (kv_end - kv_begin) // need.min_keys)
             nsplit = max(1, min(-(-(kv_end - kv_begin) // target), fit, MAX_SPLITS))
         if nsplit == 1:
             for h0, nh in small_chunks:
@@ -266,11 +273,11 @@ class AttentionPlanner(StepPlanner):
         """Key shares per decoded token for a batch of B with at most ``max_positions`` cached keys, as
         (shares in a cluster, clusters per token and KV head): as many CTAs as are resident at once (two per
         SM), never more, so that no CTA waits for a second wave, and no share shorter than
-        MIN_KEYS_PER_SPLIT keys.  Without a cluster kernel: (shares, 1)."""
+        ``shape.min_keys`` keys.  Without a cluster kernel: (shares, 1)."""
         ctas = segments_count * self.shape.kv_heads * self.chunks
         if self.shape.window:            # a token never attends to more keys than its window holds
             max_positions = min(max_positions, self.shape.window)
-        n = max(1, min(MAX_SPLITS, (2 * self.sm_count) // ctas, max_positions // MIN_KEYS_PER_SPLIT))
+        n = max(1, min(MAX_SPLITS, (2 * self.sm_count) // ctas, max_positions // self.shape.min_keys))
         if self.clusters_of is None or self.chunks != 1 or n == 1:
             return n, 1
         # The shares of a cluster are merged in its shared memory, and a cluster is placed inside one
@@ -323,7 +330,7 @@ class AttentionPlanner(StepPlanner):
         fixed = self.decode_fixed(len(starts), max_positions)
         n0 = fixed[0] * fixed[1]
         B = len(starts)
-        limit = min(max_positions // MIN_KEYS_PER_SPLIT, self.max_cluster or MAX_SPLITS)
+        limit = min(max_positions // self.shape.min_keys, self.max_cluster or MAX_SPLITS)
         if n0 > 1 or B < 2 or limit < 2:       # fewer requests: their splits are sized for one round of CTAs
             return fixed
         tiles = (np.asarray(starts, np.int64) + KEY_TILE) // KEY_TILE
