@@ -193,7 +193,7 @@ struct SplitSmem {
     static constexpr int A_STAGE = 3 * A_TILE, B_STAGE = 3 * B_TILE;
     static constexpr int B0 = 2 * A_STAGE;
     static constexpr int BARRIERS = B0 + B_STAGES * B_STAGE;
-    static constexpr int TOTAL = BARRIERS + (5 + B_STAGES) * 8 + 16 + 1024;
+    static constexpr int TOTAL = BARRIERS + (5 + 2 * B_STAGES) * 8 + 16 + 1024;
 };
 
 // K-major tile of 64-byte rows with the 64-byte swizzle: groups of 8 rows 512 bytes apart.
@@ -219,9 +219,12 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map, const float* __re
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t base = smem_addr(smem);
-    // barriers: a block's weights are cut (a set of tiles each), its MMAs are done, its tokens are here; one for leaving early
-    const uint32_t full0 = base + S::BARRIERS, done0 = full0 + 16, here0 = full0 + 32, drain = here0 + 8 * B_STAGES;
-    uint32_t* slot = (uint32_t*)(smem + S::BARRIERS + (5 + B_STAGES) * 8);
+    // barriers: a block's weights are cut, its MMAs are done (a set of tiles and an accumulator each); its tokens are here,
+    // their stage is free again (a stage each: a wait for a phase's parity must not fall two phases behind, which a wait of
+    // the loading warp on `done` could); one for leaving early
+    const uint32_t full0 = base + S::BARRIERS, done0 = full0 + 16, here0 = full0 + 32, free0 = here0 + 8 * B_STAGES,
+                   drain = free0 + 8 * B_STAGES;
+    uint32_t* slot = (uint32_t*)(smem + S::BARRIERS + (5 + 2 * B_STAGES) * 8);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.x * BN, n0 = blockIdx.y * T_BM;
     const int total = (K + T_BK - 1) / T_BK;
@@ -231,7 +234,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map, const float* __re
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < 2; ++s) { mbar_init(full0 + 8 * s, T_WORKERS); mbar_init(done0 + 8 * s, 1); }
-        for (int s = 0; s < B_STAGES; ++s) mbar_init(here0 + 8 * s, 1);
+        for (int s = 0; s < B_STAGES; ++s) { mbar_init(here0 + 8 * s, 1); mbar_init(free0 + 8 * s, 1); }
         mbar_init(drain, 1);
         mbar_fence_init();
     }
@@ -248,8 +251,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map, const float* __re
             int i = 0;
             for (; i < count; ++i) {
                 // a stage is free when the MMAs of the block B_STAGES before have read it
-                const int old = i - B_STAGES;
-                ok = old < 0 || mbar_wait(done0 + 8 * (old & 1), (old >> 1) & 1);
+                ok = i < B_STAGES || mbar_wait(free0 + 8 * (i % B_STAGES), (i / B_STAGES - 1) & 1);
                 if (!ok) break;
                 const uint32_t bar = here0 + 8 * (i % B_STAGES), dst = base + S::B0 + (i % B_STAGES) * S::B_STAGE;
                 mbar_expect_tx(bar, S::B_STAGE);
@@ -279,6 +281,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map, const float* __re
                                   db + (order[p][1] * S::B_TILE + 32 * k) / 16, idesc, (p || k) ? 1u : 0u);
                 }
                 umma_commit(done0 + 8 * s);
+                umma_commit(free0 + 8 * (i % B_STAGES));
             }
             if (!ok) {                       // leaving early: not before what was issued has run
                 umma_commit(drain);
