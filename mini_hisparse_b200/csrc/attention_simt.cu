@@ -90,8 +90,7 @@ struct AttnArgs {
 __device__ __forceinline__ float gate_of(const AttnArgs& a, int t, int col) {
     if (!a.gate) return 1.f;
     const size_t idx = (size_t)t * a.gate_ld + col;
-    float g = a.gate[idx];
-    for (int s = 1; s < a.gate_nsplit; ++s) g += a.gate[idx + (size_t)s * a.gate_split_stride];
+    const float g = sum_parts(a.gate + idx, a.gate_nsplit, a.gate_split_stride);
     return 1.f / (1.f + expf(-g));
 }
 
@@ -424,8 +423,7 @@ __global__ void attention_combine_kernel(const float* __restrict__ part_acc,
         float g = 1.f;
         if (gate) {
             const size_t idx = (size_t)t * gate_ld + (gate_per_head ? h : h * d + e);
-            float z = gate[idx];
-            for (int s = 1; s < gate_nsplit; ++s) z += gate[idx + (size_t)s * gate_split_stride];
+            const float z = sum_parts(gate + idx, gate_nsplit, gate_split_stride);
             g = 1.f / (1.f + expf(-z));
         }
         out[((size_t)t * nq + h) * d + e] = from_float<OT>(o * inv * g);

@@ -77,6 +77,62 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return scratch[32];
 }
 
+// The same with one barrier: every warp adds the warps' sums for itself.  `scratch` holds 32 floats that no other sum of
+// the kernel uses (nothing keeps a fast warp from writing it again while a slow one still reads).
+__device__ __forceinline__ float block_sum_once(float v, float* scratch) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nwarps = (blockDim.x + 31) >> 5;
+    v = warp_sum(v);
+    if (lane == 0) scratch[warp] = v;
+    __syncthreads();
+    return warp_sum(lane < nwarps ? scratch[lane] : 0.f);
+}
+
+// ---- split-K parts ------------------------------------------------------------------------------
+// The sum of `n` parts `stride` elements apart, in index order.  Eight loads are asked for before the first is added: in a
+// decode step these sums are what a kernel waits for, and one round trip to the L2 per part (18 parts behind a down
+// projection) was most of its time.  A single part costs one load.
+template <typename T>
+__device__ __forceinline__ float sum_parts(const T* p, int n, size_t stride) {
+    float v = to_float(p[0]);
+    for (int s = 1; s < n; s += 8) {
+        float d[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (s + q < n) d[q] = to_float(p[(size_t)(s + q) * stride]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (s + q < n) v += d[q];
+    }
+    return v;
+}
+__device__ __forceinline__ float4 vec4(const float* p) { return *(const float4*)p; }
+__device__ __forceinline__ float4 vec4(const __nv_bfloat16* p) {
+    const uint2 u = *(const uint2*)p;
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+                       __uint_as_float(u.y & 0xffff0000u));
+}
+// four neighbours at once, B loads in flight (four registers each: fewer where a kernel is for many rows and a single part);
+// with a start value that the parts are added to, one after the other
+template <int B, typename T>
+__device__ __forceinline__ void add_parts4(float4& v, const T* p, int n, size_t stride) {
+    for (int s = 0; s < n; s += B) {
+        float4 d[B];
+#pragma unroll
+        for (int q = 0; q < B; ++q)
+            if (s + q < n) d[q] = vec4(p + (size_t)(s + q) * stride);
+#pragma unroll
+        for (int q = 0; q < B; ++q)
+            if (s + q < n) { v.x += d[q].x; v.y += d[q].y; v.z += d[q].z; v.w += d[q].w; }
+    }
+}
+template <int B, typename T>
+__device__ __forceinline__ float4 sum_parts4(const T* p, int n, size_t stride) {
+    float4 v = vec4(p);
+    if (n > 1) add_parts4<B>(v, p + stride, n - 1, stride);
+    return v;
+}
+
 }  // namespace mhb
 
 // ---- programmatic dependent launch -----------------------------------------------------------

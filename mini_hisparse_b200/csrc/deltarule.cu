@@ -32,10 +32,7 @@ struct Parts {
     size_t stride;
     int ld;
     __device__ __forceinline__ float at(size_t row, int col) const {
-        const size_t idx = row * ld + col;
-        float v = p[idx];
-        for (int s = 1; s < nsplit; ++s) v += p[idx + (size_t)s * stride];
-        return v;
+        return sum_parts(p + row * ld + col, nsplit, stride);
     }
 };
 

@@ -17,9 +17,17 @@ MHB_EXPORT const char* mhb_last_error() { return error_buffer(); }
 // ---- load helpers -----------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ float load_split(const T* p, size_t idx, int nsplit, size_t split_stride) {
-    float v = to_float(p[idx]);
-    for (int s = 1; s < nsplit; ++s) v += to_float(p[idx + (size_t)s * split_stride]);
-    return v;
+    return sum_parts(p + idx, nsplit, split_stride);
+}
+
+template <typename T> __device__ __forceinline__ void store4(T* p, float4 v);
+template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *(float4*)p = v; }
+template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    uint2 u;
+    u.x = *(const uint32_t*)&a;
+    u.y = *(const uint32_t*)&b;
+    *(uint2*)p = u;
 }
 
 // ---- embedding ---------------------------------------------------------------------------
@@ -50,10 +58,37 @@ __global__ void embed_kernel(const WT* __restrict__ table, const int* __restrict
     }
 }
 
+// The same with every element of the row asked for at once: four elements a thread (H % 4 == 0, rows on 16 bytes).  One
+// element a thread and step was a chain of memory round trips, 11 us for a row of 3584.
+template <typename WT>
+__global__ void embed_vec_kernel(const WT* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ out, int H,
+                                 int V, int* __restrict__ status, float scale, __nv_bfloat16* __restrict__ copy) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.x, i = 4 * (blockIdx.y * blockDim.x + threadIdx.x);
+    if (i >= H) return;
+    const int tok = tokens[t];
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tok >= 0 && tok < V) {
+        v = vec4(table + (size_t)tok * H + i);
+        v.x *= scale; v.y *= scale; v.z *= scale; v.w *= scale;
+    } else if (i == 0 && status) {
+        atomicOr(status, 1);
+    }
+    *(float4*)(out + (size_t)t * H + i) = v;
+    if (copy) store4<__nv_bfloat16>(copy + (size_t)t * H + i, v);
+}
+
 static int launch_embed(const void* table, int table_dtype, const int* tokens, float* out, int T, int H, int V,
                         int* status, float scale, void* copy, cudaStream_t stream) {
     if (T <= 0) return 0;
     const int threads = H >= 1024 ? 256 : 128;
+    if (H % 4 == 0 && !(((uintptr_t)table | (uintptr_t)out | (uintptr_t)copy) & 15)) {
+        MHB_DISPATCH_DTYPE(table_dtype, WT,
+            launch_kernel(embed_vec_kernel<WT>, dim3(T, (H / 4 + threads - 1) / threads), dim3(threads), 0, stream,
+                          (const WT*)table, tokens, out, H, V, status, scale, (__nv_bfloat16*)copy));
+        return check_launch("embed");
+    }
     MHB_DISPATCH_DTYPE(table_dtype, WT,
         launch_kernel(embed_kernel<WT>, dim3(T), dim3(threads), 0, stream, (const WT*)table, tokens, out, H, V, status,
                       scale, (__nv_bfloat16*)copy));
@@ -145,27 +180,11 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ x, const DT* __restrict__
 // (rows of up to 4 * VEC_CACHE * blockDim elements; H % 4 == 0, 16-byte aligned rows).
 constexpr int VEC_CACHE = 4;
 
-template <typename T> __device__ __forceinline__ float4 load4(const T* p);
-template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *(const float4*)p; }
-template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
-    const uint2 u = *(const uint2*)p;
-    const __nv_bfloat162 a = *(const __nv_bfloat162*)&u.x, b = *(const __nv_bfloat162*)&u.y;
-    return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
-}
-template <typename T> __device__ __forceinline__ void store4(T* p, float4 v);
-template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *(float4*)p = v; }
-template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
-    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-    uint2 u;
-    u.x = *(const uint32_t*)&a;
-    u.y = *(const uint32_t*)&b;
-    *(uint2*)p = u;
-}
-
 // VC vectors per thread: 4 for many rows; 1 for few rows (a decode step), where the kernel's time is
 // the chain of memory round trips of one thread and more threads make that chain shorter.
 template <typename DT, typename OT, int VC>
-__global__ void add_rmsnorm_vec_kernel(float* __restrict__ x, const DT* __restrict__ delta, int nsplit,
+__global__ void __launch_bounds__(1024)
+add_rmsnorm_vec_kernel(float* __restrict__ x, const DT* __restrict__ delta, int nsplit,
                                        size_t split_stride, const float* __restrict__ weight, float eps,
                                        const int* __restrict__ rows, OT* __restrict__ out, int H) {
     __shared__ float scratch[33];
@@ -190,36 +209,14 @@ __global__ void add_rmsnorm_vec_kernel(float* __restrict__ x, const DT* __restri
         if (i < nvec) {
             float4 a = *(const float4*)(xr + 4 * i);
             if (delta) {
-                const DT* dp = delta + (size_t)s * H + 4 * i;
-                int sp = 0;
-                for (; sp + 8 <= nsplit; sp += 8) {      // eight loads in flight; summed in order
-                    float4 d[8];
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) d[q] = load4<DT>(dp + (size_t)(sp + q) * split_stride);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) { a.x += d[q].x; a.y += d[q].y; a.z += d[q].z; a.w += d[q].w; }
-                }
-                for (; sp + 4 <= nsplit; sp += 4) {      // four loads in flight; summed in order
-                    const float4 d0 = load4<DT>(dp + (size_t)(sp + 0) * split_stride);
-                    const float4 d1 = load4<DT>(dp + (size_t)(sp + 1) * split_stride);
-                    const float4 d2 = load4<DT>(dp + (size_t)(sp + 2) * split_stride);
-                    const float4 d3 = load4<DT>(dp + (size_t)(sp + 3) * split_stride);
-                    a.x += d0.x; a.y += d0.y; a.z += d0.z; a.w += d0.w;
-                    a.x += d1.x; a.y += d1.y; a.z += d1.z; a.w += d1.w;
-                    a.x += d2.x; a.y += d2.y; a.z += d2.z; a.w += d2.w;
-                    a.x += d3.x; a.y += d3.y; a.z += d3.z; a.w += d3.w;
-                }
-                for (; sp < nsplit; ++sp) {
-                    const float4 d = load4<DT>(dp + (size_t)sp * split_stride);
-                    a.x += d.x; a.y += d.y; a.z += d.z; a.w += d.w;
-                }
+                add_parts4<VC == 1 ? 8 : 4>(a, delta + (size_t)s * H + 4 * i, nsplit, split_stride);
                 if (write_back) *(float4*)(xr + 4 * i) = a;
             }
             v[c] = a;
             ss += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
         }
     }
-    const float total = block_sum(ss, scratch);
+    const float total = block_sum_once(ss, scratch);
     const float rstd = rsqrtf(total / (float)H + eps);
     OT* o = out + (size_t)r * H;
 #pragma unroll
@@ -256,7 +253,7 @@ add_rmsnorm_rows_kernel(float* __restrict__ x, const DT* __restrict__ delta, con
             const int i = threadIdx.x + c * blockDim.x;
             if (i < nvec) {
                 a[c] = *(const float4*)(x + (size_t)r * H + 4 * i);
-                d[c] = delta ? load4<DT>(delta + (size_t)r * H + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                d[c] = delta ? vec4(delta + (size_t)r * H + 4 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
     };
@@ -459,20 +456,7 @@ __global__ void rope_append_kernel(const IT* __restrict__ qkv, int nsplit, size_
 // row, bias and cache row is 16-byte aligned then): 16-byte loads, 8- or 16-byte stores.
 template <typename IT>
 __device__ __forceinline__ float4 load4_split(const IT* p, size_t idx, int nsplit, size_t split_stride) {
-    float4 v = load4<IT>(p + idx);
-    int s = 1;
-    for (; s + 4 <= nsplit; s += 4) {       // four loads in flight; summed in order
-        float4 w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) w[q] = load4<IT>(p + idx + (size_t)(s + q) * split_stride);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) { v.x += w[q].x; v.y += w[q].y; v.z += w[q].z; v.w += w[q].w; }
-    }
-    for (; s < nsplit; ++s) {
-        const float4 w = load4<IT>(p + idx + (size_t)s * split_stride);
-        v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
-    }
-    return v;
+    return sum_parts4<4>(p + idx, nsplit, split_stride);
 }
 __device__ __forceinline__ void add4(float4& a, const float4 b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
 

@@ -42,10 +42,7 @@ struct Parts {            // a float32 product, possibly split-K parts
     int ld;
 };
 __device__ __forceinline__ float load(const Parts& a, size_t t, int col) {
-    const size_t idx = t * a.ld + col;
-    float v = a.p[idx];
-    for (int s = 1; s < a.nsplit; ++s) v += a.p[idx + (size_t)s * a.stride];
-    return v;
+    return sum_parts(a.p + t * a.ld + col, a.nsplit, a.stride);
 }
 
 // ---- prep ---------------------------------------------------------------------------------------------

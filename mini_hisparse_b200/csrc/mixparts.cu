@@ -22,10 +22,7 @@ namespace {
 
 template <typename T>
 __device__ __forceinline__ float load_parts(const T* p, size_t idx, int nsplit, size_t split_stride) {
-    float v = to_float(p[idx]);
-#pragma unroll 4              // the parts' loads in flight together; they are still added in order
-    for (int s = 1; s < nsplit; ++s) v += to_float(p[idx + (size_t)s * split_stride]);
-    return v;
+    return sum_parts(p + idx, nsplit, split_stride);
 }
 
 __device__ __forceinline__ float sigmoidf(float z) { return 1.f / (1.f + expf(-z)); }

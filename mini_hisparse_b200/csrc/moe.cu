@@ -26,9 +26,7 @@ namespace {
 constexpr int TILE_ROWS = 64;
 
 __device__ __forceinline__ float load_parts(const float* p, size_t idx, int nsplit, size_t stride) {
-    float v = p[idx];
-    for (int s = 1; s < nsplit; ++s) v += p[idx + (size_t)s * stride];
-    return v;
+    return sum_parts(p + idx, nsplit, stride);
 }
 
 // ---- router ---------------------------------------------------------------------------------------------

@@ -22,16 +22,11 @@ MHB_EXPORT const char* mhb_last_error() { return error_buffer(); }
 namespace {
 
 __device__ __forceinline__ float load_parts(const float* p, size_t idx, int nsplit, size_t split_stride) {
-    float v = p[idx];
-#pragma unroll 4
-    for (int s = 1; s < nsplit; ++s) v += p[idx + (size_t)s * split_stride];
-    return v;
+    return sum_parts(p + idx, nsplit, split_stride);
 }
 template <typename T>
 __device__ __forceinline__ float load_parts_t(const T* p, size_t idx, int nsplit, size_t split_stride) {
-    float v = to_float(p[idx]);
-    for (int s = 1; s < nsplit; ++s) v += to_float(p[idx + (size_t)s * split_stride]);
-    return v;
+    return sum_parts(p + idx, nsplit, split_stride);
 }
 
 __device__ __forceinline__ float sigmoidf(float z) { return 1.f / (1.f + expf(-z)); }
@@ -41,13 +36,6 @@ __device__ __forceinline__ float gelu_tanhf(float z) {
     return 0.5f * z * (1.f + tanhf(c * (z + 0.044715f * z * z * z)));
 }
 
-template <typename T> __device__ __forceinline__ float4 load4(const T* p);
-template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return *(const float4*)p; }
-template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
-    const uint2 u = *(const uint2*)p;
-    const __nv_bfloat162 a = *(const __nv_bfloat162*)&u.x, b = *(const __nv_bfloat162*)&u.y;
-    return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
-}
 template <typename T> __device__ __forceinline__ void store4(T* p, float4 v);
 template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *(float4*)p = v; }
 template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
@@ -57,16 +45,6 @@ template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16*
     u.y = *(const uint32_t*)&b;
     *(uint2*)p = u;
 }
-template <typename T>
-__device__ __forceinline__ float4 load4_parts(const T* p, size_t idx, int nsplit, size_t split_stride) {
-    float4 v = load4<T>(p + idx);
-    for (int s = 1; s < nsplit; ++s) {
-        const float4 w = load4<T>(p + idx + (size_t)s * split_stride);
-        v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
-    }
-    return v;
-}
-
 // ---- x <- keep x + rms(alpha x + delta) w ---------------------------------------------------------
 template <typename DT, typename OT>
 __global__ void norm_mix_kernel(float* __restrict__ x, const DT* __restrict__ delta, int nsplit,
@@ -95,42 +73,55 @@ __global__ void norm_mix_kernel(float* __restrict__ x, const DT* __restrict__ de
     }
 }
 
-// The same with four elements per thread and step (H % 4 == 0, every row 16-byte aligned).
-template <typename DT, typename OT>
-__global__ void norm_mix_vec_kernel(float* __restrict__ x, const DT* __restrict__ delta, int nsplit,
+// The same with the row in registers, VC vectors of four elements a thread (H % 4 == 0, every row 16-byte aligned): one
+// vector where rows are few and a thread's chain of loads is the kernel's time, four where there are many.
+template <typename DT, typename OT, int VC, int MOST>
+__global__ void __launch_bounds__(MOST)
+norm_mix_vec_kernel(float* __restrict__ x, const DT* __restrict__ delta, int nsplit,
                                     size_t split_stride, const float* __restrict__ weight, float eps,
                                     float alpha, float keep, OT* __restrict__ copy, int H) {
-    extern __shared__ float row[];
-    __shared__ float scratch[33];
+    __shared__ float scratch[32];
     pdl_launch_dependents();
+    const int nvec = H >> 2;
+    float4 w[VC];                            // constant: fetched while the kernel before this one still runs
+#pragma unroll
+    for (int c = 0; c < VC; ++c) {
+        const int i = threadIdx.x + c * blockDim.x;
+        if (VC == 1 && i < nvec) w[c] = vec4(weight + 4 * i);
+    }
     pdl_wait();
     const size_t r = blockIdx.x;
     float* xr = x + r * H;
+    float4 v[VC], s[VC];
     float ss = 0.f;
-    for (int i = 4 * threadIdx.x; i < H; i += 4 * blockDim.x) {
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (alpha != 0.f) {
-            const float4 v = *(const float4*)(xr + i);
-            s = make_float4(alpha * v.x, alpha * v.y, alpha * v.z, alpha * v.w);
-        }
-        if (delta) {
-            const float4 d = load4_parts(delta, r * H + i, nsplit, split_stride);
-            s.x += d.x; s.y += d.y; s.z += d.z; s.w += d.w;
-        }
-        *(float4*)(row + i) = s;
-        ss += s.x * s.x + s.y * s.y + s.z * s.z + s.w * s.w;
+#pragma unroll
+    for (int c = 0; c < VC; ++c) {
+        const int i = threadIdx.x + c * blockDim.x;
+        if (i >= nvec) continue;
+        v[c] = s[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (alpha != 0.f || keep != 0.f) v[c] = vec4(xr + 4 * i);
+        if (delta) s[c] = sum_parts4<VC == 1 ? 8 : 2>(delta + r * H + 4 * i, nsplit, split_stride);
     }
-    const float total = block_sum(ss, scratch);
-    const float rstd = 1.f / sqrtf(total / (float)H + eps);
-    for (int i = 4 * threadIdx.x; i < H; i += 4 * blockDim.x) {
-        const float4 s = *(const float4*)(row + i), w = *(const float4*)(weight + i);
-        float4 n = make_float4(s.x * rstd * w.x, s.y * rstd * w.y, s.z * rstd * w.z, s.w * rstd * w.w);
-        if (keep != 0.f) {
-            const float4 v = *(const float4*)(xr + i);
-            n.x += keep * v.x; n.y += keep * v.y; n.z += keep * v.z; n.w += keep * v.w;
+#pragma unroll
+    for (int c = 0; c < VC; ++c) {
+        const int i = threadIdx.x + c * blockDim.x;
+        if (i >= nvec) continue;
+        if (alpha != 0.f) {
+            s[c].x += alpha * v[c].x; s[c].y += alpha * v[c].y; s[c].z += alpha * v[c].z; s[c].w += alpha * v[c].w;
         }
-        *(float4*)(xr + i) = n;
-        if (copy) store4<OT>(copy + r * H + i, n);
+        ss += s[c].x * s[c].x + s[c].y * s[c].y + s[c].z * s[c].z + s[c].w * s[c].w;
+    }
+    const float total = block_sum_once(ss, scratch);
+    const float rstd = 1.f / sqrtf(total / (float)H + eps);
+#pragma unroll
+    for (int c = 0; c < VC; ++c) {
+        const int i = threadIdx.x + c * blockDim.x;
+        if (i >= nvec) continue;
+        const float4 wv = VC == 1 ? w[c] : vec4(weight + 4 * i);
+        float4 n = make_float4(s[c].x * rstd * wv.x, s[c].y * rstd * wv.y, s[c].z * rstd * wv.z, s[c].w * rstd * wv.w);
+        if (keep != 0.f) { n.x += keep * v[c].x; n.y += keep * v[c].y; n.z += keep * v[c].z; n.w += keep * v[c].w; }
+        *(float4*)(xr + 4 * i) = n;
+        if (copy) store4<OT>(copy + r * H + 4 * i, n);
     }
 }
 
@@ -157,14 +148,14 @@ __global__ void act_rows_kernel(const IT* __restrict__ z, int nsplit, size_t spl
 }
 
 // four elements per thread (n % 4 == 0, 16-byte aligned, parts a multiple of four elements apart)
-template <typename IT, typename OT>
+template <typename IT, typename OT, int B>
 __global__ void act_rows_vec_kernel(const IT* __restrict__ z, int nsplit, size_t split_stride, OT* __restrict__ out,
                                     size_t n, int act) {
     pdl_launch_dependents();
     pdl_wait();
     const size_t i = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= n) return;
-    const float4 v = load4_parts(z, i, nsplit, split_stride);
+    const float4 v = sum_parts4<B>(z + i, nsplit, split_stride);
     store4<OT>(out + i, make_float4(act_of(v.x, act), act_of(v.y, act), act_of(v.z, act), act_of(v.w, act)));
 }
 
@@ -204,6 +195,43 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const float* _
         float n = orow[i] * rstd * weight[i];
         if (gate) n *= sigmoidf(load_parts(gate, r * gate_ld + i, gate_nsplit, gate_split_stride));
         out[r * N + i] = from_float<OT>(n);
+    }
+}
+
+// The same with the row and its gate in registers, VC vectors a thread (N, strides and addresses in 16-byte steps).
+template <typename OT, int VC>
+__global__ void __launch_bounds__(1024)
+gated_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_nsplit,
+                                         size_t gate_split_stride, int gate_ld, const float* __restrict__ weight,
+                                         float eps, OT* __restrict__ out, int N) {
+    __shared__ float scratch[32];
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t r = blockIdx.x;
+    const int nvec = N >> 2;
+    float4 v[VC], g[VC];
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < VC; ++c) {
+        const int i = threadIdx.x + c * blockDim.x;
+        if (i >= nvec) continue;
+        v[c] = vec4(o + r * N + 4 * i);
+        if (gate) g[c] = sum_parts4<VC == 1 ? 8 : 2>(gate + r * gate_ld + 4 * i, gate_nsplit, gate_split_stride);
+    }
+#pragma unroll
+    for (int c = 0; c < VC; ++c)
+        if ((int)(threadIdx.x + c * blockDim.x) < nvec)
+            ss += v[c].x * v[c].x + v[c].y * v[c].y + v[c].z * v[c].z + v[c].w * v[c].w;
+    const float total = block_sum_once(ss, scratch);
+    const float rstd = 1.f / sqrtf(total / (float)N + eps);
+#pragma unroll
+    for (int c = 0; c < VC; ++c) {
+        const int i = threadIdx.x + c * blockDim.x;
+        if (i >= nvec) continue;
+        const float4 w = vec4(weight + 4 * i);
+        float4 n = make_float4(v[c].x * rstd * w.x, v[c].y * rstd * w.y, v[c].z * rstd * w.z, v[c].w * rstd * w.w);
+        if (gate) { n.x *= sigmoidf(g[c].x); n.y *= sigmoidf(g[c].y); n.z *= sigmoidf(g[c].z); n.w *= sigmoidf(g[c].w); }
+        store4<OT>(out + r * N + 4 * i, n);
     }
 }
 
@@ -332,6 +360,151 @@ __global__ void qknorm_rope_append_kernel(const float* __restrict__ qkv, int nsp
     }
 }
 
+// The same four elements at a time (head sizes and the rotated width in steps of 4 and 8, rows and strides on 16 bytes): a
+// thread asks for all its loads at once, both norms' sums cross the CTA at one barrier, and angles, pages and the
+// destination are worked out before the kernel waits for the product.  One element a thread and step, with two block-wide
+// sums in turn and the values loaded after them, took 10.6 us for 8 tokens of 16 heads and 62 us for 2,048 of 32.
+template <typename CT>
+__global__ void __launch_bounds__(1024)
+qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t split_stride, int ld,
+                                              const float* __restrict__ q_weight, const float* __restrict__ k_weight,
+                                              float eps, const int* __restrict__ positions,
+                                              const int* __restrict__ tok_seg, const int* __restrict__ block_table,
+                                              int table_width, const float* __restrict__ inv_freq, int rdim,
+                                              CT* __restrict__ q_out, CT* __restrict__ cache, int nq, int nkv, int dk,
+                                              int dv, int P, int num_pages, int has_kv, int* __restrict__ status,
+                                              int per_head, float v_eps, size_t page_extra, float temp_coef,
+                                              double temp_every, float v_scale, const float* __restrict__ bias,
+                                              int v_from_k) {
+    extern __shared__ __align__(16) float sh[];            // q and k rows, cos, sin, the v row if it is kept
+    __shared__ float sums[2][32];
+    pdl_launch_dependents();
+    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int qw = nq * dk, kw = has_kv ? nkv * dk : 0, vw = has_kv ? nkv * dv : 0, rhalf = rdim >> 1;
+    float* cs = sh + qw + kw;
+    float* sn = cs + rhalf;
+    float* vs = sn + rhalf;
+    // positions and block tables do not change during a step
+    const int pos = positions[t], within = pos % P;
+    for (int i = threadIdx.x; i < rhalf; i += blockDim.x) {
+        float sine, cosine;
+        sincosf((float)pos * inv_freq[i], &sine, &cosine);
+        cs[i] = cosine;
+        sn[i] = sine;
+    }
+    CT* page_k = nullptr;
+    CT* page_v = nullptr;
+    bool outside = false;
+    if (has_kv) {
+        const int page = block_table[(size_t)tok_seg[t] * table_width + pos / P];
+        outside = page < 0 || page >= num_pages;          // never write outside the pool
+        if (!outside) {
+            page_k = cache + (size_t)page * ((size_t)nkv * P * (dk + dv) + page_extra);
+            page_v = page_k + (size_t)nkv * P * dk;
+        }
+    }
+    pdl_wait();
+    if (outside && threadIdx.x == 0 && status) atomicOr(status, 2);
+    const float* row = qkv + (size_t)t * ld;
+    const bool keep_v = v_eps > 0.f || v_from_k;
+    const int loads = (qw + kw + (v_from_k ? 0 : vw)) >> 2;
+    float ssq = 0.f, ssk = 0.f;
+#pragma unroll 2
+    for (int u = threadIdx.x; u < loads; u += blockDim.x) {
+        const int i = 4 * u;
+        float4 v = sum_parts4<8>(row + i, nsplit, split_stride);
+        if (i < qw + kw) {
+            if (bias) { const float4 b = vec4(bias + i); v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
+            *(float4*)(sh + i) = v;
+            const float ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            if (i < qw) ssq += ss;
+            else {
+                ssk += ss;
+                if (v_from_k) *(float4*)(vs + i - qw) = v;
+            }
+        } else if (keep_v) {
+            *(float4*)(vs + i - qw - kw) = v;
+        } else if (page_v) {
+            const int e = i - qw - kw, g = e / dv;
+            store4<CT>(page_v + ((size_t)g * P + within) * dv + (e - g * dv),
+                       make_float4(v_scale * v.x, v_scale * v.y, v_scale * v.z, v_scale * v.w));
+        }
+    }
+    float rq = 1.f, rk = 1.f;
+    if (per_head) {
+        __syncthreads();
+        const float temp = temp_coef != 0.f ? 1.f + temp_coef * log1pf((float)floor((double)(pos + 1) / temp_every)) : 1.f;
+        for (int head = warp; head < (qw + kw) / dk; head += nwarps) {
+            float* hr = sh + head * dk;
+            const float* w = head < nq ? q_weight : k_weight;
+            float ss = 0.f;
+            for (int e = 4 * lane; e < dk; e += 128) {
+                const float4 v = vec4(hr + e);
+                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+            }
+            const float r = 1.f / sqrtf(warp_sum(ss) / (float)dk + eps);
+            const float f = head < nq ? temp : 1.f;
+            for (int e = 4 * lane; e < dk; e += 128) {
+                float4 v = vec4(hr + e);
+                const float4 m = w ? vec4(w + e) : make_float4(1.f, 1.f, 1.f, 1.f);
+                v.x = v.x * r * m.x * f; v.y = v.y * r * m.y * f; v.z = v.z * r * m.z * f; v.w = v.w * r * m.w * f;
+                *(float4*)(hr + e) = v;
+            }
+        }
+    } else {
+        ssq = warp_sum(ssq);
+        ssk = warp_sum(ssk);
+        if (lane == 0) { sums[0][warp] = ssq; sums[1][warp] = ssk; }
+        __syncthreads();
+        const float tq = warp_sum(lane < nwarps ? sums[0][lane] : 0.f), tk = warp_sum(lane < nwarps ? sums[1][lane] : 0.f);
+        rq = 1.f / sqrtf(tq / (float)qw + eps);
+        rk = kw ? 1.f / sqrtf(tk / (float)kw + eps) : 0.f;
+    }
+    if (v_eps > 0.f) {
+        for (int head = warp; head < (has_kv ? nkv : 0); head += nwarps) {
+            float* hr = vs + head * dv;
+            float ss = 0.f;
+            for (int e = lane; e < dv; e += 32) ss += hr[e] * hr[e];
+            const float r = 1.f / sqrtf(warp_sum(ss) / (float)dv + v_eps);
+            for (int e = lane; e < dv; e += 32) hr[e] *= r;
+        }
+    }
+    if (per_head || v_eps > 0.f) __syncthreads();
+    // a thread per four rotated pairs, or four elements that are not rotated
+    auto scaled = [&](int head, int e) {
+        float4 v = vec4(sh + head * dk + e);
+        if (!per_head) {
+            const float r = head < nq ? rq : rk;
+            const float4 w = head < nq ? vec4(q_weight + head * dk + e) : vec4(k_weight + (head - nq) * dk + e);
+            v.x = v.x * r * w.x; v.y = v.y * r * w.y; v.z = v.z * r * w.z; v.w = v.w * r * w.w;
+        }
+        return v;
+    };
+    const int pairs4 = rhalf >> 2, units = pairs4 + ((dk - rdim) >> 2), heads = nq + (has_kv ? nkv : 0);
+    for (int idx = threadIdx.x; idx < heads * units; idx += blockDim.x) {
+        const int head = idx / units, u = idx - head * units;
+        CT* dst = head < nq ? q_out + (size_t)t * qw + head * dk
+                  : page_k  ? page_k + ((size_t)(head - nq) * P + within) * dk : nullptr;
+        if (!dst) continue;
+        if (u < pairs4) {
+            const float4 a = scaled(head, 4 * u), b = scaled(head, 4 * u + rhalf), c = vec4(cs + 4 * u), n = vec4(sn + 4 * u);
+            store4<CT>(dst + 4 * u, make_float4(a.x * c.x - b.x * n.x, a.y * c.y - b.y * n.y, a.z * c.z - b.z * n.z, a.w * c.w - b.w * n.w));
+            store4<CT>(dst + 4 * u + rhalf, make_float4(b.x * c.x + a.x * n.x, b.y * c.y + a.y * n.y, b.z * c.z + a.z * n.z, b.w * c.w + a.w * n.w));
+        } else {
+            const int e = rdim + 4 * (u - pairs4);
+            store4<CT>(dst + e, scaled(head, e));
+        }
+    }
+    if (page_v && keep_v) {
+        for (int i = 4 * threadIdx.x; i < vw; i += 4 * blockDim.x) {
+            const int g = i / dv;
+            const float4 v = vec4(vs + i);
+            store4<CT>(page_v + ((size_t)g * P + within) * dv + (i - g * dv),
+                       make_float4(v_scale * v.x, v_scale * v.y, v_scale * v.z, v_scale * v.w));
+        }
+    }
+}
+
 int row_threads(int H) {
     int t = (H + 31) / 32 * 32;
     if (t > 512) t = 512;
@@ -341,7 +514,7 @@ int row_threads(int H) {
 
 template <typename Kern>
 int allow_smem(Kern kern, size_t smem, const char* what) {
-    if (smem > 48 * 1024) {
+    if (smem > 47 * 1024) {                  // 48 KB without being asked, the static part included
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail("%s: shared memory %zu: %s", what, smem, cudaGetErrorString(e));
     }
@@ -357,16 +530,19 @@ MHB_EXPORT int mhb_norm_mix(float* x, const void* delta, int delta_dtype, int ns
     const size_t smem = sizeof(float) * (size_t)H;
     const bool vec = H % 4 == 0 && !((uintptr_t)x & 15) && !((uintptr_t)delta & 15) && !((uintptr_t)weight & 15) &&
                      !((uintptr_t)copy & 15) && split_stride % 4 == 0;
-    if (vec) {
-        int threads = (H / 4 + 31) / 32 * 32;
-        if (threads > 512) threads = 512;
-        if (threads < 64) threads = 64;
-        MHB_DISPATCH_DTYPE(delta_dtype, DT, MHB_DISPATCH_DTYPE(copy_dtype, OT, {
-            auto kern = norm_mix_vec_kernel<DT, OT>;
-            if (allow_smem(kern, smem, "norm_mix")) return -1;
-            launch_kernel(kern, dim3(R), dim3(threads), smem, stream, x, (const DT*)delta, nsplit,
-                          (size_t)split_stride, weight, eps, alpha, keep, (OT*)copy, H);
-        }));
+    // one vector a thread for up to 128 rows, four beyond: 8 rows of 2048 with 18 parts 6.0 us before
+    const int wide = (H / 4 + 31) / 32 * 32, narrow = ((H / 4 + 3) / 4 + 31) / 32 * 32;
+    if (vec && R <= 128 && wide <= 1024) {
+        MHB_DISPATCH_DTYPE(delta_dtype, DT, MHB_DISPATCH_DTYPE(copy_dtype, OT,
+            launch_kernel((norm_mix_vec_kernel<DT, OT, 1, 1024>), dim3(R), dim3(wide < 64 ? 64 : wide), 0, stream, x,
+                          (const DT*)delta, nsplit, (size_t)split_stride, weight, eps, alpha, keep, (OT*)copy, H)));
+        return check_launch("norm_mix");
+    }
+    if (vec && narrow <= 1024) {
+        MHB_DISPATCH_DTYPE(delta_dtype, DT, MHB_DISPATCH_DTYPE(copy_dtype, OT,
+            launch_kernel((narrow <= 256 ? norm_mix_vec_kernel<DT, OT, 4, 256> : norm_mix_vec_kernel<DT, OT, 4, 1024>), dim3(R),
+                          dim3(narrow < 64 ? 64 : narrow), 0, stream, x, (const DT*)delta, nsplit, (size_t)split_stride,
+                          weight, eps, alpha, keep, (OT*)copy, H)));
         return check_launch("norm_mix");
     }
     MHB_DISPATCH_DTYPE(delta_dtype, DT, MHB_DISPATCH_DTYPE(copy_dtype, OT, {
@@ -387,7 +563,7 @@ MHB_EXPORT int mhb_act_rows(const void* z, int in_dtype, int nsplit, long long s
     if (n % 4 == 0 && !((uintptr_t)z & 15) && !((uintptr_t)out & 15) && split_stride % 4 == 0) {
         const unsigned vblocks = (unsigned)((n / 4 + threads - 1) / threads);
         MHB_DISPATCH_DTYPE(in_dtype, IT, MHB_DISPATCH_DTYPE(out_dtype, OT,
-            launch_kernel((act_rows_vec_kernel<IT, OT>), dim3(vblocks), dim3(threads), 0, stream, (const IT*)z, nsplit,
+            launch_kernel((nsplit == 1 ? act_rows_vec_kernel<IT, OT, 1> : act_rows_vec_kernel<IT, OT, 8>), dim3(vblocks), dim3(threads), 0, stream, (const IT*)z, nsplit,
                           (size_t)split_stride, (OT*)out, (size_t)n, act)));
         return check_launch("act_rows");
     }
@@ -417,6 +593,19 @@ MHB_EXPORT int mhb_gated_rmsnorm(const float* o, const float* gate, int gate_nsp
                                  int gate_ld, const float* weight, float eps, void* out, int out_dtype, int R, int N,
                                  cudaStream_t stream) {
     if (R <= 0) return 0;
+    const bool vec = N % 4 == 0 && gate_ld % 4 == 0 && gate_split_stride % 4 == 0 &&
+                     !(((uintptr_t)o | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out) & 15);
+    const int wide = (N / 4 + 31) / 32 * 32, narrow = ((N / 4 + 3) / 4 + 31) / 32 * 32;
+    if (vec && narrow <= 1024) {
+        const bool few = R <= 128 && wide <= 1024;
+        const dim3 threads(few ? (wide < 64 ? 64 : wide) : (narrow < 64 ? 64 : narrow));
+        MHB_DISPATCH_DTYPE(out_dtype, OT, {
+            auto kern = few ? gated_rmsnorm_vec_kernel<OT, 1> : gated_rmsnorm_vec_kernel<OT, 4>;
+            launch_kernel(kern, dim3(R), threads, 0, stream, o, gate, gate_nsplit, (size_t)gate_split_stride, gate_ld,
+                          weight, eps, (OT*)out, N);
+        });
+        return check_launch("gated_rmsnorm");
+    }
     MHB_DISPATCH_DTYPE(out_dtype, OT,
         launch_kernel(gated_rmsnorm_kernel<OT>, dim3(R), dim3(row_threads(N)), 0, stream, o, gate, gate_nsplit,
                       (size_t)gate_split_stride, gate_ld, weight, eps, (OT*)out, N));
@@ -445,6 +634,25 @@ MHB_EXPORT int mhb_qknorm_rope_append_opts(const float* qkv, int nsplit, long lo
     if (rdim < 0 || rdim > dk || (rdim & 1)) return fail("qknorm_rope_append: %d rotated elements of a head of %d", rdim, dk);
     const int qw = nq * dk, kw = has_kv ? nkv * dk : 0;
     const size_t smem = sizeof(float) * ((size_t)qw + kw + rdim + ((v_eps > 0.f || v_from_k) && has_kv ? (size_t)nkv * dv : 0));
+    const uintptr_t addresses = (uintptr_t)qkv | (uintptr_t)q_weight | (uintptr_t)k_weight | (uintptr_t)q_out |
+                                (uintptr_t)cache | (uintptr_t)bias;
+    if (dk % 4 == 0 && dv % 4 == 0 && rdim % 8 == 0 && ld % 4 == 0 && split_stride % 4 == 0 && page_extra % 4 == 0 &&
+        !(addresses & 15)) {
+        // few tokens: a thread for every four elements; many: half as many, so that several tokens share an SM
+        const int quads = (qw + kw + (has_kv && !v_from_k ? nkv * dv : 0)) / 4, want = T <= 64 ? quads : (quads + 1) / 2;
+        const int most = T <= 64 ? 1024 : 512;
+        int threads = (want + 31) / 32 * 32;
+        threads = threads < 64 ? 64 : threads > most ? most : threads;
+        MHB_DISPATCH_DTYPE(dtype, CT, {
+            auto kern = qknorm_rope_append_vec_kernel<CT>;
+            if (allow_smem(kern, smem, "qknorm_rope_append")) return -1;
+            launch_kernel(kern, dim3(T), dim3(threads), smem, stream, qkv, nsplit, (size_t)split_stride, ld, q_weight,
+                          k_weight, eps, positions, tok_seg, block_table, table_width, inv_freq, rdim, (CT*)q_out,
+                          (CT*)cache, nq, nkv, dk, dv, P, num_pages, has_kv, status, per_head, v_eps, (size_t)page_extra,
+                          temp_coef, temp_every, v_scale, bias, v_from_k);
+        });
+        return check_launch("qknorm_rope_append");
+    }
     MHB_DISPATCH_DTYPE(dtype, CT, {
         auto kern = qknorm_rope_append_kernel<CT, CT>;
         if (allow_smem(kern, smem, "qknorm_rope_append")) return -1;

@@ -48,6 +48,20 @@ def test_embed(dtype):
     assert torch.equal(out3[0], table.float()[3])
 
 
+@pytest.mark.parametrize("H", [4, 1028, 3584, 30])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_embed_forms(H, dtype):
+    """Rows in steps of four elements and others, with a scale and a second copy, and an id outside the table."""
+    table = rnd(50, H, dtype=dtype, seed=2)
+    tokens = torch.tensor([3, 49, -1, 0], dtype=torch.int32, device=DEV)
+    out, copy = torch.empty(4, H, device=DEV), torch.empty(4, H, dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    K().embed(table, tokens, out, status, scale=1.5, copy=copy)
+    want = table.float()[tokens.clamp(min=0).long()] * 1.5
+    want[2] = 0
+    assert int(status) == 1 and torch.equal(out, want) and torch.equal(copy, want.bfloat16())
+
+
 # ---- RMSNorm ------------------------------------------------------------------------------------
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("H", [80, 1000, 3584])
@@ -631,6 +645,17 @@ def test_attention_tensor_core_splits_window_and_far_key(kernel):
     torch.testing.assert_close(out, ref, **tol(bf, 2))
     out2, ref2, _ = run_attention(4, 2, 64, 16, [(0, 641)], bf, edit=edit, kernel=kernel)
     torch.testing.assert_close(out2, ref2, **tol(bf, 2))
+
+
+@pytest.mark.parametrize("d,P_", [(64, 16), (128, 32), (128, 4)])
+@pytest.mark.parametrize("hist", [0, 63, 64, 130, 191, 192, 300, 700, 1500])
+def test_attention_tma_few_ctas(d, P_, hist):
+    """A launch with no more CTAs than SMs works on several key tiles at once: from less than one tile to several rounds of
+    the ring of stages, unsplit and split, decode tokens and a short portion."""
+    for nsplit in (1, 3):
+        out, ref, plan = run_attention(6, 2, d, P_, [(hist, 1), (hist, 5)], torch.bfloat16, fixed_nsplit=nsplit, kernel="tc")
+        assert len(plan.items) * 2 <= 148 and plan.n_small
+        torch.testing.assert_close(out, ref, **tol(torch.bfloat16, 2))
 
 
 @pytest.mark.parametrize("nq,nkv,d,P_,nsplit,qkv_nsplit,rdim,interleaved,window,ngroups", [

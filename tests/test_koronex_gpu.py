@@ -177,6 +177,118 @@ def test_activations_and_table_gate():
     torch.testing.assert_close(o2.cpu().double(), ref, atol=1e-6, rtol=1e-5)
 
 
+# ---- the decode forms: rows in registers, four elements at a time; their limits and the general forms beside them ----------
+@pytest.mark.parametrize("R,H,nsplit", [(1, 4, 1), (128, 4096, 18), (129, 4096, 1), (3, 4100, 9), (130, 5000, 2), (2, 16384, 1),
+                                        (5, 16388, 3), (7, 66, 8), (64, 2048, 10)])
+def test_norm_and_gate_forms(R, H, nsplit):
+    """norm_mix and gated_rmsnorm at the row counts and widths where their forms change.  float32 with up to 18 parts: the sum
+    of n numbers of size 1 is within n 2^-24 of its own magnitude, a norm's relative error is of that order: 1e-5."""
+    from mini_hisparse_b200.kernels import api as K
+
+    g = torch.Generator(device="cuda").manual_seed(R * H + nsplit)
+    x, w = (torch.randn(*n, device="cuda", generator=g) for n in ((R, H), (H,)))
+    parts = torch.randn(nsplit, R, H, device="cuda", generator=g)
+    for alpha, keep in ((1.5, 0.0), (0.0, 1.0), (0.5, 2.0)):
+        xr, copy = x.clone(), torch.empty(R, H, dtype=torch.bfloat16, device="cuda")
+        K.norm_mix(xr, w, 1e-5, delta=parts, nsplit=nsplit, split_stride=parts.stride(0), alpha=alpha, keep=keep, copy=copy)
+        s = alpha * x.double() + parts.double().sum(0)
+        want = keep * x.double() + s / torch.sqrt((s * s).mean(-1, keepdim=True) + 1e-5) * w.double()
+        torch.testing.assert_close(xr.double(), want, atol=1e-5, rtol=1e-5)
+        assert torch.equal(copy, xr.bfloat16())
+    wide = torch.randn(nsplit, R, H + 8, device="cuda", generator=g)
+    out = torch.empty(R, H, device="cuda")
+    K.gated_rmsnorm(x, w, 1e-5, out, gate=wide[0][:, 8:], gate_nsplit=nsplit, gate_split_stride=wide.stride(0))
+    want = x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-5) * w.double()
+    torch.testing.assert_close(out.double(), want * torch.sigmoid(wide.double().sum(0)[:, 8:]), atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("dk,dv,rdim,nsplit,T", [(64, 64, 32, 1, 70), (64, 64, 32, 9, 3), (24, 36, 8, 2, 5), (24, 36, 4, 2, 5),
+                                                 (16, 16, 16, 18, 64), (20, 20, 0, 3, 65), (22, 30, 6, 2, 4)])
+@pytest.mark.parametrize("per_head", [False, True])
+def test_qk_norm_forms(dk, dv, rdim, nsplit, T, per_head):
+    """The q/k norm with rotation and append: sizes that the four-element form takes and sizes that it does not, with every
+    option a caller combines; pages of 3 positions.  float32 throughout: 2e-5 as above, and the angles' rounding."""
+    from mini_hisparse_b200.kernels import api as K
+
+    nq, nkv, P_ = 6, 2, 3
+    g = torch.Generator(device="cuda").manual_seed(dk * T + nsplit)
+    def rand(*n):
+        return torch.randn(*n, device="cuda", generator=g)
+    ld = nq * dk + nkv * (dk + dv) + 4
+    qkv, bias = rand(nsplit, T, ld), rand((nq + nkv) * dk)
+    qw, kw = (rand(dk if per_head else n * dk) for n in (nq, nkv))
+    pos = torch.arange(7, 7 + T, dtype=torch.int32, device="cuda")
+    width = (7 + T) // P_ + 1
+    table = torch.randperm(width, generator=torch.Generator().manual_seed(1)).int().cuda().view(1, -1)
+    seg = torch.zeros(T, dtype=torch.int32, device="cuda")
+    inv = 10.0 ** -torch.arange(rdim // 2, device="cuda").float()
+    extra = 4 if dk % 4 == 0 else 2
+    page = nkv * P_ * (dk + dv) + extra
+    cache, q = torch.full((width, page), 9.0, device="cuda"), torch.empty(T, nq * dk, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    opts = dict(per_head=True, q_temp=(0.3, 5.0), v_eps=1e-5) if per_head else {}
+    K.qknorm_rope_append(qkv, qw, kw, 1e-6, pos, seg, table, inv, rdim, q, cache, nq=nq, nkv=nkv, dk=dk, dv=dv, page_size=P_,
+                         nsplit=nsplit, split_stride=qkv.stride(0), status=status, page_extra=extra, v_scale=0.5, bias=bias, **opts)
+    assert int(status) == 0
+    row = qkv.double().sum(0)
+    a = [(row[:, :nq * dk] + bias[:nq * dk].double()), row[:, nq * dk:(nq + nkv) * dk] + bias[nq * dk:].double()]
+    v = row[:, (nq + nkv) * dk:(nq + nkv) * dk + nkv * dv].view(T, nkv, dv)
+    if per_head:
+        a = [y.view(T, -1, dk) for y in a]
+        v = v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5)
+    a = [y / torch.sqrt((y * y).mean(-1, keepdim=True) + 1e-6) * w.double() for y, w in zip(a, (qw, kw))]
+    a = [y.reshape(T, -1, dk) for y in a]
+    if per_head:
+        a[0] = a[0] * (1 + 0.3 * torch.log(torch.floor((pos.double() + 1) / 5.0) + 1))[:, None, None]
+    ang = (pos.float()[:, None] * inv).double()
+    for y in a:
+        u, w2 = y[..., :rdim // 2].clone(), y[..., rdim // 2:rdim].clone()
+        y[..., :rdim // 2] = u * ang.cos()[:, None] - w2 * ang.sin()[:, None]
+        y[..., rdim // 2:rdim] = w2 * ang.cos()[:, None] + u * ang.sin()[:, None]
+    torch.testing.assert_close(q.double().view(T, nq, dk), a[0], atol=2e-5, rtol=2e-5)
+    for t in range(T):
+        pg = cache[int(table[0, int(pos[t]) // P_])]
+        k_got = pg[:nkv * P_ * dk].view(nkv, P_, dk)[:, int(pos[t]) % P_]
+        v_got = pg[nkv * P_ * dk:nkv * P_ * (dk + dv)].view(nkv, P_, dv)[:, int(pos[t]) % P_]
+        torch.testing.assert_close(k_got.double(), a[1][t], atol=2e-5, rtol=2e-5)
+        torch.testing.assert_close(v_got.double(), 0.5 * v[t], atol=2e-5, rtol=2e-5)
+        assert (pg[nkv * P_ * (dk + dv):] == 9.0).all()                  # what lies behind keys and values is left alone
+
+
+@pytest.mark.parametrize("dk,dv", [(32, 32), (64, 96), (96, 32), (128, 128), (160, 64), (256, 32), (48, 32), (64, 40)])
+@pytest.mark.parametrize("counts", [[1, 1, 1], [3, 1, 16, 2], [2, 1]])
+def test_lightning_scan_forms(dk, dv, counts):
+    """The scan with the state in registers (dk and dv in steps of 32) and the general one: single tokens, where the search for
+    a segment is skipped, and short portions; a segment that starts at position 0 over a slot with something in it."""
+    from mini_hisparse_b200.kernels import api as K
+
+    H, T, S = 3, sum(counts), len(counts)
+    g = torch.Generator(device="cuda").manual_seed(dk + dv + T)
+    proj = torch.randn(5, T, H * (2 * dk + dv), device="cuda", generator=g) * 0.4
+    state = torch.randn(S + 2, H, dk, dv, device="cuda", generator=g)
+    lam = torch.tensor([0.5, 0.9, 0.999], device="cuda")
+    slots = torch.tensor([s + 1 for s in range(S)][::-1], dtype=torch.int32, device="cuda")
+    seg = torch.tensor(sum(([s] * n for s, n in enumerate(counts)), []), dtype=torch.int32, device="cuda")
+    pos = torch.tensor(sum((list(range(0 if s == 1 else 40, (0 if s == 1 else 40) + n)) for s, n in enumerate(counts)), []),
+                       dtype=torch.int32, device="cuda")
+    before, out = state.clone(), torch.empty(T, H * dv, device="cuda")
+    K.lightning_scan(proj, 0, H * dk, 2 * H * dk, lam, state, out, seg, slots, pos, heads=H, dk=dk, dv=dv, nsplit=5,
+                     split_stride=proj.stride(0))
+    z = proj.double().sum(0)
+    z = z * torch.sigmoid(z)
+    q, k, v = (y.view(T, H, -1) for y in z.split([H * dk, H * dk, H * dv], -1))
+    t = 0
+    for s, n in enumerate(counts):
+        St = before[slots[s]].double() * (0.0 if s == 1 else 1.0)
+        for _ in range(n):
+            St = lam.double()[:, None, None] * St + k[t][:, :, None] * v[t][:, None, :]
+            torch.testing.assert_close(out[t].double().view(H, dv), (St * q[t][:, :, None]).sum(1), atol=1e-5 * math.sqrt(dk), rtol=1e-5)
+            t += 1
+        torch.testing.assert_close(state[slots[s]].double(), St, atol=1e-5, rtol=1e-5)
+    for other in (0, S + 1):
+        assert torch.equal(state[other], before[other])
+
+
 def plain_lightning(q, k, v, lam, S0):
     """o_t = S_t^T q_t with S_t = lam S_(t-1) + k_t v_t^T, for one head; returns (o, S)."""
     S, out = S0.clone(), []
