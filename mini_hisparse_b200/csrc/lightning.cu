@@ -49,9 +49,7 @@ struct LightArgs {
 __device__ __forceinline__ float siluf(float z) { return z / (1.f + expf(-z)); }
 
 __device__ __forceinline__ float load_silu(const LightArgs& a, size_t idx) {
-    float v = a.proj[idx];
-    for (int s = 1; s < a.nsplit; ++s) v += a.proj[idx + (size_t)s * a.split_stride];
-    return siluf(v);
+    return siluf(sum_parts(a.proj + idx, a.nsplit, a.split_stride));
 }
 
 // first token of segment `seg` and one past its last, by bisection of the ascending tok_seg
@@ -114,6 +112,78 @@ lightning_scan_kernel(const LightArgs a, int max_tokens) {
     __syncthreads();
     if (a.writable)
         for (int i = threadIdx.x; i < dk * dv; i += blockDim.x) slot[i] = St[i];
+}
+
+// The same with the state in registers and a head's value columns dealt to gridDim.z CTAs of 32 (dk in steps of 32 up to
+// 256, dv in steps of 32, rows on 16 bytes).  A thread holds four columns of every 32nd row.  What a decode step waits
+// for is the state's way from memory and back: with a CTA per head that walked it one element a thread and step through
+// shared memory, 41 us for 8 requests of 16 heads of 128 x 128 (16 MB to move, 3 us of copy bandwidth).
+template <int RPT>
+__global__ void __launch_bounds__(256)
+lightning_scan_vec_kernel(const LightArgs a, int max_tokens) {
+    constexpr int DK = 32 * RPT;
+    __shared__ __align__(16) float qs[DK], ks[DK], vs[32];
+    __shared__ float4 po[8][8];                       // [warp][column quad]
+    pdl_launch_dependents();
+    const int seg = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * 32, dv = a.dv;
+    const int c4 = threadIdx.x & 7, r0 = threadIdx.x >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the index arrays and the decay do not change during a step
+    int t0 = seg, t1 = seg + 1;
+    // as many segments as tokens, and this one's only token at its place (a decode step): no search
+    if (a.T != (int)gridDim.x || a.tok_seg[seg] != seg || a.tok_seg[max(seg - 1, 0)] == (seg ? seg : -1) ||
+        a.tok_seg[min(seg + 1, a.T - 1)] == (seg + 1 < a.T ? seg : -1))
+        segment_range(a.tok_seg, a.T, seg, t0, t1);
+    const bool skip = t1 <= t0 || (max_tokens > 0 && t1 - t0 > max_tokens);      // longer segments go the chunked way
+    const float lam = a.decay[h];
+    float* slot = a.state + ((size_t)a.seg_slot[seg] * a.H + h) * DK * dv + col0 + 4 * c4;
+    const bool fresh = !skip && a.positions[t0] == 0;
+    if (!skip && !fresh && c4 == 0) {                 // towards the L2 while the kernel before this one still runs
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(slot + (size_t)(r0 + 32 * i) * dv));
+    }
+    pdl_wait();
+    if (skip) return;
+    float4 S[RPT];
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) S[i] = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : vec4(slot + (size_t)(r0 + 32 * i) * dv);
+    for (int t = t0; t < t1; ++t) {
+        const float* row = a.proj + (size_t)t * a.ld;
+        for (int u = threadIdx.x; u < 2 * (DK / 4) + 8; u += 256) {
+            const bool q = u < DK / 4, k = !q && u < DK / 2;
+            const int e = 4 * (q ? u : k ? u - DK / 4 : u - DK / 2);
+            const int col = q ? a.q0 + h * DK + e : k ? a.k0 + h * DK + e : a.v0 + h * dv + col0 + e;
+            const float4 v = sum_parts4<8>(row + col, a.nsplit, a.split_stride);
+            *(float4*)((q ? qs : k ? ks : vs) + e) = make_float4(siluf(v.x), siluf(v.y), siluf(v.z), siluf(v.w));
+        }
+        __syncthreads();
+        const float4 v = vec4(vs + 4 * c4);
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const float k = ks[r0 + 32 * i], q = qs[r0 + 32 * i];
+            S[i].x = fmaf(lam, S[i].x, k * v.x); S[i].y = fmaf(lam, S[i].y, k * v.y);
+            S[i].z = fmaf(lam, S[i].z, k * v.z); S[i].w = fmaf(lam, S[i].w, k * v.w);
+            o.x = fmaf(S[i].x, q, o.x); o.y = fmaf(S[i].y, q, o.y);
+            o.z = fmaf(S[i].z, q, o.z); o.w = fmaf(S[i].w, q, o.w);
+        }
+#pragma unroll
+        for (int m = 8; m < 32; m <<= 1) {            // the warp's four rows of a column
+            o.x += __shfl_xor_sync(0xffffffffu, o.x, m); o.y += __shfl_xor_sync(0xffffffffu, o.y, m);
+            o.z += __shfl_xor_sync(0xffffffffu, o.z, m); o.w += __shfl_xor_sync(0xffffffffu, o.w, m);
+        }
+        if (lane < 8) po[warp][lane] = o;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            float sum = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) sum += ((const float*)po[w])[threadIdx.x];
+            a.out[(size_t)t * a.H * dv + h * dv + col0 + threadIdx.x] = sum;
+        }
+    }
+    if (a.writable) {
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) *(float4*)(slot + (size_t)(r0 + 32 * i) * dv) = S[i];
+    }
 }
 
 // ---- chunked: (1) every chunk's own contribution -----------------------------------------------------
@@ -616,6 +686,22 @@ MHB_EXPORT int mhb_lightning_scan(const float* proj, int nsplit, long long split
     if (H > 65535) return fail("lightning: too many heads");
     const LightArgs a = make_args(proj, nsplit, split_stride, ld, q0, k0, v0, decay, state, out, tok_seg, seg_slot,
                                   positions, T, H, dk, dv, writable);
+    if (dk % 32 == 0 && dk <= 256 && dv % 32 == 0 && dv / 32 <= 65535 && ((ld | q0 | k0 | v0) & 3) == 0 &&
+        (split_stride & 3) == 0 && !(((uintptr_t)proj | (uintptr_t)state) & 15)) {
+        auto kern = lightning_scan_vec_kernel<8>;
+        switch (dk / 32) {
+            case 1: kern = lightning_scan_vec_kernel<1>; break;
+            case 2: kern = lightning_scan_vec_kernel<2>; break;
+            case 3: kern = lightning_scan_vec_kernel<3>; break;
+            case 4: kern = lightning_scan_vec_kernel<4>; break;
+            case 5: kern = lightning_scan_vec_kernel<5>; break;
+            case 6: kern = lightning_scan_vec_kernel<6>; break;
+            case 7: kern = lightning_scan_vec_kernel<7>; break;
+            default: break;
+        }
+        launch_kernel(kern, dim3(S, H, dv / 32), dim3(256), 0, stream, a, max_tokens);
+        return check_launch("lightning_scan");
+    }
     const int R = 256 / dv > 1 ? 256 / dv : 1;
     const size_t smem = sizeof(float) * ((size_t)dk * dv + 2 * dk + dv + (size_t)R * dv);
     if (allow_smem(lightning_scan_kernel, smem, "lightning_scan")) return -1;
