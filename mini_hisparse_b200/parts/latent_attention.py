@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .attention import ITEM_INTS, ROW_TILE, AttentionPlanner, AttentionShape
+from .attention import ITEM_INTS, ROW_TILE, SPLIT_MAX_TOKENS, AttentionPlanner, AttentionShape
 from .base import CacheView, Mixer, Product, StepContext
 from .multimap_attention import _pad_rows
 from .registry import POSITIONS, register_mixer
@@ -156,7 +156,7 @@ class LatentAttention(Mixer):
                     K.attention_tma_ext(*args, meta["items"], n_small, 16, *tail, nq=self.heads, nkv=1, d=self.width,
                                         page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                         shared_kv=True, **opts, tok_nsplit=meta["tok_nsplit"], counters=counters,
-                                        status=ctx.status)
+                                        status=ctx.status, fresh=SPLIT_MAX_TOKENS)
                 else:
                     K.attention_mma_ext(*args, meta["items"], n_small, 16, *tail, **common,
                                         tok_nsplit=meta["tok_nsplit"], counters=counters)

@@ -6,7 +6,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .attention import ITEM_INTS, ROW_TILE, AttentionPlanner, AttentionShape
+from .attention import ITEM_INTS, ROW_TILE, SPLIT_MAX_TOKENS, AttentionPlanner, AttentionShape
 from .base import CacheView, Mixer, Product, StepContext
 from .registry import POSITIONS, register_mixer
 from .spec import PagedKVNeed, ParamSpec, PartSpec
@@ -144,7 +144,7 @@ class DifferentialAttention(Mixer):
                 K.attention_tma_ext(*args, meta["items"], n_small, 16, *tail, nq=self.nq, nkv=self.nkv, d=self.dv,
                                     page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                     softcap=self.softcap, tok_nsplit=meta["tok_nsplit"], counters=counters,
-                                    status=ctx.status)
+                                    status=ctx.status, fresh=SPLIT_MAX_TOKENS)
             if n_big:
                 K.attention_tc_ext(q, cache.storage, maps, big_items, n_big, ctx.positions, meta["block_table"],
                                    nq=self.nq, nkv=self.nkv, d=self.dv, page_size=cache.page_size,

@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .attention import ITEM_INTS, ROW_TILE, AttentionPlanner, AttentionShape
+from .attention import ITEM_INTS, ROW_TILE, SPLIT_MAX_TOKENS, AttentionPlanner, AttentionShape
 from .base import CacheView, Mixer, Product, StepContext
 from .registry import POSITIONS, register_mixer
 from .spec import PagedKVNeed, ParamSpec, PartSpec
@@ -143,7 +143,7 @@ class SinkAttention(Mixer):
                     K.attention_tma_ext(*args, meta["items"], n_small, 16, *tail, nq=self.nq, nkv=self.nkv, d=self.dk,
                                         page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                         sink=sink, slopes=slopes, **gate, tok_nsplit=meta["tok_nsplit"], counters=counters,
-                                        status=ctx.status)
+                                        status=ctx.status, fresh=SPLIT_MAX_TOKENS)
                 else:
                     K.attention_mma_ext(*args, meta["items"], n_small, 16, *tail, **common,
                                         tok_nsplit=meta["tok_nsplit"], counters=counters)
