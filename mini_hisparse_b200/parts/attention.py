@@ -34,11 +34,14 @@ class AttentionShape:
     window: int | None = None
     tile_rows: int = ROW_TILE
 
-    @property
-    def min_keys(self) -> int:
-        """The shortest key split.  The tensor-core kernels walk 256 keys in the time a split costs to start and to merge;
-        the CUDA-core kernel (ROW_TILE rows for every portion) takes that long for two of its 32-key tiles."""
-        return MIN_KEYS_PER_SIMT_SPLIT if self.tile_rows == ROW_TILE else MIN_KEYS_PER_SPLIT
+    def max_splits(self, keys: int) -> int:
+        """How many splits ``keys`` keys are worth.  The tensor-core kernels walk 256 keys in the time a split costs to start
+        and to merge.  The CUDA-core kernel (ROW_TILE rows for every portion) takes about 1 us for a tile of 32 keys, and its
+        merge is a launch of 2.3 us: splits of 64 keys, once there are three (a turn of short histories that were cut
+        in two took 6 % longer than uncut)."""
+        if self.tile_rows == ROW_TILE:
+            return max(1, keys // MIN_KEYS_PER_SIMT_SPLIT) if keys >= 3 * MIN_KEYS_PER_SIMT_SPLIT else 1
+        return max(1, keys // MIN_KEYS_PER_SPLIT)
 
 
 @dataclass
@@ -100,7 +103,7 @@ def plan_attention(need: AttentionShape, segments, T: int, sm_count: int = 148,
     # SM, so that a long history beside short ones is cut into more parts and no CTA runs alone at
     # the end
     small_keys = sum(t[4] - t[3] for t in small_tiles) * len(small_chunks) * need.kv_heads
-    target = max(need.min_keys, -(-small_keys // (2 * sm_count)))
+    target = max(MIN_KEYS_PER_SIMT_SPLIT if need.tile_rows == ROW_TILE else MIN_KEYS_PER_SPLIT, -(-small_keys // (2 * sm_count)))
     target = -(-target // KEY_TILE) * KEY_TILE
     items = []
     tok_part_row = np.zeros(T, np.int32)
@@ -111,7 +114,7 @@ def plan_attention(need: AttentionShape, segments, T: int, sm_count: int = 148,
         if fixed_nsplit is not None:
             nsplit = fixed_nsplit
         else:
-            fit = max(1, (kv_end - kv_begin) // need.min_keys)
+            fit = need.max_splits(kv_end - kv_begin)
             nsplit = max(1, min(-(-(kv_end - kv_begin) // target), fit, MAX_SPLITS))
         if nsplit == 1:
             for h0, nh in small_chunks:
@@ -273,11 +276,11 @@ class AttentionPlanner(StepPlanner):
         """Key shares per decoded token for a batch of B with at most ``max_positions`` cached keys, as
         (shares in a cluster, clusters per token and KV head): as many CTAs as are resident at once (two per
         SM), never more, so that no CTA waits for a second wave, and no share shorter than
-        ``shape.min_keys`` keys.  Without a cluster kernel: (shares, 1)."""
+        ``shape.max_splits`` allows.  Without a cluster kernel: (shares, 1)."""
         ctas = segments_count * self.shape.kv_heads * self.chunks
         if self.shape.window:            # a token never attends to more keys than its window holds
             max_positions = min(max_positions, self.shape.window)
-        n = max(1, min(MAX_SPLITS, (2 * self.sm_count) // ctas, max_positions // self.shape.min_keys))
+        n = max(1, min(MAX_SPLITS, (2 * self.sm_count) // ctas, self.shape.max_splits(max_positions)))
         if self.clusters_of is None or self.chunks != 1 or n == 1:
             return n, 1
         # The shares of a cluster are merged in its shared memory, and a cluster is placed inside one
@@ -330,7 +333,7 @@ class AttentionPlanner(StepPlanner):
         fixed = self.decode_fixed(len(starts), max_positions)
         n0 = fixed[0] * fixed[1]
         B = len(starts)
-        limit = min(max_positions // self.shape.min_keys, self.max_cluster or MAX_SPLITS)
+        limit = min(self.shape.max_splits(max_positions), self.max_cluster or MAX_SPLITS)
         if n0 > 1 or B < 2 or limit < 2:       # fewer requests: their splits are sized for one round of CTAs
             return fixed
         tiles = (np.asarray(starts, np.int64) + KEY_TILE) // KEY_TILE
