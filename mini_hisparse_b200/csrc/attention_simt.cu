@@ -107,7 +107,7 @@ __device__ __forceinline__ float4 tile4(const __nv_bfloat16* p) {
 // buffered and arrive by 16-byte cp.async (a.vec: widths and pages allow it) while the tile before is attended to, their
 // pages are looked up a tile earlier, by one lane a key, and scores read four elements at once, for all of a warp's rows.
 // A decode step of 4 requests with up to 281 cached positions (3 heads of 32, float32) took 44 us a layer here before; the
-// whole step, with the products of gemm_f32.cu, went from 292 to 139 us.  Splits may now be as short as 64 keys.
+// whole step, with the products of gemm_f32.cu, went from 292 to 139 us.  Splits may now be as short as 128 keys.
 template <typename CT, int DPL>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_simt_kernel(const AttnArgs a) {

@@ -255,6 +255,53 @@ lightning_chunk_prefix_kernel(const LightArgs a, const int* __restrict__ seg_chu
     if (a.writable) slot[idx] = S;
 }
 
+// The same with four elements a thread (dk dv in steps of 4, slots on 16 bytes): a quarter of the requests for the same
+// bytes in flight.
+__global__ void __launch_bounds__(256)
+lightning_chunk_prefix_vec_kernel(const LightArgs a, const int* __restrict__ seg_chunks, const int* __restrict__ chunks,
+                                  float* __restrict__ U) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int s = blockIdx.x, h = blockIdx.y;
+    const int seg = seg_chunks[4 * s], c0 = seg_chunks[4 * s + 1], nc = seg_chunks[4 * s + 2], t0 = seg_chunks[4 * s + 3];
+    const size_t size = (size_t)a.dk * a.dv, idx = 4 * ((size_t)blockIdx.z * blockDim.x + threadIdx.x);
+    if (idx >= size) return;
+    const float lam = a.decay[h];
+    float* slot = a.state + ((size_t)a.seg_slot[seg] * a.H + h) * size + idx;
+    const int n_full = chunks[4 * c0 + 2];
+    const float lam_full = powf(lam, (float)n_full);
+    const size_t stride = (size_t)a.H * size;
+    float* u = U + ((size_t)c0 * a.H + h) * size + idx;
+    float4 S = a.positions[t0] == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : vec4(slot);
+    for (int c = 0; c < nc; c += 8) {
+        float4 own[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (c + i < nc) own[i] = vec4(u + (size_t)(c + i) * stride);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (c + i < nc) {
+                *(float4*)(u + (size_t)(c + i) * stride) = S;
+                const int n = chunks[4 * (c0 + c + i) + 2];
+                const float l = n == n_full ? lam_full : powf(lam, (float)n);
+                S.x = fmaf(l, S.x, own[i].x); S.y = fmaf(l, S.y, own[i].y);
+                S.z = fmaf(l, S.z, own[i].z); S.w = fmaf(l, S.w, own[i].w);
+            }
+        }
+    }
+    if (a.writable) *(float4*)slot = S;
+}
+
+void launch_prefix(const LightArgs& a, const int* seg_chunks, int num_segs, const int* chunks, float* U, cudaStream_t stream) {
+    const int size = a.dk * a.dv;
+    if (size % 4 == 0 && !(((uintptr_t)a.state | (uintptr_t)U) & 15))
+        launch_kernel(lightning_chunk_prefix_vec_kernel, dim3(num_segs, a.H, (size / 4 + 255) / 256), dim3(256), 0, stream, a,
+                      seg_chunks, chunks, U);
+    else
+        launch_kernel(lightning_chunk_prefix_kernel, dim3(num_segs, a.H, (size + 255) / 256), dim3(256), 0, stream, a,
+                      seg_chunks, chunks, U);
+}
+
 // ---- chunked: (3) outputs -----------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 lightning_chunk_out_kernel(const LightArgs a, const int* __restrict__ chunks, const float* __restrict__ U, int C) {
@@ -732,7 +779,7 @@ MHB_EXPORT int mhb_lightning_chunked(const float* proj, int nsplit, long long sp
     if (allow_smem(lightning_chunk_out_kernel, s3, "lightning_chunk_out")) return -1;
     launch_kernel(lightning_chunk_state_kernel, dim3(num_chunks, H), dim3(256), s1, stream, a, chunks, U, C);
     if (check_launch("lightning_chunk_state")) return -1;
-    launch_kernel(lightning_chunk_prefix_kernel, dim3(num_segs, H, (dk * dv + 255) / 256), dim3(256), 0, stream, a, seg_chunks, chunks, U);
+    launch_prefix(a, seg_chunks, num_segs, chunks, U, stream);
     if (check_launch("lightning_chunk_prefix")) return -1;
     launch_kernel(lightning_chunk_out_kernel, dim3(num_chunks, H), dim3(256), s3, stream, a, chunks, (const float*)U, C);
     return check_launch("lightning_chunk_out");
@@ -755,7 +802,7 @@ int launch_chunked_tc(const LightArgs& a, const int* chunks, int num_chunks, con
     if (allow_smem(lightning_chunk_out_tc_kernel<DK, DV>, s3_used, "lightning_chunk_out_tc")) return -1;
     launch_kernel(lightning_chunk_state_tc_kernel<DK, DV>, dim3(num_chunks, a.H), dim3(STATE_THREADS), s1, stream, a, chunks, U);
     if (check_launch("lightning_chunk_state_tc")) return -1;
-    launch_kernel(lightning_chunk_prefix_kernel, dim3(num_segs, a.H, (a.dk * a.dv + 255) / 256), dim3(256), 0, stream, a, seg_chunks, chunks, U);
+    launch_prefix(a, seg_chunks, num_segs, chunks, U, stream);
     if (check_launch("lightning_chunk_prefix")) return -1;
     launch_kernel(lightning_chunk_out_tc_kernel<DK, DV>, dim3(num_chunks, a.H), dim3(OUT_THREADS), s3_used, stream, a, chunks,
                   (const float*)U, staged ? 1 : 0);

@@ -364,8 +364,8 @@ __global__ void qknorm_rope_append_kernel(const float* __restrict__ qkv, int nsp
 // thread asks for all its loads at once, both norms' sums cross the CTA at one barrier, and angles, pages and the
 // destination are worked out before the kernel waits for the product.  One element a thread and step, with two block-wide
 // sums in turn and the values loaded after them, took 10.6 us for 8 tokens of 16 heads and 62 us for 2,048 of 32.
-template <typename CT>
-__global__ void __launch_bounds__(1024)
+template <typename CT, int B, int MOST>
+__global__ void __launch_bounds__(MOST)
 qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t split_stride, int ld,
                                               const float* __restrict__ q_weight, const float* __restrict__ k_weight,
                                               float eps, const int* __restrict__ positions,
@@ -409,10 +409,10 @@ qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t 
     const bool keep_v = v_eps > 0.f || v_from_k;
     const int loads = (qw + kw + (v_from_k ? 0 : vw)) >> 2;
     float ssq = 0.f, ssk = 0.f;
-#pragma unroll 2
+#pragma unroll (B == 1 ? 4 : 1)
     for (int u = threadIdx.x; u < loads; u += blockDim.x) {
         const int i = 4 * u;
-        float4 v = sum_parts4<8>(row + i, nsplit, split_stride);
+        float4 v = sum_parts4<B>(row + i, nsplit, split_stride);
         if (i < qw + kw) {
             if (bias) { const float4 b = vec4(bias + i); v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
             *(float4*)(sh + i) = v;
@@ -638,13 +638,16 @@ MHB_EXPORT int mhb_qknorm_rope_append_opts(const float* qkv, int nsplit, long lo
                                 (uintptr_t)cache | (uintptr_t)bias;
     if (dk % 4 == 0 && dv % 4 == 0 && rdim % 8 == 0 && ld % 4 == 0 && split_stride % 4 == 0 && page_extra % 4 == 0 &&
         !(addresses & 15)) {
-        // few tokens: a thread for every four elements; many: half as many, so that several tokens share an SM
-        const int quads = (qw + kw + (has_kv && !v_from_k ? nkv * dv : 0)) / 4, want = T <= 64 ? quads : (quads + 1) / 2;
-        const int most = T <= 64 ? 1024 : 512;
+        // few tokens: a thread for every four elements; many: a quarter as many, with four loads of its own in flight, so
+        // that several tokens share an SM
+        const int quads = (qw + kw + (has_kv && !v_from_k ? nkv * dv : 0)) / 4, want = T <= 64 ? quads : (quads + 3) / 4;
+        const int most = T <= 64 ? 1024 : 256;
         int threads = (want + 31) / 32 * 32;
         threads = threads < 64 ? 64 : threads > most ? most : threads;
         MHB_DISPATCH_DTYPE(dtype, CT, {
-            auto kern = qknorm_rope_append_vec_kernel<CT>;
+            auto kern = T <= 64       ? qknorm_rope_append_vec_kernel<CT, 8, 1024>
+                        : nsplit > 1 ? qknorm_rope_append_vec_kernel<CT, 8, 256>
+                                     : qknorm_rope_append_vec_kernel<CT, 1, 256>;
             if (allow_smem(kern, smem, "qknorm_rope_append")) return -1;
             launch_kernel(kern, dim3(T), dim3(threads), smem, stream, qkv, nsplit, (size_t)split_stride, ld, q_weight,
                           k_weight, eps, positions, tok_seg, block_table, table_width, inv_freq, rdim, (CT*)q_out,

@@ -15,7 +15,7 @@ ROW_TILE = 16          # query rows (tokens x heads of one group) per CTA of the
 KEY_TILE = 64          # split boundaries are multiples of the kernels' key tile
 ITEM_INTS = 8
 MIN_KEYS_PER_SPLIT = 256
-MIN_KEYS_PER_SIMT_SPLIT = 64
+MIN_KEYS_PER_SIMT_SPLIT = 128
 SPLIT_MAX_TOKENS = 16  # only short segments (decode tokens, tiny portions) are split along the keys
 MAX_SPLITS = 64
 MAX_BIG_SPLITS = 8       # key splits of a long portion's tile (tcgen05 kernel only)
@@ -36,11 +36,11 @@ class AttentionShape:
 
     def max_splits(self, keys: int) -> int:
         """How many splits ``keys`` keys are worth.  The tensor-core kernels walk 256 keys in the time a split costs to start
-        and to merge.  The CUDA-core kernel (ROW_TILE rows for every portion) takes about 1 us for a tile of 32 keys, and its
-        merge is a launch of 2.3 us: splits of 64 keys, once there are three (a turn of short histories that were cut
-        in two took 6 % longer than uncut)."""
+        and to merge.  The CUDA-core kernel (ROW_TILE rows for every portion) takes about 1 us for a tile of 32 keys; its merge
+        is a launch of 2.5 to 3.7 us, and a plan with splits costs the host 15 us a step more: splits of 128 keys, once
+        there are four (histories of 20 keys in a graph for 256, cut in four, took 13 % longer than uncut)."""
         if self.tile_rows == ROW_TILE:
-            return max(1, keys // MIN_KEYS_PER_SIMT_SPLIT) if keys >= 3 * MIN_KEYS_PER_SIMT_SPLIT else 1
+            return keys // MIN_KEYS_PER_SIMT_SPLIT if keys >= 4 * MIN_KEYS_PER_SIMT_SPLIT else 1
         return max(1, keys // MIN_KEYS_PER_SPLIT)
 
 
