@@ -83,12 +83,16 @@ template <int VEC> __device__ __forceinline__ void store_f(__nv_bfloat16* p, con
     } else *p = __float2bfloat16_rn(v[0]);
 }
 template <int VEC> __device__ __forceinline__ void add_parts(const float* p, int nsplit, size_t stride, float (&v)[VEC]) {
-#pragma unroll 4
-    for (int s = 0; s < nsplit; ++s) {
-        float d[VEC];
-        load_f<VEC>(p + (size_t)s * stride, d);
+    for (int s = 0; s < nsplit; s += 8) {            // eight parts' loads in flight; added in order
+        float d[8][VEC];
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) v[i] += d[i];
+        for (int q = 0; q < 8; ++q)
+            if (s + q < nsplit) load_f<VEC>(p + (size_t)(s + q) * stride, d[q]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (s + q < nsplit)
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) v[i] += d[q][i];
     }
 }
 
@@ -107,8 +111,43 @@ __device__ __forceinline__ void raw_input(const ConvArgs& a, int t, int c, float
     }
 }
 
+// The raw inputs of the tokens t .. t + n - 1 (n <= N).  SINGLE: no product comes in parts; then every token's loads are asked
+// for before the first sum (a loop over parts between them made a token wait for the one before: 28 us for 2,000 tokens of
+// 2048 channels).
+template <int MODE, typename IT, int VEC, bool SINGLE, int N>
+__device__ __forceinline__ void raw_inputs(const ConvArgs& a, int t, int n, int c, float (&v)[N][VEC]) {
+    if constexpr (!SINGLE) {
+#pragma unroll
+        for (int u = 0; u < N; ++u)
+            if (u < n) raw_input<MODE, IT, VEC>(a, t + u, c, v[u]);
+        return;
+    }
+    float d[N][VEC], e[N][VEC];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        if (u >= n) continue;
+        const size_t at = (size_t)(t + u) * a.ld + c;
+        load_f<VEC>((const IT*)a.src + at, v[u]);
+        if constexpr (MODE == STREAM) {
+            if (a.d1.p) load_f<VEC>(a.d1.p + at, d[u]);
+            if (a.d2.p) load_f<VEC>(a.d2.p + at, e[u]);
+        }
+    }
+    if constexpr (MODE == STREAM) {
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            if (u >= n) continue;
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) {
+                if (a.d1.p) v[u][i] += d[u][i];
+                if (a.d2.p) v[u][i] += e[u][i];
+            }
+        }
+    }
+}
+
 // TAPS >= ntaps: the filters are padded with zeros at the old end
-template <int MODE, typename IT, typename OT, int VEC, int TAPS>
+template <int MODE, typename IT, typename OT, int VEC, int TAPS, bool SINGLE>
 __global__ void __launch_bounds__(128)
 conv_kernel(const ConvArgs a) {
     pdl_launch_dependents();
@@ -153,32 +192,44 @@ conv_kernel(const ConvArgs a) {
 #pragma unroll
             for (int i = 0; i < VEC; ++i) v[i] = tanhf(alpha * v[i]) * gain[i] + shift[i];
     };
+    auto raw_one = [&](int t, float (&v)[VEC]) {
+        float one[1][VEC];
+        raw_inputs<MODE, IT, VEC, SINGLE, 1>(a, t, 1, c, one);
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) v[i] = one[0][i];
+    };
     // win[j]: the input TAPS - 1 - j tokens before the one that is next
-    float win[TAPS > 1 ? TAPS - 1 : 1][VEC];
+    constexpr int WIN = TAPS > 1 ? TAPS - 1 : 1;
+    float win[WIN][VEC];
+    const bool small = TAPS <= 4 && TAPS > 1 && !first && R == TAPS - 1;      // the whole window lies before a later tile
+    if (small) {
+        raw_inputs<MODE, IT, VEC, SINGLE, WIN>(a, begin - R, WIN, c, win);
+#pragma unroll
+        for (int j = 0; j < WIN; ++j) activate(win[j]);
+    }
 #pragma unroll
     for (int j = 0; j < TAPS - 1; ++j) {
+        if (small) break;
         const int back = TAPS - 1 - j;
 #pragma unroll
         for (int i = 0; i < VEC; ++i) win[j][i] = 0.f;
         if (back > R) continue;
         if (begin - back >= t0) {
-            raw_input<MODE, IT, VEC>(a, begin - back, c, win[j]);
+            raw_one(begin - back, win[j]);
             activate(win[j]);
         } else if (!fresh) load_f<VEC>(kept + (size_t)(R - back) * a.C + c, win[j]);      // only the first tile gets here
     }
     if (first && a.writable && end < t1) {       // a segment of several tiles: its last R inputs are all its own (TILE >= R)
         for (int r = 0; r < R; ++r) {
             float v[VEC];
-            raw_input<MODE, IT, VEC>(a, t1 - R + r, c, v);
+            raw_one(t1 - R + r, v);
             activate(v);
             store_f<VEC>(kept + (size_t)r * a.C + c, v);
         }
     }
     for (int t = begin; t < end; t += AHEAD) {
         float raw[AHEAD][VEC];
-#pragma unroll
-        for (int u = 0; u < AHEAD; ++u)
-            if (t + u < end) raw_input<MODE, IT, VEC>(a, t + u, c, raw[u]);
+        raw_inputs<MODE, IT, VEC, SINGLE, AHEAD>(a, t, end - t, c, raw);
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u) {
             if (t + u >= end) break;
@@ -229,9 +280,11 @@ int launch_conv(const ConvArgs& a, int S, int longest, bool vec, const char* wha
     // few tokens: small CTAs, so that more SMs take part
     int threads = (long long)S * tiles * a.C / (per * 128) < 296 ? 32 : 128;
     dim3 grid((a.C + per * threads - 1) / (per * threads), S, tiles);
-    if (per == 4) launch_kernel(conv_kernel<MODE, IT, OT, 4, 4>, grid, dim3(threads), 0, stream, a);
-    else if (a.ntaps <= 4) launch_kernel(conv_kernel<MODE, IT, OT, 1, 4>, grid, dim3(threads), 0, stream, a);
-    else launch_kernel(conv_kernel<MODE, IT, OT, 1, MAX_TAPS>, grid, dim3(threads), 0, stream, a);
+    const bool single = (!a.d1.p || a.d1.nsplit == 1) && (!a.d2.p || a.d2.nsplit == 1) && a.nsplit == 1;
+    auto kern = conv_kernel<MODE, IT, OT, 1, MAX_TAPS, false>;
+    if (per == 4) kern = single ? conv_kernel<MODE, IT, OT, 4, 4, true> : conv_kernel<MODE, IT, OT, 4, 4, false>;
+    else if (a.ntaps <= 4) kern = single ? conv_kernel<MODE, IT, OT, 1, 4, true> : conv_kernel<MODE, IT, OT, 1, 4, false>;
+    launch_kernel(kern, grid, dim3(threads), 0, stream, a);
     return check_launch(what);
 }
 

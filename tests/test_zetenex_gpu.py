@@ -186,6 +186,30 @@ def test_norm_and_convolution_in_one_kernel(C, taps, batch):
                 close(kept[slot, 1, :taps - 1], both[n:], 0, f"rows, kept inputs of segment {i}")
 
 
+@pytest.mark.parametrize("C,taps", [(96, 4), (100, 3), (33, 2), (64, 1), (24, 16)])
+@pytest.mark.parametrize("batch", range(len(BATCHES)))
+def test_convolution_with_products_that_are_whole(C, taps, batch):
+    """One part a product (a prompt portion): loads of several tokens at once.  The same numbers as from the summed stream, up
+    to the order of two additions (3 x 2^-24 of values of size 1, through tanh, filters of size 1 and at most 16 taps)."""
+    from mini_hisparse_b200.kernels import api as K
+
+    b = Batch(*BATCHES[batch])
+    g = torch.Generator().manual_seed(C + taps)
+    x, d1, d2 = (torch.randn(b.T, C, generator=g).cuda() for _ in range(3))
+    f, w, shift = torch.randn(taps, C, generator=g).cuda(), torch.randn(C, generator=g).cuda(), torch.randn(C, generator=g).cuda()
+    alpha, keep = torch.tensor([0.7]).cuda(), torch.randn(7, 2, max(taps - 1, 1), C, generator=g).cuda()
+    for deltas in ((d1, None), (d1, d2)):
+        total = x + d1 if deltas[1] is None else x + d1 + d2
+        got, kept, ref, ref_kept = torch.empty_like(x), keep.clone(), torch.empty_like(x), keep.clone()
+        x_out = torch.full_like(x, 7.0)
+        side = [k[:, 1] if taps > 1 else None for k in (kept, ref_kept)]
+        K.stream_conv(x, alpha, w, shift, f, side[0], b, got, delta=Parts(deltas[0]), x_out=x_out,
+                      delta2=Parts(deltas[1]) if deltas[1] is not None else None)
+        K.stream_conv(total, alpha, w, shift, f, side[1], b, ref)
+        for have, want in ((x_out, total), (got, ref), (kept, ref_kept)):
+            torch.testing.assert_close(have, want, atol=4e-6, rtol=4e-6)
+
+
 @pytest.mark.parametrize("C,taps,nsplit,c0", [(96, 4, 1, 16), (96, 4, 3, 3), (20, 1, 2, 0), (36, 2, 1, 8), (24, 7, 2, 4)])
 @pytest.mark.parametrize("batch", range(len(BATCHES)))
 def test_convolution_of_a_products_columns(C, taps, nsplit, c0, batch):
