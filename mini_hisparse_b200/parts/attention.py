@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 from dataclasses import dataclass
+from functools import lru_cache
 
 import numpy as np
 import torch
@@ -177,39 +178,40 @@ def plan_attention(need: AttentionShape, segments, T: int, sm_count: int = 148,
     return AttentionPlan(arr, n_small, len(big_items), tok_part_row, tok_nsplit, part_rows, big_split)
 
 
+@lru_cache(maxsize=64)
+def _decode_template(chunks: tuple, B: int, nsplit: int):
+    """What plan_decode's arrays hold whatever the positions: (items without their key ranges, splits, first partial rows)."""
+    items = np.zeros((B, nsplit, len(chunks), ITEM_INTS), np.int32)
+    seg = np.arange(B, dtype=np.int32)
+    items[..., 0] = items[..., 1] = seg[:, None, None]
+    items[..., 2] = 1
+    items[..., 3:5] = np.asarray(chunks, np.int32)[None, None]
+    items[..., 7] = np.arange(nsplit, dtype=np.int32)[None, :, None] if nsplit > 1 else -1
+    splits = np.full(B, nsplit if nsplit > 1 else 0, np.int32)
+    return items, splits, seg * splits
+
+
 def plan_decode(need: AttentionShape, starts: np.ndarray, nsplit: int) -> AttentionPlan:
     """The plan of a batch of single decoded tokens (token i belongs to segment i and sits at
     position starts[i]) with exactly ``nsplit`` key splits each: what plan_attention gives for such
     a batch with fixed_nsplit, computed with arrays instead of loops."""
     B = len(starts)
-    groups = need.q_heads // need.kv_heads
-    chunks, _ = _tiling(groups, ROW_TILE)
-    C = len(chunks)
+    chunks, _ = _tiling(need.q_heads // need.kv_heads, ROW_TILE)
+    template, splits, part_row = _decode_template(tuple(chunks), B, nsplit)
+    items = template.copy()
     kv_end = starts.astype(np.int64) + 1
-    kv_begin = np.maximum(0, starts - need.window + 1) if need.window else np.zeros(B, np.int64)
-    items = np.empty((B, nsplit, C, ITEM_INTS), np.int32)
-    seg = np.arange(B, dtype=np.int32)
-    items[..., 0] = seg[:, None, None]
-    items[..., 1] = seg[:, None, None]
-    items[..., 2] = 1
-    items[..., 3] = np.asarray([h for h, _ in chunks], np.int32)[None, None, :]
-    items[..., 4] = np.asarray([n for _, n in chunks], np.int32)[None, None, :]
+    kv_begin = np.maximum(0, kv_end - need.window) if need.window else 0
     if nsplit == 1:
-        items[..., 5] = kv_begin[:, None, None]
+        items[..., 5] = kv_begin[:, None, None] if need.window else 0
         items[..., 6] = kv_end[:, None, None]
-        items[..., 7] = -1
-        return AttentionPlan(items.reshape(-1, ITEM_INTS), B * C, 0, np.zeros(B, np.int32),
-                             np.zeros(B, np.int32), 0)
-    span = kv_end - kv_begin
-    chunk = -(-(-(-span // nsplit)) // KEY_TILE) * KEY_TILE
-    ks = np.arange(nsplit, dtype=np.int64)
-    b = np.minimum(kv_end[:, None], kv_begin[:, None] + ks[None, :] * chunk[:, None])
-    e = np.minimum(kv_end[:, None], b + chunk[:, None])
+        return AttentionPlan(items.reshape(-1, ITEM_INTS), B * len(chunks), 0, part_row.copy(), splits.copy(), 0)
+    step = nsplit * KEY_TILE                    # every split gets the same whole number of tiles, the last ones what is left
+    chunk = ((kv_end - kv_begin + step - 1) // step * KEY_TILE)[:, None]
+    end = kv_end[:, None]
+    b = np.minimum(end, chunk * np.arange(nsplit) + (kv_begin[:, None] if need.window else 0))
     items[..., 5] = b[:, :, None]
-    items[..., 6] = e[:, :, None]
-    items[..., 7] = ks[None, :, None]
-    return AttentionPlan(items.reshape(-1, ITEM_INTS), B * nsplit * C, 0,
-                         (seg * nsplit).astype(np.int32), np.full(B, nsplit, np.int32), B * nsplit)
+    items[..., 6] = np.minimum(end, b + chunk)[:, :, None]
+    return AttentionPlan(items.reshape(-1, ITEM_INTS), B * nsplit * len(chunks), 0, part_row.copy(), splits.copy(), B * nsplit)
 
 
 def plan_capacity(need: AttentionShape, max_tokens: int, max_segments: int,
