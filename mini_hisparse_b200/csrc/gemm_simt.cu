@@ -1,8 +1,8 @@
 // C[M,N] = A[M,K] * W[N,K]^T (+ bias) on the CUDA cores with float32 accumulation.
 //
-// This is the matrix product of the true 32-bit path (plain FFMA: no TF32, no tensor core,
-// no reduced-precision intermediate) and the any-shape product of the bfloat16 path for sizes
-// the tensor-core kernel refuses.  A and W are row-major with K contiguous, the layout of
+// Plain FFMA: no TF32, no tensor core, no reduced-precision intermediate.  This is the any-shape
+// product of both dtypes, for sizes that the float32 kernels of gemm_f32.cu and the bfloat16
+// tensor-core kernel refuse, and for products with a bias.  A and W are row-major with K contiguous, the layout of
 // nn.Linear (mini_hisparse/model.py:57-60: y = x W^T + b).
 //
 // With nsplit > 1 the K range is cut into nsplit parts; part z writes a float32 partial
