@@ -73,55 +73,106 @@ __global__ void norm_mix_kernel(float* __restrict__ x, const DT* __restrict__ de
     }
 }
 
-// The same with the row in registers, VC vectors of four elements a thread (H % 4 == 0, every row 16-byte aligned): one
-// vector where rows are few and a thread's chain of loads is the kernel's time, four where there are many.
-template <typename DT, typename OT, int VC, int MOST>
-__global__ void __launch_bounds__(MOST)
+// What the four-element forms below do to a vector.  Every product that is added to something is fused as written here, not
+// as a compiler may choose in each kernel, so that all forms round alike.
+__device__ __forceinline__ void add_scaled(float4& s, float alpha, const float4& v) {
+    s.x = fmaf(alpha, v.x, s.x); s.y = fmaf(alpha, v.y, s.y); s.z = fmaf(alpha, v.z, s.z); s.w = fmaf(alpha, v.w, s.w);
+}
+__device__ __forceinline__ float squares(const float4& s) {
+    return fmaf(s.w, s.w, fmaf(s.z, s.z, fmaf(s.x, s.x, __fmul_rn(s.y, s.y))));
+}
+__device__ __forceinline__ float normed(float s, float rstd, float weight, float keep, float x) {
+    const float n = __fmul_rn(s, rstd);
+    return keep != 0.f ? fmaf(n, weight, __fmul_rn(keep, x)) : __fmul_rn(n, weight);
+}
+__device__ __forceinline__ float4 normed(const float4& s, float rstd, const float4& weight, float keep, const float4& x) {
+    return make_float4(normed(s.x, rstd, weight.x, keep, x.x), normed(s.y, rstd, weight.y, keep, x.y),
+                       normed(s.z, rstd, weight.z, keep, x.z), normed(s.w, rstd, weight.w, keep, x.w));
+}
+
+// The same with the row in registers (H % 4 == 0, every row 16-byte aligned).  The sum of squares is `sums` partial sums in the
+// order of norm_mix_wide_kernel below, so that a row's result does not depend on the form: partial sum j takes the vectors j,
+// j + sums, ..., M of them.  A thread holds Q partial sums: one where rows are few and a thread's chain of loads is the
+// kernel's time (8 rows of 2048 with 18 parts: 6.0 us in the wide form, 4.9 here), up to four where rows are many.
+template <typename DT, typename OT, int Q, int M>
+__global__ void __launch_bounds__(512 / Q)
 norm_mix_vec_kernel(float* __restrict__ x, const DT* __restrict__ delta, int nsplit,
                                     size_t split_stride, const float* __restrict__ weight, float eps,
-                                    float alpha, float keep, OT* __restrict__ copy, int H) {
-    __shared__ float scratch[32];
+                                    float alpha, float keep, OT* __restrict__ copy, int H, int sums) {
+    __shared__ float scratch[16];
     pdl_launch_dependents();
-    const int nvec = H >> 2;
-    float4 w[VC];                            // constant: fetched while the kernel before this one still runs
-#pragma unroll
-    for (int c = 0; c < VC; ++c) {
-        const int i = threadIdx.x + c * blockDim.x;
-        if (VC == 1 && i < nvec) w[c] = vec4(weight + 4 * i);
-    }
+    const int nvec = H >> 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    // vector c = q M + m of this thread; past the end: none
+    auto at = [&](int c) {
+        const int j = ((c / M) * nwarps + warp) * 32 + lane;
+        return j < sums ? j + (c % M) * sums : nvec;
+    };
+    float4 w = make_float4(0.f, 0.f, 0.f, 0.f);         // constant: fetched while the kernel before this one still runs
+    if (Q * M == 1 && at(0) < nvec) w = vec4(weight + 4 * at(0));
     pdl_wait();
     const size_t r = blockIdx.x;
     float* xr = x + r * H;
-    float4 v[VC], s[VC];
-    float ss = 0.f;
+    float4 v[Q * M], s[Q * M];
 #pragma unroll
-    for (int c = 0; c < VC; ++c) {
-        const int i = threadIdx.x + c * blockDim.x;
+    for (int c = 0; c < Q * M; ++c) {
+        const int i = at(c);
         if (i >= nvec) continue;
         v[c] = s[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (alpha != 0.f || keep != 0.f) v[c] = vec4(xr + 4 * i);
-        if (delta) s[c] = sum_parts4<VC == 1 ? 8 : 2>(delta + r * H + 4 * i, nsplit, split_stride);
+        if (delta) s[c] = sum_parts4<Q * M == 1 ? 8 : 2>(delta + r * H + 4 * i, nsplit, split_stride);
     }
 #pragma unroll
-    for (int c = 0; c < VC; ++c) {
-        const int i = threadIdx.x + c * blockDim.x;
-        if (i >= nvec) continue;
-        if (alpha != 0.f) {
-            s[c].x += alpha * v[c].x; s[c].y += alpha * v[c].y; s[c].z += alpha * v[c].z; s[c].w += alpha * v[c].w;
+    for (int q = 0; q < Q; ++q) {
+        float ss = 0.f;
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const int c = q * M + m;
+            if (at(c) >= nvec) continue;
+            if (alpha != 0.f) add_scaled(s[c], alpha, v[c]);
+            ss = __fadd_rn(ss, squares(s[c]));
         }
-        ss += s[c].x * s[c].x + s[c].y * s[c].y + s[c].z * s[c].z + s[c].w * s[c].w;
+        ss = warp_sum(ss);
+        if (lane == 0 && q * nwarps + warp < sums / 32) scratch[q * nwarps + warp] = ss;
+    }
+    __syncthreads();
+    const float total = warp_sum(lane < sums / 32 ? scratch[lane] : 0.f);
+    const float rstd = 1.f / sqrtf(total / (float)H + eps);
+#pragma unroll
+    for (int c = 0; c < Q * M; ++c) {
+        const int i = at(c);
+        if (i >= nvec) continue;
+        const float4 n = normed(s[c], rstd, Q * M == 1 ? w : vec4(weight + 4 * i), keep, v[c]);
+        *(float4*)(xr + 4 * i) = n;
+        if (copy) store4<OT>(copy + r * H + 4 * i, n);
+    }
+}
+
+// Rows of more vectors than 512 threads hold in registers (H > 16384): the row waits in shared memory.
+template <typename DT, typename OT>
+__global__ void __launch_bounds__(512)
+norm_mix_wide_kernel(float* __restrict__ x, const DT* __restrict__ delta, int nsplit,
+                                    size_t split_stride, const float* __restrict__ weight, float eps,
+                                    float alpha, float keep, OT* __restrict__ copy, int H) {
+    extern __shared__ __align__(16) float row[];
+    __shared__ float scratch[32];
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t r = blockIdx.x;
+    float* xr = x + r * H;
+    float ss = 0.f;
+    for (int i = 4 * threadIdx.x; i < H; i += 4 * blockDim.x) {
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (delta) s = sum_parts4<8>(delta + r * H + i, nsplit, split_stride);
+        if (alpha != 0.f) add_scaled(s, alpha, vec4(xr + i));
+        *(float4*)(row + i) = s;
+        ss = __fadd_rn(ss, squares(s));
     }
     const float total = block_sum_once(ss, scratch);
     const float rstd = 1.f / sqrtf(total / (float)H + eps);
-#pragma unroll
-    for (int c = 0; c < VC; ++c) {
-        const int i = threadIdx.x + c * blockDim.x;
-        if (i >= nvec) continue;
-        const float4 wv = VC == 1 ? w[c] : vec4(weight + 4 * i);
-        float4 n = make_float4(s[c].x * rstd * wv.x, s[c].y * rstd * wv.y, s[c].z * rstd * wv.z, s[c].w * rstd * wv.w);
-        if (keep != 0.f) { n.x += keep * v[c].x; n.y += keep * v[c].y; n.z += keep * v[c].z; n.w += keep * v[c].w; }
-        *(float4*)(xr + 4 * i) = n;
-        if (copy) store4<OT>(copy + r * H + 4 * i, n);
+    for (int i = 4 * threadIdx.x; i < H; i += 4 * blockDim.x) {
+        const float4 s = vec4(row + i), n = normed(s, rstd, vec4(weight + i), keep, keep != 0.f ? vec4(xr + i) : s);
+        *(float4*)(xr + i) = n;
+        if (copy) store4<OT>(copy + r * H + i, n);
     }
 }
 
@@ -198,31 +249,37 @@ __global__ void gated_rmsnorm_kernel(const float* __restrict__ o, const float* _
     }
 }
 
-// The same with the row and its gate in registers, VC vectors a thread (N, strides and addresses in 16-byte steps).
+// The same with the row and its gate in registers, VC vectors of four elements a thread (N, strides and addresses in 16-byte
+// steps).  The sum of squares is that of the kernel above, element by element in its order (`sums`: its threads): a thread reads
+// the elements of its partial sums once more, from L1, at the same time as its vectors.
 template <typename OT, int VC>
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(512)
 gated_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_nsplit,
                                          size_t gate_split_stride, int gate_ld, const float* __restrict__ weight,
-                                         float eps, OT* __restrict__ out, int N) {
-    __shared__ float scratch[32];
+                                         float eps, OT* __restrict__ out, int N, int sums) {
+    __shared__ float scratch[16];
     pdl_launch_dependents();
     pdl_wait();
     const size_t r = blockIdx.x;
-    const int nvec = N >> 2;
+    const int nvec = N >> 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const float* row = o + r * N;
     float4 v[VC], g[VC];
-    float ss = 0.f;
 #pragma unroll
     for (int c = 0; c < VC; ++c) {
         const int i = threadIdx.x + c * blockDim.x;
         if (i >= nvec) continue;
-        v[c] = vec4(o + r * N + 4 * i);
+        v[c] = vec4(row + 4 * i);
         if (gate) g[c] = sum_parts4<VC == 1 ? 8 : 2>(gate + r * gate_ld + 4 * i, gate_nsplit, gate_split_stride);
     }
-#pragma unroll
-    for (int c = 0; c < VC; ++c)
-        if ((int)(threadIdx.x + c * blockDim.x) < nvec)
-            ss += v[c].x * v[c].x + v[c].y * v[c].y + v[c].z * v[c].z + v[c].w * v[c].w;
-    const float total = block_sum_once(ss, scratch);
+    for (int u = warp; u < sums / 32; u += nwarps) {
+        float ss = 0.f;
+#pragma unroll 4
+        for (int i = u * 32 + lane; i < N; i += sums) { const float e = row[i]; ss = fmaf(e, e, ss); }
+        ss = warp_sum(ss);
+        if (lane == 0) scratch[u] = ss;
+    }
+    __syncthreads();
+    const float total = warp_sum(lane < sums / 32 ? scratch[lane] : 0.f);
     const float rstd = 1.f / sqrtf(total / (float)N + eps);
 #pragma unroll
     for (int c = 0; c < VC; ++c) {
@@ -530,19 +587,25 @@ MHB_EXPORT int mhb_norm_mix(float* x, const void* delta, int delta_dtype, int ns
     const size_t smem = sizeof(float) * (size_t)H;
     const bool vec = H % 4 == 0 && !((uintptr_t)x & 15) && !((uintptr_t)delta & 15) && !((uintptr_t)weight & 15) &&
                      !((uintptr_t)copy & 15) && split_stride % 4 == 0;
-    // one vector a thread for up to 128 rows, four beyond: 8 rows of 2048 with 18 parts 6.0 us before
-    const int wide = (H / 4 + 31) / 32 * 32, narrow = ((H / 4 + 3) / 4 + 31) / 32 * 32;
-    if (vec && R <= 128 && wide <= 1024) {
-        MHB_DISPATCH_DTYPE(delta_dtype, DT, MHB_DISPATCH_DTYPE(copy_dtype, OT,
-            launch_kernel((norm_mix_vec_kernel<DT, OT, 1, 1024>), dim3(R), dim3(wide < 64 ? 64 : wide), 0, stream, x,
-                          (const DT*)delta, nsplit, (size_t)split_stride, weight, eps, alpha, keep, (OT*)copy, H)));
-        return check_launch("norm_mix");
-    }
-    if (vec && narrow <= 1024) {
-        MHB_DISPATCH_DTYPE(delta_dtype, DT, MHB_DISPATCH_DTYPE(copy_dtype, OT,
-            launch_kernel((narrow <= 256 ? norm_mix_vec_kernel<DT, OT, 4, 256> : norm_mix_vec_kernel<DT, OT, 4, 1024>), dim3(R),
-                          dim3(narrow < 64 ? 64 : narrow), 0, stream, x, (const DT*)delta, nsplit, (size_t)split_stride,
-                          weight, eps, alpha, keep, (OT*)copy, H)));
+    if (vec) {
+        // up to 512 partial sums of M vectors each; a thread takes one of them for up to 128 rows, four vectors beyond
+        const int sums = row_threads(H / 4), m = (H / 4 + sums - 1) / sums;
+        const bool few = R <= 128;
+        MHB_DISPATCH_DTYPE(delta_dtype, DT, MHB_DISPATCH_DTYPE(copy_dtype, OT, {
+            if (m > 8) {
+                auto kern = norm_mix_wide_kernel<DT, OT>;
+                if (allow_smem(kern, smem, "norm_mix")) return -1;
+                launch_kernel(kern, dim3(R), dim3(sums), smem, stream, x, (const DT*)delta, nsplit, (size_t)split_stride, weight,
+                              eps, alpha, keep, (OT*)copy, H);
+            } else {
+                const int q = few || m > 2 ? 1 : m == 2 ? 2 : 4;
+                auto kern = m > 4 ? norm_mix_vec_kernel<DT, OT, 1, 8> : m > 2 ? norm_mix_vec_kernel<DT, OT, 1, 4>
+                            : m == 2 ? (few ? norm_mix_vec_kernel<DT, OT, 1, 2> : norm_mix_vec_kernel<DT, OT, 2, 2>)
+                                     : (few ? norm_mix_vec_kernel<DT, OT, 1, 1> : norm_mix_vec_kernel<DT, OT, 4, 1>);
+                launch_kernel(kern, dim3(R), dim3((sums / 32 + q - 1) / q * 32), 0, stream, x, (const DT*)delta, nsplit,
+                              (size_t)split_stride, weight, eps, alpha, keep, (OT*)copy, H, sums);
+            }
+        }));
         return check_launch("norm_mix");
     }
     MHB_DISPATCH_DTYPE(delta_dtype, DT, MHB_DISPATCH_DTYPE(copy_dtype, OT, {
@@ -595,14 +658,15 @@ MHB_EXPORT int mhb_gated_rmsnorm(const float* o, const float* gate, int gate_nsp
     if (R <= 0) return 0;
     const bool vec = N % 4 == 0 && gate_ld % 4 == 0 && gate_split_stride % 4 == 0 &&
                      !(((uintptr_t)o | (uintptr_t)gate | (uintptr_t)weight | (uintptr_t)out) & 15);
-    const int wide = (N / 4 + 31) / 32 * 32, narrow = ((N / 4 + 3) / 4 + 31) / 32 * 32;
-    if (vec && narrow <= 1024) {
-        const bool few = R <= 128 && wide <= 1024;
-        const dim3 threads(few ? (wide < 64 ? 64 : wide) : (narrow < 64 ? 64 : narrow));
+    // a thread for every four elements of up to 128 rows, a quarter as many beyond; 512 at most
+    const int sums = row_threads(N), want = R <= 128 ? N / 4 : (N / 4 + 3) / 4;
+    const int threads = row_threads(want), vc = (N / 4 + threads - 1) / threads;
+    if (vec && vc <= 8) {
         MHB_DISPATCH_DTYPE(out_dtype, OT, {
-            auto kern = few ? gated_rmsnorm_vec_kernel<OT, 1> : gated_rmsnorm_vec_kernel<OT, 4>;
-            launch_kernel(kern, dim3(R), threads, 0, stream, o, gate, gate_nsplit, (size_t)gate_split_stride, gate_ld,
-                          weight, eps, (OT*)out, N);
+            auto kern = vc == 1 ? gated_rmsnorm_vec_kernel<OT, 1> : vc == 2 ? gated_rmsnorm_vec_kernel<OT, 2>
+                        : vc <= 4 ? gated_rmsnorm_vec_kernel<OT, 4> : gated_rmsnorm_vec_kernel<OT, 8>;
+            launch_kernel(kern, dim3(R), dim3(threads), 0, stream, o, gate, gate_nsplit, (size_t)gate_split_stride, gate_ld,
+                          weight, eps, (OT*)out, N, sums);
         });
         return check_launch("gated_rmsnorm");
     }

@@ -202,6 +202,70 @@ def test_norm_and_gate_forms(R, H, nsplit):
     torch.testing.assert_close(out.double(), want * torch.sigmoid(wide.double().sum(0)[:, 8:]), atol=1e-5, rtol=1e-5)
 
 
+def off16(t):
+    """The same numbers at an address that is not on 16 bytes: what keeps a call on the general kernels."""
+    room = torch.empty(t.numel() + 4, dtype=t.dtype, device=t.device)
+    out = room[1:1 + t.numel()].view(t.shape)
+    out.copy_(t)
+    return out
+
+
+@pytest.mark.parametrize("H,nsplit", [(4, 1), (320, 3), (2048, 18), (2052, 1), (4096, 8), (6000, 2), (16384, 1), (16388, 3)])
+@pytest.mark.parametrize("alpha,keep", [(1.0, 0.0), (1.5, 0.0), (0.0, 1.0), (0.5, 1.7)])
+def test_norm_mix_rounds_the_same_in_every_form(H, nsplit, alpha, keep):
+    """norm_mix has forms for few and for many rows and for rows too wide for registers.  All of them give, bit for bit, what
+    is worked out here: up to 512 partial sums, partial sum j of the vectors of four elements j, j + 512, ...; a warp's and
+    then the warps' sums by halves; fused multiplications where fma() stands."""
+    from mini_hisparse_b200.kernels import api as K
+
+    def fma(a, b, c):          # exact product, one rounding to 53 bits on the way to 24: a second one changes nothing here
+        return (a.double() * b.double() + c.double()).float()
+
+    def halves(v):
+        for o in (16, 8, 4, 2, 1):
+            v = v + v[..., torch.arange(32, device="cuda") ^ o]
+        return v[..., 0]
+
+    R, sums = 131, min(512, max(64, -(-H // 128) * 32))
+    g = torch.Generator(device="cuda").manual_seed(H + nsplit)
+    x, w = (torch.randn(*n, device="cuda", generator=g) for n in ((R, H), (H,)))
+    parts = torch.randn(nsplit, R, H, device="cuda", generator=g)
+    s = parts[0]
+    for p in parts[1:]:
+        s = s + p
+    al, ke, n = (torch.tensor(v, device="cuda") for v in (alpha, keep, float(H)))
+    s = fma(al, x, s) if alpha else s
+    quads, total = s.view(R, H // 4, 4), torch.zeros(R, sums, device="cuda")
+    for at in range(0, H // 4, sums):
+        a, b, c, d = quads[:, at:at + sums].unbind(-1)
+        total[:, :a.shape[1]] += fma(d, d, fma(c, c, fma(a, a, b * b)))
+    warps = torch.zeros(R, 32, device="cuda")
+    warps[:, :sums // 32] = halves(total.view(R, -1, 32))
+    rstd = 1.0 / torch.sqrt(halves(warps) / n + torch.tensor(1e-5, device="cuda"))
+    s = s * rstd[:, None]
+    want = fma(s, w.expand_as(s), ke * x) if keep else s * w
+    for rows in (1, 128, R):
+        got = x[:rows].clone()
+        K.norm_mix(got, w, 1e-5, delta=parts, nsplit=nsplit, split_stride=parts.stride(0), alpha=alpha, keep=keep)
+        assert torch.equal(got, want[:rows])
+
+
+@pytest.mark.parametrize("R,N,nsplit", [(1, 4, 1), (8, 2048, 18), (128, 4096, 8), (129, 4096, 1), (300, 2048, 2), (3, 4100, 9), (130, 5000, 2),
+                                        (2, 16384, 1), (150, 16384, 1), (200, 96, 2)])
+def test_gated_norm_forms_give_the_same_bits(R, N, nsplit):
+    """The four-element forms add a row's squares in the general kernel's order."""
+    from mini_hisparse_b200.kernels import api as K
+
+    g = torch.Generator(device="cuda").manual_seed(R * N + nsplit)
+    x, w = (torch.randn(*n, device="cuda", generator=g) for n in ((R, N), (N,)))
+    wide = torch.randn(nsplit, R, N + 8, device="cuda", generator=g)
+    for opts in ({}, dict(gate=wide[0][:, 8:], gate_nsplit=nsplit, gate_split_stride=wide.stride(0))):
+        got, want = torch.empty(R, N, device="cuda"), torch.empty(R, N, device="cuda")
+        K.gated_rmsnorm(x, w, 1e-5, got, **opts)
+        K.gated_rmsnorm(x, off16(w), 1e-5, want, **opts)
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("dk,dv,rdim,nsplit,T", [(64, 64, 32, 1, 70), (64, 64, 32, 9, 3), (24, 36, 8, 2, 5), (24, 36, 4, 2, 5),
                                                  (16, 16, 16, 18, 64), (20, 20, 0, 3, 65), (22, 30, 6, 2, 4)])
 @pytest.mark.parametrize("per_head", [False, True])
