@@ -292,6 +292,10 @@ gated_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ 
     }
 }
 
+// A rotated pair, fused the same way wherever it is computed
+__device__ __forceinline__ float turned_first(float a, float b, float c, float s) { return fmaf(a, c, -__fmul_rn(b, s)); }
+__device__ __forceinline__ float turned_second(float a, float b, float c, float s) { return fmaf(a, s, __fmul_rn(b, c)); }
+
 // ---- q/k norm over the whole projection, rotation, append ------------------------------------------
 // A row of the product holds [q: nq * dk | k: nkv * dk | v: nkv * dv | anything else]; a layer that
 // reads another layer's cache has [q | anything else] and has_kv = 0.  With v_from_k the row holds [q | k | anything
@@ -398,8 +402,8 @@ __global__ void qknorm_rope_append_kernel(const float* __restrict__ qkv, int nsp
         CT* kdst = (head >= nq && page_k) ? page_k + ((size_t)(head - nq) * P + within) * dk : nullptr;
         if (u < rhalf) {
             const float a = src[u], b = src[u + rhalf];
-            const float oa = a * cs[u] - b * sn[u];
-            const float ob = b * cs[u] + a * sn[u];
+            const float oa = turned_first(a, b, cs[u], sn[u]);
+            const float ob = turned_second(a, b, cs[u], sn[u]);
             if (qdst) { qdst[u] = from_float<QT>(oa); qdst[u + rhalf] = from_float<QT>(ob); }
             else if (kdst) { kdst[u] = from_float<CT>(oa); kdst[u + rhalf] = from_float<CT>(ob); }
         } else {
@@ -432,7 +436,7 @@ qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t 
                                               int dv, int P, int num_pages, int has_kv, int* __restrict__ status,
                                               int per_head, float v_eps, size_t page_extra, float temp_coef,
                                               double temp_every, float v_scale, const float* __restrict__ bias,
-                                              int v_from_k) {
+                                              int v_from_k, int nsums) {
     extern __shared__ __align__(16) float sh[];            // q and k rows, cos, sin, the v row if it is kept
     __shared__ float sums[2][32];
     pdl_launch_dependents();
@@ -465,20 +469,15 @@ qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t 
     const float* row = qkv + (size_t)t * ld;
     const bool keep_v = v_eps > 0.f || v_from_k;
     const int loads = (qw + kw + (v_from_k ? 0 : vw)) >> 2;
-    float ssq = 0.f, ssk = 0.f;
 #pragma unroll (B == 1 ? 4 : 1)
     for (int u = threadIdx.x; u < loads; u += blockDim.x) {
         const int i = 4 * u;
         float4 v = sum_parts4<B>(row + i, nsplit, split_stride);
         if (i < qw + kw) {
-            if (bias) { const float4 b = vec4(bias + i); v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w; }
+            const float4 b = bias ? vec4(bias + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
             *(float4*)(sh + i) = v;
-            const float ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            if (i < qw) ssq += ss;
-            else {
-                ssk += ss;
-                if (v_from_k) *(float4*)(vs + i - qw) = v;
-            }
+            if (v_from_k && i >= qw) *(float4*)(vs + i - qw) = v;
         } else if (keep_v) {
             *(float4*)(vs + i - qw - kw) = v;
         } else if (page_v) {
@@ -488,19 +487,17 @@ qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t 
         }
     }
     float rq = 1.f, rk = 1.f;
+    __syncthreads();
     if (per_head) {
-        __syncthreads();
         const float temp = temp_coef != 0.f ? 1.f + temp_coef * log1pf((float)floor((double)(pos + 1) / temp_every)) : 1.f;
         for (int head = warp; head < (qw + kw) / dk; head += nwarps) {
             float* hr = sh + head * dk;
             const float* w = head < nq ? q_weight : k_weight;
             float ss = 0.f;
-            for (int e = 4 * lane; e < dk; e += 128) {
-                const float4 v = vec4(hr + e);
-                ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
-            }
+            for (int e = lane; e < dk; e += 32) ss = fmaf(hr[e], hr[e], ss);
             const float r = 1.f / sqrtf(warp_sum(ss) / (float)dk + eps);
             const float f = head < nq ? temp : 1.f;
+            __syncwarp();
             for (int e = 4 * lane; e < dk; e += 128) {
                 float4 v = vec4(hr + e);
                 const float4 m = w ? vec4(w + e) : make_float4(1.f, 1.f, 1.f, 1.f);
@@ -509,11 +506,20 @@ qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t 
             }
         }
     } else {
-        ssq = warp_sum(ssq);
-        ssk = warp_sum(ssk);
-        if (lane == 0) { sums[0][warp] = ssq; sums[1][warp] = ssk; }
+        // both sums cross the CTA at one barrier; partial sum j takes the elements j, j + nsums, ...
+        for (int u = warp; u < nsums / 32; u += nwarps) {
+            float ssq = 0.f, ssk = 0.f;
+            for (int i = u * 32 + lane; i < qw + kw; i += nsums) {
+                const float v = sh[i];
+                if (i < qw) ssq = fmaf(v, v, ssq);
+                else ssk = fmaf(v, v, ssk);
+            }
+            ssq = warp_sum(ssq);
+            ssk = warp_sum(ssk);
+            if (lane == 0) { sums[0][u] = ssq; sums[1][u] = ssk; }
+        }
         __syncthreads();
-        const float tq = warp_sum(lane < nwarps ? sums[0][lane] : 0.f), tk = warp_sum(lane < nwarps ? sums[1][lane] : 0.f);
+        const float tq = warp_sum(lane < nsums / 32 ? sums[0][lane] : 0.f), tk = warp_sum(lane < nsums / 32 ? sums[1][lane] : 0.f);
         rq = 1.f / sqrtf(tq / (float)qw + eps);
         rk = kw ? 1.f / sqrtf(tk / (float)kw + eps) : 0.f;
     }
@@ -521,7 +527,7 @@ qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t 
         for (int head = warp; head < (has_kv ? nkv : 0); head += nwarps) {
             float* hr = vs + head * dv;
             float ss = 0.f;
-            for (int e = lane; e < dv; e += 32) ss += hr[e] * hr[e];
+            for (int e = lane; e < dv; e += 32) ss = fmaf(hr[e], hr[e], ss);
             const float r = 1.f / sqrtf(warp_sum(ss) / (float)dv + v_eps);
             for (int e = lane; e < dv; e += 32) hr[e] *= r;
         }
@@ -545,8 +551,10 @@ qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t 
         if (!dst) continue;
         if (u < pairs4) {
             const float4 a = scaled(head, 4 * u), b = scaled(head, 4 * u + rhalf), c = vec4(cs + 4 * u), n = vec4(sn + 4 * u);
-            store4<CT>(dst + 4 * u, make_float4(a.x * c.x - b.x * n.x, a.y * c.y - b.y * n.y, a.z * c.z - b.z * n.z, a.w * c.w - b.w * n.w));
-            store4<CT>(dst + 4 * u + rhalf, make_float4(b.x * c.x + a.x * n.x, b.y * c.y + a.y * n.y, b.z * c.z + a.z * n.z, b.w * c.w + a.w * n.w));
+            store4<CT>(dst + 4 * u, make_float4(turned_first(a.x, b.x, c.x, n.x), turned_first(a.y, b.y, c.y, n.y),
+                                                turned_first(a.z, b.z, c.z, n.z), turned_first(a.w, b.w, c.w, n.w)));
+            store4<CT>(dst + 4 * u + rhalf, make_float4(turned_second(a.x, b.x, c.x, n.x), turned_second(a.y, b.y, c.y, n.y),
+                                                        turned_second(a.z, b.z, c.z, n.z), turned_second(a.w, b.w, c.w, n.w)));
         } else {
             const int e = rdim + 4 * (u - pairs4);
             store4<CT>(dst + e, scaled(head, e));
@@ -698,6 +706,8 @@ MHB_EXPORT int mhb_qknorm_rope_append_opts(const float* qkv, int nsplit, long lo
     if (rdim < 0 || rdim > dk || (rdim & 1)) return fail("qknorm_rope_append: %d rotated elements of a head of %d", rdim, dk);
     const int qw = nq * dk, kw = has_kv ? nkv * dk : 0;
     const size_t smem = sizeof(float) * ((size_t)qw + kw + rdim + ((v_eps > 0.f || v_from_k) && has_kv ? (size_t)nkv * dv : 0));
+    // how many partial sums the norms over whole projections have, whichever form sums them
+    const int nsums = T <= 64 && qw + kw > 512 ? 1024 : row_threads(qw + kw);
     const uintptr_t addresses = (uintptr_t)qkv | (uintptr_t)q_weight | (uintptr_t)k_weight | (uintptr_t)q_out |
                                 (uintptr_t)cache | (uintptr_t)bias;
     if (dk % 4 == 0 && dv % 4 == 0 && rdim % 8 == 0 && ld % 4 == 0 && split_stride % 4 == 0 && page_extra % 4 == 0 &&
@@ -716,14 +726,14 @@ MHB_EXPORT int mhb_qknorm_rope_append_opts(const float* qkv, int nsplit, long lo
             launch_kernel(kern, dim3(T), dim3(threads), smem, stream, qkv, nsplit, (size_t)split_stride, ld, q_weight,
                           k_weight, eps, positions, tok_seg, block_table, table_width, inv_freq, rdim, (CT*)q_out,
                           (CT*)cache, nq, nkv, dk, dv, P, num_pages, has_kv, status, per_head, v_eps, (size_t)page_extra,
-                          temp_coef, temp_every, v_scale, bias, v_from_k);
+                          temp_coef, temp_every, v_scale, bias, v_from_k, nsums);
         });
         return check_launch("qknorm_rope_append");
     }
     MHB_DISPATCH_DTYPE(dtype, CT, {
         auto kern = qknorm_rope_append_kernel<CT, CT>;
         if (allow_smem(kern, smem, "qknorm_rope_append")) return -1;
-        launch_kernel(kern, dim3(T), dim3(T <= 64 && qw + kw > 512 ? 1024 : row_threads(qw + kw)), smem, stream, qkv, nsplit, (size_t)split_stride, ld,
+        launch_kernel(kern, dim3(T), dim3(nsums), smem, stream, qkv, nsplit, (size_t)split_stride, ld,
                       q_weight, k_weight, eps, positions, tok_seg, block_table, table_width, inv_freq, rdim,
                       (CT*)q_out, (CT*)cache, nq, nkv, dk, dv, P, num_pages, has_kv, status, per_head, v_eps,
                       (size_t)page_extra, temp_coef, temp_every, v_scale, bias, v_from_k);

@@ -266,6 +266,38 @@ def test_gated_norm_forms_give_the_same_bits(R, N, nsplit):
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("nq,nkv,dk,dv,rdim,nsplit,T", [(6, 2, 64, 64, 32, 1, 70), (6, 2, 24, 36, 8, 2, 5), (6, 2, 20, 20, 0, 3, 65), (16, 4, 128, 128, 64, 8, 8),
+                                                        (32, 8, 128, 128, 64, 1, 300), (32, 8, 128, 128, 128, 12, 33), (2, 1, 64, 64, 64, 1, 5)])
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_qk_norm_forms_give_the_same_bits(nq, nkv, dk, dv, rdim, nsplit, T, per_head, dtype):
+    """The four-element form against the general kernel, which a bias off 16 bytes chooses: with and without keys of its own,
+    with a norm, a temperature and a scale on the values, and with keys that serve as values."""
+    from mini_hisparse_b200.kernels import api as K
+
+    g = torch.Generator(device="cuda").manual_seed(dk * T + nsplit + nq)
+    P_, width = 3, (7 + T) // 3 + 1
+    qkv = torch.randn(nsplit, T, nq * dk + nkv * (dk + dv) + 4, device="cuda", generator=g)
+    bias = torch.randn((nq + nkv) * dk, device="cuda", generator=g)
+    qw, kw = (torch.randn(dk if per_head else n * dk, device="cuda", generator=g) for n in (nq, nkv))
+    pos = torch.arange(7, 7 + T, dtype=torch.int32, device="cuda")
+    table = torch.randperm(width, generator=torch.Generator().manual_seed(1)).int().cuda().view(1, -1)
+    seg = torch.zeros(T, dtype=torch.int32, device="cuda")
+    inv = 10.0 ** -torch.arange(rdim // 2, device="cuda").float()
+    options = [{}, dict(has_kv=False)]
+    options += [dict(q_temp=(0.3, 5.0), v_eps=1e-5)] if per_head else []
+    options += [dict(v_from_k=True)] if dv == dk else []
+    for opts in options:
+        results = []
+        for b in (bias, off16(bias)):
+            cache = torch.full((width, nkv * P_ * (dk + dv)), 9.0, device="cuda", dtype=dtype)
+            q, status = torch.empty(T, nq * dk, device="cuda", dtype=dtype), torch.zeros(1, dtype=torch.int32, device="cuda")
+            K.qknorm_rope_append(qkv, qw, kw, 1e-6, pos, seg, table, inv, rdim, q, cache, nq=nq, nkv=nkv, dk=dk, dv=dv, page_size=P_,
+                                 nsplit=nsplit, split_stride=qkv.stride(0), status=status, v_scale=0.5, bias=b, per_head=per_head, **opts)
+            results += [q, cache]
+        assert torch.equal(results[0], results[2]) and torch.equal(results[1], results[3])
+
+
 @pytest.mark.parametrize("dk,dv,rdim,nsplit,T", [(64, 64, 32, 1, 70), (64, 64, 32, 9, 3), (24, 36, 8, 2, 5), (24, 36, 4, 2, 5),
                                                  (16, 16, 16, 18, 64), (20, 20, 0, 3, 65), (22, 30, 6, 2, 4)])
 @pytest.mark.parametrize("per_head", [False, True])
