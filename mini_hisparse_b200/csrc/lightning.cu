@@ -114,19 +114,19 @@ lightning_scan_kernel(const LightArgs a, int max_tokens) {
         for (int i = threadIdx.x; i < dk * dv; i += blockDim.x) slot[i] = St[i];
 }
 
-// The same with the state in registers and a head's value columns dealt to gridDim.z CTAs of 32 (dk in steps of 32 up to
-// 256, dv in steps of 32, rows on 16 bytes).  A thread holds four columns of every 32nd row.  What a decode step waits
-// for is the state's way from memory and back: with a CTA per head that walked it one element a thread and step through
-// shared memory, 41 us for 8 requests of 16 heads of 128 x 128 (16 MB to move, 3 us of copy bandwidth).
-template <int RPT>
+// The same with the state in registers and a head's value columns dealt to gridDim.z CTAs of `cols` (32 or 64; dv a multiple of
+// it, dk in steps of 32, rows on 16 bytes).  What a decode step waits for is the state's way from memory and back: with a CTA per
+// head that walked it one element a thread and step through shared memory, 41 us for 8 requests of 16 heads of 128 x 128 (16 MB
+// to move, 3 us of copy bandwidth).  A thread holds one column of the rows r, r + R, ..., the ones that a thread of the kernel
+// above walks in turn (R = 1 << lr = 256 / dv, rounded down to a power of two as there), so that both give the same bits.
+template <int ROWS>
 __global__ void __launch_bounds__(256)
-lightning_scan_vec_kernel(const LightArgs a, int max_tokens) {
-    constexpr int DK = 32 * RPT;
-    __shared__ __align__(16) float qs[DK], ks[DK], vs[32];
-    __shared__ float4 po[8][8];                       // [warp][column quad]
+lightning_scan_vec_kernel(const LightArgs a, int max_tokens, int cols, int lr) {
+    __shared__ __align__(16) float qs[512], ks[512], vs[64];        // q and k by [r][row of the thread], zeros up to ROWS
+    __shared__ float po[256];                                       // [r][column]
     pdl_launch_dependents();
-    const int seg = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * 32, dv = a.dv;
-    const int c4 = threadIdx.x & 7, r0 = threadIdx.x >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int seg = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * cols, dk = a.dk, dv = a.dv;
+    const int j = threadIdx.x % cols, r = threadIdx.x / cols, R = 1 << lr, rows = dk >> lr;
     // the index arrays and the decay do not change during a step
     int t0 = seg, t1 = seg + 1;
     // as many segments as tokens, and this one's only token at its place (a decode step): no search
@@ -135,54 +135,67 @@ lightning_scan_vec_kernel(const LightArgs a, int max_tokens) {
         segment_range(a.tok_seg, a.T, seg, t0, t1);
     const bool skip = t1 <= t0 || (max_tokens > 0 && t1 - t0 > max_tokens);      // longer segments go the chunked way
     const float lam = a.decay[h];
-    float* slot = a.state + ((size_t)a.seg_slot[seg] * a.H + h) * DK * dv + col0 + 4 * c4;
+    float* slot = a.state + (((size_t)a.seg_slot[seg] * a.H + h) * dk + r) * dv + col0 + j;
+    const size_t next = (size_t)R * dv;                                              // to the thread's next row
     const bool fresh = !skip && a.positions[t0] == 0;
-    if (!skip && !fresh && c4 == 0) {                 // towards the L2 while the kernel before this one still runs
-#pragma unroll
-        for (int i = 0; i < RPT; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(slot + (size_t)(r0 + 32 * i) * dv));
+    if (!skip && !fresh && (j & 7) == 0) {            // towards the L2 while the kernel before this one still runs
+#pragma unroll 1
+        for (int i = 0; i < rows; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(slot + i * next));
     }
     pdl_wait();
     if (skip) return;
-    float4 S[RPT];
+    if (rows < ROWS)
+        for (int u = threadIdx.x; u < R * (ROWS - rows); u += blockDim.x) {
+            const int at = u / (ROWS - rows) * ROWS + rows + u % (ROWS - rows);
+            qs[at] = ks[at] = 0.f;
+        }
+    float S[ROWS];
+    {
+        const float* p = slot;
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) S[i] = fresh ? make_float4(0.f, 0.f, 0.f, 0.f) : vec4(slot + (size_t)(r0 + 32 * i) * dv);
+        for (int i = 0; i < ROWS; ++i, p += next) S[i] = fresh || i >= rows ? 0.f : *p;
+    }
     for (int t = t0; t < t1; ++t) {
         const float* row = a.proj + (size_t)t * a.ld;
-        for (int u = threadIdx.x; u < 2 * (DK / 4) + 8; u += 256) {
-            const bool q = u < DK / 4, k = !q && u < DK / 2;
-            const int e = 4 * (q ? u : k ? u - DK / 4 : u - DK / 2);
-            const int col = q ? a.q0 + h * DK + e : k ? a.k0 + h * DK + e : a.v0 + h * dv + col0 + e;
+        for (int u = threadIdx.x; u < 2 * (dk / 4) + cols / 4; u += blockDim.x) {
+            const bool q = u < dk / 4, k = !q && u < dk / 2;
+            const int e = 4 * (q ? u : k ? u - dk / 4 : u - dk / 2);
+            const int col = q ? a.q0 + h * dk + e : k ? a.k0 + h * dk + e : a.v0 + h * dv + col0 + e;
             const float4 v = sum_parts4<8>(row + col, a.nsplit, a.split_stride);
-            *(float4*)((q ? qs : k ? ks : vs) + e) = make_float4(siluf(v.x), siluf(v.y), siluf(v.z), siluf(v.w));
+            const float x[4] = {siluf(v.x), siluf(v.y), siluf(v.z), siluf(v.w)};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int at = ((e + i) & (R - 1)) * ROWS + ((e + i) >> lr);
+                if (q) qs[at] = x[i];
+                else if (k) ks[at] = x[i];
+                else vs[e + i] = x[i];
+            }
         }
         __syncthreads();
-        const float4 v = vec4(vs + 4 * c4);
-        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float vj = vs[j];
+        float part = 0.f;
 #pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-            const float k = ks[r0 + 32 * i], q = qs[r0 + 32 * i];
-            S[i].x = fmaf(lam, S[i].x, k * v.x); S[i].y = fmaf(lam, S[i].y, k * v.y);
-            S[i].z = fmaf(lam, S[i].z, k * v.z); S[i].w = fmaf(lam, S[i].w, k * v.w);
-            o.x = fmaf(S[i].x, q, o.x); o.y = fmaf(S[i].y, q, o.y);
-            o.z = fmaf(S[i].z, q, o.z); o.w = fmaf(S[i].w, q, o.w);
-        }
+        for (int i0 = 0; i0 < ROWS; i0 += 16) {
+            asm volatile("" ::: "memory");            // sixteen rows' q and k in registers at a time
 #pragma unroll
-        for (int m = 8; m < 32; m <<= 1) {            // the warp's four rows of a column
-            o.x += __shfl_xor_sync(0xffffffffu, o.x, m); o.y += __shfl_xor_sync(0xffffffffu, o.y, m);
-            o.z += __shfl_xor_sync(0xffffffffu, o.z, m); o.w += __shfl_xor_sync(0xffffffffu, o.w, m);
+            for (int i = i0; i < i0 + 16; ++i) {
+                S[i] = fmaf(lam, S[i], ks[r * ROWS + i] * vj);
+                part = fmaf(S[i], qs[r * ROWS + i], part);
+            }
         }
-        if (lane < 8) po[warp][lane] = o;
+        po[r * cols + j] = part;
         __syncthreads();
-        if (threadIdx.x < 32) {
-            float sum = 0.f;
-#pragma unroll
-            for (int w = 0; w < 8; ++w) sum += ((const float*)po[w])[threadIdx.x];
-            a.out[(size_t)t * a.H * dv + h * dv + col0 + threadIdx.x] = sum;
+        if (r == 0) {
+            float o = 0.f;
+            for (int x = 0; x < R; ++x) o += po[x * cols + j];
+            a.out[(size_t)t * a.H * dv + h * dv + col0 + j] = o;
         }
     }
     if (a.writable) {
+        asm volatile("" : "+l"(slot));                // the addresses anew instead of kept since the loads
 #pragma unroll
-        for (int i = 0; i < RPT; ++i) *(float4*)(slot + (size_t)(r0 + 32 * i) * dv) = S[i];
+        for (int i = 0; i < ROWS; ++i, slot += next)
+            if (i < rows) *slot = S[i];
     }
 }
 
@@ -733,24 +746,23 @@ MHB_EXPORT int mhb_lightning_scan(const float* proj, int nsplit, long long split
     if (H > 65535) return fail("lightning: too many heads");
     const LightArgs a = make_args(proj, nsplit, split_stride, ld, q0, k0, v0, decay, state, out, tok_seg, seg_slot,
                                   positions, T, H, dk, dv, writable);
-    if (dk % 32 == 0 && dk <= 256 && dv % 32 == 0 && dv / 32 <= 65535 && ((ld | q0 | k0 | v0) & 3) == 0 &&
-        (split_stride & 3) == 0 && !(((uintptr_t)proj | (uintptr_t)state) & 15)) {
-        auto kern = lightning_scan_vec_kernel<8>;
-        switch (dk / 32) {
-            case 1: kern = lightning_scan_vec_kernel<1>; break;
-            case 2: kern = lightning_scan_vec_kernel<2>; break;
-            case 3: kern = lightning_scan_vec_kernel<3>; break;
-            case 4: kern = lightning_scan_vec_kernel<4>; break;
-            case 5: kern = lightning_scan_vec_kernel<5>; break;
-            case 6: kern = lightning_scan_vec_kernel<6>; break;
-            case 7: kern = lightning_scan_vec_kernel<7>; break;
-            default: break;
-        }
-        launch_kernel(kern, dim3(S, H, dv / 32), dim3(256), 0, stream, a, max_tokens);
-        return check_launch("lightning_scan");
-    }
     const int R = 256 / dv > 1 ? 256 / dv : 1;
     const size_t smem = sizeof(float) * ((size_t)dk * dv + 2 * dk + dv + (size_t)R * dv);
+    if (dk % 32 == 0 && dk <= 256 && dv % 32 == 0 && dv / 32 <= 65535 && ((ld | q0 | k0 | v0) & 3) == 0 &&
+        (split_stride & 3) == 0 && !(((uintptr_t)proj | (uintptr_t)state) & 15)) {
+        // more rows than registers hold: half as many a thread where the other form has no room for the state either
+        int lr = R >= 8 ? 3 : R >= 4 ? 2 : R >= 2 ? 1 : 0;
+        if (dk >> lr > 128 && smem > 227 * 1024) ++lr;
+        const int cols = dv % 64 == 0 && lr <= 2 ? 64 : 32, rows = dk >> lr;
+        if (rows <= 128) {
+            auto kern = rows <= 16   ? lightning_scan_vec_kernel<16>
+                        : rows <= 32 ? lightning_scan_vec_kernel<32>
+                        : rows <= 64 ? lightning_scan_vec_kernel<64>
+                                     : lightning_scan_vec_kernel<128>;
+            launch_kernel(kern, dim3(S, H, dv / cols), dim3(cols << lr), 0, stream, a, max_tokens, cols, lr);
+            return check_launch("lightning_scan");
+        }
+    }
     if (allow_smem(lightning_scan_kernel, smem, "lightning_scan")) return -1;
     launch_kernel(lightning_scan_kernel, dim3(S, H), dim3(256), smem, stream, a, max_tokens);
     return check_launch("lightning_scan");

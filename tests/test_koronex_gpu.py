@@ -351,7 +351,31 @@ def test_qk_norm_forms(dk, dv, rdim, nsplit, T, per_head):
         assert (pg[nkv * P_ * (dk + dv):] == 9.0).all()                  # what lies behind keys and values is left alone
 
 
-@pytest.mark.parametrize("dk,dv", [(32, 32), (64, 96), (96, 32), (128, 128), (160, 64), (256, 32), (48, 32), (64, 40)])
+@pytest.mark.parametrize("dk,dv", [(32, 32), (64, 64), (64, 96), (96, 128), (128, 128), (128, 256), (160, 64), (256, 32), (256, 128)])
+def test_lightning_scan_forms_give_the_same_bits(dk, dv):
+    """The state in registers against the state in shared memory, which a product whose columns start off 16 bytes chooses."""
+    from mini_hisparse_b200.kernels import api as K
+
+    H, counts = 3, [3, 1, 16, 2]
+    T, S = sum(counts), len(counts)
+    g = torch.Generator(device="cuda").manual_seed(dk + dv)
+    proj = torch.randn(5, T, 4 + H * (2 * dk + dv), device="cuda", generator=g) * 0.4
+    state = torch.randn(S, H, dk, dv, device="cuda", generator=g)
+    lam, slots = torch.tensor([0.5, 0.9, 0.999], device="cuda"), torch.arange(S, dtype=torch.int32, device="cuda")
+    seg = torch.tensor(sum(([s] * n for s, n in enumerate(counts)), []), dtype=torch.int32, device="cuda")
+    pos = torch.tensor(sum((list(range(0 if s == 1 else 40, (0 if s == 1 else 40) + n)) for s, n in enumerate(counts)), []),
+                       dtype=torch.int32, device="cuda")
+    results = []
+    for col in (4, 1):
+        there, out = state.clone(), torch.empty(T, H * dv, device="cuda")
+        p = proj if col == 4 else torch.cat((proj[..., 3:], proj[..., :3]), -1).contiguous()      # the columns at 1 instead of 4
+        K.lightning_scan(p, col, col + H * dk, col + 2 * H * dk, lam, there, out, seg, slots, pos, heads=H, dk=dk, dv=dv, nsplit=5,
+                         split_stride=p.stride(0))
+        results += [out, there]
+    assert torch.equal(results[0], results[2]) and torch.equal(results[1], results[3])
+
+
+@pytest.mark.parametrize("dk,dv", [(32, 32), (64, 96), (96, 32), (128, 128), (160, 64), (256, 32), (48, 32), (64, 40), (256, 256)])
 @pytest.mark.parametrize("counts", [[1, 1, 1], [3, 1, 16, 2], [2, 1]])
 def test_lightning_scan_forms(dk, dv, counts):
     """The scan with the state in registers (dk and dv in steps of 32) and the general one: single tokens, where the search for
