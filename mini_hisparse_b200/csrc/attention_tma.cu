@@ -23,7 +23,8 @@ MHB_EXPORT const char* mhb_last_error() { return error_buffer(); }
 
 namespace {
 constexpr int KT = 64;
-constexpr int CWARPS = 4;                    // compute warps that share a tile's keys
+constexpr int CWARPS = 4;                    // compute warps
+constexpr int THREADS = (CWARPS + 1) * 32;   // + the TMA warp
 constexpr int ITEM_INTS = 8;
 constexpr int MAX_MERGE_SPLITS = 64;
 
@@ -67,26 +68,16 @@ __device__ __forceinline__ float gate_of(const AttnArgs& a, int t, int col) {
     return 1.f / (1.f + expf(-sum_parts(a.gate + idx, a.gate_nsplit, a.gate_split_stride)));
 }
 
-// GROUPS: how many tiles are worked on at once, each by four warps of its own.  One, and two CTAs an SM, where a launch has
-// CTAs enough; three or four (what the registers leave for rows 128 and 64 wide) where it has no more CTAs than SMs, as in
-// decoding with a few requests: a tile is a chain of shared-memory reads, products and exponentials that four warps cannot
-// fill an SM with, and a CTA alone on its SM walked its tiles one after the other (14 us for 32 CTAs of 5 tiles, 22 us for
-// 8 CTAs of 6).
-template <int D, int ROWS, int GROUPS>
+template <int D, int ROWS>
 struct Layout {
-    static constexpr int WARPS = CWARPS * GROUPS, THREADS = (WARPS + 1) * 32;      // + the TMA warp
     static constexpr int HALVES = D / 64;
-    // A stage belongs to one group (STAGES is a multiple of GROUPS): a group that waits for a stage's next tile has then seen
-    // the one before.  Were the one before another group's, still on its way, the wait for the next phase's parity would
-    // take the phase before that for it and let the group through to a stage that is not there yet.
-    static constexpr int STAGES = GROUPS > 1 ? 2 * GROUPS : ROWS == 16 ? 3 : 2;
-    static_assert(STAGES % GROUPS == 0, "see above");
+    static constexpr int STAGES = ROWS == 16 ? 3 : 2;
     static constexpr int Q_BYTES = ROWS * D * 2;            // [HALVES][ROWS][128 B], swizzled
     static constexpr int KV_BYTES = KT * D * 2;             // K or V of one stage: [HALVES][64][128 B]
     static constexpr int STAGE_BYTES = 2 * KV_BYTES;
     static constexpr int BAR_OFFSET = Q_BYTES + STAGES * STAGE_BYTES;
     static constexpr int LOOP_BYTES = BAR_OFFSET + 2 * STAGES * 8;
-    static constexpr int MERGE_BYTES = ROWS == 16 ? WARPS * 16 * (D + 2) * 4 : 0;
+    static constexpr int MERGE_BYTES = ROWS == 16 ? CWARPS * 16 * (D + 2) * 4 : 0;
     static constexpr int TOTAL = (LOOP_BYTES > MERGE_BYTES ? LOOP_BYTES : MERGE_BYTES) + 1024;
 };
 
@@ -95,19 +86,16 @@ struct Layout {
 __device__ __forceinline__ uint32_t swz(uint32_t base, int rows_per_half, int r, int e) {
     return base + (e >> 6) * rows_per_half * 128 + r * 128 + ((((e & 63) >> 3) ^ (r & 7)) << 4);
 }
-template <int THREADS>
-__device__ __forceinline__ void compute_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }
+__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CWARPS * 32) : "memory"); }
 
 // EXT: the options.  The sink starts ONE thread's running (max, sum) of a row at (sink / scale, 1), in the
 // unsplit item or in split 0 only; the softmax's weights enter the value product as two bfloat16 numbers (the
 // weight and what rounding it lost: 16 bits instead of 8); the output is multiplied by sigmoid(gate).
-template <int D, int ROWS, bool EXT, int GROUPS>
-__global__ void __launch_bounds__((CWARPS * GROUPS + 1) * 32, GROUPS == 1 ? 2 : 1)
+template <int D, int ROWS, bool EXT>
+__global__ void __launch_bounds__(THREADS, 2)
 attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs a) {
-    static_assert(GROUPS == 1 || ROWS == 16, "tiles in parallel share their rows");
-    using L = Layout<D, ROWS, GROUPS>;
-    constexpr int STAGES = L::STAGES, WARPS = L::WARPS;
-    auto compute_sync = [] { compute_barrier<WARPS * 32>(); };
+    using L = Layout<D, ROWS>;
+    constexpr int STAGES = L::STAGES;
     constexpr int KSTEPS = D / 16;
     constexpr int DTILES = D / 8;
     constexpr bool SPLIT_KEYS = ROWS == 16;
@@ -147,7 +135,7 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
     }
     __syncthreads();
 
-    if (warp == WARPS) {
+    if (warp == CWARPS) {
         // ---- TMA warp: one lane per page of the tile ----------------------------------------------
         const int pages_per_tile = KT / a.P;
         bool ok = true, waited = false;
@@ -202,7 +190,7 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
     // ---- compute warps ---------------------------------------------------------------------------------
     if (tid < ROWS) row_pos[tid] = tid < nrows ? a.positions[tok0 + tid / nheads] : -1;
     pdl_wait();         // the queries come from the kernel before this one
-    for (int c = tid; c < ROWS * (D / 8); c += WARPS * 32) {
+    for (int c = tid; c < ROWS * (D / 8); c += CWARPS * 32) {
         const int r = c / (D / 8), ch = c % (D / 8);
         const bool live = r < nrows;
         const int t = tok0 + (live ? r / nheads : 0), h = kvh * groups + head0 + (live ? r % nheads : 0);
@@ -247,14 +235,14 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
     const float scale_log2 = a.scale * 1.4426950408889634f;
     bool ok = true;
 
-    for (int itile = GROUPS > 1 ? warp / CWARPS : 0; itile < ntiles; itile += GROUPS) {
+    for (int itile = 0; itile < ntiles; ++itile) {
         const int stage = itile % STAGES;
         ok = mbar_wait(full_bar(stage), (itile / STAGES) & 1);
         if (!ok) break;
         const uint32_t k_s = kv_s + stage * L::STAGE_BYTES;
         const uint32_t v_s = k_s + L::KV_BYTES;
         const int t0 = tile_begin + itile * KT;
-        const int key0 = SPLIT_KEYS ? (warp % CWARPS) * 16 : 0;
+        const int key0 = SPLIT_KEYS ? warp * 16 : 0;
 
         float s[NT][4];
 #pragma unroll
@@ -377,14 +365,14 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
             if ((lane & 3) == 0) { dst[D] = m_run[h]; dst[D + 1] = l_run[h]; }
         }
         compute_sync();
-        for (int idx = tid; idx < nrows * D; idx += WARPS * 32) {
+        for (int idx = tid; idx < nrows * D; idx += CWARPS * 32) {
             const int row = idx / D, e = idx - row * D;
             float M = -INFINITY;
 #pragma unroll
-            for (int w = 0; w < WARPS; ++w) M = fmaxf(M, mg[(w * 16 + row) * MS + D]);
+            for (int w = 0; w < CWARPS; ++w) M = fmaxf(M, mg[(w * 16 + row) * MS + D]);
             float acc = 0.f, lsum = 0.f;
 #pragma unroll
-            for (int w = 0; w < WARPS; ++w) {
+            for (int w = 0; w < CWARPS; ++w) {
                 const float mw = mg[(w * 16 + row) * MS + D];
                 const float wgt = mw == -INFINITY ? 0.f : exp2f((mw - M) * scale_log2);
                 acc += wgt * mg[(w * 16 + row) * MS + e];
@@ -433,7 +421,7 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
                 float2 (*ml_s)[MAX_MERGE_SPLITS] = (float2 (*)[MAX_MERGE_SPLITS])(smem + 16 * MAX_MERGE_SPLITS * 4);
                 float* inv_s = (float*)(smem + 16 * MAX_MERGE_SPLITS * 12);
                 const int ns = min(a.tok_nsplit[tok0], MAX_MERGE_SPLITS);
-                for (int idx = tid; idx < nrows * ns; idx += WARPS * 32) {     // all (maximum, sum) pairs at once
+                for (int idx = tid; idx < nrows * ns; idx += CWARPS * 32) {     // all (maximum, sum) pairs at once
                     const int row = idx / ns, sp = idx - row * ns;
                     const int t = tok0 + row / nheads, hq = kvh * groups + head0 + row % nheads;
                     ml_s[row][sp] = __ldcg((const float2*)(a.part_ml + (((size_t)a.tok_part_row[t] + sp) * a.nq + hq) * 2));
@@ -453,7 +441,7 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
                 }
                 compute_sync();
                 // four elements per thread and step, eight splits in flight; summed in the splits' order
-                for (int idx = tid; idx < nrows * (D / 4); idx += WARPS * 32) {
+                for (int idx = tid; idx < nrows * (D / 4); idx += CWARPS * 32) {
                     const int row = idx / (D / 4), e = (idx - row * (D / 4)) * 4;
                     const int t = tok0 + row / nheads, hq = kvh * groups + head0 + row % nheads;
                     const float* src = a.part_acc + ((size_t)a.tok_part_row[t] * a.nq + hq) * D + e;
@@ -523,10 +511,10 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
     }
 }
 
-template <int D, int ROWS, bool EXT, int GROUPS>
-int launch_groups(const CUtensorMap& map, const AttnArgs& a, int launch_items, cudaStream_t stream) {
-    auto kern = attention_tma_kernel<D, ROWS, EXT, GROUPS>;
-    constexpr int smem = Layout<D, ROWS, GROUPS>::TOTAL;
+template <int D, int ROWS, bool EXT>
+int launch(const CUtensorMap& map, const AttnArgs& a, int launch_items, cudaStream_t stream) {
+    auto kern = attention_tma_kernel<D, ROWS, EXT>;
+    constexpr int smem = Layout<D, ROWS>::TOTAL;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -535,20 +523,8 @@ int launch_groups(const CUtensorMap& map, const AttnArgs& a, int launch_items, c
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
         configured = true;
     }
-    launch_kernel(kern, dim3(launch_items, a.nkv), dim3(Layout<D, ROWS, GROUPS>::THREADS), smem, stream, map, a);
+    launch_kernel(kern, dim3(launch_items, a.nkv), dim3(THREADS), smem, stream, map, a);
     return check_launch("attention_tma");
-}
-template <int D, int ROWS, bool EXT>
-int launch(const CUtensorMap& map, const AttnArgs& a, int launch_items, cudaStream_t stream) {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-    }
-    if ((long long)launch_items * a.nkv <= sms) return launch_groups<D, ROWS, EXT, D == 128 ? 3 : 4>(map, a, launch_items, stream);
-    return launch_groups<D, ROWS, EXT, 1>(map, a, launch_items, stream);
 }
 }  // namespace
 

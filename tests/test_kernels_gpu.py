@@ -650,12 +650,92 @@ def test_attention_tensor_core_splits_window_and_far_key(kernel):
 @pytest.mark.parametrize("d,P_", [(64, 16), (128, 32), (128, 4)])
 @pytest.mark.parametrize("hist", [0, 63, 64, 130, 191, 192, 300, 700, 1500])
 def test_attention_tma_few_ctas(d, P_, hist):
-    """A launch with no more CTAs than SMs works on several key tiles at once: from less than one tile to several rounds of
-    the ring of stages, unsplit and split, decode tokens and a short portion."""
+    """Few CTAs with few or many tiles each: from less than one tile to several rounds of the ring of stages, unsplit and
+    split, decode tokens and a short portion."""
     for nsplit in (1, 3):
         out, ref, plan = run_attention(6, 2, d, P_, [(hist, 1), (hist, 5)], torch.bfloat16, fixed_nsplit=nsplit, kernel="tc")
         assert len(plan.items) * 2 <= 148 and plan.n_small
         torch.testing.assert_close(out, ref, **tol(torch.bfloat16, 2))
+
+
+@pytest.mark.parametrize("d,P_", [(64, 16), (128, 32)])
+@pytest.mark.parametrize("nsplit", [1, 3])
+@pytest.mark.parametrize("ext", [False, True])
+def test_attention_tma_alone_and_in_a_busy_batch(d, P_, nsplit, ext):
+    """A launch with more CTAs than SMs (64 decode tokens and a short portion), against the oracle, and its first segments
+    launched alone: the same bits, whatever else is in the launch.  ``ext``: with a sink, a cap and a gate."""
+    from mini_hisparse_b200.parts.attention import AttentionShape, plan_attention
+
+    nq, nkv, bf = 8, 4, torch.bfloat16
+    specs = [(130, 1), (64, 1)] + [(i % 150, 1) for i in range(62)] + [(70, 5)]
+    cache, table, segments, qs, ks, vs, positions = paged_case(nq, nkv, d, P_, specs, bf)
+    T = sum(n for _, n in specs)
+    plan = plan_attention(AttentionShape(nq, nkv, None, 128), segments, T, 148, fixed_nsplit=nsplit)
+    assert not plan.n_big and plan.n_small * nkv > 148
+    q = torch.cat([qq[h:] for qq, (h, n) in zip(qs, specs)]).reshape(T, nq * d).to(DEV)
+    sink, gate = (torch.randn(*n, generator=torch.Generator().manual_seed(d)).to(DEV) for n in ((nq,), (T, nq * d)))
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(items):
+        out = torch.full((T, nq * d), float("nan"), dtype=bf, device=DEV)
+        rows = max(1, plan.part_rows)
+        part_acc, part_ml = torch.full((rows, nq, d), float("nan"), device=DEV), torch.full((rows, nq, 2), float("nan"), device=DEV)
+        counters = torch.zeros(T * nkv, dtype=torch.int32, device=DEV)
+        opts = dict(sink=sink, gate=gate, softcap=20.0) if ext else {}
+        (K().attention_tma_ext if ext else K().attention_tma)(
+            q, cache, out, part_acc, part_ml, torch.from_numpy(items).to(DEV).reshape(-1), len(items), 16, positions, table,
+            torch.from_numpy(plan.tok_part_row).to(DEV), nq=nq, nkv=nkv, d=d, page_size=P_,
+            tok_nsplit=torch.from_numpy(plan.tok_nsplit).to(DEV), counters=counters, status=status, **opts)
+        assert int(status) == 0 and int(counters.abs().sum()) == 0
+        return out
+
+    out = run(plan.items)
+    few = plan.items[plan.items[:, 0] < 2]                      # the items of the first two segments
+    assert len(few) * nkv <= 148
+    assert torch.equal(run(few)[:2], out[:2])
+    ref = []
+    for qq, kk, vv, (h, n) in zip(qs, ks, vs, specs):
+        qq, kk, vv = (y.double() for y in (qq, kk, vv))
+        kk, vv = (y.repeat_interleave(nq // nkv, 1) for y in (kk, vv))
+        z = torch.einsum("qhd,khd->hqk", qq[h:], kk) * d ** -0.5
+        z = 20.0 * torch.tanh(z / 20.0) if ext else z
+        z.masked_fill_(torch.arange(h + n) > torch.arange(h, h + n)[:, None], -math.inf)
+        if ext:
+            z = torch.cat((z, sink.cpu().double()[:, None, None].expand(-1, n, 1)), -1)
+        ref.append(torch.einsum("hqk,khd->qhd", torch.softmax(z, -1)[..., :h + n], vv).reshape(n, nq * d))
+    ref = torch.cat(ref)
+    ref = ref * torch.sigmoid(gate.cpu().double()) if ext else ref
+    torch.testing.assert_close(out.double().cpu(), ref, **tol(bf, 2))
+
+
+@pytest.mark.parametrize("ext", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 16])
+def test_attention_tma_early_keys_behind_the_append(ext, n):
+    """``fresh``: keys older than the step are read before the kernel that appends the step's own is done.  Straight behind
+    that kernel, with histories around the edges of tiles and of what counts as fresh, the result is that of a launch that
+    waits for every key."""
+    from mini_hisparse_b200.parts.attention import AttentionShape, plan_attention
+
+    nq, nkv, d, P_, bf = 8, 2, 64, 16, torch.bfloat16
+    specs = [(h, n) for h in (0, 15, 16, 63, 64, 79, 80, 200)]
+    cache, table, segments, _, _, _, positions = paged_case(nq, nkv, d, P_, specs, bf)
+    T = n * len(specs)
+    plan = plan_attention(AttentionShape(nq, nkv, None, 128), segments, T, 148, fixed_nsplit=1)
+    assert plan.n_small == len(plan.items)
+    items, status = torch.from_numpy(plan.items).to(DEV).reshape(-1), torch.zeros(1, dtype=torch.int32, device=DEV)
+    seg = torch.arange(len(specs), dtype=torch.int32, device=DEV).repeat_interleave(n)
+    qkv = rnd(T, (nq + 2 * nkv) * d, seed=3)
+    parts = torch.zeros(1, nq, d, device=DEV), torch.zeros(1, nq, 2, device=DEV)
+    tpr, tns = (torch.from_numpy(y).to(DEV) for y in (plan.tok_part_row, plan.tok_nsplit))
+    launch = K().attention_tma_ext if ext else K().attention_tma
+    results = []
+    for fresh in (0, 16) * 10:
+        pool, q, out = cache.clone(), torch.empty(T, nq * d, dtype=bf, device=DEV), torch.empty(T, nq * d, dtype=bf, device=DEV)
+        K().rope_append(qkv, None, positions, seg, table, None, q, pool, nq=nq, nkv=nkv, d=d, page_size=P_, status=status)
+        launch(q, pool, out, *parts, items, plan.n_small, 16, positions, table, tpr, nq=nq, nkv=nkv, d=d, page_size=P_, tok_nsplit=tns,
+               status=status, fresh=fresh)
+        results.append(out)
+    assert int(status) == 0 and all(torch.equal(y, results[0]) for y in results)
 
 
 @pytest.mark.parametrize("nq,nkv,d,P_,nsplit,qkv_nsplit,rdim,interleaved,window,ngroups", [
