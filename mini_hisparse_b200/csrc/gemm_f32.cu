@@ -5,25 +5,30 @@
 //    pace, so a warp keeps NR feature rows of 16-byte loads in flight, all its lanes run along K, and the activations
 //    come through L1.
 //
-//  * more: the tensor cores.  A float32 number is EXACTLY the sum of three bfloat16 numbers (8 bits each, cut from
-//    the top, so nothing rounds and nothing overflows): x = h + m + l.  Of the nine products of two such sums six are
-//    taken, l*h, h*l, m*m, m*h, h*m, h*h; the three that are left out are below 2^-24 of h*h, what one rounding of a
-//    float32 product costs.  The tensor core adds in float32 but does not round to nearest, an error that would grow
-//    with the length of the sum; so an accumulator in tensor memory only ever holds ONE block of 32 elements of K
-//    (products of small parts first), and the warps add it to sums of their own in registers, rounded to nearest.
-//    The 7B shape's products (K = 3584 and 18944, 750 tokens) come out nearer to the 64-bit result than the
-//    FFMA chain over K that they replace.  No operand is held or read in less than 32 bits outside of a
-//    CTA: the cut happens between the load and shared memory.
+//  * more: the tensor cores.  A float32 number is EXACTLY the sum of three bfloat16 numbers x = h + m + l: h is x rounded to 8
+//    bits, m what is left rounded to 8 bits, l the rest, which has 8 bits or fewer (the splitting of a number by rounding of
+//    Dekker, "A floating-point technique for extending the available precision", 1971).  |m| is at most 2^-8 and |l| at most
+//    2^-17 of |h|, both of either sign.  Operands are multiplied by 2^16 first, so that the parts of the smallest float32
+//    number are bfloat16 numbers too; finished sums by 2^-32.  Of the nine products of two such sums six are taken, l*h, h*l,
+//    m*m, m*h, h*m, h*h; the three that are left out, m*l, l*m and l*l, come to at most 1.002 x 2^-24 of h*h, what one rounding
+//    of a float32 product may cost, and have either sign.  The tensor core adds in float32 but does not round to nearest, an
+//    error that would grow with the length of the sum; so an accumulator in tensor memory only ever holds ONE block of 32
+//    elements of K (products of small parts first), and the warps add it to sums of their own in registers, rounded to nearest.
+//    No operand is held or read in less than 32 bits outside of a CTA but as all three of its parts.
 //
 // Measured (us; in brackets the 64 x 64 FFMA tiles that served before), tokens x K x features: 4 x 3584 x 37888 102 [622],
-// 8 x 18944 x 3584 81 [1433], 16 x 3584 x 37888 149 [740], 100 x 3584 x 37888 225 [1346], 750 x 3584 x 37888 1162 [8238] =
-// 175 TFLOP/s, 750 x 18944 x 3584 574 [4645].  Relative errors against 64 bits at those: 2.2e-7 to 4.5e-7 [1.1e-6 to 2.5e-6].
+// 8 x 18944 x 3584 82 [1435], 16 x 3584 x 3584 40 [210], 100 x 3584 x 37888 219 [1343], 750 x 3584 x 37888 1059 [8764] =
+// 192 TFLOP/s, 750 x 18944 x 3584 564 [4936].  Errors against 64 bits there (2-norm, relative): 1.0e-7 to 2.3e-7 [1.1e-6 to
+// 2.5e-6].  At K = 64, 256 and 3584 and random numbers, in units of 2^-24: 1.07, 1.34, 3.4 [2.4, 4.8, 18], of one sign 1.02, 1.13,
+// 2.8 [2.0, 3.9, 15].  Parts cut from the top instead of rounded leave out up to 2^-21 of a product, always towards zero
+// (1.8, 2.0, 3.7 and 1.7, 1.7, 3.1 there), and took 1168 us where 1059 stands.
 //
 // What bounds the second: six tensor-core products for one, i.e. 2.25 / 6 = 0.37 PFLOP/s at best, and before that shared
 // memory: a 128 x 128 x 16 MMA reads 8 KB in the 64 cycles it takes, and 192 bytes a row are written per block.
 //
-// A result that is NaN is computed once more by one thread as a plain FFMA chain: an infinite operand is not the
-// sum of its three parts (inf - inf), and the chain says what the product of infinities is.
+// A result that is not finite is computed once more by one thread as a plain FFMA chain: an infinite operand is not the
+// sum of its three parts (inf - inf), an operand from 2^112 or a sum from 2^96 on leaves the range when it is scaled, and the
+// chain says what the result is.
 #include "common.cuh"
 #include "tc_helpers.cuh"
 #include "tma_helpers.cuh"
@@ -141,20 +146,24 @@ int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, l
 }
 
 // ---- more tokens: three bfloat16 parts on the tensor cores ----------------------------------------------------------------
+constexpr float CUT_SCALE = 65536.f, SUM_SCALE = 1.f / (65536.f * 65536.f);
+
+__device__ __forceinline__ uint32_t round_pair(float a, float b) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+    return *(const uint32_t*)&p;
+}
 // 8 numbers' parts as 16 bytes each
 __device__ __forceinline__ void cut(const float4& p, const float4& q, uint4& h, uint4& m, uint4& l) {
     const float x[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
     uint32_t hh[4], mm[4], ll[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const float a = x[2 * i], b = x[2 * i + 1];
-        const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-        hh[i] = __byte_perm(ua, ub, 0x7632);
-        const float a1 = a - __uint_as_float(ua & 0xffff0000u), b1 = b - __uint_as_float(ub & 0xffff0000u);
-        const uint32_t va = __float_as_uint(a1), vb = __float_as_uint(b1);
-        mm[i] = __byte_perm(va, vb, 0x7632);
-        const float a2 = a1 - __uint_as_float(va & 0xffff0000u), b2 = b1 - __uint_as_float(vb & 0xffff0000u);
-        ll[i] = __byte_perm(__float_as_uint(a2), __float_as_uint(b2), 0x7632);
+        float a = x[2 * i] * CUT_SCALE, b = x[2 * i + 1] * CUT_SCALE;
+        hh[i] = round_pair(a, b);
+        a -= __uint_as_float(hh[i] << 16);
+        b -= __uint_as_float(hh[i] & 0xffff0000u);
+        mm[i] = round_pair(a, b);
+        ll[i] = round_pair(a - __uint_as_float(mm[i] << 16), b - __uint_as_float(mm[i] & 0xffff0000u));
     }
     h = make_uint4(hh[0], hh[1], hh[2], hh[3]);
     m = make_uint4(mm[0], mm[1], mm[2], mm[3]);
@@ -362,8 +371,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map, const float* __re
             for (int c = 0; c < COLS; ++c) {
                 const int m = m0 + half * COLS + c;
                 if (m >= M) continue;
-                float v = acc[c];
-                if (v != v) {                    // see the top: an infinite operand, or a true NaN
+                float v = acc[c] * SUM_SCALE;
+                if (!isfinite(v)) {              // see the top
                     const int k1 = min(K, last * T_BK);
                     v = 0.f;
                     for (int k = first * T_BK; k < k1; ++k) v = fmaf(A[(size_t)m * lda + k], W[(size_t)n * ldw + k], v);

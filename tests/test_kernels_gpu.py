@@ -155,6 +155,47 @@ def test_gemm_is_true_float32():
     assert abs(float(out[0, 0]) - exact) < 1e-4
 
 
+def float32_operands(kind, M, N, K_):
+    """Operands of a float32 product: random ones, and ones that tell a kernel of fewer bits from one of 24."""
+    a, w = rnd(M, K_, seed=1), rnd(N, K_, seed=2)
+    if kind == "positive":
+        a, w = a.abs(), w.abs()
+    if kind == "one to two":
+        a, w = 1 + a.abs().clamp(max=1), 1 + w.abs().clamp(max=1)
+    if kind == "one number":                   # bits at the edge of every 8: cut from the top, parts 1, 2^-7 - 2^-15 and 2^-15 - 2^-23
+        a, w = torch.full_like(a, 1 + 2.0 ** -7 - 2.0 ** -23), torch.full_like(w, 1 + 2.0 ** -7 - 2.0 ** -23)
+    if kind == "tiny tokens":                  # their last bits are subnormal bfloat16 numbers, or below these
+        a = a * 2.0 ** -118
+    if kind == "tiny weights":
+        w = w * 2.0 ** -118
+    if kind == "huge":                         # parts and sums out of a scaled range
+        a, w = a * 2.0 ** 113, w * 2.0 ** -20
+    return a, w
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 130])
+@pytest.mark.parametrize("K_", [8, 16, 32, 40, 64, 104, 256, 3584])
+@pytest.mark.parametrize("kind", ["signed", "positive", "one to two", "one number", "tiny tokens", "tiny weights", "huge"])
+def test_float32_path_is_true_float32(M, K_, kind):
+    """What the float32 path's products launch, on both sides of 8 tokens and of the shortest sum for the tensor cores, is no
+    further from 64 bits than the chain of FFMA over K, in the largest error of an element and in the 2-norm."""
+    from mini_hisparse_b200.kernels.runtime import Float32Runtime
+    from mini_hisparse_b200.parts.base import Workspace
+
+    N = 4096
+    a, w = float32_operands(kind, M, N, K_)
+    rt = Float32Runtime(DEV)
+    rt.status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    p = rt.linear(a, w, Workspace(rt.device), "out")
+    got = p.tensor.double().view(-1, M, N).sum(0)
+    chain = torch.empty(M, N, device=DEV)
+    K().gemm_simt(a, w, chain)
+    ref = a.double() @ w.double().T
+    assert int(rt.status) == 0 and got.isfinite().all()
+    got, chain = (got - ref).abs(), (chain.double() - ref).abs()
+    assert got.max() <= chain.max() and got.norm() <= chain.norm()
+
+
 @pytest.mark.parametrize("M,N,K_,bn,nsplit", [
     (1, 5, 8, 0, 1), (2, 2400, 136, 0, 1), (3, 97, 1000, 0, 1), (4, 2369, 2056, 0, 1), (8, 130, 4104, 0, 1), (7, 2400, 520, 0, 1),
     (9, 130, 8, 64, 1), (64, 128, 32, 64, 1), (65, 127, 40, 64, 2), (33, 300, 1000, 64, 5), (128, 129, 96, 128, 1),
@@ -162,10 +203,12 @@ def test_gemm_is_true_float32():
 ])
 @pytest.mark.parametrize("kind", ["signed", "positive", "special"])
 def test_gemm_f32(M, N, K_, bn, nsplit, kind):
-    """The float32 products at the edges of their tiles.  Bound, element by element, in units of S = sum |a||w|: the kernel
-    adds at most 14 tensor-core steps of 2^-23 S inside a block of 32, one rounding of 2^-24 per block, three parts' products
-    below 2^-24 that are left out; the CUDA-core kernel at most K / 128 + 9 roundings a lane and the sums across lanes and
-    splits.  "special": infinities and NaN come out where a chain of multiplications and additions puts them."""
+    """The float32 products at the edges of their tiles.  Bound, element by element, in units of 2^-24 S with S = sum |a||w|.
+    Tensor cores: 1 for the parts' products that are left out; 2 for each of the two steps of a block of 32 that add products of
+    first parts, of which a truncating sum of the block loses less than its last bit (2^-23), and less than 1 for the ten steps
+    before them, which add at most 2^-7 as much; 1 per block for its rounded addition; 1 per split.  CUDA cores: 1 for every
+    multiplication and addition of a lane (K / 32 of them at most), 5 across lanes, 8 across warps.  "special": infinities
+    and NaN come out where a chain of multiplications and additions puts them."""
     a, w = rnd(M, K_, seed=1), rnd(N, K_, seed=2)
     if kind == "positive":
         a, w = a.abs(), w.abs()
@@ -173,7 +216,7 @@ def test_gemm_f32(M, N, K_, bn, nsplit, kind):
         a[M // 2, K_ // 2] = math.inf
         a[0, 0] = math.nan
         w[N - 1, K_ // 2] = -math.inf
-        a[M - 1, K_ - 1] = 3.4e38          # its first 8 bits round to infinity
+        a[M - 1, K_ - 1] = 3.4e38          # rounded to 8 bits it is infinite
         w[:, K_ - 1] = 2.0 ** -20          # ... and none of its products overflows, which 64 bits would not show
     out = torch.full((nsplit, M, N), math.nan, device=DEV)
     status = torch.zeros(1, dtype=torch.int32, device=DEV)
@@ -184,7 +227,7 @@ def test_gemm_f32(M, N, K_, bn, nsplit, kind):
     if kind == "special":
         ref = ref.float().double()
         assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got[got.isinf()], ref[ref.isinf()])
-    room = (14 * 2.0 ** -23 + (K_ / 32 + 20) * 2.0 ** -24) * (a.abs().double() @ w.abs().double().T)
+    room = (6 + -(-K_ // 32) + nsplit if bn else -(-K_ // 32) + 4 + 5 + 8) * 2.0 ** -24 * (a.abs().double() @ w.abs().double().T)
     fine = ref.isfinite()
     assert ((got - ref).abs() <= room)[fine].all()
 
