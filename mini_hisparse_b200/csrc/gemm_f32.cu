@@ -28,7 +28,7 @@
 //
 // A result that is not finite is computed once more by one thread as a plain FFMA chain: an infinite operand is not the
 // sum of its three parts (inf - inf), an operand from 2^112 or a sum from 2^96 on leaves the range when it is scaled, and the
-// chain says what the result is.
+// chain says what the result is.  The chain ends at the first NaN.
 #include "common.cuh"
 #include "tc_helpers.cuh"
 #include "tma_helpers.cuh"
@@ -375,7 +375,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map, const float* __re
                 if (!isfinite(v)) {              // see the top
                     const int k1 = min(K, last * T_BK);
                     v = 0.f;
-                    for (int k = first * T_BK; k < k1; ++k) v = fmaf(A[(size_t)m * lda + k], W[(size_t)n * ldw + k], v);
+                    for (int k = first * T_BK; k < k1 && v == v; ++k) v = fmaf(A[(size_t)m * lda + k], W[(size_t)n * ldw + k], v);
                 }
                 Cz[(size_t)m * ldc] = v;
             }
