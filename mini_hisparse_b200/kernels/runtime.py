@@ -10,6 +10,8 @@ multiple of 8) go to the CUDA-core product, which takes any shape.
 """
 from __future__ import annotations
 
+from functools import lru_cache
+
 import torch
 
 from ..parts.base import Product, Runtime, Workspace
@@ -17,6 +19,35 @@ from . import api as K
 
 BK = 64            # K elements per pipeline stage of the tensor-core kernel
 MIN_KB_PER_SPLIT = 4
+
+
+F32_BLOCK = 32          # elements of K in a block of the float32 tensor-core product
+# a CTA's time per block in us, measured at 7B-shape sizes, by its tokens: with tiles of 64 two CTAs share an SM
+F32_BLOCK_US = {64: 1.3, 128: 1.0, 192: 1.3}
+
+
+@lru_cache(maxsize=1024)
+def _f32_tile(sm_count: int, M: int, N: int, Kd: int, allow_split: bool) -> tuple[int, int]:
+    """(tokens a CTA, K splits) of the float32 product with more than 8 tokens: the pair whose rounds of CTAs, each as long
+    as its blocks and 6 blocks' time for its start and end, are done first, counting 8 bytes at 5 TB/s for every number
+    of a further partial matrix.  Measured (us, with a block 9 % longer than now): 750 x 3584 x 4608 147 with (192, 1)
+    against 209 (128, 1) and 210 (64, 2); 64 x 18944 x 3584 87 with (64, 10) against 573 (64, 1); 400 x 3584 x 4608 110 with
+    (128, 1), 136 (192, 1)."""
+    blocks = -(-Kd // F32_BLOCK)
+    best, best_us = (64, 1), None
+    for bn, us in F32_BLOCK_US.items():
+        if bn > 64 and M <= bn - 64:
+            break
+        tiles = -(-M // bn) * -(-N // 128)
+        slots = sm_count * (2 if bn == 64 else 1)
+        for n in range(1, (min(12, max(1, blocks // 8)) if allow_split else 1) + 1):
+            per = -(-blocks // n)
+            if (n - 1) * per >= blocks:
+                continue
+            t = -(-tiles * n // slots) * (per + 6) * us + (n - 1) * M * N * 8 / 5e6
+            if best_us is None or t < best_us:
+                best, best_us = (bn, n), t
+    return best
 
 
 class Float32Runtime(Runtime):
@@ -28,31 +59,6 @@ class Float32Runtime(Runtime):
     def kernel_modules(self):
         return ("elementwise", "gemm_simt", "gemm_f32", "sampling")
 
-    F32_BLOCK = 32          # elements of K in a block of the tensor-core product
-    # a CTA's time per block in us, measured at 7B-shape sizes, by its tokens: with tiles of 64 two CTAs share an SM
-    F32_BLOCK_US = {64: 1.3, 128: 1.0, 192: 1.3}
-
-    def _tile(self, M: int, N: int, Kd: int, allow_split: bool) -> tuple[int, int]:
-        """(tokens a CTA, K splits) of the product with more than 8 tokens: the pair whose rounds of CTAs, each as long as
-        its blocks and 6 blocks' time for its start and end, are done first, counting 8 bytes at 5 TB/s for every number
-        of a further partial matrix.  Measured (us, with a block 9 % longer than now): 750 x 3584 x 4608 147 with (192, 1)
-        against 209 (128, 1) and 210 (64, 2); 64 x 18944 x 3584 87 with (64, 10) against 573 (64, 1); 400 x 3584 x 4608 110 with (128, 1), 136 (192, 1)."""
-        blocks = -(-Kd // self.F32_BLOCK)
-        best, best_us = (64, 1), None
-        for bn, us in self.F32_BLOCK_US.items():
-            if bn > 64 and M <= bn - 64:
-                break
-            tiles = -(-M // bn) * -(-N // 128)
-            slots = self.sm_count * (2 if bn == 64 else 1)
-            for n in range(1, (min(12, max(1, blocks // 8)) if allow_split else 1) + 1):
-                per = -(-blocks // n)
-                if (n - 1) * per >= blocks:
-                    continue
-                t = -(-tiles * n // slots) * (per + 6) * us + (n - 1) * M * N * 8 / 5e6
-                if best_us is None or t < best_us:
-                    best, best_us = (bn, n), t
-        return best
-
     def linear(self, x, weight, ws: Workspace, name: str, out_dtype=None, bias=None, allow_split: bool = True) -> Product:
         """K in steps of 8 and aligned rows: the kernels of gemm_f32 (CUDA cores up to 8 tokens, three bfloat16 parts on
         the tensor cores beyond); any other shape, and a product with a bias: the general CUDA-core kernel.  It also takes
@@ -60,14 +66,14 @@ class Float32Runtime(Runtime):
         2-norm of the errors of numbers of one sign (0.81 against 0.75 x 2^-24), can be a little above the plain chain's;
         from 40 numbers on both kernels are nearer to the 64-bit result in either (at 64: 1.02 against 1.96)."""
         M, N, Kd = x.shape[0], weight.shape[0], x.shape[1]
-        if (bias is not None or (out_dtype or self.dtype) != torch.float32 or Kd <= self.F32_BLOCK
+        if (bias is not None or (out_dtype or self.dtype) != torch.float32 or Kd <= F32_BLOCK
                 or not K.gemm_f32_takes(x, weight)):
             return super().linear(x, weight, ws, name, out_dtype, bias, allow_split)
         if M <= 8:
             out = ws.get(name, (M, N), torch.float32)
             K.gemm_f32(x, weight, out)
             return Product(out)
-        bn, nsplit = self._tile(M, N, Kd, allow_split)
+        bn, nsplit = _f32_tile(self.sm_count, M, N, Kd, allow_split)
         parts = ws.get(name + "_parts", (3, M, Kd), torch.bfloat16)
         out = ws.get(name, (nsplit, M, N) if nsplit > 1 else (M, N), torch.float32)
         K.gemm_f32(x, weight, out, bn=bn, nsplit=nsplit, split_stride=out.stride(0) if nsplit > 1 else 0, parts=parts,
