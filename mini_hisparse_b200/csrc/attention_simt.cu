@@ -239,7 +239,6 @@ attention_simt_kernel(const AttnArgs a) {
         page = look_up(1);
     }
 
-    // l: this lane's share of the sum; the lanes' shares are added at the end
     float m[ROWS_PER_WARP], l[ROWS_PER_WARP], acc[ROWS_PER_WARP][DPL], slope[ROWS_PER_WARP];
 #pragma unroll
     for (int rs = 0; rs < ROWS_PER_WARP; ++rs) {
@@ -251,7 +250,7 @@ attention_simt_kernel(const AttnArgs a) {
         slope[rs] = a.slopes && r < nrows ? a.slopes[(kvh * groups + head0 + r % nheads) * kparts + map] : 0.f;
         if (a.sink && split <= 0 && r < nrows) {      // a single time per token: here or in split 0
             m[rs] = a.sink[(kvh * groups + head0 + r % nheads) * kparts + map];
-            l[rs] = lane == 0 ? 1.f : 0.f;
+            l[rs] = 1.f;
         }
     }
     // rows of this warp: rs * WARPS + warp < nrows
@@ -327,7 +326,7 @@ attention_simt_kernel(const AttnArgs a) {
                 p[rs] = valid ? expf(x - m_new) : 0.f;
                 alpha = m[rs] > -INFINITY ? expf(m[rs] - m_new) : 0.f;
             }
-            l[rs] = l[rs] * alpha + p[rs];
+            l[rs] = l[rs] * alpha + warp_sum(p[rs]);
             m[rs] = m_new;
 #pragma unroll
             for (int i = 0; i < DPL; ++i) acc[rs][i] *= alpha;
@@ -352,9 +351,6 @@ attention_simt_kernel(const AttnArgs a) {
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int rs = 0; rs < ROWS_PER_WARP; ++rs) l[rs] = warp_sum(l[rs]);
-
 #pragma unroll
     for (int rs = 0; rs < ROWS_PER_WARP; ++rs) {
         const int r = rs * WARPS + warp;

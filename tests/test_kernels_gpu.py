@@ -1,6 +1,7 @@
 """Each CUDA kernel alone against a plain PyTorch float32 reference of the same operation, at
 sizes other than the engine's test models (widths and vocabularies that are no power of two,
 head sizes in steps of 16, odd group counts)."""
+import hashlib
 import math
 
 import pytest
@@ -623,6 +624,18 @@ def test_attention_simt_staging(nq, nkv, d, P_, dtype):
     torch.testing.assert_close(out, ref, **tol(dtype, 4))
     out, ref, _ = run_attention(nq, nkv, d, P_, specs, dtype, window=33, fixed_nsplit=3)
     torch.testing.assert_close(out, ref, **tol(dtype, 4))
+
+
+@pytest.mark.parametrize("nq,nkv,d,P_,dtype,window,digest", [
+    (4, 2, 16, 16, torch.float32, None, "ff3db8955cc0fb31"), (3, 1, 32, 32, torch.float32, None, "eacb959b9b6a0da5"),
+    (4, 2, 23, 3, torch.float32, None, "c8026b0b6d11cead"), (6, 2, 24, 16, torch.bfloat16, 33, "0e40358704170298"),
+    (6, 1, 256, 16, torch.bfloat16, None, "6dc225df5a5a1fd7")])
+def test_attention_simt_bits(nq, nkv, d, P_, dtype, window, digest):
+    """The bits of the CUDA-core kernel's outputs: a digest of what the kernel gave that staged one tile at a time, element by
+    element.  However tiles are staged, scores, maxima and sums are taken in that kernel's order (a tile's weights are added
+    across the warp before they meet the running sum)."""
+    out, _, plan = run_attention(nq, nkv, d, P_, [(0, 1), (30, 1), (31, 1), (63, 1), (200, 17), (250, 1)], dtype, window=window)
+    assert plan.part_rows == 0 and hashlib.sha256(out.numpy().tobytes()).hexdigest()[:16] == digest
 
 
 @pytest.mark.parametrize("nq,nkv,d,P_", [(4, 2, 32, 16), (3, 1, 32, 32), (28, 4, 128, 16), (20, 1, 96, 8),
