@@ -119,7 +119,7 @@ norm_mix_vec_kernel(float* __restrict__ x, const DT* __restrict__ delta, int nsp
         if (i >= nvec) continue;
         v[c] = s[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (alpha != 0.f || keep != 0.f) v[c] = vec4(xr + 4 * i);
-        if (delta) s[c] = sum_parts4<Q * M == 1 ? 8 : 2>(delta + r * H + 4 * i, nsplit, split_stride);
+        if (delta) s[c] = sum_parts4<Q == 1 && M <= 2 ? 8 : 2>(delta + r * H + 4 * i, nsplit, split_stride);
     }
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
@@ -269,11 +269,11 @@ gated_rmsnorm_vec_kernel(const float* __restrict__ o, const float* __restrict__ 
         const int i = threadIdx.x + c * blockDim.x;
         if (i >= nvec) continue;
         v[c] = vec4(row + 4 * i);
-        if (gate) g[c] = sum_parts4<VC == 1 ? 8 : 2>(gate + r * gate_ld + 4 * i, gate_nsplit, gate_split_stride);
+        if (gate) g[c] = sum_parts4<VC <= 2 ? 8 : 2>(gate + r * gate_ld + 4 * i, gate_nsplit, gate_split_stride);
     }
     for (int u = warp; u < sums / 32; u += nwarps) {
         float ss = 0.f;
-#pragma unroll 4
+#pragma unroll 8
         for (int i = u * 32 + lane; i < N; i += sums) { const float e = row[i]; ss = fmaf(e, e, ss); }
         ss = warp_sum(ss);
         if (lane == 0) scratch[u] = ss;
