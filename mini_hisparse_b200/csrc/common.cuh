@@ -140,8 +140,16 @@ __device__ __forceinline__ float4 sum_parts4(const T* p, int n, size_t stride) {
 // begins with pdl_launch_dependents(); pdl_wait().  The first lets the NEXT kernel's CTAs start as
 // soon as SM resources allow (its start-up, and in the matrix products the first weight tiles,
 // overlap this kernel's tail); the second holds this kernel until its predecessor has completed
-// and its writes are visible.  Before pdl_wait() a kernel touches constant data only (weights,
-// tensor maps).  Since every kernel waits for its predecessor, completion stays in stream order.
+// and its writes are visible.  Since every kernel waits for its predecessor, completion stays in
+// stream order; but what a kernel does before pdl_wait() may run beside ANY earlier kernel that was
+// launched like this, not only the one before it.  So before pdl_wait() a kernel reads only what none
+// of them writes:
+//   * weights and tensor maps;
+//   * the step's index arrays (positions, segments, slots, block tables, work items): the host copies
+//     them before the step's first kernel, and a copy is a full dependency.  A kernel that makes one of
+//     them inside a step may only be followed by readers behind their pdl_wait();
+//   * cached keys and values older than the step, as far as the attention kernels' `fresh` says.
+// Anything else may at most be prefetched into the L2.
 // MHB_PDL=0 in the environment switches the attribute off (then both calls are no-ops).
 namespace mhb {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

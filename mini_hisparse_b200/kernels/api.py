@@ -185,7 +185,8 @@ def qknorm_rope_append(qkv, q_weight, k_weight, eps, positions, tok_seg, block_t
     the weights may be None, and ``q_temp`` = (coef, every) multiplies q by
     1 + coef ln(floor((position + 1) / every) + 1).  ``v_scale``: a factor on the stored values.  ``bias`` float32
     [nq dk + nkv dk] is added to q and k first; with ``v_from_k`` a row is [q | k | ...] and the values are the keys as
-    projected (with the bias, before norm and rotation)."""
+    projected (with the bias, before norm and rotation).  ``positions``, ``tok_seg`` and ``block_table`` must not be written
+    by kernels of the same step: they are read while the kernels before this one still run."""
     lib = build.load("postnorm")
     T = q_out.shape[0]
     if qkv.dtype != torch.float32 or qkv.stride(-1) != 1:
@@ -219,7 +220,8 @@ def lightning_scan(proj, q0, k0, v0, decay, state, out, tok_seg, seg_slot, posit
                    split_stride=0, writable=True, max_tokens=0):
     """Linear attention with decay, token by token, for every segment of at most ``max_tokens`` tokens
     (0: all).  ``proj`` float32 [.., T, ld] holds silu's inputs: q at column q0, k at k0, v at v0, heads
-    side by side; ``state`` [slots, heads, dk, dv]; ``out`` float32 [T, heads * dv]."""
+    side by side; ``state`` [slots, heads, dk, dv]; ``out`` float32 [T, heads * dv].  ``tok_seg``, ``seg_slot``, ``positions``
+    and ``decay`` must not be written by kernels of the same step: they are read while the kernels before this one run."""
     lib = build.load("lightning")
     T, S = out.shape[0], seg_slot.shape[0]
     head = _lightning_head(proj, q0, k0, v0, decay, state, out, (tok_seg, seg_slot, positions), heads, dk, dv,
