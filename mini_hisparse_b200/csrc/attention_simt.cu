@@ -94,14 +94,6 @@ __device__ __forceinline__ float gate_of(const AttnArgs& a, int t, int col) {
     return 1.f / (1.f + expf(-g));
 }
 
-// Four elements of a tile as float32 (the address is a multiple of four elements)
-__device__ __forceinline__ float4 tile4(const float* p) { return *(const float4*)p; }
-__device__ __forceinline__ float4 tile4(const __nv_bfloat16* p) {
-    const uint2 u = *(const uint2*)p;
-    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
-                       __uint_as_float(u.y & 0xffff0000u));
-}
-
 // What set the pace of a decoded token here was latency, tile after tile: a page looked up and a key loaded for each of a
 // warp's eight keys in turn, then the dot product's reads of shared memory one element at a time.  So tiles are double
 // buffered and arrive by 16-byte cp.async (a.vec: widths and pages allow it) while the tile before is attended to, their
@@ -285,7 +277,7 @@ attention_simt_kernel(const AttnArgs a) {
         if (a.vec) {
 #pragma unroll 4
             for (int e = 0; e < d; e += 4) {
-                const float4 k4 = tile4(kr + e);
+                const float4 k4 = vec4(kr + e);
 #pragma unroll
                 for (int rs = 0; rs < ROWS_PER_WARP; ++rs) {
                     if (rs >= my_rows) break;

@@ -42,7 +42,6 @@ namespace {
 // ---- up to 8 tokens ---------------------------------------------------------------------------------------------------
 constexpr int R_WARPS = 8;
 
-__device__ __forceinline__ float4 load4(const float* p) { return *(const float4*)p; }
 __device__ __forceinline__ float4 load4_stream(const float* p) {
     float4 v;
     asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
@@ -182,7 +181,7 @@ cut_rows_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ parts, 
         const int r = (int)(i / per_row), k = (int)(i - (size_t)r * per_row) * 8;
         const float* src = A + (size_t)r * lda + k;
         uint4 h, m, l;
-        cut(load4(src), load4(src + 4), h, m, l);
+        cut(vec4(src), vec4(src + 4), h, m, l);
         __nv_bfloat16* dst = parts + (size_t)r * K + k;
         *(uint4*)dst = h;
         *(uint4*)(dst + plane) = m;
@@ -309,8 +308,8 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map, const float* __re
             for (int j = 0; j < ITEMS; ++j) {
                 const bool in = i < count && n0 + row0 + 64 * j < N && k + run * 8 < K;
                 const float* p = wsrc + (size_t)(64 * j) * ldw + k;
-                v[j][0] = in ? load4(p) : make_float4(0.f, 0.f, 0.f, 0.f);
-                v[j][1] = in ? load4(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[j][0] = in ? vec4(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[j][1] = in ? vec4(p + 4) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         };
 #pragma unroll
