@@ -116,8 +116,8 @@ lightning_scan_kernel(const LightArgs a, int max_tokens) {
 
 // The same with the state in registers and a head's value columns dealt to gridDim.z CTAs of `cols` (32 or 64; dv a multiple of
 // it, dk in steps of 32, rows on 16 bytes).  What a decode step waits for is the state's way from memory and back: with a CTA per
-// head that walked it one element a thread and step through shared memory, 41 us for 8 requests of 16 heads of 128 x 128 (16 MB
-// to move, 3 us of copy bandwidth).  A thread holds one column of the rows r, r + R, ..., the ones that a thread of the kernel
+// head that walked it one element a thread and step through shared memory, 47 us for 8 requests of 16 heads of 128 x 128 (16 MB
+// to move, 3 us of copy bandwidth); here 12 (caches cold, launch included; 32 requests 87 and 29, one 45 and 10).  A thread holds one column of the rows r, r + R, ..., the ones that a thread of the kernel
 // above walks in turn (R = 1 << lr = 256 / dv, rounded down to a power of two as there), so that both give the same bits.
 template <int ROWS>
 __global__ void __launch_bounds__(256)

@@ -424,7 +424,9 @@ __global__ void qknorm_rope_append_kernel(const float* __restrict__ qkv, int nsp
 // The same four elements at a time (head sizes and the rotated width in steps of 4 and 8, rows and strides on 16 bytes): a
 // thread asks for all its loads at once, both norms' sums cross the CTA at one barrier, and angles, pages and the
 // destination are worked out before the kernel waits for the product.  One element a thread and step, with two block-wide
-// sums in turn and the values loaded after them, took 10.6 us for 8 tokens of 16 heads and 62 us for 2,048 of 32.
+// sums in turn and the values loaded after them, took 18.4 us for 8 tokens of 16 heads and 67 us for 2,048 of 32; this form
+// 12.3 and 45 (caches cold, launch included).  The norms' sums are those of the general kernel, `nsums` partial sums in its order,
+// read back from shared memory.
 template <typename CT, int B, int MOST>
 __global__ void __launch_bounds__(MOST)
 qknorm_rope_append_vec_kernel(const float* __restrict__ qkv, int nsplit, size_t split_stride, int ld,

@@ -1,7 +1,8 @@
 """The runtime of each compute dtype: which kernel a part's matrix product runs on.
 
 float32: every operand enters with all of its 24 bits and every sum is float32.  Up to 8 tokens the weights stream through
-the CUDA cores; with more, the tensor cores multiply exact sums of three bfloat16 parts (csrc/gemm_f32.cu).
+the CUDA cores; with more, the tensor cores multiply exact sums of three bfloat16 parts (csrc/gemm_f32.cu); sums of up to 32
+numbers and odd shapes go to the general CUDA-core product.
 bfloat16: the tcgen05 tensor-core product; with up to 64 tokens the weights stream through the
 128-row operand and the K range is split over enough CTAs to fill the GPU (the consumer sums
 the partial matrices in order); with more, a persistent kernel gives every SM the same share
