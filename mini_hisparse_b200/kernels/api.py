@@ -151,6 +151,33 @@ def table_gate(z, table, column0, tokens, out, nsplit=1, split_stride=0, status=
            "table_gate")
 
 
+def side_branch_takes(x, gate, proj, table) -> bool:
+    """Sizes, dtypes and addresses that side_branch is built for."""
+    (T, W), D = x.shape, gate.shape[0]
+    if any(t.dtype != torch.bfloat16 or not t.is_contiguous() for t in (gate, proj, table)) or not 1 <= T <= 64:
+        return False
+    if (x.data_ptr() | gate.data_ptr() | proj.data_ptr()) & 15:
+        return False
+    return bool(build.load("sidebranch").mhb_side_branch_supports(c_int(T), c_int(W), c_int(D)))
+
+
+def side_branch(x, w1, eps1, gate, proj, table, column0, tokens, w2, eps2, copy, *, delta, nsplit=1, split_stride=0,
+                alpha=1.0, keep=0.0, status=None):
+    """A post-norm and the token's own input behind it, for few tokens (the same as norm_mix, a product with ``gate``,
+    table_gate, a product with ``proj`` and norm_mix with alpha 0 and keep 1):
+    x1 = keep x + rms(alpha x + delta) w1;  x <- x1 + rms(proj (gelu_tanh(gate x1) table[token])) w2;  copy = x in bfloat16."""
+    lib = build.load("sidebranch")
+    T, W = x.shape
+    if x.dtype != torch.float32 or not x.is_contiguous() or delta.dtype != torch.float32 or not delta.is_contiguous():
+        raise KernelError("side_branch: the stream and what is added to it must be contiguous float32 matrices")
+    if copy.dtype != torch.bfloat16 or not copy.is_contiguous() or gate.shape[1] != W or tuple(proj.shape) != (W, gate.shape[0]):
+        raise KernelError("side_branch: the copy is bfloat16 [T, W], the weights are [D, W] and [W, D]")
+    _check(lib, lib.mhb_side_branch(
+        _ptr(x), _ptr(delta), c_int(nsplit), c_longlong(split_stride), _ptr(w1), c_float(eps1), c_float(alpha), c_float(keep),
+        _ptr(gate), _ptr(proj), _ptr(table), c_int(table.shape[1]), c_int(column0), c_int(table.shape[0]), _ptr(tokens),
+        _ptr(w2), c_float(eps2), _ptr(copy), c_int(T), c_int(W), c_int(gate.shape[0]), _ptr(status), _stream()), "side_branch")
+
+
 def _gate_args(gate, gate_nsplit, gate_split_stride):
     """(pointer, parts, stride between parts, row stride) of a gate that is a run of columns of a float32 product."""
     if gate is None:

@@ -5,6 +5,8 @@ import torch
 
 from ..kernels import api as K
 from .base import Block, CacheView, Product, StepContext
+from .feed_forward import TokenSide
+from .norm import RMSNorm
 from .registry import FEED_FORWARDS, GATES, INPUT_CONVS, MIXERS, NORMS, register_block
 from .spec import LayerSpec, StateNeed
 
@@ -95,13 +97,17 @@ class PostNormBlock(Block):
             if ctx.rt.dtype != x.dtype:
                 h = ctx.ws.get("x_copy", tuple(x.shape), ctx.rt.dtype)
                 K.act_rows(x, h, "copy")
-        a = self.mixer.forward(h, ctx, cache)
-        h = self.mixer_norm.forward_post(x, ctx, a, alpha=self.alpha, keep=self.keep)
+        last, out = self.mixer_norm, self.mixer.forward(h, ctx, cache)
         if self.feed_forward is not None:
-            f = self.feed_forward.forward(h, ctx)
-            h = self.ff_norm.forward_post(x, ctx, f, alpha=self.alpha, keep=self.keep)
-        if self.side is not None:
-            h = self.side.forward_into(x, h, ctx)
+            h = last.forward_post(x, ctx, out, alpha=self.alpha, keep=self.keep)
+            last, out = self.ff_norm, self.feed_forward.forward(h, ctx)
+        h = None
+        if self.side is not None and isinstance(last, RMSNorm) and isinstance(self.side, TokenSide):
+            h = self.side.forward_behind(last, x, out, ctx, self.alpha, self.keep)
+        if h is None:
+            h = last.forward_post(x, ctx, out, alpha=self.alpha, keep=self.keep)
+            if self.side is not None:
+                h = self.side.forward_into(x, h, ctx)
         ctx.extras["x_copy"] = h
         return None
 

@@ -114,7 +114,7 @@ class TokenSide(FeedForward):
         self.gate = self.proj = self.norm = None
 
     def kernel_modules(self):
-        return ("postnorm",)
+        return ("postnorm", "sidebranch")
 
     def parameters(self):
         return {"gate": ParamSpec((self.dim, self.hidden)), "proj": ParamSpec((self.hidden, self.dim)),
@@ -143,6 +143,22 @@ class TokenSide(FeedForward):
         if not keep_copy:
             return None
         return x if copy is None else copy
+
+    def forward_behind(self, norm, x, delta: Product, ctx: StepContext, alpha: float, keep: float):
+        """The post-norm ``norm`` and this branch in one kernel: x <- x1 + branch(x1) with x1 = keep x + norm(alpha x + delta).
+        Returns the new rows in the compute dtype, or None where the kernel is not built for the step (more than 64
+        tokens, float32, odd widths): then nothing has been done."""
+        rt = ctx.rt
+        if (rt.dtype != torch.bfloat16 or delta is None or delta.also is not None or delta.tensor.dtype != torch.float32
+                or not delta.tensor.is_contiguous() or (delta.nsplit > 1 and delta.split_stride % 4)
+                or any(w.dtype != torch.float32 or w.data_ptr() % 16 for w in (norm.weight, self.norm))
+                or not K.side_branch_takes(x, self.gate, self.proj, self.table.weight)):
+            return None
+        copy = ctx.ws.get("x_copy", tuple(x.shape), rt.dtype)
+        K.side_branch(x, norm.weight, norm.eps, self.gate, self.proj, self.table.weight, self.column0, ctx.tokens, self.norm,
+                      self.eps, copy, delta=delta.tensor, nsplit=delta.nsplit, split_stride=delta.split_stride, alpha=alpha,
+                      keep=keep, status=ctx.status)
+        return copy
 
     def forward(self, h, ctx):
         raise NotImplementedError("a token_side part adds into the stream: call forward_into")

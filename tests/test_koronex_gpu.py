@@ -831,3 +831,42 @@ def test_trace_run_picks_the_model_by_its_config(models, tmp_path):
             row += len(e["want"])
     assert run.close() == 0
     check_against_plain({k: torch.cat(v) for k, v in got.items()}, refs, "float32", "B")
+
+
+@pytest.mark.parametrize("T,W,D,nsplit,alpha,keep", [(1, 1024, 8, 1, 1.0, 0.0), (3, 2048, 64, 5, 1.5, 0.0), (16, 4096, 64, 18, 1.0, 0.0),
+                                                     (17, 2048, 64, 2, 0.0, 1.0), (32, 1024, 136, 9, 1.0, 0.5),
+                                                     (33, 2048, 40, 1, 1.0, 0.0), (64, 3072, 64, 4, 2.0, 0.0)])
+def test_side_branch_in_one_kernel(T, W, D, nsplit, alpha, keep):
+    """The post-norm and the token's own input behind it in one kernel, one to four tokens a cluster with a ragged last one,
+    against the same steps in 64 bits with the same two roundings to bfloat16.  A value that lies on the edge of one of them may
+    round the other way: 2^-8 of one of D (or W) terms of a row whose root mean square is about one."""
+    from mini_hisparse_b200.kernels import api as K
+
+    g = torch.Generator().manual_seed(T * W + D)
+    x, parts = torch.randn(T, W, generator=g), torch.randn(nsplit, T, W, generator=g)
+    w1, w2 = 1 + 0.1 * torch.randn(W, generator=g), 1 + 0.1 * torch.randn(W, generator=g)
+    gate, proj = (0.5 / D ** 0.5 * torch.randn(D, W, generator=g)).bfloat16(), torch.randn(W, D, generator=g).bfloat16()
+    table = torch.randn(50, 3 * D, generator=g).bfloat16()
+    tokens = torch.randint(0, 50, (T,), generator=g, dtype=torch.int32)
+    xd, copy = x.cuda(), torch.full((T + 1, W), float("nan"), dtype=torch.bfloat16, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    assert K.side_branch_takes(xd, gate.cuda(), proj.cuda(), table.cuda())
+    K.side_branch(xd, w1.cuda(), 1e-5, gate.cuda(), proj.cuda(), table.cuda(), D, tokens.cuda(), w2.cuda(), 1e-5, copy[:T],
+                  delta=parts.cuda(), nsplit=nsplit, split_stride=T * W, alpha=alpha, keep=keep, status=status)
+
+    def rms(t):
+        return t / torch.sqrt((t * t).mean(-1, keepdim=True) + 1e-5)
+
+    x1 = keep * x.double() + rms(alpha * x.double() + parts.double().sum(0)) * w1.double()
+    z = x1.bfloat16().double() @ gate.double().T
+    e = table[tokens.long(), D:2 * D].double()
+    y = (torch.nn.functional.gelu(z, approximate="tanh") * e).bfloat16().double() @ proj.double().T
+    ref = x1 + rms(y) * w2.double()
+    assert int(status) == 0 and bool(copy[T].isnan().all()) and bool((copy[:T] == xd.bfloat16()).all())
+    assert float((xd.cpu().double() - ref).abs().max()) < 2.0 ** -8 * float(ref.abs().max())
+    assert not K.side_branch_takes(torch.empty(65, W, device="cuda"), gate.cuda(), proj.cuda(), table.cuda())
+    assert not K.side_branch_takes(torch.empty(T, W + 512, device="cuda"), gate.cuda(), proj.cuda(), table.cuda())
+    tokens[0] = 50          # outside the table: reported, and its row gets no branch
+    K.side_branch(x.cuda(), w1.cuda(), 1e-5, gate.cuda(), proj.cuda(), table.cuda(), D, tokens.cuda(), w2.cuda(), 1e-5, copy[:T],
+                  delta=parts.cuda(), nsplit=nsplit, split_stride=T * W, alpha=alpha, keep=keep, status=status)
+    assert int(status) == 1
