@@ -670,6 +670,167 @@ __device__ __forceinline__ void store_tile(uint32_t acc, int ra0, int rb0, int b
     }
 }
 
+// The epilogue of a tile whose ROWS are features (two SMs on one tile, see gemm_tc_pair_kernel): a thread's lane of tensor
+// memory holds one feature of 16 tokens at a time, so the sums cross shared memory (`buf`, 16 tokens of 128 features)
+// and a warp takes whole tokens: 128 neighbouring features, four a lane, stored in one row.  The four warps move
+// together; they have agreed before that none of them gave up.
+constexpr int FT_LD = BM + 4;                     // floats between two tokens in `buf`
+constexpr int FT_TOKENS = 16;
+__device__ __forceinline__ void epilogue_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ bool epilogue_all(bool ok) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.and.pred q, 1, 128, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r) : "r"((uint32_t)ok) : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void store4_out(float* p, float4 v) { *(float4*)p = v; }
+__device__ __forceinline__ void store4_out(__nv_bfloat16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *(uint2*)p = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
+}
+
+// `ready` waits for the accumulator (false: give up); what does not depend on it is fetched before.
+template <typename OT, int EPI, typename Ready>
+__device__ __forceinline__ bool store_tile_features(Ready ready, uint32_t acc, int f0, int t0, int bn, int quarter, int lane,
+                                                    float* __restrict__ buf, int* __restrict__ slot, OT* __restrict__ C,
+                                                    long long ldc, int N, int M, const QkvRopeArgs& qr,
+                                                    int* __restrict__ status) {
+    const int mine = quarter * 32 + lane;
+    // this lane's four features (of a gated tile: the two outputs whose gate sums start at `f` and whose up sums 16 behind)
+    const int fl = is_glu(EPI) ? (lane >> 3) * 32 + (lane & 7) * 2 : lane * 4;
+    const int f = f0 + fl;
+    int head = 0, e = 0;
+    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f), bias2 = bias;
+    bool is_q = false, is_v = false, turned = false;
+    int partner = 0;                                  // where the other element of a half-split pair lies
+    float4 cs[EPI == 2 ? FT_TOKENS / 4 : 1], sn[EPI == 2 ? FT_TOKENS / 4 : 1];
+    // the angles of the token in turn i of a chunk (asked for a chunk ahead: a round trip to the L2 each)
+    auto angles = [&](int i, int c0) {
+        const int half = qr.rdim >> 1, t = min(t0 + c0 + quarter + 4 * i, M - 1);
+        const float* row = qr.cos_sin + (size_t)t * qr.rdim;
+        if (qr.interleaved) {
+            const float2 c = *(const float2*)(row + (e >> 1)), s = *(const float2*)(row + half + (e >> 1));
+            cs[i] = make_float4(c.x, c.y, 0.f, 0.f);
+            sn[i] = make_float4(s.x, s.y, 0.f, 0.f);
+        } else {
+            const int at = partner > 0 ? e : e - half;
+            cs[i] = *(const float4*)(row + at);
+            sn[i] = *(const float4*)(row + half + at);
+        }
+    };
+    if constexpr (EPI == 2) {
+        const int d = qr.d;
+        head = f / d;
+        e = f - head * d;
+        is_q = head < qr.nq;
+        is_v = head >= qr.nq + qr.nkv;
+        turned = f < N && !is_v && e < qr.rdim;
+        if (!qr.interleaved) partner = e < (qr.rdim >> 1) ? qr.rdim >> 1 : -(qr.rdim >> 1);
+        if (qr.bias && f < N) bias = *(const float4*)(qr.bias + f);
+        if (qr.bias && turned) bias2 = *(const float4*)(qr.bias + f + partner);
+        pdl_wait();             // the table of angles was made in this step
+        if (turned) {
+#pragma unroll
+            for (int i = 0; i < FT_TOKENS / 4; ++i) angles(i, 0);
+        }
+        // the places in the cache of this tile's tokens: page * P + offset, or -1
+        if (f0 + BM > qr.nq * d)
+            for (int i = mine; i < bn; i += 128) {
+                int s = -1;
+                if (t0 + i < M && qr.write_kv) {
+                    const int pos = qr.positions[t0 + i];
+                    const int page = qr.block_table[(size_t)qr.tok_seg[t0 + i] * qr.table_width + pos / qr.P];
+                    if (page >= 0 && page < qr.num_pages) s = page * qr.P + pos % qr.P;
+                    else if (status) atomicOr(status, 2);           // never write outside the pool
+                }
+                slot[i] = s;
+            }
+    }
+    if (!ready()) return false;
+    const bool wide = EPI != 2 && ldc % (is_glu(EPI) ? 2 : 4) == 0 &&
+                      ((uintptr_t)C & (is_glu(EPI) ? 3 : 4 * sizeof(OT) - 1)) == 0;
+    // two buffers: the next chunk is on its way out of tensor memory while this one is stored, and the warps meet once a chunk
+    uint32_t r[16];
+    tmem_ld16(acc, r);
+#pragma unroll 1
+    for (int c0 = 0; c0 < bn && t0 + c0 < M; c0 += FT_TOKENS) {
+        float* half_buf = buf + (c0 / FT_TOKENS & 1) * (FT_TOKENS * FT_LD);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            float v = __uint_as_float(r[j]);
+            if constexpr (EPI >= 4 && EPI <= 6) v = plain_act<EPI>(v);
+            half_buf[j * FT_LD + mine] = v;
+        }
+        if (c0 + FT_TOKENS < bn && t0 + c0 + FT_TOKENS < M) tmem_ld16(acc + c0 + FT_TOKENS, r);
+        epilogue_sync();
+#pragma unroll
+        for (int i = 0; i < FT_TOKENS / 4; ++i) {
+            const int j = quarter + 4 * i, t = t0 + c0 + j;
+            if (t >= M || f >= N) continue;
+            const float* row = half_buf + j * FT_LD;
+            if constexpr (EPI == 2) {
+                const int d = qr.d;
+                float4 v = *(const float4*)(row + fl);
+                v.x += bias.x; v.y += bias.y; v.z += bias.z; v.w += bias.w;
+                if (turned) {
+                    const float4 c = cs[i], s = sn[i];
+                    if (qr.interleaved) {
+                        v = make_float4(v.x * c.x - v.y * s.x, v.y * c.x + v.x * s.x, v.z * c.y - v.w * s.y, v.w * c.y + v.z * s.y);
+                    } else {
+                        float4 w = *(const float4*)(row + fl + partner);
+                        w.x += bias2.x; w.y += bias2.y; w.z += bias2.z; w.w += bias2.w;
+                        v = partner > 0 ? make_float4(v.x * c.x - w.x * s.x, v.y * c.y - w.y * s.y, v.z * c.z - w.z * s.z, v.w * c.w - w.w * s.w)
+                                        : make_float4(v.x * c.x + w.x * s.x, v.y * c.y + w.y * s.y, v.z * c.z + w.z * s.z, v.w * c.w + w.w * s.w);
+                    }
+                }
+                if (is_q) {
+                    store4_out(qr.q_out + (size_t)t * qr.nq * d + f, v);
+                } else {
+                    const int s = slot[c0 + j];
+                    const int kvh = head - qr.nq - (is_v ? qr.nkv : 0);
+                    if (s >= 0)
+                        store4_out(qr.cache + ((((size_t)(s / qr.P) * 2 + (is_v ? 1 : 0)) * qr.nkv + kvh) * qr.P + s % qr.P) * d + e, v);
+                }
+            } else if constexpr (is_glu(EPI)) {
+                const float2 g = *(const float2*)(row + fl), u = *(const float2*)(row + fl + 16);
+                OT* dst = C + (size_t)t * ldc + (f0 >> 1) + lane * 2;
+                const float a = glu_mul<EPI>(g.x, u.x), b = glu_mul<EPI>(g.y, u.y);
+                if (wide && sizeof(OT) == 2) {
+                    const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+                    *(uint32_t*)dst = *(const uint32_t*)&p;
+                } else {
+                    store_out<OT>(dst, a);
+                    store_out<OT>(dst + 1, b);
+                }
+            } else {
+                const float4 v = *(const float4*)(row + fl);
+                OT* dst = C + (size_t)t * ldc + f;
+                if (wide && f + 4 <= N) {
+                    store4_out(dst, v);
+                } else {
+                    store_out<OT>(dst, v.x);
+                    if (f + 1 < N) store_out<OT>(dst + 1, v.y);
+                    if (f + 2 < N) store_out<OT>(dst + 2, v.z);
+                    if (f + 3 < N) store_out<OT>(dst + 3, v.w);
+                }
+            }
+        }
+        if constexpr (EPI == 2) {
+            if (turned && c0 + FT_TOKENS < bn) {
+#pragma unroll
+                for (int i = 0; i < FT_TOKENS / 4; ++i) angles(i, c0 + FT_TOKENS);
+            }
+        }
+    }
+    epilogue_sync();        // the buffers and places may be written again
+    return true;
+}
+
 template <typename OT, int EPI>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -946,6 +1107,10 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 //     barrier before the end keeps either CTA's shared and tensor memory alive while the other may use it.
 // Whole tiles only (no sharing of a tile's K range); every wait is bounded as above.
 //
+// FEATURES: the roles of the operands change, a tile is 256 features x bn tokens.  A tile's 256 rows are all paid for,
+// its bn columns can be any multiple of 16: with 543 tokens (a portion of 512 beside 31 decoding requests) three tiles of
+// 256 tokens are 768 rows of work, three of 192 are 576.  (see choose_features_bn).
+//
 // A stage of the ring holds one or two K blocks of 64 (`kbs`).  The thread that issues the MMAs pays some
 // 250 cycles for the barrier it looks at before a stage, whatever the stage holds: with tiles 256 wide
 // the four MMAs of one K block (512 cycles) hide that, with narrower tiles they do not (a K block took
@@ -955,11 +1120,18 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // [A block 0 | A block 1 | B block 0 | B block 1] with each CTA's half of the B rows.
 constexpr int PAIR_MAX_STAGES = 8;
 constexpr int PAIR_DATA_BYTES = 216 * 1024;     // operand stages of one CTA
+constexpr int PAIR_FEATURES_DATA_BYTES = 208 * 1024;   // ... beside the buffers of an epilogue that transposes
 constexpr uint32_t PEER_MASK = 0xFEFFFFFFu;     // clears the bit that tells the pair's second CTA from its first
 struct PairSmem {
     static constexpr int A_BYTES = BM * BK * 2;
     static constexpr int BARRIER_OFFSET = PAIR_DATA_BYTES;
     static constexpr int TOTAL = BARRIER_OFFSET + (2 * PAIR_MAX_STAGES + 5) * 8 + 16 + 1024;
+    // where rows are features: two buffers of the epilogue and the tokens' places lie behind a shorter ring
+    static constexpr int BUF_OFFSET = PAIR_FEATURES_DATA_BYTES;
+    static constexpr int SLOT_OFFSET = BUF_OFFSET + 2 * FT_TOKENS * FT_LD * 4;
+    static constexpr int FEATURES_BARRIER_OFFSET = SLOT_OFFSET + P_BN_MAX * 4;
+    static constexpr int FEATURES_TOTAL = FEATURES_BARRIER_OFFSET + (2 * PAIR_MAX_STAGES + 5) * 8 + 16 + 1024;
+    static_assert(FEATURES_TOTAL <= 227 * 1024 && TOTAL <= 227 * 1024, "more shared memory than a CTA may have");
 };
 struct PairRing {
     int kbs;                 // K blocks of 64 per stage: 1 or 2
@@ -1013,7 +1185,7 @@ __host__ __device__ constexpr uint32_t make_idesc_pair(int bn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 }
 
-template <typename OT, int EPI>
+template <typename OT, int EPI, bool FEATURES>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     OT* __restrict__ C, int Ra, int Rb, int K, long long ldc, int bn, int tiles_m, int num_tiles,
@@ -1023,13 +1195,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t smem_base = smem_u32(smem);
-    const uint32_t bar_base = smem_base + S::BARRIER_OFFSET;
+    constexpr int BARRIERS = FEATURES ? S::FEATURES_BARRIER_OFFSET : S::BARRIER_OFFSET;
+    const uint32_t bar_base = smem_base + BARRIERS;
     auto full_bar = [&](int s) { return bar_base + 8 * s; };                                  // the leader's counts
     auto empty_bar = [&](int s) { return bar_base + 8 * (PAIR_MAX_STAGES + s); };                 // each CTA's own
     auto acc_full_bar = [&](int b) { return bar_base + 8 * (2 * PAIR_MAX_STAGES + b); };          // each CTA's own
     auto acc_empty_bar = [&](int b) { return bar_base + 8 * (2 * PAIR_MAX_STAGES + 2 + b); };     // the leader's counts
     const uint32_t drain_bar = bar_base + 8 * (2 * PAIR_MAX_STAGES + 4);
-    uint32_t* tmem_slot = (uint32_t*)(smem + S::BARRIER_OFFSET + 8 * (2 * PAIR_MAX_STAGES + 5));
+    uint32_t* tmem_slot = (uint32_t*)(smem + BARRIERS + 8 * (2 * PAIR_MAX_STAGES + 5));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = (int)pair_rank();
     const bool leader = rank == 0;
@@ -1040,7 +1213,13 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int total_st = (total_kb + kbs - 1) / kbs;              // stages a tile takes (the last may hold a K block of zeros)
     const uint32_t b_bytes = half_bn * BK * 2;                    // this CTA's rows of one K block of the weights
     const uint32_t half_tx = kbs * (S::A_BYTES + b_bytes);        // what one CTA loads per stage
-    const uint32_t b_offset = kbs * S::A_BYTES;                   // the weights' place in a stage
+    const uint32_t b_offset = kbs * S::A_BYTES;                   // the second operand's place in a stage
+    // first rows of tile t: of operand A (this CTA's 128 of 256) and of operand B (tiles that share weights are neighbours)
+    auto tile_rows = [&](int t, int& ra0, int& rb0) {
+        const int m = t % tiles_m, n = t / tiles_m;               // tiles_m tiles along the tokens
+        ra0 = (FEATURES ? n : m) * 2 * BM + rank * BM;
+        rb0 = (FEATURES ? m : n) * bn;
+    };
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
@@ -1064,15 +1243,24 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
             const uint32_t count_bar0 = full_bar(0) & PEER_MASK;      // the leader's barrier of stage 0
             int it = 0, early = 0;
-            // the weight halves of the first stages are asked for while the kernel before this one still runs
+            int ra0, rb0;
+            auto load_a = [&](int s, int kk, int kb) {
+                tma_load_2d_pair(smem_base + s * ring.stage_bytes + kk * S::A_BYTES, &map_a, kb * BK, ra0, count_bar0 + 8 * s);
+            };
+            auto load_b = [&](int s, int kk, int kb) {
+                tma_load_2d_pair(smem_base + s * ring.stage_bytes + b_offset + kk * b_bytes, &map_b, kb * BK,
+                                 rb0 + rank * half_bn, count_bar0 + 8 * s);
+            };
+            // the weights' part of the first stages is asked for while the kernel before this one still runs
             // (a K block beyond the matrix is a box outside the tensor map: zeros, counted like any other)
             if (pair < num_tiles) {
-                const int rbh0 = (pair / tiles_m) * bn + rank * half_bn;
+                tile_rows(pair, ra0, rb0);
                 for (int st = 0; st < total_st && early < nstages; ++st, ++early) {
                     if (leader) mbar_expect_tx(full_bar(early), 2 * half_tx);
-                    for (int kk = 0; kk < kbs; ++kk)
-                        tma_load_2d_pair(smem_base + early * ring.stage_bytes + b_offset + kk * b_bytes, &map_b,
-                                         (st * kbs + kk) * BK, rbh0, count_bar0 + 8 * early);
+                    for (int kk = 0; kk < kbs; ++kk) {
+                        if (FEATURES) load_a(early, kk, st * kbs + kk);
+                        else load_b(early, kk, st * kbs + kk);
+                    }
                 }
             }
             pdl_wait();
@@ -1081,20 +1269,21 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             int s = 0;
             uint32_t turn = 0;
             for (int t = pair; ok && t < num_tiles; t += npairs) {
-                const int ra0 = (t % tiles_m) * 2 * BM + rank * BM, rbh0 = (t / tiles_m) * bn + rank * half_bn;
+                tile_rows(t, ra0, rb0);
                 for (int st = 0; st < total_st; ++st, ++it, turn ^= (s + 1 == nstages), s = (s + 1 == nstages) ? 0 : s + 1) {
-                    const uint32_t a_dst = smem_base + s * ring.stage_bytes;
-                    if (it < early) {                   // the weight half is on its way already
-                        for (int kk = 0; kk < kbs; ++kk)
-                            tma_load_2d_pair(a_dst + kk * S::A_BYTES, &map_a, (st * kbs + kk) * BK, ra0, count_bar0 + 8 * s);
+                    if (it < early) {                   // the weights are on their way already
+                        for (int kk = 0; kk < kbs; ++kk) {
+                            if (FEATURES) load_b(s, kk, st * kbs + kk);
+                            else load_a(s, kk, st * kbs + kk);
+                        }
                         continue;
                     }
                     ok = mbar_wait(empty_bar(s), turn ^ 1, wait_limit);
                     if (!ok) break;
                     if (leader) mbar_expect_tx(full_bar(s), 2 * half_tx);
                     for (int kk = 0; kk < kbs; ++kk) {
-                        tma_load_2d_pair(a_dst + kk * S::A_BYTES, &map_a, (st * kbs + kk) * BK, ra0, count_bar0 + 8 * s);
-                        tma_load_2d_pair(a_dst + b_offset + kk * b_bytes, &map_b, (st * kbs + kk) * BK, rbh0, count_bar0 + 8 * s);
+                        load_a(s, kk, st * kbs + kk);
+                        load_b(s, kk, st * kbs + kk);
                     }
                 }
             }
@@ -1152,12 +1341,23 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         int j = 0;
         for (int t = pair; ok && t < num_tiles; t += npairs, ++j) {
             const int b = j & 1;
-            const int ra0 = (t % tiles_m) * 2 * BM + rank * BM, rb0 = (t / tiles_m) * bn;
-            ok = mbar_wait(acc_full_bar(b), (j >> 1) & 1, wait_limit);
-            if (!ok) break;
-            tc_fence_after();
+            int ra0, rb0;
+            tile_rows(t, ra0, rb0);
             const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + b * P_BN_MAX;
-            store_tile<OT, EPI>(acc, ra0, rb0, bn, row_in_tile, C, ldc, Ra, Rb, qr, status);
+            auto ready = [&]() {
+                bool full = mbar_wait(acc_full_bar(b), (j >> 1) & 1, wait_limit);
+                if (FEATURES) full = epilogue_all(full);        // the warps meet inside the epilogue: all of them or none
+                tc_fence_after();
+                return full;
+            };
+            if constexpr (FEATURES) {
+                ok = store_tile_features<OT, EPI>(ready, acc, ra0, rb0, bn, quarter, lane, (float*)(smem + S::BUF_OFFSET),
+                                                  (int*)(smem + S::SLOT_OFFSET), C, ldc, Ra, Rb, qr, status);
+            } else {
+                ok = ready();
+                if (ok) store_tile<OT, EPI>(acc, ra0, rb0, bn, row_in_tile, C, ldc, Ra, Rb, qr, status);
+            }
+            if (!ok) break;
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_leader(acc_empty_bar(b));    // this warp has read its quarter
@@ -1290,6 +1490,76 @@ int choose_persistent_bn(int tiles_m, int N, int sms, int step) {
     return best;
 }
 
+// What a launch of the two-SM kernel takes, in rows of 64 operand elements that a pair loads: its rounds of tiles, each
+// (256 + bn) rows per K block and a fixed cost, or what reading the weights takes if that is longer.  Fitted to 2,048 and
+// 543 tokens at the 14B, 7B and 2,048-wide shapes (0.74 ns a row; 14B down of 2,048 tokens: 228 us measured, 228 counted; 7B
+// gate/up: 350, 371; 2,048-wide gate/up: 106, 99).  The epilogue that rotates and appends takes longer where rows are features.
+constexpr double PAIR_ROUND_ROWS = 2800.0, PAIR_HEADS_ROWS = 12000.0, PAIR_WEIGHT_BYTES = 4800.0;
+double pair_cost(long long tiles, int bn, int N, int K, int pairs, double fixed) {
+    const double rows = (double)((tiles + pairs - 1) / pairs) * ((256 + bn) * (double)((K + BK - 1) / BK) + fixed);
+    const double weights = (double)N * K * 2 / PAIR_WEIGHT_BYTES;
+    return rows > weights ? rows : weights;
+}
+long long features_tiles(int bn, int M, int N) { return (long long)((M + bn - 1) / bn) * ((N + 2 * BM - 1) / (2 * BM)); }
+// Tokens of a tile whose rows are features: the multiple of 16 that takes least.
+int choose_features_bn(int M, int N, int K, int pairs, double fixed) {
+    int best = P_BN_MAX;
+    double best_cost = 1e30;
+    for (int bn = P_BN_MAX; bn >= 96; bn -= 16) {
+        const double cost = pair_cost(features_tiles(bn, M, N), bn, N, K, pairs, fixed);
+        if (cost < best_cost * (1 - 1e-9)) { best_cost = cost; best = bn; }
+    }
+    return best;
+}
+// Tiles of features are taken when they are this much shorter by that count.  Measured beside tiles of tokens (us): 543
+// tokens, 14B: gate/up 134 instead of 154, q/k/v 52 for 68, down 70 for 77; 257 tokens, 14B gate/up 77 for 99, 2,048 wide 28 for
+// 43; 2,048 tokens, 14B q/k/v 129 for 168.  Between 0.9 and 1 either may win (2,048-wide gate/up of 2,079 tokens: 0.91 counted,
+// 156 for 130: with K short the epilogue's pace counts).
+constexpr double FEATURES_GAIN = 0.905;
+
+template <typename OT, int EPI, bool FEATURES>
+int launch_pair(const void* X, const void* W, void* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
+                int bn, int tiles_m, long long tiles, int pairs, int* status, cudaStream_t stream, const QkvRopeArgs* qr) {
+    // two K blocks per stage (see PairRing): three stages of 64 KB with tiles 256 wide, four or more below 176
+    PairRing ring;
+    ring.kbs = pair_kbs() ? pair_kbs() : 2;
+    ring.stage_bytes = (uint32_t)ring.kbs * (PairSmem::A_BYTES + (bn / 2) * BK * 2);
+    ring.stages = (FEATURES ? PAIR_FEATURES_DATA_BYTES : PAIR_DATA_BYTES) / (int)ring.stage_bytes;
+    constexpr int smem = FEATURES ? PairSmem::FEATURES_TOTAL : PairSmem::TOTAL;
+    if (ring.stages > PAIR_MAX_STAGES) ring.stages = PAIR_MAX_STAGES;
+    if (ring.stages < 2) return fail("gemm_tc: a stage of %u bytes leaves no ring", ring.stage_bytes);
+    CUtensorMap pa, pb;
+    int prc;
+    if ((prc = FEATURES ? make_map(&pa, W, N, K, ldw, BM) : make_map(&pa, X, M, K, lda, BM))) return prc;
+    if ((prc = FEATURES ? make_map(&pb, X, M, K, lda, bn / 2) : make_map(&pb, W, N, K, ldw, bn / 2))) return prc;
+    auto pkern = gemm_tc_pair_kernel<OT, EPI, FEATURES>;
+    static bool pair_configured = false;
+    if (!pair_configured) {
+        cudaError_t e = cudaFuncSetAttribute(pkern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return fail("gemm_tc: cannot set %d bytes of shared memory: %s", smem, cudaGetErrorString(e));
+        pair_configured = true;
+    }
+    QkvRopeArgs none = {};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, pkern, pa, pb, (OT*)C, FEATURES ? N : M, FEATURES ? M : N, K, ldc, bn, tiles_m,
+                                       (int)tiles, ring, status, qr ? *qr : none, g_wait_limit);
+    if (e != cudaSuccess) return fail("gemm_tc: launch of the two-SM kernel: %s", cudaGetErrorString(e));
+    return check_launch("gemm_tc_pair");
+}
+
 // `partials` (2 P_MAX_CTAS tiles of 128 x 256 floats) and `flags` (4 P_FLAG_CAP ints, zero; the kernel
 // leaves them zero) let CTAs share a tile's K range; without them the ranges are cut at tile
 // boundaries only.
@@ -1345,43 +1615,15 @@ int launch_persistent(const void* X, const void* W, void* C, int M, int N, int K
             if (narrow < wide) pbn = 128;
         }
         const long long pair_tiles = (long long)tiles_m2 * ((N + pbn - 1) / pbn);
-        // two K blocks per stage (see PairRing): three stages of 64 KB with tiles 256 wide, four or more below 176
-        PairRing ring;
-        ring.kbs = pair_kbs() ? pair_kbs() : 2;
-        ring.stage_bytes = (uint32_t)ring.kbs * (PairSmem::A_BYTES + (pbn / 2) * BK * 2);
-        ring.stages = PAIR_DATA_BYTES / (int)ring.stage_bytes;
-        if (ring.stages > PAIR_MAX_STAGES) ring.stages = PAIR_MAX_STAGES;
-        if (ring.stages < 2) return fail("gemm_tc: a stage of %u bytes leaves no ring", ring.stage_bytes);
-        CUtensorMap pa, pb;
-        int prc;
-        if ((prc = make_map(&pa, X, M, K, lda, BM))) return prc;
-        if ((prc = make_map(&pb, W, N, K, ldw, pbn / 2))) return prc;
-        auto pkern = gemm_tc_pair_kernel<OT, EPI>;
-        static bool pair_configured = false;
-        if (!pair_configured) {
-            cudaError_t e = cudaFuncSetAttribute(pkern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::TOTAL);
-            if (e != cudaSuccess) return fail("gemm_tc: cannot set %d bytes of shared memory: %s", PairSmem::TOTAL, cudaGetErrorString(e));
-            pair_configured = true;
+        if (M > 2 * BM) {       // up to 256 tokens fit one tile's rows
+            const double fixed = EPI == 2 ? PAIR_HEADS_ROWS : PAIR_ROUND_ROWS;
+            const int fbn = choose_features_bn(M, N, K, pairs, fixed);
+            const long long tiles = features_tiles(fbn, M, N);
+            if (pair_cost(tiles, fbn, N, K, pairs, fixed) < FEATURES_GAIN * pair_cost(pair_tiles, pbn, N, K, pairs, PAIR_ROUND_ROWS))
+                return launch_pair<OT, EPI, true>(X, W, C, M, N, K, lda, ldw, ldc, fbn, (M + fbn - 1) / fbn, tiles, pairs, status,
+                                                  stream, qr);
         }
-        QkvRopeArgs none = {};
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(2 * (pair_tiles < pairs ? pair_tiles : pairs)));
-        cfg.blockDim = dim3(THREADS);
-        cfg.dynamicSmemBytes = PairSmem::TOTAL;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = pdl_enabled() ? 2 : 1;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, pkern, pa, pb, (OT*)C, M, N, K, ldc, pbn, tiles_m2, (int)pair_tiles, ring,
-                                           status, qr ? *qr : none, g_wait_limit);
-        if (e != cudaSuccess) return fail("gemm_tc: launch of the two-SM kernel: %s", cudaGetErrorString(e));
-        return check_launch("gemm_tc_pair");
+        return launch_pair<OT, EPI, false>(X, W, C, M, N, K, lda, ldw, ldc, pbn, tiles_m2, pair_tiles, pairs, status, stream, qr);
     }
     if (EPI != 2 && !share && N >= P_BN_MAX) {     // (epilogue 2 needs tiles that begin and end on heads)
         // whole tiles only: a narrower tile may fill the last round better

@@ -359,6 +359,67 @@ def test_gemm_tensor_core_swiglu_epilogue(M, I, K_, swap, bn):
     torch.testing.assert_close(out2.float(), ref, atol=2e-2 * float(ref.abs().max()), rtol=2e-2)
 
 
+@pytest.mark.parametrize("M,N,K_", [(257, 19000, 136), (272, 27648, 64), (543, 27648, 200), (543, 7168, 1024), (321, 14001, 72),
+                                    (781, 13826, 64)])
+@pytest.mark.parametrize("epilogue", ["float32", "bfloat16", "silu", "gelu_tanh", "gelu_act", "heads128", "heads64"])
+def test_gemm_tiles_of_features(M, N, K_, epilogue):
+    """Token counts that fill tiles of 256 tokens badly: the two-SM kernel with 256 features a tile and every epilogue,
+    ragged in tokens and features, output rows on and off 16 bytes."""
+    x = rnd(M, K_, dtype=torch.bfloat16, seed=1)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    scratch = K().stream_k_scratch(DEV)
+    if epilogue.startswith("heads"):
+        d = int(epilogue[5:])
+        nkv, P_ = 3, 16
+        nq = N // d - 2 * nkv
+        n = (nq + 2 * nkv) * d
+        w, bias = rnd(n, K_, dtype=torch.bfloat16, seed=2, scale=K_ ** -0.5), rnd(n, seed=3)
+        pos = torch.arange(5, 5 + M, dtype=torch.int32, device=DEV)
+        seg = torch.zeros(M, dtype=torch.int32, device=DEV)
+        pages = (M + 5) // P_ + 1
+        table = torch.randperm(pages, generator=torch.Generator().manual_seed(5)).to(torch.int32).to(DEV)[None]
+        inv = (10000.0 ** (-torch.arange(0, d, 2).float() / d)).to(DEV)
+        for rdim, interleaved in ((d, False), (d // 2, True)):
+            cs = torch.empty(M, rdim, device=DEV)
+            K().rope_table(pos, inv[: rdim // 2], cs)
+            q, cache = torch.full((M + 1, nq * d), float("nan"), dtype=torch.bfloat16, device=DEV), torch.zeros(pages, 2, nkv, P_, d, dtype=torch.bfloat16, device=DEV)
+            K().gemm_tc_qkv_rope(x, w, bias, cs, pos, seg, table, q[:M], cache, nq=nq, nkv=nkv, d=d, page_size=P_, rotary_dim=rdim,
+                                 interleaved=interleaved, status=status)
+            y = (x.float() @ w.float().T + bias).view(M, -1, d)
+            h, c, s = rdim // 2, cs[:, None, : rdim // 2], cs[:, None, rdim // 2:]
+            a, b = (y[..., 0:rdim:2], y[..., 1:rdim:2]) if interleaved else (y[..., :h], y[..., h:rdim])
+            turned = torch.stack((a * c - b * s, b * c + a * s), -1).flatten(-2) if interleaved else torch.cat((a * c - b * s, b * c + a * s), -1)
+            y = torch.cat((torch.cat((turned, y[..., rdim:]), -1)[:, : nq + nkv], y[:, nq + nkv:]), 1)
+            page, at = table[0][(pos // P_).long()].long(), (pos % P_).long()
+            top = float(y.abs().max())
+            assert int(status) == 0 and bool(q[M].isnan().all())
+            torch.testing.assert_close(q[:M].float(), y[:, :nq].flatten(1), atol=2.0 ** -8 * top, rtol=2.0 ** -8)
+            for plane in (0, 1):
+                got = cache[page, plane, :, at].float()
+                torch.testing.assert_close(got, y[:, nq + plane * nkv: nq + (plane + 1) * nkv], atol=2.0 ** -8 * top, rtol=2.0 ** -8)
+            assert int((cache[:, 0].abs().sum(-1) > 0).sum()) == M * nkv
+        return
+    gated = epilogue in ("silu", "gelu_tanh")
+    n = N // 32 * 32 if gated else N
+    w = rnd(n, K_, dtype=torch.bfloat16, seed=2, scale=0.2)
+    out = torch.full((M + 1, n // 2 if gated else n), float("nan"), dtype=torch.float32 if epilogue == "float32" else torch.bfloat16, device=DEV)
+    y = x.float() @ w.float().T
+    if gated:
+        K().gemm_tc_glu(x, w, out[:M], epilogue, swap=False, bn=0, status=status, scratch=scratch)
+        g, u = y.view(M, -1, 2, 16).unbind(2)
+        y = ((torch.nn.functional.silu(g) if epilogue == "silu" else torch.nn.functional.gelu(g, approximate="tanh")) * u).flatten(1)
+    elif epilogue == "gelu_act":
+        K().gemm_tc_act(x, w, out[:M], "gelu_tanh", status=status, scratch=scratch)
+        y = torch.nn.functional.gelu(y, approximate="tanh")
+    else:
+        K().gemm_tc(x, w, out[:M], swap=False, bn=0, status=status, scratch=scratch)
+    assert int(status) == 0 and bool(out[M].isnan().all())
+    if epilogue == "float32":       # two float32 sums of K exact products
+        torch.testing.assert_close(out[:M], y, atol=2.0 * K_ * 2.0 ** -24 * float((x.float().abs() @ w.float().abs().T).max()), rtol=0)
+    else:
+        torch.testing.assert_close(out[:M].float(), y, atol=2.0 ** -8 * float(y.abs().max()), rtol=2.0 ** -8)
+
+
 def test_gemm_tensor_core_refuses_unaligned_k():
     from mini_hisparse_b200.kernels.api import KernelError
 
