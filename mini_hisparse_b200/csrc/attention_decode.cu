@@ -16,6 +16,10 @@
 //     the 7B shape) from the product's partials, and the CTA that owns the token's own position
 //     builds the new k and v, patches them into its last tile in shared memory and, when it has
 //     walked its keys, stores them into the page for the steps to come.
+//   * the products have the KEYS (or the head's elements) along the 16 rows of an mma and the heads along its 8 columns:
+//     S^T = K Q^T and O^T = V^T P^T.  With the heads along the rows, a KV head's 4 to 7 query heads left more than half of
+//     every product to padding; groups of up to 8 heads now take half the mmas, with half the accumulators (steps of 1, 8 and
+//     64 tokens at the 7B shape: 1.4, 1.3 and 1.7 % shorter; 8 to 40 tokens of 70 to 2,400 keys, 4,096 wide: 2 to 3 %).
 //   * the splits' (max, sum, accumulator) meet in distributed shared memory: a CTA that has walked
 //     its keys sends every row of its part to the CTA that owns that row (CTA r owns the rows r,
 //     r + nsplit, ...; plain st.shared::cluster), one cluster barrier follows, and each owner merges
@@ -164,13 +168,12 @@ __device__ __forceinline__ void head_unit(const DecodeArgs& a, const float* row,
     }
 }
 
-template <int D>
+// NB: columns of 8 heads (groups of up to 8, or 16 heads).
+template <int D, int NB>
 __global__ void __launch_bounds__(THREADS, 2)
 attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const DecodeArgs a) {
     using L = Layout<D>;
-    constexpr int KSTEPS = D / 16;
-    constexpr int DTILES = D / 8;
-    constexpr int NT = 2;                       // each warp takes 16 of a tile's 64 keys
+    constexpr int KSTEPS = D / 16;              // also the tiles of 16 elements of an output row
     constexpr int MS = L::MS;
     extern __shared__ uint8_t smem_raw[];
     __shared__ int cta_failed;          // a bounded wait ran out somewhere in this CTA: it stores nothing
@@ -320,15 +323,20 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const Decode
         }
         prologue_sync();      // q, the new key and (from the TMA warp) the new value are in shared memory
 
-        float o[DTILES][4];
+        // sums of the outputs, transposed: tile i of column block b holds elements 16 i + (lane >> 2) (+ 8: [2], [3]) of the
+        // heads 8 b + 2 (lane & 3) ([0], [2]) and the one after it ([1], [3])
+        float o[NB][KSTEPS][4];
+        float m_run[NB][2], l_run[NB][2];
+        uint32_t qf[NB][KSTEPS][2];
 #pragma unroll
-        for (int i = 0; i < DTILES; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-        float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-        uint32_t qf[KSTEPS][4];
+        for (int b = 0; b < NB; ++b) {
 #pragma unroll
-        for (int k = 0; k < KSTEPS; ++k) {
-            const int r = (lane & 7) + 8 * ((lane >> 3) & 1), c = k * 16 + 8 * (lane >> 4);
-            ldmatrix_x4(swz(q_s, ROWS, r, c), qf[k][0], qf[k][1], qf[k][2], qf[k][3]);
+            for (int i = 0; i < KSTEPS; ++i) o[b][i][0] = o[b][i][1] = o[b][i][2] = o[b][i][3] = 0.f;
+            m_run[b][0] = m_run[b][1] = -INFINITY;
+            l_run[b][0] = l_run[b][1] = 0.f;
+#pragma unroll
+            for (int k = 0; k < KSTEPS; k += 2)
+                ldmatrix_x4(swz(q_s, ROWS, 8 * b + (lane & 7), k * 16 + 8 * (lane >> 3)), qf[b][k][0], qf[b][k][1], qf[b][k + 1][0], qf[b][k + 1][1]);
         }
         const float scale_log2 = a.scale * 1.4426950408889634f;
         const int key0 = warp * 16;
@@ -351,76 +359,58 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const Decode
                 __syncwarp();
             }
 
-            // scores: two accumulators per key group (even and odd steps along the head), so that the
-            // chain of dependent products is half as long; their sum is the score
-            float s[NT][4], s2[NT][4];
+            // scores of 16 keys: two accumulators (even and odd steps along the head), so that the chain of
+            // dependent products is half as long; their sum is the score
+            float s[NB][4], s2[NB][4];
 #pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-                s2[j][0] = s2[j][1] = s2[j][2] = s2[j][3] = 0.f;
+            for (int b = 0; b < NB; ++b) {
+                s[b][0] = s[b][1] = s[b][2] = s[b][3] = 0.f;
+                s2[b][0] = s2[b][1] = s2[b][2] = s2[b][3] = 0.f;
             }
+            const int kr = key0 + (lane & 7);
 #pragma unroll
-            for (int k = 0; k < KSTEPS; k += 2) {
+            for (int k = 0; k < KSTEPS; ++k) {
+                uint32_t ka[4];
+                ldmatrix_x4(swz(k_s, KT, kr + 8 * ((lane >> 3) & 1), k * 16 + 8 * (lane >> 4)), ka[0], ka[1], ka[2], ka[3]);
 #pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    uint32_t b0, b1, b2, b3;
-                    const int r = key0 + j * 8 + (lane & 7), c = k * 16 + 8 * (lane >> 3);
-                    ldmatrix_x4(swz(k_s, KT, r, c), b0, b1, b2, b3);
-                    mma_bf16(s[j], qf[k], b0, b1);
-                    mma_bf16(s2[j], qf[k + 1], b2, b3);
+                for (int b = 0; b < NB; ++b) mma_bf16((k & 1) ? s2[b] : s[b], ka, qf[b][k][0], qf[b][k][1]);
+            }
+            const int kp = t0 + key0 + (lane >> 2);
+            const bool valid0 = kp >= kv_begin && kp < kv_stop, valid1 = kp + 8 >= kv_begin && kp + 8 < kv_stop;   // causal and window limits are the split's
+            uint32_t pf[NB][2];
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+#pragma unroll
+                for (int x = 0; x < 4; ++x) s[b][x] = (x < 2 ? valid0 : valid1) ? s[b][x] + s2[b][x] : -INFINITY;
+                float alpha[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float mx = fmaxf(s[b][h], s[b][2 + h]);
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                    const float m_new = fmaxf(m_run[b][h], mx);
+                    const float m_use = m_new == -INFINITY ? 0.f : m_new;
+                    alpha[h] = exp2f((m_run[b][h] - m_use) * scale_log2);
+                    m_run[b][h] = m_new;
+                    s[b][h] = exp2f((s[b][h] - m_use) * scale_log2);
+                    s[b][2 + h] = exp2f((s[b][2 + h] - m_use) * scale_log2);
+                    l_run[b][h] = l_run[b][h] * alpha[h] + (s[b][h] + s[b][2 + h]);
+                }
+                pf[b][0] = transposed(pack_bf16(s[b][0], s[b][1]));
+                pf[b][1] = transposed(pack_bf16(s[b][2], s[b][3]));
+#pragma unroll
+                for (int i = 0; i < KSTEPS; ++i) {
+                    o[b][i][0] *= alpha[0]; o[b][i][1] *= alpha[1];
+                    o[b][i][2] *= alpha[0]; o[b][i][3] *= alpha[1];
                 }
             }
 #pragma unroll
-            for (int j = 0; j < NT; ++j) {
+            for (int i = 0; i < KSTEPS; ++i) {
+                uint32_t va[4];
+                ldmatrix_x4_trans(swz(v_s, KT, kr + 8 * (lane >> 4), i * 16 + 8 * ((lane >> 3) & 1)), va[0], va[1], va[2], va[3]);
 #pragma unroll
-                for (int x = 0; x < 4; ++x) s[j][x] += s2[j][x];
-            }
-            float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    const int kp = t0 + key0 + j * 8 + (lane & 3) * 2 + (x & 1);
-                    const bool valid = kp >= kv_begin && kp < kv_stop;      // causal and window limits are the split's
-                    s[j][x] = valid ? s[j][x] : -INFINITY;
-                    mx[x >> 1] = fmaxf(mx[x >> 1], s[j][x]);
-                }
-            }
-            float alpha[2], m_use[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-                mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-                const float m_new = fmaxf(m_run[h], mx[h]);
-                m_use[h] = m_new == -INFINITY ? 0.f : m_new;
-                alpha[h] = exp2f((m_run[h] - m_use[h]) * scale_log2);
-                m_run[h] = m_new;
-                l_run[h] *= alpha[h];
-            }
-            uint32_t pf[NT / 2][4];
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                float p[4];
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    p[x] = exp2f((s[j][x] - m_use[x >> 1]) * scale_log2);
-                    l_run[x >> 1] += p[x];
-                }
-                pf[j >> 1][(j & 1) * 2 + 0] = pack_bf16(p[0], p[1]);
-                pf[j >> 1][(j & 1) * 2 + 1] = pack_bf16(p[2], p[3]);
-            }
-#pragma unroll
-            for (int i = 0; i < DTILES; ++i) {
-                o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
-                o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
-            }
-#pragma unroll
-            for (int i = 0; i < DTILES; i += 2) {
-                uint32_t b0, b1, b2, b3;
-                const int r = key0 + (lane & 7) + 8 * ((lane >> 3) & 1), c = i * 8 + 8 * (lane >> 4);
-                ldmatrix_x4_trans(swz(v_s, KT, r, c), b0, b1, b2, b3);
-                mma_bf16(o[i], pf[0], b0, b1);
-                mma_bf16(o[i + 1], pf[0], b2, b3);
+                for (int b = 0; b < NB; ++b) mma_bf16(o[b][i], va, pf[b][0], pf[b][1]);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(empty_bar(stage));     // this warp is done with the stage
@@ -431,10 +421,13 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const Decode
         }
 
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
-            l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
-        }
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                l_run[b][h] += __shfl_xor_sync(0xffffffffu, l_run[b][h], 4);
+                l_run[b][h] += __shfl_xor_sync(0xffffffffu, l_run[b][h], 8);
+                l_run[b][h] += __shfl_xor_sync(0xffffffffu, l_run[b][h], 16);
+            }
         // the four warps' parts meet in the ring (every tile has been consumed; if a wait ran out the
         // TMA warp waits for its armed copies itself and nothing below is stored to global memory)
         compute_sync();
@@ -442,14 +435,18 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const Decode
         float* mg = (float*)(smem + L::Q_BYTES);
         if (ok) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int r = (lane >> 2) + 8 * h;
-                float* dst = mg + (warp * ROWS + r) * MS;
+            for (int b = 0; b < NB; ++b)
 #pragma unroll
-                for (int i = 0; i < DTILES; ++i)
-                    *(float2*)(dst + i * 8 + (lane & 3) * 2) = make_float2(o[i][2 * h + 0], o[i][2 * h + 1]);
-                if ((lane & 3) == 0) *(float2*)(dst + D) = make_float2(m_run[h], l_run[h]);
-            }
+                for (int h = 0; h < 2; ++h) {
+                    const int r = 8 * b + 2 * (lane & 3) + h;
+                    float* dst = mg + (warp * ROWS + r) * MS;
+#pragma unroll
+                    for (int i = 0; i < KSTEPS; ++i) {
+                        dst[16 * i + (lane >> 2)] = o[b][i][h];
+                        dst[16 * i + (lane >> 2) + 8] = o[b][i][2 + h];
+                    }
+                    if (lane < 4) *(float2*)(dst + D) = make_float2(m_run[b][h], l_run[b][h]);
+                }
         }
         compute_sync();
         // four columns of a row per thread and turn: the row's weights are worked out once per turn
@@ -527,9 +524,9 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap kv_map, const Decode
     // no second barrier: after the one above nobody touches another CTA's shared memory
 }
 
-template <int D>
+template <int D, int NB>
 int configure() {
-    auto kern = attention_decode_kernel<D>;
+    auto kern = attention_decode_kernel<D, NB>;
     constexpr int smem = Layout<D>::TOTAL;
     static bool configured = false;
     if (!configured) {
@@ -547,7 +544,7 @@ int configure() {
 // cluster share a GPC, so this is not the number of CTA slots divided by nsplit).
 template <int D>
 int max_clusters(int nsplit) {
-    int rc = configure<D>();
+    int rc = configure<D, 1>();
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nsplit, 1);
@@ -561,16 +558,16 @@ int max_clusters(int nsplit) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    cudaError_t e = cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel<D>, &cfg);
+    cudaError_t e = cudaOccupancyMaxActiveClusters(&n, attention_decode_kernel<D, 1>, &cfg);
     if (e != cudaSuccess) return fail("attention_decode: clusters of %d: %s", nsplit, cudaGetErrorString(e));
     return n;
 }
 
-template <int D>
+template <int D, int NB>
 int launch(const CUtensorMap& map, const DecodeArgs& a, cudaStream_t stream) {
-    auto kern = attention_decode_kernel<D>;
+    auto kern = attention_decode_kernel<D, NB>;
     constexpr int smem = Layout<D>::TOTAL;
-    int rc = configure<D>();
+    int rc = configure<D, NB>();
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.T * a.ngroups * a.nsplit, a.nkv);
@@ -638,5 +635,6 @@ MHB_EXPORT int mhb_attention_decode(const float* qkv, int qkv_nsplit, long long 
     a.qkv_nsplit = qkv_nsplit; a.rdim = rotary_dim; a.interleaved = interleaved ? 1 : 0; a.T = T; a.width = width;
     a.nq = nq; a.nkv = nkv; a.P = P; a.num_pages = num_pages; a.window = window; a.nsplit = nsplit; a.scale = scale;
     a.ngroups = ngroups; a.part_acc = part_acc; a.part_ml = part_ml;
-    return d == 128 ? launch<128>(map, a, stream) : launch<64>(map, a, stream);
+    if (nq / nkv <= 8) return d == 128 ? launch<128, 1>(map, a, stream) : launch<64, 1>(map, a, stream);
+    return d == 128 ? launch<128, 2>(map, a, stream) : launch<64, 2>(map, a, stream);
 }

@@ -232,9 +232,12 @@ class AttentionPlanner(StepPlanner):
     """The plan of grouped-query attention for the step function: work items, and for every token
     the first of its partial rows and the number of its key splits."""
 
-    def __init__(self, shape: AttentionShape, sm_count: int, clusters_of=None, max_cluster: int = 0):
+    def __init__(self, shape: AttentionShape, sm_count: int, clusters_of=None, max_cluster: int = 0,
+                 min_share: int = MIN_KEYS_PER_SPLIT):
         """``clusters_of(n)``: how many clusters of n CTAs the mixer's decode kernel can run at once, if
-        it merges a token's key splits inside a cluster of up to ``max_cluster`` CTAs (None: it does not)."""
+        it merges a token's key splits inside a cluster of up to ``max_cluster`` CTAs (None: it does not).
+        ``min_share``: keys that a share of a cluster has at least."""
+        self.min_share = min_share
         self.shape, self.sm_count = shape, sm_count
         self.clusters_of, self.max_cluster = clusters_of, max_cluster
         self._uneven = {}        # decode_fixed_for's answers
@@ -282,7 +285,9 @@ class AttentionPlanner(StepPlanner):
         ctas = segments_count * self.shape.kv_heads * self.chunks
         if self.shape.window:            # a token never attends to more keys than its window holds
             max_positions = min(max_positions, self.shape.window)
-        n = max(1, min(MAX_SPLITS, (2 * self.sm_count) // ctas, self.shape.max_splits(max_positions)))
+        plain = n = max(1, min(MAX_SPLITS, (2 * self.sm_count) // ctas, self.shape.max_splits(max_positions)))
+        if self.clusters_of is not None and self.chunks == 1:
+            n = max(n, min((2 * self.sm_count) // ctas, self.max_cluster, max_positions // self.min_share))
         if self.clusters_of is None or self.chunks != 1 or n == 1:
             return n, 1
         # The shares of a cluster are merged in its shared memory, and a cluster is placed inside one
@@ -321,7 +326,7 @@ class AttentionPlanner(StepPlanner):
                     if cost(c, g) < best_cost:
                         best, best_cost = (c, g), cost(c, g)
         # no cluster fits: the shares go through the kernels that merge through global memory
-        return best if best is not None else (n, 1)
+        return best if best is not None else (plain, 1)
 
     UNEVEN_CANDIDATES = (2, 3, 4, 6, 8, 12, 16)
 
@@ -441,8 +446,9 @@ class GQAttention(Mixer):
     def planner(self, page_size: int, sm_count: int):
         shape = AttentionShape(self.nq, self.nkv, self.window, self.big_tile_rows(page_size))
         if self.kernel_family(page_size) == "tc" and self.nq // self.nkv <= ROW_TILE:
+            # a cluster's merge pays for shares of two key tiles
             return AttentionPlanner(shape, sm_count, lambda n: K.attention_decode_max_clusters(self.d, n),
-                                    K.DECODE_MAX_SPLITS)
+                                    K.DECODE_MAX_SPLITS, min_share=2 * KEY_TILE)
         return AttentionPlanner(shape, sm_count)
 
     def parameters(self):
