@@ -7,10 +7,11 @@
 // In a decode step these are five launches (norm, product, gate, product, norm) of 2.3 to 3 us each that hardly move any
 // bytes: what they cost is handing over.  Here a cluster of 8 CTAs holds the rows of TB tokens, an eighth of the columns
 // each.  Both weights' parts of a CTA (Wg: D rows of its columns; Wp: the rows of its columns) and the table's rows are
-// fetched while the kernel before this one still runs; the three sums that need whole rows (two norms, z) cross the
+// fetched while the kernel before this one still runs, into REGISTERS: that kernel is a product whose two CTAs leave an SM
+// 7 KB of shared memory, and a CTA that needs more cannot start before they are gone (with the weights in shared memory
+// a launch took 11.5 us of the step instead of 7.6).  The three sums that need whole rows (two norms, z) cross the
 // cluster through distributed shared memory, every CTA adding the eight parts in rank order.
-// 24 decode steps of 8 requests through 8 layers 2,048 wide took 13.19 ms instead of 14.01: 4.3 us a layer less.  (One CTA per
-// token walked 1 MB of weights at its loads' latency: 47 us.)
+// (One CTA per token walked 1 MB of weights at its loads' latency: 47 us.)
 //
 // Precision is that of the five kernels: float32 sums, x1 and g rounded to bfloat16 where they enter a product.
 #include "common.cuh"
@@ -91,24 +92,23 @@ __device__ __forceinline__ float warp_sum8(float (&v)[8], int lane) {
     return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-// Shared memory: [gate D x S][proj S x (D + 8)] bfloat16, then floats [rows TB x S][second TB x S][e TB x D][g TB x D]
-// [z parts CLUSTER x TB x D][two sums CLUSTER x TB][warp sums TB x 32]
-template <int TB>
-size_t smem_bytes(int S, int D) {
-    return 2 * ((size_t)D * S + (size_t)S * (D + 8)) +
-           4 * ((size_t)2 * TB * S + 2 * TB * D + CLUSTER * TB * D + 2 * CLUSTER * TB + 32 * TB);
+// Shared memory, floats: [rows TB x S][second TB x S][e TB x D][g TB x D][z parts CLUSTER x TB x D][two sums CLUSTER x TB]
+// [warp sums TB x 32]
+size_t smem_bytes(int TB, int S, int D) {
+    return 4 * ((size_t)2 * TB * S + 2 * TB * D + CLUSTER * TB * D + 2 * CLUSTER * TB + 32 * TB);
 }
+__device__ __forceinline__ float low(uint32_t u) { return __uint_as_float(u << 16); }
+__device__ __forceinline__ float high(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
 
-template <int TB>
+// CH: a CTA's columns are CH runs of 128
+template <int TB, int CH>
 __global__ void __launch_bounds__(THREADS)
 side_branch_kernel(const SideArgs a) {
-    extern __shared__ __align__(16) uint8_t smem[];
-    const int W = a.W, D = a.D, S = W / CLUSTER, LP = D + 8;
+    extern __shared__ __align__(16) float rows[];      // alpha x + delta, then x1
+    constexpr int S = CH * 128, CP = (S + THREADS - 1) / THREADS;
+    const int W = a.W, D = a.D;
     const int rank = (int)cluster_rank(), t0 = ((int)blockIdx.x / CLUSTER) * TB, col0 = rank * S;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    __nv_bfloat16* wg = (__nv_bfloat16*)smem;
-    __nv_bfloat16* wp = wg + D * S;
-    float* rows = (float*)(wp + S * LP);          // alpha x + delta, then x1
     float* second = rows + TB * S;                // x1 rounded, then y
     float* es = second + TB * S;
     float* gs = es + TB * D;
@@ -118,16 +118,20 @@ side_branch_kernel(const SideArgs a) {
     float* wsum = sum2 + CLUSTER * TB;            // [TB][32]
 
     pdl_launch_dependents();
-    // constant: the weights' parts and the table's rows
-    for (int i = tid; i < D * (S / 8); i += THREADS) {
-        const int j = i / (S / 8), c = (i - j * (S / 8)) * 8;
-        cp_async16((uint32_t)__cvta_generic_to_shared(wg + j * S + c), a.gate + (size_t)j * W + col0 + c, 16);
-    }
-    for (int i = tid; i < S * (D / 8); i += THREADS) {
-        const int c = i / (D / 8), j = (i - c * (D / 8)) * 8;
-        cp_async16((uint32_t)__cvta_generic_to_shared(wp + c * LP + j), a.proj + (size_t)(col0 + c) * D + j, 16);
-    }
-    cp_async_commit();
+    // constant: this warp's eight rows of the gate weight (four columns a lane and run), this thread's rows of the projection
+    uint2 wg[8][CH];
+    uint4 wp[CP][8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int k = 0; k < CH; ++k)
+            wg[j][k] = 8 * warp < D ? __ldg((const uint2*)(a.gate + (size_t)(8 * warp + j) * W + col0 + k * 128 + 4 * lane)) : make_uint2(0, 0);
+#pragma unroll
+    for (int i = 0; i < CP; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            wp[i][j] = 8 * j < D && tid + i * THREADS < S ? __ldg((const uint4*)(a.proj + (size_t)(col0 + tid + i * THREADS) * D + 8 * j))
+                                                           : make_uint4(0, 0, 0, 0);
     bool outside = false;
     for (int i = tid; i < TB * D; i += THREADS) {
         const int tb = i / D, j = i - tb * D;
@@ -144,7 +148,7 @@ side_branch_kernel(const SideArgs a) {
     if (outside && rank == 0 && a.status) atomicOr(a.status, 1);
 
     // ---- s and its squares: a warp takes 128 columns of one token at a time
-    const int chunks = S / 128;
+    constexpr int chunks = CH;
     for (int u = warp; u < TB * chunks; u += WARPS) {
         const int tb = u / chunks, c = (u - tb * chunks) * 128 + 4 * lane;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -165,8 +169,7 @@ side_branch_kernel(const SideArgs a) {
         for (int i = 0; i < chunks; ++i) ss += wsum[tb * 32 + i];
         st_peer(sum1 + rank * TB + tb, peer, ss);
     }
-    cp_async_wait<0>();
-    cluster_sync();            // (also the CTA's barrier for the weights)
+    cluster_sync();
     for (int u = warp; u < TB * chunks; u += WARPS) {
         const int tb = u / chunks, c = (u - tb * chunks) * 128 + 4 * lane;
         float total = 0.f;
@@ -183,30 +186,30 @@ side_branch_kernel(const SideArgs a) {
     }
     __syncthreads();
 
-    // ---- this CTA's part of z: a warp takes eight rows of the gate weight at a time
-    for (int jb = warp; jb < D / 8; jb += WARPS) {
+    // ---- this CTA's part of z: a warp takes eight rows of the gate weight
+    if (8 * warp < D) {
         float acc[TB][8];
 #pragma unroll
         for (int tb = 0; tb < TB; ++tb)
 #pragma unroll
             for (int j = 0; j < 8; ++j) acc[tb][j] = 0.f;
-        for (int k = 0; k < chunks; ++k) {
-            const int c = k * 128 + 4 * lane;
+#pragma unroll
+        for (int k = 0; k < CH; ++k) {
             float4 h[TB];
 #pragma unroll
-            for (int tb = 0; tb < TB; ++tb) h[tb] = vec4(second + tb * S + c);
+            for (int tb = 0; tb < TB; ++tb) h[tb] = vec4(second + tb * S + k * 128 + 4 * lane);
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const float4 w = vec4(wg + (jb * 8 + j) * S + c);
+                const uint2 w = wg[j][k];
 #pragma unroll
                 for (int tb = 0; tb < TB; ++tb)
-                    acc[tb][j] = fmaf(h[tb].w, w.w, fmaf(h[tb].z, w.z, fmaf(h[tb].y, w.y, fmaf(h[tb].x, w.x, acc[tb][j]))));
+                    acc[tb][j] = fmaf(h[tb].w, high(w.y), fmaf(h[tb].z, low(w.y), fmaf(h[tb].y, high(w.x), fmaf(h[tb].x, low(w.x), acc[tb][j]))));
             }
         }
 #pragma unroll
         for (int tb = 0; tb < TB; ++tb) {
             const float z = warp_sum8(acc[tb], lane);
-            float* slot = zp + (rank * TB + tb) * D + jb * 8 + (lane >> 2);
+            float* slot = zp + (rank * TB + tb) * D + warp * 8 + (lane >> 2);
             st_peer(slot, 2 * (lane & 3), z);
             st_peer(slot, 2 * (lane & 3) + 1, z);
         }
@@ -224,17 +227,22 @@ side_branch_kernel(const SideArgs a) {
     float ss[TB];
 #pragma unroll
     for (int tb = 0; tb < TB; ++tb) ss[tb] = 0.f;
-    for (int c = tid; c < S; c += THREADS) {
+#pragma unroll
+    for (int i = 0; i < CP; ++i) {
+        const int c = tid + i * THREADS;
+        if (c >= S) break;
         float y[TB];
 #pragma unroll
         for (int tb = 0; tb < TB; ++tb) y[tb] = 0.f;
-        for (int j = 0; j < D; j += 8) {
-            const float4 w0 = vec4(wp + c * LP + j), w1 = vec4(wp + c * LP + j + 4);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (8 * j >= D) break;
+            const uint4 w = wp[i][j];
 #pragma unroll
             for (int tb = 0; tb < TB; ++tb) {
-                const float4 g0 = vec4(gs + tb * D + j), g1 = vec4(gs + tb * D + j + 4);
-                y[tb] = fmaf(w0.w, g0.w, fmaf(w0.z, g0.z, fmaf(w0.y, g0.y, fmaf(w0.x, g0.x, y[tb]))));
-                y[tb] = fmaf(w1.w, g1.w, fmaf(w1.z, g1.z, fmaf(w1.y, g1.y, fmaf(w1.x, g1.x, y[tb]))));
+                const float4 g0 = vec4(gs + tb * D + 8 * j), g1 = vec4(gs + tb * D + 8 * j + 4);
+                y[tb] = fmaf(high(w.y), g0.w, fmaf(low(w.y), g0.z, fmaf(high(w.x), g0.y, fmaf(low(w.x), g0.x, y[tb]))));
+                y[tb] = fmaf(high(w.w), g1.w, fmaf(low(w.w), g1.z, fmaf(high(w.z), g1.y, fmaf(low(w.z), g1.x, y[tb]))));
             }
         }
 #pragma unroll
@@ -270,17 +278,15 @@ side_branch_kernel(const SideArgs a) {
     }
 }
 
-// Tokens a cluster: one while 16 clusters (128 CTAs) take them all, up to four.
-int tokens_per_cluster(int T) { return T <= 16 ? 1 : T <= 32 ? 2 : 4; }
+// Tokens a cluster: one while 16 clusters (128 CTAs) take them all, up to four.  Beyond 2,048 columns an SM's registers hold
+// one CTA and 8 clusters are what runs at once (16 tokens of 4,096: 13.8 us with 16 clusters, 8.3 with 8).
+int most_clusters(int W) { return W > 2048 ? 8 : 16; }
+int tokens_per_cluster(int T, int W) { return T <= most_clusters(W) ? 1 : T <= 2 * most_clusters(W) ? 2 : 4; }
 
-template <int TB>
+template <int TB, int CH>
 int launch(const SideArgs& a, cudaStream_t stream) {
-    auto kern = side_branch_kernel<TB>;
-    const size_t smem = smem_bytes<TB>(a.W / CLUSTER, a.D);
-    if (smem > 47 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail("side_branch: shared memory %zu: %s", smem, cudaGetErrorString(e));
-    }
+    auto kern = side_branch_kernel<TB, CH>;
+    const size_t smem = smem_bytes(TB, a.W / CLUSTER, a.D);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(CLUSTER * ((a.T + TB - 1) / TB));
     cfg.blockDim = dim3(THREADS);
@@ -301,11 +307,19 @@ int launch(const SideArgs& a, cudaStream_t stream) {
 }
 }  // namespace
 
-// Widths in steps of 1024 (an eighth is whole warps' 128 columns), up to 64 tokens, D in steps of 8, all of it in a CTA's
-// shared memory.
+// Widths of 1024 to 4096 in steps of 1024 (an eighth is whole warps' 128 columns), up to 64 tokens (32 beyond 2,048), D in steps of 8 up to 64
+// (eight warps' eight rows): what a CTA's registers hold.
 MHB_EXPORT int mhb_side_branch_supports(int T, int W, int D) {
-    return T >= 1 && T <= 64 && W >= 1024 && W % 1024 == 0 && D >= 8 && D % 8 == 0 &&
-           (T <= 16 ? smem_bytes<1>(W / CLUSTER, D) : T <= 32 ? smem_bytes<2>(W / CLUSTER, D) : smem_bytes<4>(W / CLUSTER, D)) <= 220 * 1024;
+    return T >= 1 && W >= 1024 && W <= 4096 && T <= 4 * most_clusters(W) && W % 1024 == 0 && D >= 8 && D <= 64 && D % 8 == 0;
+}
+
+template <int CH>
+static int by_tokens(const SideArgs& a, cudaStream_t stream) {
+    switch (tokens_per_cluster(a.T, a.W)) {
+        case 1: return launch<1, CH>(a, stream);
+        case 2: return launch<2, CH>(a, stream);
+        default: return launch<4, CH>(a, stream);
+    }
 }
 
 MHB_EXPORT int mhb_side_branch(float* x, const float* delta, int nsplit, long long split_stride, const float* w1, float eps1,
@@ -322,9 +336,10 @@ MHB_EXPORT int mhb_side_branch(float* x, const float* delta, int nsplit, long lo
     a.alpha = alpha; a.keep = keep; a.gate = (const __nv_bfloat16*)gate; a.proj = (const __nv_bfloat16*)proj;
     a.table = (const __nv_bfloat16*)table; a.table_width = table_width; a.column0 = column0; a.vocab = vocab;
     a.tokens = tokens; a.w2 = w2; a.eps2 = eps2; a.copy = (__nv_bfloat16*)copy; a.status = status; a.T = T; a.W = W; a.D = D;
-    switch (tokens_per_cluster(T)) {
-        case 1: return launch<1>(a, stream);
-        case 2: return launch<2>(a, stream);
-        default: return launch<4>(a, stream);
+    switch (W / 1024) {
+        case 1: return by_tokens<1>(a, stream);
+        case 2: return by_tokens<2>(a, stream);
+        case 3: return by_tokens<3>(a, stream);
+        default: return by_tokens<4>(a, stream);
     }
 }

@@ -146,7 +146,7 @@ class TokenSide(FeedForward):
 
     def forward_behind(self, norm, x, delta: Product, ctx: StepContext, alpha: float, keep: float):
         """The post-norm ``norm`` and this branch in one kernel: x <- x1 + branch(x1) with x1 = keep x + norm(alpha x + delta).
-        Returns the new rows in the compute dtype, or None where the kernel is not built for the step (more than 64
+        Returns the new rows in the compute dtype, or None where the kernel is not built for the step (more than 32 or 64
         tokens, float32, odd widths): then nothing has been done."""
         rt = ctx.rt
         if (rt.dtype != torch.bfloat16 or delta is None or delta.also is not None or delta.tensor.dtype != torch.float32
