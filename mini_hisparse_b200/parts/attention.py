@@ -8,7 +8,7 @@ import numpy as np
 import torch
 
 from ..kernels import api as K
-from .base import CacheView, Mixer, Product, StepContext, StepPlanner
+from .base import CacheView, Mixer, Product, StepContext, StepPlanner, join_branch
 from .registry import POSITIONS, register_mixer
 from .spec import PagedKVNeed, ParamSpec, PartSpec
 
@@ -559,7 +559,7 @@ class GQAttention(Mixer):
                     long_portions()
                     join.record(side)
                 short_segments()
-                main.wait_event(join)
+                join_branch(main, join, ws)
             else:
                 if n_small:
                     short_segments()

@@ -119,6 +119,16 @@ class Workspace:
         return sum(b.numel() for b in self._buffers.values())
 
 
+def join_branch(main, done, ws: Workspace) -> None:
+    """The main stream waits for a second stream's event ``done``, and its next kernel starts only when BOTH streams have
+    finished.  Every kernel of a step may start before the one in front of it has finished (csrc/common.cuh); behind a join
+    there are two in front, one of each stream.  Should one of them be enough, the kernels behind the join could take every
+    SM's shared memory while they wait for a kernel of the other stream that still has CTAs to place.  Something that
+    is no kernel stands in between, so there is no early start across a join (1.5 us each)."""
+    main.wait_event(done)
+    ws.get("join", (1,), torch.int32).zero_()
+
+
 class Runtime:
     """Device, compute dtype and the matrix product for that dtype."""
 

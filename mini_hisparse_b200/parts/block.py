@@ -4,7 +4,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .base import Block, CacheView, Product, StepContext
+from .base import Block, CacheView, Product, StepContext, join_branch
 from .feed_forward import TokenSide
 from .norm import RMSNorm
 from .registry import FEED_FORWARDS, GATES, INPUT_CONVS, MIXERS, NORMS, register_block
@@ -158,7 +158,7 @@ class ParallelBlock(Block):
             f = self.feed_forward.forward(h, ctx)
             join.record(branch)
         a = self.mixer.forward(h, ctx, cache)
-        main.wait_event(join)
+        join_branch(main, join, ctx.ws)
         return Product(a.tensor, a.nsplit, also=f)
 
 

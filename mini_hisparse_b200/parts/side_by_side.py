@@ -4,7 +4,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .base import CacheView, Mixer, Product, StepContext
+from .base import CacheView, Mixer, Product, StepContext, join_branch
 from .multimap_attention import _pad_rows
 from .registry import MIXERS, register_mixer
 from .spec import PartSpec
@@ -99,5 +99,5 @@ class SideBySide(Mixer):
             b = self.right.forward_projected(proj, self.col, ctx, right_view, "mix_out_right")
             join.record(branch)
         a = self.left.forward_projected(proj, 0, ctx, left_view, "mix_out")
-        main.wait_event(join)
+        join_branch(main, join, ctx.ws)
         return Product(a.tensor, a.nsplit, also=b)
