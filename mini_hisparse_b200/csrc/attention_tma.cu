@@ -12,6 +12,12 @@
 // ring stays full while they work, which is what a decode step needs: it is bound by how many
 // bytes are in flight.  ldmatrix reads the swizzled tiles without bank conflicts.
 //
+// A step of decoded tokens alone can have the splits of a token and KV head merged in a thread-block cluster instead
+// (AttnArgs::cluster): every CTA sends its rows to the CTA that owns them (CTA r the rows r, r + cluster, ...) through
+// distributed shared memory, and each owner merges in split order.  A merge through global memory (partials, a fence, a
+// counter, the last CTA's loads) costs as much as 200 keys, so shares were 256 keys long at least and 8 requests of 300
+// keys ran on 32 of 148 SMs; the cluster's merge pays for shares of 64.
+//
 // Needs head_dim 64 or 128 and a page size that divides 64; other shapes use attention_mma.cu or
 // attention_simt.cu.  Every mbarrier wait is bounded (status bit 8 when one runs out).
 #include "mma_helpers.cuh"
@@ -54,13 +60,10 @@ struct AttnArgs {
     int shared_kv;              // a latent cache: the pool is [pages][P][d] rows (one KV head), a row is key AND value
     float softcap;              // s <- softcap * tanh(s / softcap) on the scaled score (0: none)
     int out_f32;                // `out` is float32 (a sum of the outputs is still to be taken in 32 bits)
+    int cluster;                // > 1: blockIdx.x = token * cluster + split, and a cluster of that many CTAs merges them
+    int gate_vec;               // the gate's columns can be read four at a time
     const float* slopes;        // [nq] or null: slope_h * (query position - key position) is taken off the scaled score
 };
-
-__device__ __forceinline__ void store_out(const AttnArgs& a, size_t idx, float v) {
-    if (a.out_f32) ((float*)a.out)[idx] = v;
-    else a.out[idx] = __float2bfloat16_rn(v);
-}
 
 __device__ __forceinline__ float gate_of(const AttnArgs& a, int t, int col) {
     if (!a.gate) return 1.f;
@@ -68,17 +71,54 @@ __device__ __forceinline__ float gate_of(const AttnArgs& a, int t, int col) {
     return 1.f / (1.f + expf(-sum_parts(a.gate + idx, a.gate_nsplit, a.gate_split_stride)));
 }
 
+// four neighbouring columns of a gate (or one head's, four times)
+__device__ __forceinline__ float4 gate4_of(const AttnArgs& a, int t, int hq, int D, int e) {
+    if (!a.gate) return make_float4(1.f, 1.f, 1.f, 1.f);
+    if (a.gate_per_head) {
+        const float g = gate_of(a, t, hq);
+        return make_float4(g, g, g, g);
+    }
+    const int col = hq * D + e;
+    if (!a.gate_vec) {
+        float g[4];
+#pragma unroll 1
+        for (int i = 0; i < 4; ++i) g[i] = gate_of(a, t, col + i);
+        return make_float4(g[0], g[1], g[2], g[3]);
+    }
+    float4 z = sum_parts4<8>(a.gate + (size_t)t * a.gate_ld + col, a.gate_nsplit, a.gate_split_stride);
+    z.x = 1.f / (1.f + expf(-z.x)); z.y = 1.f / (1.f + expf(-z.y)); z.z = 1.f / (1.f + expf(-z.z)); z.w = 1.f / (1.f + expf(-z.w));
+    return z;
+}
+__device__ __forceinline__ void store4_out(const AttnArgs& a, size_t idx, float4 v) {
+    if (a.out_f32) *(float4*)((float*)a.out + idx) = v;
+    else *(uint2*)(a.out + idx) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+}
+__device__ __forceinline__ float4 times(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
+__device__ __forceinline__ float4 over(float4 acc, float lsum) {
+    return lsum > 0.f ? make_float4(acc.x / lsum, acc.y / lsum, acc.z / lsum, acc.w / lsum) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 template <int D, int ROWS>
 struct Layout {
     static constexpr int HALVES = D / 64;
-    static constexpr int STAGES = ROWS == 16 ? 3 : 2;
+    static constexpr int STAGES = 3;
     static constexpr int Q_BYTES = ROWS * D * 2;            // [HALVES][ROWS][128 B], swizzled
     static constexpr int KV_BYTES = KT * D * 2;             // K or V of one stage: [HALVES][64][128 B]
     static constexpr int STAGE_BYTES = 2 * KV_BYTES;
     static constexpr int BAR_OFFSET = Q_BYTES + STAGES * STAGE_BYTES;
     static constexpr int LOOP_BYTES = BAR_OFFSET + 2 * STAGES * 8;
-    static constexpr int MERGE_BYTES = ROWS == 16 ? CWARPS * 16 * (D + 2) * 4 : 0;
-    static constexpr int TOTAL = (LOOP_BYTES > MERGE_BYTES ? LOOP_BYTES : MERGE_BYTES) + 1024;
+    static constexpr int MS = D + 4;                        // a partial row: accumulator, maximum, sum (16-byte rows)
+    static constexpr int MERGE_BYTES = CWARPS * 16 * MS * 4;
+    static constexpr int RECV_ROWS = 17;                    // splits x rows a cluster's CTA owns, and the gates of these
+    static constexpr int RECV_OFFSET = ((LOOP_BYTES > MERGE_BYTES ? LOOP_BYTES : MERGE_BYTES) + 15) / 16 * 16;
+    static constexpr int TOTAL = RECV_OFFSET + RECV_ROWS * MS * 4 + 1024;
 };
 
 // Address of element (row r, column e) of a tile stored as halves of 64 columns, rows of 128 bytes,
@@ -97,9 +137,7 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
     using L = Layout<D, ROWS>;
     constexpr int STAGES = L::STAGES;
     constexpr int KSTEPS = D / 16;
-    constexpr int DTILES = D / 8;
-    constexpr bool SPLIT_KEYS = ROWS == 16;
-    constexpr int NT = SPLIT_KEYS ? 2 : 8;
+    static_assert(ROWS == 16, "two blocks of 8 query rows");
     extern __shared__ uint8_t smem_raw[];
     __shared__ int row_pos[ROWS];
     __shared__ int cta_failed;      // a bounded wait ran out somewhere in this CTA: it merges and stores nothing
@@ -134,6 +172,8 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
         cta_failed = 0;
     }
     __syncthreads();
+    const bool clustered = EXT && a.cluster > 1;
+    if (clustered) cluster_arrive();        // this CTA runs: its shared memory may be written
 
     if (warp == CWARPS) {
         // ---- TMA warp: one lane per page of the tile ----------------------------------------------
@@ -184,6 +224,12 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
             for (int i = max(0, armed - STAGES); i < armed; ++i) mbar_wait(full_bar(i % STAGES), (i / STAGES) & 1);
             if (a.status) atomicOr(a.status, 8);
         }
+        if (clustered) {                // the two meetings of the compute warps' merge
+            __syncwarp();
+            cluster_wait();
+            cluster_arrive();
+            cluster_wait();
+        }
         return;
     }
 
@@ -198,39 +244,58 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
         cp_async16(swz(q_s, ROWS, r, ch * 8), src, live ? 16 : 0);
     }
     cp_async_commit();
-    cp_async_wait<0>();
-    compute_sync();
-
-    const int wrow = SPLIT_KEYS ? 0 : warp * 16;
-    float o[DTILES][4];
-#pragma unroll
-    for (int i = 0; i < DTILES; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
-    float slope[2] = {0.f, 0.f};          // in the raw products' units
+    // The rows that this CTA will write, four columns a thread and turn, and their gates: asked for while the queries come
+    // (at the end, each of these was a round trip to the L2 that the whole launch waited for).
+    const int rank = clustered ? split : 0, nranks = clustered ? a.cluster : 1;
+    const int own_rows = nrows > rank ? (nrows - rank + nranks - 1) / nranks : 0;
+    const int owned = (nrows + nranks - 1) / nranks;
+    float* recv = (float*)(smem + L::RECV_OFFSET);          // [split][row this CTA owns][MS], then the gates of these rows
+    float* gates = recv + (clustered ? nranks * owned * L::MS : 0);
     if constexpr (EXT) {
-        if (a.slopes) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int row = wrow + (lane >> 2) + 8 * h;
-                if (row < nrows) slope[h] = a.slopes[kvh * groups + head0 + row % nheads] / a.scale;
-            }
-        }
-        if (a.sink && split <= 0 && (!SPLIT_KEYS || warp == 0)) {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int row = wrow + (lane >> 2) + 8 * h;
-                if (row < nrows) {
-                    m_run[h] = a.sink[kvh * groups + head0 + row % nheads] / a.scale;
-                    l_run[h] = (lane & 3) == 0 ? 1.f : 0.f;
-                }
+        if (a.gate && (split < 0 || clustered)) {
+#pragma unroll 1
+            for (int idx = tid; idx < own_rows * (D / 4); idx += CWARPS * 32) {
+                const int l = idx / (D / 4), e = (idx - l * (D / 4)) * 4, row = rank + l * nranks;
+                *(float4*)(gates + l * L::MS + e) = gate4_of(a, tok0 + row / nheads, kvh * groups + head0 + row % nheads, D, e);
             }
         }
     }
-    uint32_t qf[KSTEPS][4];
+    cp_async_wait<0>();
+    compute_sync();
+
+    // The products have the KEYS (or the head's elements) along the 16 rows of an mma and the tile's query rows along its 8
+    // columns: S^T = K Q^T, O^T = V^T P^T, in two blocks of 8 query rows.  A decoded token has 4 to 8 heads per KV head in
+    // most models: the second block is left out, which halves the mmas of a launch of decoded tokens.
+    const bool both = nrows > 8;
+    // sums of the outputs, transposed: tile i of block b holds elements 16 i + (lane >> 2) (+ 8: [2], [3]) of the query rows
+    // 8 b + 2 (lane & 3) ([0], [2]) and the one after it ([1], [3])
+    float o[2][KSTEPS][4];
+    float m_run[2][2], l_run[2][2];
+    float slope[2][2];          // in the raw products' units
+    int qp[2][2];               // the rows' positions
+    uint32_t qf[2][KSTEPS][2];
 #pragma unroll
-    for (int k = 0; k < KSTEPS; ++k) {
-        const int r = wrow + (lane & 7) + 8 * ((lane >> 3) & 1), c = k * 16 + 8 * (lane >> 4);
-        ldmatrix_x4(swz(q_s, ROWS, r, c), qf[k][0], qf[k][1], qf[k][2], qf[k][3]);
+    for (int b = 0; b < 2; ++b) {
+#pragma unroll
+        for (int i = 0; i < KSTEPS; ++i) o[b][i][0] = o[b][i][1] = o[b][i][2] = o[b][i][3] = 0.f;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int row = 8 * b + 2 * (lane & 3) + h;
+            m_run[b][h] = -INFINITY;
+            l_run[b][h] = slope[b][h] = 0.f;
+            qp[b][h] = row_pos[row];
+            if constexpr (EXT) {
+                const int hq = kvh * groups + head0 + row % nheads;
+                if (a.slopes && row < nrows) slope[b][h] = a.slopes[hq] / a.scale;
+                if (a.sink && split <= 0 && warp == 0 && row < nrows) {
+                    m_run[b][h] = a.sink[hq] / a.scale;
+                    l_run[b][h] = lane < 4 ? 1.f : 0.f;
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < KSTEPS; k += 2)
+            ldmatrix_x4(swz(q_s, ROWS, 8 * b + (lane & 7), k * 16 + 8 * (lane >> 3)), qf[b][k][0], qf[b][k][1], qf[b][k + 1][0], qf[b][k + 1][1]);
     }
     const float scale_log2 = a.scale * 1.4426950408889634f;
     bool ok = true;
@@ -241,95 +306,76 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
         if (!ok) break;
         const uint32_t k_s = kv_s + stage * L::STAGE_BYTES;
         const uint32_t v_s = k_s + L::KV_BYTES;
-        const int t0 = tile_begin + itile * KT;
-        const int key0 = SPLIT_KEYS ? warp * 16 : 0;
+        const int key0 = warp * 16, kr = key0 + (lane & 7);
+        const int kp0 = tile_begin + itile * KT + key0 + (lane >> 2);      // this lane's keys: kp0 and kp0 + 8
 
-        float s[NT][4];
+        float s[2][4];
 #pragma unroll
-        for (int j = 0; j < NT; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+        for (int b = 0; b < 2; ++b) s[b][0] = s[b][1] = s[b][2] = s[b][3] = 0.f;
 #pragma unroll
-        for (int k = 0; k < KSTEPS; k += 2) {
-#pragma unroll
-            for (int j = 0; j < NT; ++j) {
-                uint32_t b0, b1, b2, b3;
-                const int r = key0 + j * 8 + (lane & 7), c = k * 16 + 8 * (lane >> 3);
-                ldmatrix_x4(swz(k_s, KT, r, c), b0, b1, b2, b3);
-                mma_bf16(s[j], qf[k], b0, b1);
-                mma_bf16(s[j], qf[k + 1], b2, b3);
-            }
+        for (int k = 0; k < KSTEPS; ++k) {
+            uint32_t ka[4];
+            ldmatrix_x4(swz(k_s, KT, kr + 8 * ((lane >> 3) & 1), k * 16 + 8 * (lane >> 4)), ka[0], ka[1], ka[2], ka[3]);
+            mma_bf16(s[0], ka, qf[0][k][0], qf[0][k][1]);
+            if (both) mma_bf16(s[1], ka, qf[1][k][0], qf[1][k][1]);
         }
-        if constexpr (EXT) {
-            if (a.softcap > 0.f) {      // the cap works on the scaled score; the tile stays in the raw products' units
-                const float to_cap = a.scale / a.softcap, from_cap = a.softcap / a.scale;
+        uint32_t pf[2][2], pl[EXT ? 2 : 1][2];
 #pragma unroll
-                for (int j = 0; j < NT; ++j)
+        for (int b = 0; b < 2; ++b) {
+            if (b == 1 && !both) break;
+            if constexpr (EXT) {
+                if (a.softcap > 0.f) {      // the cap works on the scaled score; the tile stays in the raw products' units
+                    const float to_cap = a.scale / a.softcap, from_cap = a.softcap / a.scale;
 #pragma unroll
-                    for (int x = 0; x < 4; ++x) s[j][x] = from_cap * tanhf(s[j][x] * to_cap);
+                    for (int x = 0; x < 4; ++x) s[b][x] = from_cap * tanhf(s[b][x] * to_cap);
+                }
             }
-        }
-        float mx[2] = {-INFINITY, -INFINITY};
+            float alpha[2];
 #pragma unroll
-        for (int j = 0; j < NT; ++j) {
+            for (int h = 0; h < 2; ++h) {
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const int row = wrow + (lane >> 2) + 8 * (x >> 1);
-                const int kp = t0 + key0 + j * 8 + (lane & 3) * 2 + (x & 1);
-                const int qp = row_pos[row];
-                const bool valid = kp >= kv_begin && kp < kv_end && kp <= qp && (a.window <= 0 || kp > qp - a.window);
-                if (EXT && a.slopes) s[j][x] = fmaf(-slope[x >> 1], (float)(qp - kp), s[j][x]);
-                s[j][x] = valid ? s[j][x] : -INFINITY;
-                mx[x >> 1] = fmaxf(mx[x >> 1], s[j][x]);
+                for (int x = h; x < 4; x += 2) {
+                    const int kp = kp0 + 4 * (x & 2);
+                    const bool valid = kp >= kv_begin && kp < kv_end && kp <= qp[b][h] && (a.window <= 0 || kp > qp[b][h] - a.window);
+                    if (EXT && a.slopes) s[b][x] = fmaf(-slope[b][h], (float)(qp[b][h] - kp), s[b][x]);
+                    s[b][x] = valid ? s[b][x] : -INFINITY;
+                }
+                float mx = fmaxf(s[b][h], s[b][2 + h]);
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+                const float m_new = fmaxf(m_run[b][h], mx);
+                const float m_use = m_new == -INFINITY ? 0.f : m_new;
+                alpha[h] = exp2f((m_run[b][h] - m_use) * scale_log2);
+                m_run[b][h] = m_new;
+                s[b][h] = exp2f((s[b][h] - m_use) * scale_log2);
+                s[b][2 + h] = exp2f((s[b][2 + h] - m_use) * scale_log2);
+                l_run[b][h] = l_run[b][h] * alpha[h] + (s[b][h] + s[b][2 + h]);
             }
-        }
-        float alpha[2], m_use[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 1));
-            mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xffffffffu, mx[h], 2));
-            const float m_new = fmaxf(m_run[h], mx[h]);
-            m_use[h] = m_new == -INFINITY ? 0.f : m_new;
-            alpha[h] = exp2f((m_run[h] - m_use[h]) * scale_log2);
-            m_run[h] = m_new;
-            l_run[h] *= alpha[h];
-        }
-        uint32_t pf[NT / 2][4];
-        uint32_t pl[EXT ? NT / 2 : 1][4];
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            float p[4];
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                p[x] = exp2f((s[j][x] - m_use[x >> 1]) * scale_log2);
-                l_run[x >> 1] += p[x];
-            }
-            pf[j >> 1][(j & 1) * 2 + 0] = pack_bf16(p[0], p[1]);
-            pf[j >> 1][(j & 1) * 2 + 1] = pack_bf16(p[2], p[3]);
+            pf[b][0] = transposed(pack_bf16(s[b][0], s[b][1]));
+            pf[b][1] = transposed(pack_bf16(s[b][2], s[b][3]));
             if constexpr (EXT) {
                 float r[4];
 #pragma unroll
-                for (int x = 0; x < 4; ++x) r[x] = p[x] - __bfloat162float(__float2bfloat16_rn(p[x]));
-                pl[j >> 1][(j & 1) * 2 + 0] = pack_bf16(r[0], r[1]);
-                pl[j >> 1][(j & 1) * 2 + 1] = pack_bf16(r[2], r[3]);
+                for (int x = 0; x < 4; ++x) r[x] = s[b][x] - __bfloat162float(__float2bfloat16_rn(s[b][x]));
+                pl[b][0] = transposed(pack_bf16(r[0], r[1]));
+                pl[b][1] = transposed(pack_bf16(r[2], r[3]));
+            }
+#pragma unroll
+            for (int i = 0; i < KSTEPS; ++i) {
+                o[b][i][0] *= alpha[0]; o[b][i][1] *= alpha[1];
+                o[b][i][2] *= alpha[0]; o[b][i][3] *= alpha[1];
             }
         }
 #pragma unroll
-        for (int i = 0; i < DTILES; ++i) {
-            o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
-            o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
-        }
-#pragma unroll
-        for (int kk = 0; kk < NT / 2; ++kk) {
-#pragma unroll
-            for (int i = 0; i < DTILES; i += 2) {
-                uint32_t b0, b1, b2, b3;
-                const int r = key0 + kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1), c = i * 8 + 8 * (lane >> 4);
-                ldmatrix_x4_trans(swz(v_s, KT, r, c), b0, b1, b2, b3);
-                mma_bf16(o[i], pf[kk], b0, b1);
-                mma_bf16(o[i + 1], pf[kk], b2, b3);
-                if constexpr (EXT) {
-                    mma_bf16(o[i], pl[kk], b0, b1);
-                    mma_bf16(o[i + 1], pl[kk], b2, b3);
-                }
+        for (int i = 0; i < KSTEPS; ++i) {
+            uint32_t va[4];
+            ldmatrix_x4_trans(swz(v_s, KT, kr + 8 * (lane >> 4), i * 16 + 8 * ((lane >> 3) & 1)), va[0], va[1], va[2], va[3]);
+            mma_bf16(o[0][i], va, pf[0][0], pf[0][1]);
+            if constexpr (EXT) mma_bf16(o[0][i], va, pl[0][0], pl[0][1]);
+            if (both) {
+                mma_bf16(o[1][i], va, pf[1][0], pf[1][1]);
+                if constexpr (EXT) mma_bf16(o[1][i], va, pl[1][0], pl[1][1]);
             }
         }
         __syncwarp();
@@ -344,56 +390,102 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
     }
 
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 1);
-        l_run[h] += __shfl_xor_sync(0xffffffffu, l_run[h], 2);
-    }
-    if (SPLIT_KEYS) {
-        compute_sync();     // all warps are past their last tile: the ring can become merge scratch
-        if (cta_failed) return;
-        float* mg = (float*)smem;
-        constexpr int MS = D + 2;
+    for (int b = 0; b < 2; ++b)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int row = (lane >> 2) + 8 * h;
-            float* dst = mg + (warp * 16 + row) * MS;
+            l_run[b][h] += __shfl_xor_sync(0xffffffffu, l_run[b][h], 4);
+            l_run[b][h] += __shfl_xor_sync(0xffffffffu, l_run[b][h], 8);
+            l_run[b][h] += __shfl_xor_sync(0xffffffffu, l_run[b][h], 16);
+        }
+    {
+        compute_sync();     // all warps are past their last tile: the ring can become merge scratch
+        ok = cta_failed == 0;
+        if (!ok && !clustered) return;
+        float* mg = (float*)smem;
+        constexpr int MS = L::MS;
+        if (ok) {
 #pragma unroll
-            for (int i = 0; i < DTILES; ++i) {
-                dst[i * 8 + (lane & 3) * 2 + 0] = o[i][2 * h + 0];
-                dst[i * 8 + (lane & 3) * 2 + 1] = o[i][2 * h + 1];
-            }
-            if ((lane & 3) == 0) { dst[D] = m_run[h]; dst[D + 1] = l_run[h]; }
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float* dst = mg + (warp * 16 + 8 * b + 2 * (lane & 3) + h) * MS;
+#pragma unroll
+                    for (int i = 0; i < KSTEPS; ++i) {
+                        dst[16 * i + (lane >> 2)] = o[b][i][h];
+                        dst[16 * i + (lane >> 2) + 8] = o[b][i][2 + h];
+                    }
+                    if (lane < 4) *(float2*)(dst + D) = make_float2(m_run[b][h], l_run[b][h]);
+                }
         }
         compute_sync();
-        for (int idx = tid; idx < nrows * D; idx += CWARPS * 32) {
-            const int row = idx / D, e = idx - row * D;
+        if (clustered) cluster_wait();      // the peers run (each has arrived when it started)
+#pragma unroll 1
+        for (int idx = tid; idx < nrows * (D / 4); idx += CWARPS * 32) {
+            const int row = idx / (D / 4), e = (idx - row * (D / 4)) * 4;
+            float2 ml[CWARPS];
             float M = -INFINITY;
 #pragma unroll
-            for (int w = 0; w < CWARPS; ++w) M = fmaxf(M, mg[(w * 16 + row) * MS + D]);
-            float acc = 0.f, lsum = 0.f;
+            for (int w = 0; w < CWARPS; ++w) {
+                ml[w] = *(const float2*)(mg + (w * 16 + row) * MS + D);
+                M = fmaxf(M, ml[w].x);
+            }
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            float lsum = 0.f;
 #pragma unroll
             for (int w = 0; w < CWARPS; ++w) {
-                const float mw = mg[(w * 16 + row) * MS + D];
-                const float wgt = mw == -INFINITY ? 0.f : exp2f((mw - M) * scale_log2);
-                acc += wgt * mg[(w * 16 + row) * MS + e];
-                lsum += wgt * mg[(w * 16 + row) * MS + D + 1];
+                const float wgt = ml[w].x == -INFINITY ? 0.f : exp2f((ml[w].x - M) * scale_log2);
+                const float4 v = vec4(mg + (w * 16 + row) * MS + e);
+                acc.x += wgt * v.x; acc.y += wgt * v.y; acc.z += wgt * v.z; acc.w += wgt * v.w;
+                lsum += wgt * ml[w].y;
             }
             const int t = tok0 + row / nheads, hq = kvh * groups + head0 + row % nheads;
-            if (split < 0) {
-                float res = lsum > 0.f ? acc / lsum : 0.f;
+            if (clustered) {
+                if (!ok) { M = -INFINITY; acc = make_float4(0.f, 0.f, 0.f, 0.f); lsum = 0.f; }
+                const uint32_t dst = peer_addr(recv + (split * owned + row / nranks) * MS, row % nranks);
+                asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst + e * 4), "f"(acc.x), "f"(acc.y), "f"(acc.z), "f"(acc.w) : "memory");
+                if (e == 0) asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst + D * 4), "f"(M), "f"(lsum) : "memory");
+            } else if (split < 0) {
+                float4 res = over(acc, lsum);
                 if constexpr (EXT) {
-                    res *= gate_of(a, t, a.gate_per_head ? hq : hq * D + e);
-                    store_out(a, ((size_t)t * a.nq + hq) * D + e, res);
+                    if (a.gate) res = times(res, vec4(gates + row * MS + e));
+                    store4_out(a, ((size_t)t * a.nq + hq) * D + e, res);
                 } else {
-                    a.out[((size_t)t * a.nq + hq) * D + e] = __float2bfloat16_rn(res);
+                    *(uint2*)(a.out + ((size_t)t * a.nq + hq) * D + e) = make_uint2(pack_bf16(res.x, res.y), pack_bf16(res.z, res.w));
                 }
             } else {
                 const size_t prow = (size_t)a.tok_part_row[t] + split;
-                a.part_acc[(prow * a.nq + hq) * D + e] = acc;
-                if (e == 0) {
-                    a.part_ml[(prow * a.nq + hq) * 2 + 0] = M == -INFINITY ? -INFINITY : M * a.scale;
-                    a.part_ml[(prow * a.nq + hq) * 2 + 1] = lsum;
+                *(float4*)(a.part_acc + (prow * a.nq + hq) * D + e) = acc;
+                if (e == 0)
+                    *(float2*)(a.part_ml + (prow * a.nq + hq) * 2) = make_float2(M == -INFINITY ? -INFINITY : M * a.scale, lsum);
+            }
+        }
+        if constexpr (EXT) {
+            if (clustered) {
+                __syncwarp();
+                cluster_arrive();
+                cluster_wait();         // every part has been sent; nobody writes another CTA's shared memory behind it
+                if (!ok) return;
+#pragma unroll 1
+                for (int idx = tid; idx < own_rows * (D / 4); idx += CWARPS * 32) {
+                    const int l = idx / (D / 4), e = (idx - l * (D / 4)) * 4;
+                    const int row = rank + l * nranks;
+                    float M = -INFINITY;
+                    for (int p = 0; p < nranks; ++p) M = fmaxf(M, recv[(p * owned + l) * MS + D]);
+                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                    float lsum = 0.f;
+                    for (int p = 0; p < nranks; ++p) {          // in split order
+                        const float* src = recv + (p * owned + l) * MS;
+                        const float w = src[D] == -INFINITY ? 0.f : exp2f((src[D] - M) * scale_log2);
+                        const float4 v = vec4(src + e);
+                        acc.x += w * v.x; acc.y += w * v.y; acc.z += w * v.z; acc.w += w * v.w;
+                        lsum += w * src[D + 1];
+                    }
+                    float4 res = over(acc, lsum);
+                    if (a.gate) res = times(res, vec4(gates + l * MS + e));
+                    const int t = tok0 + row / nheads, hq = kvh * groups + head0 + row % nheads;
+                    store4_out(a, ((size_t)t * a.nq + hq) * D + e, res);
                 }
+                return;
             }
         }
         if (split >= 0 && a.counters != nullptr) {
@@ -461,13 +553,8 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
                     }
                     const float inv = inv_s[row];
                     if constexpr (EXT) {
-                        if (a.gate_per_head) {
-                            const float g = gate_of(a, t, hq);
-                            acc.x *= g; acc.y *= g; acc.z *= g; acc.w *= g;
-                        } else {
-                            acc.x *= gate_of(a, t, hq * D + e); acc.y *= gate_of(a, t, hq * D + e + 1);
-                            acc.z *= gate_of(a, t, hq * D + e + 2); acc.w *= gate_of(a, t, hq * D + e + 3);
-                        }
+                        const float4 g = gate4_of(a, t, hq, D, e);
+                        acc.x *= g.x; acc.y *= g.y; acc.z *= g.z; acc.w *= g.w;
                         if (a.out_f32) {
                             *(float4*)((float*)a.out + ((size_t)t * a.nq + hq) * D + e) =
                                 make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
@@ -481,38 +568,11 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
                 }
             }
         }
-    } else {
-        if (!ok) return;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int row = wrow + (lane >> 2) + 8 * h;
-            if (row >= nrows) continue;
-            const int t = tok0 + row / nheads, hq = kvh * groups + head0 + row % nheads;
-            if (split < 0) {
-                const float inv = l_run[h] > 0.f ? 1.f / l_run[h] : 0.f;
-                __nv_bfloat16* dst = a.out + ((size_t)t * a.nq + hq) * D + (lane & 3) * 2;
-#pragma unroll
-                for (int i = 0; i < DTILES; ++i)
-                    *(uint32_t*)(dst + i * 8) = pack_bf16(o[i][2 * h] * inv, o[i][2 * h + 1] * inv);
-            } else {
-                const size_t prow = (size_t)a.tok_part_row[t] + split;
-                float* dst = a.part_acc + (prow * a.nq + hq) * D + (lane & 3) * 2;
-#pragma unroll
-                for (int i = 0; i < DTILES; ++i) {
-                    dst[i * 8] = o[i][2 * h];
-                    dst[i * 8 + 1] = o[i][2 * h + 1];
-                }
-                if ((lane & 3) == 0) {
-                    a.part_ml[(prow * a.nq + hq) * 2 + 0] = m_run[h] == -INFINITY ? -INFINITY : m_run[h] * a.scale;
-                    a.part_ml[(prow * a.nq + hq) * 2 + 1] = l_run[h];
-                }
-            }
-        }
     }
 }
 
 template <int D, int ROWS, bool EXT>
-int launch(const CUtensorMap& map, const AttnArgs& a, int launch_items, cudaStream_t stream) {
+int configure() {
     auto kern = attention_tma_kernel<D, ROWS, EXT>;
     constexpr int smem = Layout<D, ROWS>::TOTAL;
     static bool configured = false;
@@ -521,15 +581,73 @@ int launch(const CUtensorMap& map, const AttnArgs& a, int launch_items, cudaStre
         if (e != cudaSuccess) return fail("attention_tma: shared memory %d: %s", smem, cudaGetErrorString(e));
         // two CTAs per SM need the large shared-memory carve-out even when one CTA would fit a small one
         cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);     // clusters of up to 16
+        if (e != cudaSuccess) return fail("attention_tma: clusters of more than 8: %s", cudaGetErrorString(e));
         configured = true;
     }
-    launch_kernel(kern, dim3(launch_items, a.nkv), dim3(THREADS), smem, stream, map, a);
+    return 0;
+}
+
+template <int D, int ROWS, bool EXT>
+int launch(const CUtensorMap& map, const AttnArgs& a, int launch_items, cudaStream_t stream) {
+    auto kern = attention_tma_kernel<D, ROWS, EXT>;
+    constexpr int smem = Layout<D, ROWS>::TOTAL;
+    int rc = configure<D, ROWS, EXT>();
+    if (rc) return rc;
+    if (a.cluster <= 1) {
+        launch_kernel(kern, dim3(launch_items, a.nkv), dim3(THREADS), smem, stream, map, a);
+        return check_launch("attention_tma");
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(launch_items, a.nkv);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = a.cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, map, a);
+    if (e != cudaSuccess) return fail("attention_tma: launch of clusters of %d: %s", a.cluster, cudaGetErrorString(e));
     return check_launch("attention_tma");
+}
+
+// How many clusters of n CTAs of the kernel with options the device holds at once.
+template <int D>
+int max_clusters(int n) {
+    int rc = configure<D, 16, true>();
+    if (rc) return rc;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n, 1);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = Layout<D, 16>::TOTAL;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = n;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int k = 0;
+    cudaError_t e = cudaOccupancyMaxActiveClusters(&k, attention_tma_kernel<D, 16, true>, &cfg);
+    if (e != cudaSuccess) return fail("attention_tma: clusters of %d: %s", n, cudaGetErrorString(e));
+    return k;
 }
 }  // namespace
 
 MHB_EXPORT int mhb_attention_tma_supports(int d, int P) {
     return (d == 64 || d == 128) && P >= 2 && P <= KT && KT % P == 0;
+}
+
+// Clusters of n CTAs of the kernel with options that run at once on the current device (0: none); < 0: error.
+MHB_EXPORT int mhb_attention_tma_max_clusters(int d, int n) {
+    if ((d != 64 && d != 128) || n < 1 || n > 16) return fail("attention_tma: head_dim %d, %d splits", d, n);
+    return d == 128 ? max_clusters<128>(n) : max_clusters<64>(n);
 }
 
 // cache: one layer's pool [num_pages, 2, nkv, P, d] bfloat16; rows = 16 (items of short segments).
@@ -558,13 +676,15 @@ MHB_EXPORT int mhb_attention_tma(const void* q, const void* cache, void* out, fl
     a.width = width; a.nq = nq; a.nkv = nkv; a.P = P; a.num_pages = num_pages; a.window = window;
     a.scale = scale;
     a.fresh = fresh;
-    a.gate_per_head = 0; a.shared_kv = 0; a.softcap = 0.f; a.out_f32 = 0; a.slopes = nullptr;
+    a.gate_per_head = 0; a.shared_kv = 0; a.softcap = 0.f; a.out_f32 = 0; a.slopes = nullptr; a.cluster = 0; a.gate_vec = 0;
     a.sink = nullptr; a.gate = nullptr; a.gate_nsplit = 1; a.gate_ld = 0; a.gate_split_stride = 0;
     if (rows == 16) return d == 128 ? launch<128, 16, false>(map, a, launch_items, stream) : launch<64, 16, false>(map, a, launch_items, stream);
     return fail("attention_tma: tile height %d", rows);
 }
 
-// The same with the options (see EXT at the kernel); keys and values are both d wide.
+// The same with the options (see EXT at the kernel); keys and values are both d wide.  cluster > 1: the items are those of
+// single tokens cut into `cluster` splits each (item = token * cluster + split, one chunk of at most 16 heads), which a
+// cluster merges; partial buffers and counters are not used.
 MHB_EXPORT int mhb_attention_tma_ext(const void* q, const void* cache, void* out, float* part_acc, float* part_ml,
                                      const int* items, int num_items, int launch_items, int rows,
                                      const int* positions, const int* block_table, int width,
@@ -572,7 +692,7 @@ MHB_EXPORT int mhb_attention_tma_ext(const void* q, const void* cache, void* out
                                      int d, int P, int num_pages, int window, int fresh, float scale,
                                      const float* sink, const float* gate, int gate_nsplit,
                                      long long gate_split_stride, int gate_ld, int gate_per_head, int shared_kv,
-                                     float softcap, int out_f32, const float* slopes, int* status,
+                                     float softcap, int out_f32, const float* slopes, int cluster, int* status,
                                      cudaStream_t stream) {
     if (launch_items <= 0) return 0;
     if (nkv <= 0 || nq % nkv) return fail("attention: %d query heads over %d KV heads", nq, nkv);
@@ -597,6 +717,12 @@ MHB_EXPORT int mhb_attention_tma_ext(const void* q, const void* cache, void* out
     a.gate_split_stride = (size_t)gate_split_stride;
     a.gate_per_head = gate_per_head; a.shared_kv = shared_kv; a.softcap = softcap; a.out_f32 = out_f32;
     a.slopes = slopes;
+    const int heads = nq / nkv;
+    if (cluster > 1 && (cluster > 16 || heads > 16 || launch_items % cluster || launch_items != num_items ||
+                        (cluster + 1) * ((heads + cluster - 1) / cluster) > Layout<128, 16>::RECV_ROWS))
+        return fail("attention_tma: clusters of %d for %d items of %d heads are not built", cluster, launch_items, heads);
+    a.cluster = cluster;
+    a.gate_vec = gate && !gate_per_head && gate_ld % 4 == 0 && gate_split_stride % 4 == 0 && ((uintptr_t)gate & 15) == 0;
     if (rows == 16) return d == 128 ? launch<128, 16, true>(map, a, launch_items, stream) : launch<64, 16, true>(map, a, launch_items, stream);
     return fail("attention_tma: tile height %d", rows);
 }

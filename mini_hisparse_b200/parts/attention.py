@@ -233,11 +233,13 @@ class AttentionPlanner(StepPlanner):
     the first of its partial rows and the number of its key splits."""
 
     def __init__(self, shape: AttentionShape, sm_count: int, clusters_of=None, max_cluster: int = 0,
-                 min_share: int = MIN_KEYS_PER_SPLIT):
+                 min_share: int = MIN_KEYS_PER_SPLIT, max_groups: int = MAX_SPLITS,
+                 max_ctas: int = 0):
         """``clusters_of(n)``: how many clusters of n CTAs the mixer's decode kernel can run at once, if
         it merges a token's key splits inside a cluster of up to ``max_cluster`` CTAs (None: it does not).
-        ``min_share``: keys that a share of a cluster has at least."""
-        self.min_share = min_share
+        ``min_share``: keys that a share of a cluster has at least; ``max_groups``: clusters per token and KV head;
+        ``max_ctas``: CTAs of a launch of clusters (0: as many as are resident)."""
+        self.min_share, self.max_groups, self.max_ctas = min_share, max_groups, max_ctas
         self.shape, self.sm_count = shape, sm_count
         self.clusters_of, self.max_cluster = clusters_of, max_cluster
         self._uneven = {}        # decode_fixed_for's answers
@@ -316,13 +318,13 @@ class AttentionPlanner(StepPlanner):
 
         best = None
         for c in range(min(n, self.max_cluster), 1, -1):
-            if room(c) >= ctas:
+            if room(c) >= ctas and (not self.max_ctas or c * ctas <= self.max_ctas):
                 best = (c, 1)
                 break
         if best is not None:
             best_cost = 0.9 * cost(*best)
             for c in range(min(n, self.max_cluster), 3, -1):
-                for g in range(2, min(n // c, room(c) // ctas) + 1):
+                for g in range(2, min(n // c, room(c) // ctas, self.max_groups) + 1):
                     if cost(c, g) < best_cost:
                         best, best_cost = (c, g), cost(c, g)
         # no cluster fits: the shares go through the kernels that merge through global memory
@@ -381,6 +383,21 @@ class AttentionPlanner(StepPlanner):
     def plan_decode(self, starts, fixed):
         cluster, groups = fixed
         return self._out(plan_decode(self.shape, starts, cluster * groups), cluster if self.chunks == 1 else 0, groups)
+
+
+def tma_planner(shape: AttentionShape, sm_count: int, d: int) -> AttentionPlanner:
+    """The planner of a mixer whose decode tokens run on attention_tma_ext, which merges splits inside a cluster: a
+    cluster's merge pays for shares of one key tile, as long as a launch is one CTA an SM (8 requests of 300 keys, 4 KV heads:
+    8.3 us uncut, 7.2 in clusters of 4, 9.3 in clusters of 8, which wait for one another)."""
+    groups = shape.q_heads // shape.kv_heads
+    return AttentionPlanner(shape, sm_count, lambda n: K.attention_tma_max_clusters(d, groups, n), K.DECODE_MAX_SPLITS,
+                            min_share=KEY_TILE, max_groups=1, max_ctas=sm_count)
+
+
+def tma_cluster(meta: dict, d: int, groups: int) -> int:
+    """Splits that attention_tma_ext merges in a cluster in this step (0: it merges through the partial buffers)."""
+    n = meta.get("decode_nsplit", 0)
+    return n if n > 1 and meta.get("decode_groups", 1) == 1 and K.attention_tma_max_clusters(d, groups, n) > 0 else 0
 
 
 @register_mixer("gq_attention")
@@ -446,7 +463,6 @@ class GQAttention(Mixer):
     def planner(self, page_size: int, sm_count: int):
         shape = AttentionShape(self.nq, self.nkv, self.window, self.big_tile_rows(page_size))
         if self.kernel_family(page_size) == "tc" and self.nq // self.nkv <= ROW_TILE:
-            # a cluster's merge pays for shares of two key tiles
             return AttentionPlanner(shape, sm_count, lambda n: K.attention_decode_max_clusters(self.d, n),
                                     K.DECODE_MAX_SPLITS, min_share=2 * KEY_TILE)
         return AttentionPlanner(shape, sm_count)

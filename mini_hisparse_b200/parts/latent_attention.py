@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .attention import ITEM_INTS, ROW_TILE, SPLIT_MAX_TOKENS, AttentionPlanner, AttentionShape
+from .attention import ITEM_INTS, ROW_TILE, SPLIT_MAX_TOKENS, AttentionPlanner, AttentionShape, tma_cluster, tma_planner
 from .base import CacheView, Mixer, Product, StepContext
 from .multimap_attention import _pad_rows
 from .registry import POSITIONS, register_mixer
@@ -87,8 +87,9 @@ class LatentAttention(Mixer):
         return ("latent_attention", self.heads, self.window, self.width, self.rt is not None and self.rt.dtype)
 
     def planner(self, page_size: int, sm_count: int):
-        rows = {"tc": 128, "mma": 64, "simt": ROW_TILE}[self.kernel_family(page_size)]
-        return AttentionPlanner(AttentionShape(self.heads, 1, self.window, rows), sm_count)
+        family = self.kernel_family(page_size)
+        shape = AttentionShape(self.heads, 1, self.window, {"tc": 128, "mma": 64, "simt": ROW_TILE}[family])
+        return tma_planner(shape, sm_count, self.width) if family == "tc" else AttentionPlanner(shape, sm_count)
 
     def parameters(self):
         p = {"q": ParamSpec((self.qw, self.hidden)),
@@ -156,7 +157,8 @@ class LatentAttention(Mixer):
                     K.attention_tma_ext(*args, meta["items"], n_small, 16, *tail, nq=self.heads, nkv=1, d=self.width,
                                         page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                         shared_kv=True, **opts, tok_nsplit=meta["tok_nsplit"], counters=counters,
-                                        status=ctx.status, fresh=SPLIT_MAX_TOKENS)
+                                        status=ctx.status, fresh=SPLIT_MAX_TOKENS,
+                                        cluster=tma_cluster(meta, self.width, self.heads))
                 else:
                     K.attention_mma_ext(*args, meta["items"], n_small, 16, *tail, **common,
                                         tok_nsplit=meta["tok_nsplit"], counters=counters)

@@ -6,7 +6,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .attention import ITEM_INTS, ROW_TILE, SPLIT_MAX_TOKENS, AttentionPlanner, AttentionShape
+from .attention import ITEM_INTS, ROW_TILE, SPLIT_MAX_TOKENS, AttentionPlanner, AttentionShape, tma_cluster, tma_planner
 from .base import CacheView, Mixer, Product, StepContext
 from .registry import POSITIONS, register_mixer
 from .spec import PagedKVNeed, ParamSpec, PartSpec
@@ -95,7 +95,7 @@ class DifferentialAttention(Mixer):
     def planner(self, page_size: int, sm_count: int):
         family = self.kernel_family(page_size)
         if family == "tc":       # plain grouped-query attention over 2 x heads padded query maps
-            return AttentionPlanner(AttentionShape(self.nq, self.nkv, self.window, 128), sm_count)
+            return tma_planner(AttentionShape(self.nq, self.nkv, self.window, 128), sm_count, self.dv)
         rows = {"mma": 64, "simt": ROW_TILE}[family]
         return AttentionPlanner(AttentionShape(self.heads, self.nkv, self.window, rows), sm_count)
 
@@ -144,7 +144,8 @@ class DifferentialAttention(Mixer):
                 K.attention_tma_ext(*args, meta["items"], n_small, 16, *tail, nq=self.nq, nkv=self.nkv, d=self.dv,
                                     page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                     softcap=self.softcap, tok_nsplit=meta["tok_nsplit"], counters=counters,
-                                    status=ctx.status, fresh=SPLIT_MAX_TOKENS)
+                                    status=ctx.status, fresh=SPLIT_MAX_TOKENS,
+                                    cluster=tma_cluster(meta, self.dv, self.nq // self.nkv))
             if n_big:
                 K.attention_tc_ext(q, cache.storage, maps, big_items, n_big, ctx.positions, meta["block_table"],
                                    nq=self.nq, nkv=self.nkv, d=self.dv, page_size=cache.page_size,

@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .attention import ITEM_INTS, ROW_TILE, SPLIT_MAX_TOKENS, AttentionPlanner, AttentionShape
+from .attention import ITEM_INTS, ROW_TILE, SPLIT_MAX_TOKENS, AttentionPlanner, AttentionShape, tma_cluster, tma_planner
 from .base import CacheView, Mixer, Product, StepContext
 from .registry import POSITIONS, register_mixer
 from .spec import PagedKVNeed, ParamSpec, PartSpec
@@ -81,8 +81,9 @@ class SinkAttention(Mixer):
         return ("sink_attention", self.nq, self.nkv, self.window)
 
     def planner(self, page_size: int, sm_count: int):
-        rows = {"tc": 128, "mma": 64, "simt": ROW_TILE}[self.kernel_family(page_size)]
-        return AttentionPlanner(AttentionShape(self.nq, self.nkv, self.window, rows), sm_count)
+        family = self.kernel_family(page_size)
+        shape = AttentionShape(self.nq, self.nkv, self.window, {"tc": 128, "mma": 64, "simt": ROW_TILE}[family])
+        return tma_planner(shape, sm_count, self.dk) if family == "tc" else AttentionPlanner(shape, sm_count)
 
     def parameters(self):
         p = {"q": ParamSpec((self.qw, self.hidden)), "g": ParamSpec((self.ow, self.hidden)),
@@ -143,7 +144,8 @@ class SinkAttention(Mixer):
                     K.attention_tma_ext(*args, meta["items"], n_small, 16, *tail, nq=self.nq, nkv=self.nkv, d=self.dk,
                                         page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                         sink=sink, slopes=slopes, **gate, tok_nsplit=meta["tok_nsplit"], counters=counters,
-                                        status=ctx.status, fresh=SPLIT_MAX_TOKENS)
+                                        status=ctx.status, fresh=SPLIT_MAX_TOKENS,
+                                        cluster=tma_cluster(meta, self.dk, self.nq // self.nkv))
                 else:
                     K.attention_mma_ext(*args, meta["items"], n_small, 16, *tail, **common,
                                         tok_nsplit=meta["tok_nsplit"], counters=counters)

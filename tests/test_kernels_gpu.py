@@ -5,6 +5,7 @@ import hashlib
 import math
 
 import pytest
+import numpy as np
 import torch
 
 from plain import qwen2_plain as P
@@ -823,6 +824,58 @@ def test_attention_tma_alone_and_in_a_busy_batch(d, P_, nsplit, ext):
     ref = torch.cat(ref)
     ref = ref * torch.sigmoid(gate.cpu().double()) if ext else ref
     torch.testing.assert_close(out.double().cpu(), ref, **tol(bf, 2))
+
+
+@pytest.mark.parametrize("nq,nkv,d,P_,nsplit,shared,per_head", [(8, 4, 64, 16, 2, False, False), (28, 4, 128, 32, 8, False, False),
+                                                                (16, 1, 128, 16, 16, True, True), (3, 1, 64, 64, 5, False, True),
+                                                                (10, 1, 128, 4, 5, True, False), (16, 16, 128, 16, 7, False, False)])
+@pytest.mark.parametrize("window", [None, 100])
+def test_attention_tma_splits_merged_in_a_cluster(nq, nkv, d, P_, nsplit, shared, per_head, window):
+    """Decoded tokens whose key splits a thread-block cluster merges: with a sink, a cap and a gate, histories with empty
+    splits among them, bfloat16 and float32 outputs, the gate on and off 16 bytes.  The partial buffers and counters stay
+    untouched."""
+    from mini_hisparse_b200.parts.attention import AttentionShape, plan_decode
+
+    bf = torch.bfloat16
+    assert K().attention_tma_max_clusters(d, nq // nkv, nsplit) > 0
+    g = torch.Generator().manual_seed(nq * d + nsplit)
+    lengths = [1, 63, 64, 65, 130, 333, 700]
+    B, width = len(lengths), 800 // P_ + 1
+    need = [-(-n // P_) for n in lengths]
+    order = torch.randperm(sum(need), generator=g).tolist()
+    table = torch.full((B, width), -1, dtype=torch.int32)
+    for i, n in enumerate(need):
+        table[i, :n] = torch.tensor([order.pop() for _ in range(n)])
+    planes = 1 if shared else 2
+    cache = torch.randn(sum(need), planes, nkv, P_, d, generator=g).to(bf)
+    q = torch.randn(B, nq, d, generator=g).to(bf)
+    sink, gate = torch.randn(nq, generator=g), torch.randn(2, B, 2 + (nq if per_head else nq * d), generator=g)
+    plan = plan_decode(AttentionShape(nq, nkv, window, 128), np.asarray(lengths) - 1, nsplit)
+    z = gate.double().sum(0)
+    for first in (0, 1):            # the gate's first column
+        cols = z[:, first: first + (nq if per_head else nq * d)].view(B, nq, -1)
+        ref = torch.empty(B, nq, d, dtype=torch.float64)
+        for i, n in enumerate(lengths):
+            kv = cache[table[i, :need[i]].long()].double().permute(1, 0, 3, 2, 4).reshape(planes, -1, nkv, d)[:, max(0, n - (window or n)): n]
+            kk, vv = (kv[j].repeat_interleave(nq // nkv, 1) for j in (0, planes - 1))
+            x = 20.0 * torch.tanh(torch.einsum("hd,khd->hk", q[i].double(), kk) * d ** -0.5 / 20.0)
+            w = torch.softmax(torch.cat((x, sink.double()[:, None]), 1), 1)[:, :-1]
+            ref[i] = torch.einsum("hk,khd->hd", w, vv) * torch.sigmoid(cols[i])
+        for dtype in (bf, torch.float32):
+            out = torch.full((B + 1, nq * d), float("nan"), dtype=dtype, device=DEV)
+            part, counters = torch.full((B * nsplit, nq, d), 7.0, device=DEV), torch.zeros(B * nkv, dtype=torch.int32, device=DEV)
+            status = torch.zeros(1, dtype=torch.int32, device=DEV)
+            gd = gate.to(DEV)
+            K().attention_tma_ext(
+                q.to(DEV), cache.to(DEV), out[:B], part, part[..., :2].contiguous(), torch.from_numpy(plan.items).to(DEV).reshape(-1),
+                len(plan.items), 16, torch.tensor(lengths, dtype=torch.int32, device=DEV) - 1, table.to(DEV),
+                torch.from_numpy(plan.tok_part_row).to(DEV), nq=nq, nkv=nkv, d=d, page_size=P_, window=window or 0, sink=sink.to(DEV),
+                gate=gd[0][:, first:], gate_nsplit=2, gate_split_stride=gd.stride(0), gate_per_head=per_head, shared_kv=shared,
+                softcap=20.0, tok_nsplit=torch.from_numpy(plan.tok_nsplit).to(DEV), counters=counters, status=status, cluster=nsplit)
+            assert int(status) == 0 and int(counters.abs().sum()) == 0 and bool((part == 7.0).all()) and bool(out[B].isnan().all())
+            got = out[:B].double().cpu().view(B, nq, d)
+            # weights in 16 bits, float32 sums; a bfloat16 output adds its own rounding
+            torch.testing.assert_close(got, ref, atol=1e-4 if dtype == torch.float32 else 2.0 ** -8 * float(ref.abs().max()), rtol=2.0 ** -8 if dtype == bf else 0)
 
 
 @pytest.mark.parametrize("ext", [False, True])
