@@ -869,6 +869,24 @@ def attention_tc_ext(q, cache, out, items, num_items, positions, block_table, *,
         _ptr(slopes), _ptr(status), _stream()), "attention_tc_ext")
 
 
+def attention_tokens_supports(nq: int, nkv: int, d: int) -> bool:
+    """Head counts and sizes of attention_tokens."""
+    return nkv >= 1 and nq % nkv == 0 and nq // nkv <= 8 and 4 <= d <= 128 and d % 4 == 0
+
+
+def attention_tokens(q, cache, out, part_acc, part_ml, items, num_items, block_table, tok_part_row, *, nq, nkv, d, page_size,
+                     scale=None):
+    """attention_simt for items of single tokens with all heads of their KV heads, without options: the keys of an item are
+    dealt to eight warps."""
+    lib = build.load("attention_tokens")
+    if q.dtype != cache.dtype or q.dtype != out.dtype or not (q.is_contiguous() and cache.is_contiguous() and out.is_contiguous()):
+        raise KernelError("attention_tokens: q, the pool and the output must be contiguous and of one dtype")
+    _check(lib, lib.mhb_attention_tokens(
+        _ptr(q), _ptr(cache), _ptr(out), c_int(dtype_code(q.dtype)), _ptr(part_acc), _ptr(part_ml), _ptr(items), c_int(num_items),
+        _ptr(block_table), c_int(block_table.shape[-1]), _ptr(tok_part_row), c_int(nq), c_int(nkv), c_int(d), c_int(page_size),
+        c_int(cache.shape[0]), c_float(float(d) ** -0.5 if scale is None else scale), _stream()), "attention_tokens")
+
+
 def attention_combine(part_acc, part_ml, tok_part_row, tok_nsplit, out, *, nq, d, every=0, gate=None,
                       gate_nsplit=1, gate_split_stride=0, gate_per_head=False):
     """Merge the parts of every token's attention.  ``every`` > 0: each token has exactly that many parts,

@@ -17,6 +17,7 @@ KEY_TILE = 64          # split boundaries are multiples of the kernels' key tile
 ITEM_INTS = 8
 MIN_KEYS_PER_SPLIT = 256
 MIN_KEYS_PER_SIMT_SPLIT = 128
+KEYS_PER_TOKEN_SPLIT = 512     # attention_tokens: two rounds of its eight warps; a merge is a launch
 SPLIT_MAX_TOKENS = 16  # only short segments (decode tokens, tiny portions) are split along the keys
 MAX_SPLITS = 64
 MAX_BIG_SPLITS = 8       # key splits of a long portion's tile (tcgen05 kernel only)
@@ -233,13 +234,14 @@ class AttentionPlanner(StepPlanner):
     the first of its partial rows and the number of its key splits."""
 
     def __init__(self, shape: AttentionShape, sm_count: int, clusters_of=None, max_cluster: int = 0,
-                 min_share: int = MIN_KEYS_PER_SPLIT, max_groups: int = MAX_SPLITS,
+                 min_share: int = MIN_KEYS_PER_SPLIT, max_groups: int = MAX_SPLITS, token_share: int = 0,
                  max_ctas: int = 0):
         """``clusters_of(n)``: how many clusters of n CTAs the mixer's decode kernel can run at once, if
         it merges a token's key splits inside a cluster of up to ``max_cluster`` CTAs (None: it does not).
         ``min_share``: keys that a share of a cluster has at least; ``max_groups``: clusters per token and KV head;
-        ``max_ctas``: CTAs of a launch of clusters (0: as many as are resident)."""
-        self.min_share, self.max_groups, self.max_ctas = min_share, max_groups, max_ctas
+        ``max_ctas``: CTAs of a launch of clusters (0: as many as are resident); ``token_share``: a step of single tokens is cut into shares of that many keys, once there are four (0: as the
+        shape says)."""
+        self.min_share, self.max_groups, self.token_share, self.max_ctas = min_share, max_groups, token_share, max_ctas
         self.shape, self.sm_count = shape, sm_count
         self.clusters_of, self.max_cluster = clusters_of, max_cluster
         self._uneven = {}        # decode_fixed_for's answers
@@ -273,6 +275,11 @@ class AttentionPlanner(StepPlanner):
         every = None if fixed is None else fixed[0] * fixed[1]
         return self._out(plan_attention(self.shape, segments, T, self.sm_count, fixed_nsplit=every))
 
+    def _most_splits(self, keys: int) -> int:
+        if self.token_share:
+            return keys // self.token_share if keys >= 4 * self.token_share else 1
+        return self.shape.max_splits(keys)
+
     # what a CTA costs beside its keys (the query and the merge) and what a launch of attention_combine
     # costs the step, in key tiles of streaming time
     CTA_FIXED_TILES = 3.5
@@ -287,7 +294,7 @@ class AttentionPlanner(StepPlanner):
         ctas = segments_count * self.shape.kv_heads * self.chunks
         if self.shape.window:            # a token never attends to more keys than its window holds
             max_positions = min(max_positions, self.shape.window)
-        plain = n = max(1, min(MAX_SPLITS, (2 * self.sm_count) // ctas, self.shape.max_splits(max_positions)))
+        plain = n = max(1, min(MAX_SPLITS, (2 * self.sm_count) // ctas, self._most_splits(max_positions)))
         if self.clusters_of is not None and self.chunks == 1:
             n = max(n, min((2 * self.sm_count) // ctas, self.max_cluster, max_positions // self.min_share))
         if self.clusters_of is None or self.chunks != 1 or n == 1:
@@ -342,7 +349,7 @@ class AttentionPlanner(StepPlanner):
         fixed = self.decode_fixed(len(starts), max_positions)
         n0 = fixed[0] * fixed[1]
         B = len(starts)
-        limit = min(self.shape.max_splits(max_positions), self.max_cluster or MAX_SPLITS)
+        limit = min(self._most_splits(max_positions), self.max_cluster or MAX_SPLITS)
         if n0 > 1 or B < 2 or limit < 2:       # fewer requests: their splits are sized for one round of CTAs
             return fixed
         tiles = (np.asarray(starts, np.int64) + KEY_TILE) // KEY_TILE
@@ -449,7 +456,7 @@ class GQAttention(Mixer):
         kernels come in for the head sizes they are built for (which of them runs depends on the
         page size, which the cache brings)."""
         if not self.tensor_core_attention:
-            return ("attention_simt",)
+            return ("attention_simt", "attention_tokens")
         if self.d in (64, 128):
             return ("attention_simt", "attention_mma", "attention_tma", "attention_decode", "attention_tc")
         return ("attention_simt", "attention_mma")
@@ -465,6 +472,8 @@ class GQAttention(Mixer):
         if self.kernel_family(page_size) == "tc" and self.nq // self.nkv <= ROW_TILE:
             return AttentionPlanner(shape, sm_count, lambda n: K.attention_decode_max_clusters(self.d, n),
                                     K.DECODE_MAX_SPLITS, min_share=2 * KEY_TILE)
+        if self.kernel_family(page_size) == "simt" and K.attention_tokens_supports(self.nq, self.nkv, self.d):
+            return AttentionPlanner(shape, sm_count, token_share=KEYS_PER_TOKEN_SPLIT)
         return AttentionPlanner(shape, sm_count)
 
     def parameters(self):
@@ -581,6 +590,9 @@ class GQAttention(Mixer):
                     short_segments()
                 if n_big:
                     long_portions()
+        elif nsplit and K.attention_tokens_supports(self.nq, self.nkv, self.d) and cache.storage.data_ptr() % 16 == 0:
+            K.attention_tokens(*args, meta["items"], n_small, meta["block_table"], meta["tok_part_row"], nq=self.nq, nkv=self.nkv,
+                               d=self.d, page_size=cache.page_size, scale=self.scale)
         elif n_small + n_big:
             K.attention_simt(*args, meta["items"], n_small + n_big, n_small + n_big, *tail, **common)
         if meta["any_split"] and family == "simt":

@@ -673,6 +673,42 @@ def run_attention(nq, nkv, d, P_, seg_specs, dtype, window=None, fixed_nsplit=No
     return out.float().cpu(), ref, plan
 
 
+@pytest.mark.parametrize("nq,nkv,d,P_,nsplit", [(3, 1, 32, 32, 1), (4, 2, 16, 16, 3), (28, 4, 128, 16, 1), (16, 4, 64, 5, 4), (8, 1, 100, 7, 2),
+                                                (5, 5, 4, 1, 1)])
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_attention_tokens(nq, nkv, d, P_, nsplit, window, dtype):
+    """Decoded tokens on the CUDA cores with the keys dealt to warps: histories around a warp's run of 32 keys and a round of
+    256, odd pages, splits (empty ones too), a window, against 64 bits."""
+    from mini_hisparse_b200.parts.attention import AttentionShape, plan_decode
+
+    assert K().attention_tokens_supports(nq, nkv, d)
+    g = torch.Generator().manual_seed(nq * d + nsplit)
+    lengths = [1, 31, 32, 33, 255, 256, 257, 600]
+    B, need = len(lengths), [-(-n // P_) for n in lengths]
+    order = torch.randperm(sum(need), generator=g).tolist()
+    table = torch.full((B, max(need) + 1), -1, dtype=torch.int32)
+    for i, n in enumerate(need):
+        table[i, :n] = torch.tensor([order.pop() for _ in range(n)])
+    cache, q = torch.randn(sum(need), 2, nkv, P_, d, generator=g).to(dtype), torch.randn(B, nq, d, generator=g).to(dtype)
+    plan = plan_decode(AttentionShape(nq, nkv, window), np.asarray(lengths) - 1, nsplit)
+    out = torch.full((B + 1, nq * d), float("nan"), dtype=dtype, device=DEV)
+    part_acc, part_ml = (torch.full((max(1, plan.part_rows), nq, n), float("nan"), device=DEV) for n in (d, 2))
+    tpr, tns = (torch.from_numpy(y).to(DEV) for y in (plan.tok_part_row, plan.tok_nsplit))
+    K().attention_tokens(q.to(DEV), cache.to(DEV), out[:B], part_acc, part_ml, torch.from_numpy(plan.items).to(DEV).reshape(-1),
+                         len(plan.items), table.to(DEV), tpr, nq=nq, nkv=nkv, d=d, page_size=P_)
+    if nsplit > 1:
+        K().attention_combine(part_acc, part_ml, tpr, tns, out[:B], nq=nq, d=d)
+    ref = torch.empty(B, nq, d, dtype=torch.float64)
+    for i, n in enumerate(lengths):
+        kv = cache[table[i, :need[i]].long()].double().permute(1, 0, 3, 2, 4).reshape(2, -1, nkv, d)[:, max(0, n - (window or n)): n]
+        kk, vv = (y.repeat_interleave(nq // nkv, 1) for y in kv)
+        ref[i] = torch.einsum("hk,khd->hd", torch.softmax(torch.einsum("hd,khd->hk", q[i].double(), kk) * d ** -0.5, 1), vv)
+    assert bool(out[B].isnan().all())
+    torch.testing.assert_close(out[:B].double().cpu().view(B, nq, d), ref, atol=2e-6 if dtype == torch.float32 else 2.0 ** -8 * float(ref.abs().max()),
+                               rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-5)
+
+
 @pytest.mark.parametrize("nq,nkv,d,P_,dtype", [
     (3, 1, 16, 16, torch.float32), (7, 7, 20, 5, torch.float32), (4, 2, 23, 3, torch.float32), (28, 4, 128, 16, torch.float32),
     (18, 1, 256, 1, torch.float32), (5, 5, 184, 64, torch.float32), (4, 2, 24, 16, torch.bfloat16), (4, 2, 20, 7, torch.bfloat16),
