@@ -213,6 +213,8 @@ class CacheManager:
             )
         P = self.cfg.page_size
         need_pages = -(-new_length // P)
+        if all(len(g.tables[req.slot].pages) >= need_pages for g in self.page_groups):
+            return                          # most decoded tokens stay inside their last page
         plans = []
         for g in self.page_groups:
             rp = g.tables[req.slot]

@@ -108,6 +108,55 @@ class _PlanSlot:
     planner: StepPlanner
 
 
+class _DecodeBuffers:
+    """A captured step's pinned host buffers, used in turn: what does not change from step to step (the order of the tokens,
+    the items' heads and splits) is written once per buffer.  An event per half of the ring says when its copies are done: it
+    is recorded when the ring moves on to the other half, so three steps of four pay for no event at all."""
+
+    RING = 8
+
+    def __init__(self, layout: _Layout, device: torch.device):
+        host = torch.empty((self.RING, layout.total), dtype=torch.int32)
+        self.cuda = torch.cuda.is_available()
+        host = host.pin_memory() if self.cuda else host
+        B = layout.T
+        self.rows = [host[i] for i in range(self.RING)]
+        self.views = []
+        for row in self.rows:
+            a = row.numpy()
+            a[:] = 0
+            a[layout.tok_seg : layout.tok_seg + B] = a[layout.rows : layout.rows + B] = np.arange(B, dtype=np.int32)
+            a[layout.seg_offset : layout.seg_offset + B + 1] = np.arange(B + 1, dtype=np.int32)
+            self.views.append(dict(
+                tokens=a[layout.tokens : layout.tokens + B], positions=a[layout.positions : layout.positions + B],
+                seg_slot=a[layout.seg_slot : layout.seg_slot + B],
+                tables=[a[at : at + B * w].reshape(B, w) for at, w in zip(layout.tables, layout.widths)],
+                plans=[{name: a[at[name] : at[name] + n] for name, n in caps.items()} for at, caps in zip(layout.plans, layout.plan_caps)],
+                first=True))
+        self.turn = 0
+        self.events = [None, None]
+        self.device = device.index if device.index is not None or not self.cuda else torch.cuda.current_device()
+        self.stream = None          # the stream of the copies since the last event
+
+    def next(self) -> int:
+        i = self.turn
+        self.turn = (i + 1) % self.RING
+        if self.cuda:
+            half = self.RING // 2
+            now = torch._C._cuda_getCurrentRawStream(self.device)
+            if self.stream is not None and now != self.stream:
+                torch.cuda.synchronize()        # the ring's copies lie on another stream than the next ones
+            self.stream = now
+            if i % half == 0:
+                before, mine = 1 - i // half, i // half
+                if self.events[before] is None:
+                    self.events[before] = torch.cuda.Event()
+                self.events[before].record()
+                if self.events[mine] is not None:
+                    self.events[mine].synchronize()
+        return i
+
+
 class _DecodeGraph:
     """A captured step for exactly B single-token segments whose block tables are ``width`` wide, with
     what the planners hold constant in it (``fixed``, one value per plan slot)."""
@@ -121,6 +170,7 @@ class _DecodeGraph:
         caps = [slot.planner.capacity(B, B, f) for slot, f in zip(batch.slots, self.fixed)]
         self.layout = _Layout(B, B, B, [min(width, g.width) for g in runner.cache.page_groups], caps)
         self.meta = torch.zeros(self.layout.total, dtype=torch.int32, device=runner.device)
+        self.buffers = None     # made at the first step
         self.facts = None       # the plans' host facts at capture: every replay must bring the same
         self.graph = None
         self.logits = None
@@ -183,12 +233,11 @@ class BatchBuilder:
         return segments, offset
 
     @staticmethod
-    def _put(buf: np.ndarray, offsets: dict[str, int], caps: dict[str, int], arrays: dict[str, np.ndarray],
-             exact: bool = False) -> None:
+    def _put(buf: np.ndarray, offsets: dict[str, int], caps: dict[str, int], arrays: dict[str, np.ndarray]) -> None:
         for name, cap in caps.items():
             arr = arrays[name]
             n = arr.size
-            if n > cap or (exact and n != cap):
+            if n > cap:
                 raise StepError(f"plan array {name!r} has {n} words, the layout holds {cap}")
             region = buf[offsets[name]: offsets[name] + cap]
             region[:n] = arr.reshape(-1)
@@ -225,29 +274,17 @@ class BatchBuilder:
             facts.append(f)
         return len(rows), facts
 
-    def _fill_decode(self, buf: np.ndarray, layout: _Layout, entries, segments, fixed) -> list[dict]:
-        """_fill for a batch of single decoded tokens that all want their logits, without loops
-        over tokens: the arrays a captured decode graph reads.  Returns the plans' facts."""
-        B = len(segments)
-        starts = np.fromiter((s.start for s in segments), np.int64, B)
-        slots = np.fromiter((s.slot for s in segments), np.intp, B)
-        ar = np.arange(B, dtype=np.int32)
-        buf[layout.tokens : layout.tokens + B] = [e.tokens[0] for e in entries]
-        buf[layout.positions : layout.positions + B] = starts
-        buf[layout.tok_seg : layout.tok_seg + B] = ar
-        buf[layout.seg_slot : layout.seg_slot + B] = slots
-        buf[layout.seg_offset : layout.seg_offset + B] = ar
-        buf[layout.seg_offset + B] = B
-        buf[layout.rows : layout.rows + B] = ar
-        for gi, g in enumerate(self.cache.page_groups):
-            width = layout.widths[gi]
-            buf[layout.tables[gi] : layout.tables[gi] + B * width].reshape(B, width)[:] = g.table_np[slots, :width]
-        facts = []
-        for pi, slot in enumerate(self.slots):
-            arrays, f = slot.planner.plan_decode(starts, fixed[pi])
-            self._put(buf, layout.plans[pi], layout.plan_caps[pi], arrays, exact=True)
-            facts.append(f)
-        return facts
+    def _fill_decode(self, views: dict, entries, segments, fixed, starts: np.ndarray) -> list[dict]:
+        """The arrays of a batch of single decoded tokens that all want their logits, without loops over tokens, into one
+        of a captured graph's buffers (_DecodeBuffers).  Returns the plans' facts."""
+        slots = [s.slot for s in segments]
+        views["tokens"][:] = [e.tokens[0] for e in entries]
+        views["positions"][:] = starts
+        views["seg_slot"][:] = slots
+        for g, table in zip(self.cache.page_groups, views["tables"]):
+            np.take(g.table_np[:, : table.shape[1]], slots, axis=0, out=table)
+        first, views["first"] = views["first"], False
+        return [slot.planner.write_decode(starts, fixed[pi], views["plans"][pi], first) for pi, slot in enumerate(self.slots)]
 
     def _views(self, meta: torch.Tensor, layout: _Layout, T: int, S: int, R: int, facts) -> dict:
         def v(off, n):
@@ -440,11 +477,10 @@ class ModelRunner:
         self.stats["two_stream_layers"] += ctx.extras.get("two_stream_layers", 0)
         return out
 
-    def _graph_key(self, segments) -> tuple:
+    def _graph_key(self, segments, starts: np.ndarray) -> tuple:
         """What a captured decode graph is made for: the batch size, the block-table width and what the
         planners want to hold constant for these histories."""
-        B, width = len(segments), self._table_width(segments)
-        starts = np.fromiter((s.start for s in segments), np.int64, B)
+        B, width = len(segments), self._table_width(int(starts.max()))
         max_keys = width * self.cache.cfg.page_size
         return B, width, tuple(slot.planner.decode_fixed_for(starts, max_keys) for slot in self.batch.slots)
 
@@ -463,7 +499,8 @@ class ModelRunner:
         """The step through a captured graph, or None if a planner cannot hold its plan constant
         (then the step runs eagerly)."""
         B = len(segments)
-        key = self._graph_key(segments)
+        starts = np.fromiter((s.start for s in segments), np.int64, B)
+        key = self._graph_key(segments, starts)
         if key not in self.graphs and self.graph_after > 1:
             asked = self._asked.pop(key, 0) + 1
             if asked < self.graph_after:
@@ -476,21 +513,22 @@ class ModelRunner:
         if not g.capturable:
             return None
         layout = g.layout
+        if g.buffers is None:
+            g.buffers = _DecodeBuffers(layout, self.device)
         if (ahead is not None and ahead["graph"] is g and g.graph is not None
                 and ahead["who"] == [(s.request, s.slot, s.start) for s in segments]):
             # everything but the token ids was packed while the GPU ran the step before this one
-            stage, turn = ahead["stage"], ahead["turn"]
-            stage.numpy()[layout.tokens : layout.tokens + B] = [e.tokens[0] for e in entries]
+            turn = ahead["turn"]
+            g.buffers.views[turn]["tokens"][:] = [e.tokens[0] for e in entries]
             self.stats["prepared_steps"] += 1
         else:
-            stage, turn = self.batch.staging.next(layout.total)
-            facts = self.batch._fill_decode(stage.numpy(), layout, entries, segments, g.fixed)
+            turn = g.buffers.next()
+            facts = self.batch._fill_decode(g.buffers.views[turn], entries, segments, g.fixed, starts)
             if g.facts is None:
                 g.facts = facts
             elif facts != g.facts:
                 raise StepError(f"a decode plan changed after its graph was captured: {facts} vs {g.facts}")
-        g.meta.copy_(stage[: layout.total], non_blocking=True)
-        self.batch.staging.mark(turn)
+        g.meta.copy_(g.buffers.rows[turn], non_blocking=True)
         if device_tokens is not None:
             g.meta[layout.tokens : layout.tokens + B].copy_(device_tokens)
         if g.graph is None:
@@ -550,19 +588,19 @@ class ModelRunner:
             except CapacityError:
                 return          # the step itself will say so, if it comes to that
         segments, _ = self.batch.segments(entries)
-        g = self.graphs.get(self._graph_key(segments))
+        starts = np.fromiter((s.start for s in segments), np.int64, len(segments))
+        g = self.graphs.get(self._graph_key(segments, starts))
         if g is None or g.graph is None:
             return              # that step will capture its graph: nothing to gain
-        stage, turn = self.batch.staging.next(g.layout.total)
-        if self.batch._fill_decode(stage.numpy(), g.layout, entries, segments, g.fixed) != g.facts:
+        turn = g.buffers.next()
+        if self.batch._fill_decode(g.buffers.views[turn], entries, segments, g.fixed, starts) != g.facts:
             return
-        self._ahead = {"graph": g, "stage": stage, "turn": turn,
-                       "who": [(s.request, s.slot, s.start) for s in segments]}
+        self._ahead = {"graph": g, "turn": turn, "who": [(s.request, s.slot, s.start) for s in segments]}
 
-    def _table_width(self, segments) -> int:
-        """Block-table width of a decode graph: a power of two, so a graph is re-captured only when
-        contexts double."""
-        pages = max(-(-(s.start + 1) // self.cache.cfg.page_size) for s in segments)
+    def _table_width(self, last: int) -> int:
+        """Block-table width of a decode graph whose longest request sits at position ``last``: a power of two, so a graph is
+        re-captured only when contexts double."""
+        pages = -(-(last + 1) // self.cache.cfg.page_size)
         width = 16
         while width < pages:
             width *= 2

@@ -245,6 +245,7 @@ class AttentionPlanner(StepPlanner):
         self.shape, self.sm_count = shape, sm_count
         self.clusters_of, self.max_cluster = clusters_of, max_cluster
         self._uneven = {}        # decode_fixed_for's answers
+        self._fixed = {}         # decode_fixed's: they depend on two numbers
         groups = shape.q_heads // shape.kv_heads
         self.chunks = 1 if groups <= ROW_TILE else -(-groups // ROW_TILE)
 
@@ -287,6 +288,15 @@ class AttentionPlanner(StepPlanner):
     STREAMS = 240.0          # CTAs streaming at a lone CTA's rate that the memory can feed
 
     def decode_fixed(self, segments_count, max_positions):
+        key = (segments_count, max_positions)
+        hit = self._fixed.get(key)
+        if hit is None:
+            if len(self._fixed) >= 512:
+                self._fixed.clear()
+            hit = self._fixed[key] = self._decode_fixed(segments_count, max_positions)
+        return hit
+
+    def _decode_fixed(self, segments_count, max_positions):
         """Key shares per decoded token for a batch of B with at most ``max_positions`` cached keys, as
         (shares in a cluster, clusters per token and KV head): as many CTAs as are resident at once (two per
         SM), never more, so that no CTA waits for a second wave, and no share shorter than
@@ -386,6 +396,19 @@ class AttentionPlanner(StepPlanner):
         for d in order[slots:]:
             heapq.heapreplace(busy, busy[0] + d)
         return max(busy)
+
+    def write_decode(self, starts, fixed, regions, first):
+        B, nsplit = len(starts), fixed[0] * fixed[1]
+        if first or nsplit > 1 or self.shape.window:
+            return super().write_decode(starts, fixed, regions, first)
+        # whole histories: nothing but the ends of the key ranges moves
+        regions["items"].reshape(B, self.chunks, ITEM_INTS)[:, :, 6] = (starts + 1)[:, None]
+        return self._facts(B * self.chunks, fixed)
+
+    def _facts(self, n_small: int, fixed) -> dict:
+        """The facts of a step of single tokens that are not split."""
+        return {"n_small": n_small, "n_big": 0, "part_rows_cap": 0, "any_split": False, "big_split": False,
+                "decode_nsplit": fixed[0] if self.chunks == 1 else 0, "decode_groups": fixed[1]}
 
     def plan_decode(self, starts, fixed):
         cluster, groups = fixed

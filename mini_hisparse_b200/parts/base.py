@@ -320,6 +320,16 @@ class StepPlanner:
         segments = [Segment(i, i, int(p), 1, i) for i, p in enumerate(starts)]
         return self.plan(segments, len(segments), fixed)
 
+    def write_decode(self, starts: np.ndarray, fixed, regions: dict[str, np.ndarray], first: bool) -> dict:
+        """plan_decode into ``regions`` (name -> words of a host buffer that holds this graph's plans and nothing else;
+        ``first``: nothing has been written there yet).  Returns the facts."""
+        arrays, facts = self.plan_decode(starts, fixed)
+        for name, region in regions.items():
+            if arrays[name].size != region.size:
+                raise ValueError(f"plan array {name!r} has {arrays[name].size} words, the layout holds {region.size}")
+            region[:] = arrays[name].reshape(-1)
+        return facts
+
 
 class Mixer(Part):
     def cache_need(self) -> CacheNeed | None:

@@ -233,3 +233,41 @@ def test_status_bits_have_messages():
     both = ModelRunner.status_message(4 | 8)
     assert "matrix product" in both and "TMA-fed attention" in both
     assert "0x40" in ModelRunner.status_message(64 | 1) and "vocabulary" in ModelRunner.status_message(64 | 1)
+
+
+@pytest.mark.parametrize("fixed", [(1, 1), (4, 1)])
+@pytest.mark.parametrize("window", [None, 40])
+def test_decode_arrays_written_again_into_a_graphs_buffers(fixed, window):
+    """The buffers of a captured decode step are written in place step after step: every word is what a buffer written for the
+    first time holds, and the plan's words are plan_decode's, whichever buffer of the ring has its turn."""
+    from mini_hisparse_b200.engine.step import _DecodeBuffers, _Layout
+
+    part = GQAttention(PartSpec.make("gq_attention", hidden_size=32, q_heads=40, kv_heads=2, head_dim=16, window=window,
+                                     position=PartSpec.make("none")))
+    cache = CacheManager([part.cache_need()], CacheConfig(num_pages=80, page_size=4, max_requests=3, dtype=torch.float32,
+                                                          device="cpu", allocate_storage=False))
+    batch = BatchBuilder(cache, "cpu", sm_count=8)
+    batch.add_user(0, part)
+    for name, n in zip("abc", (70, 1, 33)):
+        cache.open(name), cache.ensure(name, n), cache.advance(name, n)
+    planner = batch.slots[0].planner
+    caps = [planner.capacity(3, 3, fixed)]
+    layout = _Layout(3, 3, 3, [32], caps)
+    ring = _DecodeBuffers(layout, torch.device("cpu"))
+    for step in range(2 * ring.RING + 3):
+        entries = [StepEntry(r, [step + i], [0]) for i, r in enumerate("cab")]
+        segments, _ = batch.segments(entries)
+        for s in segments:
+            cache.ensure(s.request, s.start + 1)
+        starts = np.asarray([s.start for s in segments])
+        turn, fresh = ring.next(), _DecodeBuffers(layout, torch.device("cpu"))
+        facts = batch._fill_decode(ring.views[turn], entries, segments, [fixed], starts)
+        assert turn == step % ring.RING and facts == batch._fill_decode(fresh.views[0], entries, segments, [fixed], starts)
+        assert torch.equal(ring.rows[turn], fresh.rows[0])
+        arrays, plain = planner.plan_decode(starts, fixed)
+        assert facts == [plain]
+        for name, words in ring.views[turn]["plans"][0].items():
+            assert np.array_equal(words, arrays[name].reshape(-1))
+        assert ring.views[turn]["tables"][0].tolist() == cache.table_rows(0, [s.slot for s in segments], 32).tolist()
+        for r in "abc":
+            cache.advance(r, 1)
