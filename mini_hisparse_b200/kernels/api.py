@@ -887,6 +887,25 @@ def attention_tokens(q, cache, out, part_acc, part_ml, items, num_items, block_t
         c_int(cache.shape[0]), c_float(float(d) ** -0.5 if scale is None else scale), _stream()), "attention_tokens")
 
 
+ATTENTION_ROWS = 64        # query rows of attention_rows' tiles
+
+
+def attention_rows_supports(d: int) -> bool:
+    """Head sizes of attention_rows."""
+    return 4 <= d <= 128 and d % 4 == 0
+
+
+def attention_rows(q, cache, out, items, num_items, positions, block_table, *, nq, nkv, d, page_size, window=0, scale=None):
+    """attention_simt for unsplit items of up to ATTENTION_ROWS query rows (prompt portions), without options."""
+    lib = build.load("attention_rows")
+    if q.dtype != cache.dtype or q.dtype != out.dtype or not (q.is_contiguous() and cache.is_contiguous() and out.is_contiguous()):
+        raise KernelError("attention_rows: q, the pool and the output must be contiguous and of one dtype")
+    _check(lib, lib.mhb_attention_rows(
+        _ptr(q), _ptr(cache), _ptr(out), c_int(dtype_code(q.dtype)), _ptr(items), c_int(num_items), _ptr(positions),
+        _ptr(block_table), c_int(block_table.shape[-1]), c_int(nq), c_int(nkv), c_int(d), c_int(page_size), c_int(cache.shape[0]),
+        c_int(window or 0), c_float(float(d) ** -0.5 if scale is None else scale), _stream()), "attention_rows")
+
+
 def attention_combine(part_acc, part_ml, tok_part_row, tok_nsplit, out, *, nq, d, every=0, gate=None,
                       gate_nsplit=1, gate_split_stride=0, gate_per_head=False):
     """Merge the parts of every token's attention.  ``every`` > 0: each token has exactly that many parts,

@@ -32,7 +32,8 @@ NVCC_FLAGS = [
 # Every module the package has; __graft_entry__.build() compiles all of them.
 MODULES = ("elementwise", "gemm_simt", "gemm_f32", "gemm_tc", "attention_simt", "attention_mma", "attention_tma", "attention_decode",
            "attention_tc", "sampling", "postnorm", "lightning", "attention_mma_ext", "mixparts", "gateparts", "gatedlinear",
-           "moe", "maskparts", "deltarule", "timeconv", "selscan", "headconv", "sidebranch", "attention_tokens")
+           "moe", "maskparts", "deltarule", "timeconv", "selscan", "headconv", "sidebranch", "attention_tokens",
+           "attention_rows")
 
 
 class KernelBuildError(RuntimeError):

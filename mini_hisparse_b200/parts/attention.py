@@ -35,13 +35,18 @@ class AttentionShape:
     kv_heads: int
     window: int | None = None
     tile_rows: int = ROW_TILE
+    cuda_cores: bool = False      # short segments run on the CUDA-core kernel although long portions' tiles have more rows
+
+    @property
+    def simt(self) -> bool:
+        return self.cuda_cores or self.tile_rows == ROW_TILE
 
     def max_splits(self, keys: int) -> int:
         """How many splits ``keys`` keys are worth.  The tensor-core kernels walk 256 keys in the time a split costs to start
         and to merge.  The CUDA-core kernel (ROW_TILE rows for every portion) takes about 1 us for a tile of 32 keys; its merge
         is a launch of 2.5 to 3.7 us, and a plan with splits costs the host 15 us a step more: splits of 128 keys, once
         there are four (histories of 20 keys in a graph for 256, cut in four, took 13 % longer than uncut)."""
-        if self.tile_rows == ROW_TILE:
+        if self.simt:
             return keys // MIN_KEYS_PER_SIMT_SPLIT if keys >= 4 * MIN_KEYS_PER_SIMT_SPLIT else 1
         return max(1, keys // MIN_KEYS_PER_SPLIT)
 
@@ -105,7 +110,7 @@ def plan_attention(need: AttentionShape, segments, T: int, sm_count: int = 148,
     # SM, so that a long history beside short ones is cut into more parts and no CTA runs alone at
     # the end
     small_keys = sum(t[4] - t[3] for t in small_tiles) * len(small_chunks) * need.kv_heads
-    target = max(MIN_KEYS_PER_SIMT_SPLIT if need.tile_rows == ROW_TILE else MIN_KEYS_PER_SPLIT, -(-small_keys // (2 * sm_count)))
+    target = max(MIN_KEYS_PER_SIMT_SPLIT if need.simt else MIN_KEYS_PER_SPLIT, -(-small_keys // (2 * sm_count)))
     target = -(-target // KEY_TILE) * KEY_TILE
     items = []
     tok_part_row = np.zeros(T, np.int32)
@@ -472,14 +477,17 @@ class GQAttention(Mixer):
 
     def big_tile_rows(self, page_size: int) -> int:
         """Query rows per tile for long portions."""
-        return {"tc": 128, "mma": 64, "simt": ROW_TILE}[self.kernel_family(page_size)]
+        family = self.kernel_family(page_size)
+        if family == "simt" and K.attention_rows_supports(self.d):
+            return K.ATTENTION_ROWS
+        return {"tc": 128, "mma": 64, "simt": ROW_TILE}[family]
 
     def kernel_modules(self):
         """attention_simt holds the CUDA-core kernel and the merge of key splits; the tensor-core
         kernels come in for the head sizes they are built for (which of them runs depends on the
         page size, which the cache brings)."""
         if not self.tensor_core_attention:
-            return ("attention_simt", "attention_tokens")
+            return ("attention_simt", "attention_tokens", "attention_rows")
         if self.d in (64, 128):
             return ("attention_simt", "attention_mma", "attention_tma", "attention_decode", "attention_tc")
         return ("attention_simt", "attention_mma")
@@ -491,7 +499,8 @@ class GQAttention(Mixer):
         return ("gq_attention", self.nq, self.nkv, self.d, self.window)
 
     def planner(self, page_size: int, sm_count: int):
-        shape = AttentionShape(self.nq, self.nkv, self.window, self.big_tile_rows(page_size))
+        shape = AttentionShape(self.nq, self.nkv, self.window, self.big_tile_rows(page_size),
+                               cuda_cores=self.kernel_family(page_size) == "simt")
         if self.kernel_family(page_size) == "tc" and self.nq // self.nkv <= ROW_TILE:
             return AttentionPlanner(shape, sm_count, lambda n: K.attention_decode_max_clusters(self.d, n),
                                     K.DECODE_MAX_SPLITS, min_share=2 * KEY_TILE)
@@ -616,8 +625,14 @@ class GQAttention(Mixer):
         elif nsplit and K.attention_tokens_supports(self.nq, self.nkv, self.d) and cache.storage.data_ptr() % 16 == 0:
             K.attention_tokens(*args, meta["items"], n_small, meta["block_table"], meta["tok_part_row"], nq=self.nq, nkv=self.nkv,
                                d=self.d, page_size=cache.page_size, scale=self.scale)
-        elif n_small + n_big:
-            K.attention_simt(*args, meta["items"], n_small + n_big, n_small + n_big, *tail, **common)
+        else:
+            rows = n_big if K.attention_rows_supports(self.d) else 0       # these items were planned for its tiles
+            n = n_small + n_big - rows
+            if n:
+                K.attention_simt(*args, meta["items"], n, n, *tail, **common)
+            if rows:
+                K.attention_rows(q, cache.storage, attn, meta["items"][n_small * ITEM_INTS:], rows, ctx.positions,
+                                 meta["block_table"], **common)
         if meta["any_split"] and family == "simt":
             K.attention_combine(part_acc, part_ml, meta["tok_part_row"], meta["tok_nsplit"], attn,
                                 nq=self.nq, d=self.d)

@@ -673,6 +673,37 @@ def run_attention(nq, nkv, d, P_, seg_specs, dtype, window=None, fixed_nsplit=No
     return out.float().cpu(), ref, plan
 
 
+@pytest.mark.parametrize("nq,nkv,d,P_", [(3, 1, 32, 32), (28, 4, 128, 16), (16, 4, 64, 5), (8, 1, 100, 7), (5, 5, 4, 1), (70, 1, 8, 16)])
+@pytest.mark.parametrize("window", [None, 70])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_attention_rows(nq, nkv, d, P_, window, dtype):
+    """Prompt portions on the CUDA cores in tiles of 64 query rows: portions behind a history and at the start, ragged tiles,
+    keys around a tile of 32, more heads per KV head than a tile has rows, against 64 bits."""
+    from mini_hisparse_b200.parts.attention import AttentionShape, plan_attention
+
+    specs = [(0, 17), (0, 33), (31, 40), (64, 64), (100, 65), (5, 90)]
+    cache, table, segments, qs, ks, vs, positions = paged_case(nq, nkv, d, P_, specs, dtype)
+    T = sum(n for _, n in specs)
+    plan = plan_attention(AttentionShape(nq, nkv, window, 64, cuda_cores=True), segments, T, 148)
+    assert plan.n_small == 0 and plan.n_big and not plan.big_split
+    q = torch.cat([qq[h:] for qq, (h, n) in zip(qs, specs)]).reshape(T, nq * d).to(DEV)
+    out = torch.full((T + 1, nq * d), float("nan"), dtype=dtype, device=DEV)
+    K().attention_rows(q, cache, out[:T], torch.from_numpy(plan.items).to(DEV).reshape(-1), plan.n_big, positions, table, nq=nq, nkv=nkv,
+                       d=d, page_size=P_, window=window or 0)
+    ref = []
+    for qq, kk, vv, (h, n) in zip(qs, ks, vs, specs):
+        qq, kk, vv = (y.to(dtype).double() for y in (qq, kk, vv))
+        kk, vv = (y.repeat_interleave(nq // nkv, 1) for y in (kk, vv))
+        z = torch.einsum("qhd,khd->hqk", qq[h:], kk) * d ** -0.5
+        far = torch.arange(h, h + n)[:, None] - torch.arange(h + n)
+        z.masked_fill_((far < 0) | (far >= (window or 1 << 30)), -math.inf)
+        ref.append(torch.einsum("hqk,khd->qhd", torch.softmax(z, -1), vv).reshape(n, nq * d))
+    ref = torch.cat(ref)
+    assert bool(out[T].isnan().all())
+    torch.testing.assert_close(out[:T].double().cpu(), ref, atol=4e-6 if dtype == torch.float32 else 2.0 ** -8 * float(ref.abs().max()),
+                               rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-5)
+
+
 @pytest.mark.parametrize("nq,nkv,d,P_,nsplit", [(3, 1, 32, 32, 1), (4, 2, 16, 16, 3), (28, 4, 128, 16, 1), (16, 4, 64, 5, 4), (8, 1, 100, 7, 2),
                                                 (5, 5, 4, 1, 1)])
 @pytest.mark.parametrize("window", [None, 70])
