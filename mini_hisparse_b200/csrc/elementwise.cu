@@ -662,6 +662,23 @@ __global__ void swiglu_kernel(const IT* __restrict__ gu, int nsplit, size_t spli
     out[idx] = from_float<OT>(s * u);
 }
 
+// The same four elements a thread (I and block in steps of 4, rows on 16 bytes), a row of CTAs per token: no 64-bit divisions, wide
+// loads.  562 rows of 18,944 float32: 23.4 us,
+// 54.8 with an element a thread.
+template <typename IT, typename OT>
+__global__ void swiglu_vec_kernel(const IT* __restrict__ gu, int nsplit, size_t split_stride, OT* __restrict__ out, int I, int block) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int i = 4 * ((int)blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= I) return;
+    const size_t t = blockIdx.y;
+    const int gcol = block == I ? i : (i / block) * 2 * block + i % block;
+    const IT* p = gu + t * 2 * I + gcol;
+    const float4 g = sum_parts4<2>(p, nsplit, split_stride), u = sum_parts4<2>(p + block, nsplit, split_stride);
+    store4<OT>(out + t * I + i, make_float4(g.x / (1.f + expf(-g.x)) * u.x, g.y / (1.f + expf(-g.y)) * u.y,
+                                            g.z / (1.f + expf(-g.z)) * u.z, g.w / (1.f + expf(-g.w)) * u.w));
+}
+
 MHB_EXPORT int mhb_swiglu(const void* gu, int in_dtype, int nsplit, long long split_stride,
                           void* out, int out_dtype, int T, int I, int block, cudaStream_t stream) {
     if (T <= 0) return 0;
@@ -669,6 +686,12 @@ MHB_EXPORT int mhb_swiglu(const void* gu, int in_dtype, int nsplit, long long sp
     if (nsplit > 1 && in_dtype != MHB_F32) return fail("swiglu: split partials must be float32");
     const size_t total = (size_t)T * I;
     const int threads = 256;
+    if (I % 4 == 0 && block % 4 == 0 && split_stride % 4 == 0 && T <= 65535 && !(((uintptr_t)gu | (uintptr_t)out) & 15)) {
+        MHB_DISPATCH_DTYPE(in_dtype, IT, MHB_DISPATCH_DTYPE(out_dtype, OT,
+            launch_kernel(swiglu_vec_kernel<IT, OT>, dim3((I / 4 + threads - 1) / threads, T), dim3(threads), 0, stream, (const IT*)gu,
+                          nsplit, (size_t)split_stride, (OT*)out, I, block)));
+        return check_launch("swiglu");
+    }
     const unsigned blocks = (unsigned)((total + threads - 1) / threads);
     MHB_DISPATCH_DTYPE(in_dtype, IT, MHB_DISPATCH_DTYPE(out_dtype, OT,
         launch_kernel(swiglu_kernel<IT, OT>, dim3(blocks), dim3(threads), 0, stream, (const IT*)gu, nsplit,

@@ -421,6 +421,20 @@ def test_gemm_tiles_of_features(M, N, K_, epilogue):
         torch.testing.assert_close(out[:M].float(), y, atol=2.0 ** -8 * float(y.abs().max()), rtol=2.0 ** -8)
 
 
+@pytest.mark.parametrize("T,I,block,nsplit", [(1, 4, 4, 1), (3, 1020, 1020, 1), (5, 1028, 4, 3), (562, 304, 16, 1), (2, 176, 16, 9), (7, 102, 102, 2),
+                                              (3, 30, 6, 1)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_swiglu_four_at_a_time(T, I, block, nsplit, dtype):
+    """silu(gate) * up in both layouts, in widths that are taken four elements at a time and widths that are not, from parts."""
+    parts = rnd(nsplit, T, 2 * I, seed=T + I)
+    out = torch.full((T + 1, I), float("nan"), dtype=dtype, device=DEV)
+    K().swiglu(parts if nsplit > 1 else parts[0], out[:T], nsplit=nsplit, split_stride=parts.stride(0), block=block)
+    g, u = parts.double().sum(0).view(T, -1, 2, block).unbind(2)
+    ref = (torch.nn.functional.silu(g) * u).reshape(T, I)
+    assert bool(out[T].isnan().all())
+    torch.testing.assert_close(out[:T].double(), ref, atol=1e-5, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-5)
+
+
 def test_gemm_tensor_core_refuses_unaligned_k():
     from mini_hisparse_b200.kernels.api import KernelError
 
