@@ -154,9 +154,11 @@ side_branch_kernel(const SideArgs a) {
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t0 + tb < a.T) {
             const size_t at = (size_t)(t0 + tb) * W + col0 + c;
-            const float4 v = vec4(a.x + at);
             s = sum_parts4<8>(a.delta + at, a.nsplit, a.split_stride);
-            s.x = fmaf(a.alpha, v.x, s.x); s.y = fmaf(a.alpha, v.y, s.y); s.z = fmaf(a.alpha, v.z, s.z); s.w = fmaf(a.alpha, v.w, s.w);
+            if (a.alpha != 0.f) {
+                const float4 v = vec4(a.x + at);
+                s.x = fmaf(a.alpha, v.x, s.x); s.y = fmaf(a.alpha, v.y, s.y); s.z = fmaf(a.alpha, v.z, s.z); s.w = fmaf(a.alpha, v.w, s.w);
+            }
         }
         *(float4*)(rows + tb * S + c) = s;
         const float ss = warp_sum(squares(s));

@@ -868,6 +868,13 @@ def test_side_branch_in_one_kernel(T, W, D, nsplit, alpha, keep):
     assert not K.side_branch_takes(torch.empty(65 if W <= 2048 else 33, W, device="cuda"), gate.cuda(), proj.cuda(), table.cuda())
     assert not K.side_branch_takes(torch.empty(T, W + 512, device="cuda"), gate.cuda(), proj.cuda(), table.cuda())
     assert not K.side_branch_takes(xd, torch.zeros(72, W, device="cuda").bfloat16(), proj.cuda(), table.cuda())
+    if alpha == 0.0:        # the stream is left out of the norm, whatever it holds
+        lost = x.clone()
+        lost[0, 0] = math.inf
+        again = lost.cuda()
+        K.side_branch(again, w1.cuda(), 1e-5, gate.cuda(), proj.cuda(), table.cuda(), D, tokens.cuda(), w2.cuda(), 1e-5, copy[:T],
+                      delta=parts.cuda(), nsplit=nsplit, split_stride=T * W, alpha=0.0, keep=0.0, status=status)
+        assert bool(again.isfinite().all())
     tokens[0] = 50          # outside the table: reported, and its row gets no branch
     K.side_branch(x.cuda(), w1.cuda(), 1e-5, gate.cuda(), proj.cuda(), table.cuda(), D, tokens.cuda(), w2.cuda(), 1e-5, copy[:T],
                   delta=parts.cuda(), nsplit=nsplit, split_stride=T * W, alpha=alpha, keep=keep, status=status)
