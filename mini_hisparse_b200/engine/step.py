@@ -111,16 +111,16 @@ class _PlanSlot:
 class _DecodeBuffers:
     """A captured step's pinned host buffers, used in turn: what does not change from step to step (the order of the tokens,
     the items' heads and splits) is written once per buffer.  An event per half of the ring says when its copies are done: it
-    is recorded when the ring moves on to the other half, so three steps of four pay for no event at all."""
-
-    RING = 8
+    is recorded when the ring moves on to the other half, so with eight buffers three steps of four pay for no event at all.
+    Beyond 64 KB they are two: pinned memory is not for keeping."""
 
     def __init__(self, layout: _Layout, device: torch.device):
-        host = torch.empty((self.RING, layout.total), dtype=torch.int32)
+        self.ring = 8 if layout.total <= 1 << 14 else 2
+        host = torch.empty((self.ring, layout.total), dtype=torch.int32)
         self.cuda = torch.cuda.is_available()
         host = host.pin_memory() if self.cuda else host
         B = layout.T
-        self.rows = [host[i] for i in range(self.RING)]
+        self.rows = [host[i] for i in range(self.ring)]
         self.views = []
         for row in self.rows:
             a = row.numpy()
@@ -140,9 +140,9 @@ class _DecodeBuffers:
 
     def next(self) -> int:
         i = self.turn
-        self.turn = (i + 1) % self.RING
+        self.turn = (i + 1) % self.ring
         if self.cuda:
-            half = self.RING // 2
+            half = self.ring // 2
             now = torch._C._cuda_getCurrentRawStream(self.device)
             if self.stream is not None and now != self.stream:
                 torch.cuda.synchronize()        # the ring's copies lie on another stream than the next ones

@@ -254,7 +254,7 @@ def test_decode_arrays_written_again_into_a_graphs_buffers(fixed, window):
     caps = [planner.capacity(3, 3, fixed)]
     layout = _Layout(3, 3, 3, [32], caps)
     ring = _DecodeBuffers(layout, torch.device("cpu"))
-    for step in range(2 * ring.RING + 3):
+    for step in range(2 * ring.ring + 3):
         entries = [StepEntry(r, [step + i], [0]) for i, r in enumerate("cab")]
         segments, _ = batch.segments(entries)
         for s in segments:
@@ -262,7 +262,7 @@ def test_decode_arrays_written_again_into_a_graphs_buffers(fixed, window):
         starts = np.asarray([s.start for s in segments])
         turn, fresh = ring.next(), _DecodeBuffers(layout, torch.device("cpu"))
         facts = batch._fill_decode(ring.views[turn], entries, segments, [fixed], starts)
-        assert turn == step % ring.RING and facts == batch._fill_decode(fresh.views[0], entries, segments, [fixed], starts)
+        assert turn == step % ring.ring and facts == batch._fill_decode(fresh.views[0], entries, segments, [fixed], starts)
         assert torch.equal(ring.rows[turn], fresh.rows[0])
         arrays, plain = planner.plan_decode(starts, fixed)
         assert facts == [plain]
