@@ -3,8 +3,8 @@
 //
 // attention_simt.cu deals a tile's query ROWS to its warps, which suits prompts: a decoded token has 1 to 8 rows per KV
 // head, so most warps had nothing to do and the others walked every key in turn, some 900 instructions of a lone warp
-// per 32 keys.  Here a CTA of 8 warps holds one token (or one of its key splits) and one KV head, and the KEYS are dealt:
-// a warp takes every eighth run of 32 keys with all rows, keys and values straight from the cache (a lane a key, then
+// per 32 keys.  Here a CTA of 16 warps holds one token (or one of its key splits) and one KV head, and the KEYS are dealt:
+// a warp takes every sixteenth run of 32 keys with all rows, keys and values straight from the cache (a lane a key, then
 // lanes along a value row), and the warps' (maximum, sum, accumulator) meet once at the end.
 // Items are those of attention_simt.cu with one token and all heads of the group; splits leave un-normalised partials.
 #include "common.cuh"
@@ -14,7 +14,7 @@ using namespace mhb;
 MHB_EXPORT const char* mhb_last_error() { return error_buffer(); }
 
 namespace {
-constexpr int WARPS = 8;
+constexpr int WARPS = 16;
 constexpr int RUN = 32;          // keys of a warp at a time: one per lane
 constexpr int ITEM_INTS = 8;
 
@@ -84,9 +84,9 @@ attention_tokens_kernel(const TokenArgs a) {
 #pragma unroll
         for (int r = 0; r < G; ++r) {
             const float x = lane < keys ? (row >= 0 ? s[r] * a.scale : 0.f) : -INFINITY;
-            const float m_new = fmaxf(m[r], warp_max(x));          // a run holds at least one key
-            const float alpha = expf(m[r] - m_new);
-            p[r] = expf(x - m_new);
+            const float m_new = fmaxf(m[r], warp_max(x)), m_use = m_new == -INFINITY ? 0.f : m_new;
+            const float alpha = expf(m[r] - m_use);
+            p[r] = expf(x - m_use);
             m[r] = m_new;
             l[r] = l[r] * alpha + p[r];                            // this lane's keys; the lanes' sums meet at the end
 #pragma unroll

@@ -56,7 +56,9 @@ __device__ __forceinline__ float4 load4_now(const float* p) {
 }
 
 // KS warps of a CTA share NR features (each walks every KS-th stretch of 128 elements of K); R_WARPS / KS groups a CTA.
-template <int MT, int NR>
+// GATED: W holds N / 2 gate rows and as many up rows behind them; features are pairs of one of each, and C gets
+// silu(gate) * up [M, N / 2] (a launch less behind every gate/up product of a decode step: 1.5 us).
+template <int MT, int NR, bool GATED>
 __global__ void __launch_bounds__(R_WARPS * 32, 2)
 gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C, int M, int N, int K,
                      long long lda, long long ldw, long long ldc, int KS) {
@@ -68,7 +70,10 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     int k = ks * 128 + lane * 4;
     const float* wp[NR];
 #pragma unroll
-    for (int j = 0; j < NR; ++j) wp[j] = W + (size_t)min(n0 + j, N - 1) * ldw;
+    for (int j = 0; j < NR; ++j) {
+        const int n = min(n0 + j, N - 1);
+        wp[j] = W + (size_t)(GATED ? (n >> 1) + (n & 1) * (N >> 1) : n) * ldw;
+    }
     float4 w[NR];
     pdl_launch_dependents();
 #pragma unroll
@@ -112,7 +117,12 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         for (int j = 0; j < NR; ++j)
 #pragma unroll
             for (int m = 0; m < MT; ++m)
-                if (lane == j * MT + m && n0 + j < N && m < M) C[(size_t)m * ldc + n0 + j] = acc[j][m];
+                if constexpr (GATED) {
+                    if (j % 2 == 0 && lane == j * MT + m && n0 + j < N && m < M)
+                        C[(size_t)m * ldc + (n0 + j) / 2] = acc[j][m] / (1.f + expf(-acc[j][m])) * acc[j + 1 < NR ? j + 1 : j][m];
+                } else if (lane == j * MT + m && n0 + j < N && m < M) {
+                    C[(size_t)m * ldc + n0 + j] = acc[j][m];
+                }
         return;
     }
     if (lane == 0) {
@@ -127,11 +137,18 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         const int n = (blockIdx.x * groups + g) * NR + jm / MT, m = jm % MT;
         float s = 0.f;
         for (int x = 0; x < KS; ++x) s += part[g * KS + x][jm];
-        if (n < N && m < M) C[(size_t)m * ldc + n] = s;
+        if constexpr (GATED) {
+            if (n & 1) continue;
+            float u = 0.f;
+            for (int x = 0; x < KS; ++x) u += part[g * KS + x][jm + MT];
+            if (n < N && m < M) C[(size_t)m * ldc + n / 2] = s / (1.f + expf(-s)) * u;
+        } else {
+            if (n < N && m < M) C[(size_t)m * ldc + n] = s;
+        }
     }
 }
 
-template <int MT, int NR>
+template <int MT, int NR, bool GATED = false>
 int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
                 cudaStream_t stream) {
     // Warps that share a feature's K range: enough to give every SM about two CTAs' worth of loads in flight, none with
@@ -139,7 +156,7 @@ int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, l
     int ks = 1;
     while (ks < R_WARPS && (long long)((N + NR - 1) / NR) * ks < 148 * 2 * R_WARPS && K >= 512 * ks) ks *= 2;
     const int per_cta = R_WARPS / ks * NR;
-    launch_kernel(gemm_f32_rows_kernel<MT, NR>, dim3((N + per_cta - 1) / per_cta), dim3(R_WARPS * 32), 0, stream, A, W, C,
+    launch_kernel(gemm_f32_rows_kernel<MT, NR, GATED>, dim3((N + per_cta - 1) / per_cta), dim3(R_WARPS * 32), 0, stream, A, W, C,
                   M, N, K, lda, ldw, ldc, ks);
     return check_launch("gemm_f32 (rows)");
 }
@@ -449,4 +466,21 @@ MHB_EXPORT int mhb_gemm_f32(const float* A, const float* W, float* C, int M, int
     if (bn == 128) return launch_split<128, 4, 2, 1>(A, W, C, M, N, K, lda, ldw, ldc, nsplit, split_stride, parts, status, stream);
     if (bn == 192) return launch_split<192, 4, 2, 1>(A, W, C, M, N, K, lda, ldw, ldc, nsplit, split_stride, parts, status, stream);
     return fail("gemm_f32: tiles of 64, 128 or 192 tokens, not %d", bn);
+}
+
+// C[M, I] = silu(A Wg^T) * (A Wu^T) for up to 8 tokens; W [2 I, K] holds the gate rows, then the up rows.
+MHB_EXPORT int mhb_gemm_f32_glu(const float* A, const float* W, float* C, int M, int I, int K, long long lda, long long ldw,
+                                long long ldc, cudaStream_t stream) {
+    if (M <= 0 || I <= 0) return 0;
+    if (M > 8) return fail("gemm_f32_glu: %d tokens", M);
+    if (K <= 0 || K % 8 || lda % 4 || ldw % 4 || (((uintptr_t)A | (uintptr_t)W) & 15))
+        return fail("gemm_f32_glu: K %d in steps of 8, rows (%lld, %lld) in steps of 4, operands on 16 bytes", K, lda, ldw);
+    const int N = 2 * I;
+    const bool wide = N >= 4 * 148 * 4;
+#define MHB_GLU(MT) return wide ? launch_rows<MT, 4, true>(A, W, C, M, N, K, lda, ldw, ldc, stream) : launch_rows<MT, 2, true>(A, W, C, M, N, K, lda, ldw, ldc, stream)
+    if (M == 1) MHB_GLU(1);
+    if (M == 2) MHB_GLU(2);
+    if (M <= 4) MHB_GLU(4);
+    MHB_GLU(8);
+#undef MHB_GLU
 }

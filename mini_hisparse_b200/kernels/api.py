@@ -383,6 +383,17 @@ def gemm_f32(a, w, out, bn=0, nsplit=1, split_stride=0, parts=None, status=None)
                                  c_longlong(split_stride), _ptr(parts), _ptr(status), _stream()), "gemm_f32")
 
 
+def gemm_f32_glu(a, w, out):
+    """out[M, I] = silu(a Wg^T) * (a Wu^T) in float32 for up to 8 tokens; ``w`` [2 I, K] holds the gate rows, then the up rows."""
+    lib = build.load("gemm_f32")
+    M, K = a.shape
+    I = out.shape[1]
+    if any(t.dtype != torch.float32 or t.stride(-1) != 1 for t in (a, w, out)) or tuple(w.shape) != (2 * I, K):
+        raise KernelError(f"gemm_f32_glu: a is [{M},{K}], w {list(w.shape)}, out {list(out.shape)}; float32 rows")
+    _check(lib, lib.mhb_gemm_f32_glu(_ptr(a), _ptr(w), _ptr(out), c_int(M), c_int(I), c_int(K), c_longlong(a.stride(0)),
+                                     c_longlong(w.stride(0)), c_longlong(out.stride(0)), _stream()), "gemm_f32_glu")
+
+
 STREAM_K_PARTIAL_FLOATS = 2 * 160 * 128 * 256     # workspace of the persistent product: two tiles per CTA
 STREAM_K_FLAGS = 4 << 16                            # a counter for each quarter of each tile
 
@@ -877,7 +888,7 @@ def attention_tokens_supports(nq: int, nkv: int, d: int) -> bool:
 def attention_tokens(q, cache, out, part_acc, part_ml, items, num_items, block_table, tok_part_row, *, nq, nkv, d, page_size,
                      scale=None):
     """attention_simt for items of single tokens with all heads of their KV heads, without options: the keys of an item are
-    dealt to eight warps."""
+    dealt to sixteen warps."""
     lib = build.load("attention_tokens")
     if q.dtype != cache.dtype or q.dtype != out.dtype or not (q.is_contiguous() and cache.is_contiguous() and out.is_contiguous()):
         raise KernelError("attention_tokens: q, the pool and the output must be contiguous and of one dtype")

@@ -17,7 +17,7 @@ KEY_TILE = 64          # split boundaries are multiples of the kernels' key tile
 ITEM_INTS = 8
 MIN_KEYS_PER_SPLIT = 256
 MIN_KEYS_PER_SIMT_SPLIT = 128
-KEYS_PER_TOKEN_SPLIT = 512     # attention_tokens: two rounds of its eight warps; a merge is a launch
+KEYS_PER_TOKEN_SPLIT = 512     # attention_tokens: one round of its sixteen warps; a merge is a launch
 SPLIT_MAX_TOKENS = 16  # only short segments (decode tokens, tiny portions) are split along the keys
 MAX_SPLITS = 64
 MAX_BIG_SPLITS = 8       # key splits of a long portion's tile (tcgen05 kernel only)

@@ -234,6 +234,21 @@ def test_gemm_f32(M, N, K_, bn, nsplit, kind):
     assert ((got - ref).abs() <= room)[fine].all()
 
 
+@pytest.mark.parametrize("M,I,K_", [(1, 3, 40), (2, 256, 96), (4, 256, 96), (3, 1183, 3584), (5, 1185, 200), (8, 4000, 1024), (7, 33, 4096)])
+def test_gemm_f32_gate_in_the_product(M, I, K_):
+    """silu(x Wg^T) * (x Wu^T) of few tokens in one kernel, two and four features a warp, K shared by warps or not, against 64
+    bits: each sum within its bound, carried through the gate (whose slope is below 1.1)."""
+    x, w = rnd(M, K_, seed=1), rnd(2 * I, K_, seed=2, scale=K_ ** -0.5)
+    out = torch.full((M + 1, I), float("nan"), device=DEV)
+    K().gemm_f32_glu(x, w, out[:M])
+    g, u = (x.double() @ w.double().T).split(I, 1)
+    eg, eu = ((-(-K_ // 32) + 17) * 2.0 ** -24 * (x.abs().double() @ w.abs().double().T)).split(I, 1)
+    room = 1.1 * eg * u.abs() + g.abs() * eu + 8 * 2.0 ** -24 * (g * u).abs() + 1e-30
+    assert bool(out[M].isnan().all()) and ((out[:M].double() - torch.nn.functional.silu(g) * u).abs() <= room).all()
+    with pytest.raises(Exception, match="gemm_f32_glu"):
+        K().gemm_f32_glu(rnd(9, K_, seed=1), w, torch.empty(9, I, device=DEV))
+
+
 def test_gemm_f32_takes():
     """What the float32 kernels do not take is refused by the entry point and known beforehand."""
     a, w = rnd(20, 64, seed=1), rnd(30, 64, seed=2)
@@ -716,6 +731,39 @@ def test_attention_rows(nq, nkv, d, P_, window, dtype):
     assert bool(out[T].isnan().all())
     torch.testing.assert_close(out[:T].double().cpu(), ref, atol=4e-6 if dtype == torch.float32 else 2.0 ** -8 * float(ref.abs().max()),
                                rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-5)
+
+
+def test_attention_tokens_scores_beyond_float32():
+    """A run of keys whose scores are all minus infinity leaves what the other keys give; a token with no other keys gets zeros
+    (as from attention_simt)."""
+    from mini_hisparse_b200.parts.attention import AttentionShape, plan_decode
+
+    lengths, d, P_ = [40, 20, 600], 32, 32
+    need = [-(-n // P_) for n in lengths]
+    table = torch.full((3, max(need)), -1, dtype=torch.int32)
+    for i, n in enumerate(need):
+        table[i, :n] = torch.arange(sum(need[:i]), sum(need[:i]) + n)
+    cache = torch.randn(sum(need), 2, 1, P_, d, generator=torch.Generator().manual_seed(1))
+    q = torch.zeros(3, 2, d)
+    q[..., 0], q[:, 1, 0] = 1e30, -1e30
+    cache[:, 0, ..., 0] = -1e30                 # -inf for the first head, inf for the second
+    cache[[1, 4], 0, :, :, 0] = 0.0             # the second page of the first and of the third request
+    plan = plan_decode(AttentionShape(2, 1), np.asarray(lengths) - 1, 1)
+    outs = []
+    for tokens in (True, False):
+        out, items = torch.empty(3, 2 * d, device=DEV), torch.from_numpy(plan.items).to(DEV).reshape(-1)
+        parts = torch.zeros(1, 2, d, device=DEV), torch.zeros(1, 2, 2, device=DEV)
+        tpr, pos = torch.zeros(3, dtype=torch.int32, device=DEV), torch.tensor(lengths, dtype=torch.int32, device=DEV) - 1
+        if tokens:
+            K().attention_tokens(q.to(DEV), cache.to(DEV), out, *parts, items, 3, table.to(DEV), tpr, nq=2, nkv=1, d=d, page_size=P_)
+        else:
+            K().attention_simt(q.to(DEV), cache.to(DEV), out, *parts, items, 3, 3, pos, table.to(DEV), tpr, nq=2, nkv=1, d=d, page_size=P_)
+        outs.append(out.view(3, 2, d).cpu())
+    got, ref = outs
+    assert bool(got[:, 0].isfinite().all()) and bool((got[1, 0] == 0).all())
+    torch.testing.assert_close(got[:, 0], ref[:, 0], atol=1e-5, rtol=1e-5)
+    for n, page in ((8, 1), (32, 4)):           # the mean of the keys whose scores are finite (zero)
+        torch.testing.assert_close(got[0 if page == 1 else 2, 0], cache[page, 1, 0, :n].mean(0), atol=1e-5, rtol=1e-5)
 
 
 @pytest.mark.parametrize("nq,nkv,d,P_,nsplit", [(3, 1, 32, 32, 1), (4, 2, 16, 16, 3), (28, 4, 128, 16, 1), (16, 4, 64, 5, 4), (8, 1, 100, 7, 2),
