@@ -698,3 +698,26 @@ MHB_EXPORT int mhb_swiglu(const void* gu, int in_dtype, int nsplit, long long sp
                                                             (size_t)split_stride, (OT*)out, I, block, total)));
     return check_launch("swiglu");
 }
+
+// Everything launched on `stream` from here on starts when all that is in front of it has finished, whatever its launch
+// allows (see join_branch in parts/base.py).  In a capture: an empty node, which costs the device nothing; what follows
+// depends on it alone.  Else a launch without the programmatic attribute, beside which its successor may start.
+static __global__ void mark_kernel() { pdl_launch_dependents(); }
+
+MHB_EXPORT int mhb_mark(cudaStream_t stream) {
+    cudaStreamCaptureStatus status;
+    cudaGraph_t graph = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t n = 0;
+    cudaError_t e = cudaStreamGetCaptureInfo_v2(stream, &status, nullptr, &graph, &deps, &n);
+    if (e == cudaSuccess && status == cudaStreamCaptureStatusActive) {
+        cudaGraphNode_t node;
+        e = cudaGraphAddEmptyNode(&node, graph, deps, n);
+        if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(stream, &node, 1, cudaStreamSetCaptureDependencies);
+        if (e != cudaSuccess) return fail("mark: %s", cudaGetErrorString(e));
+        return 0;
+    }
+    if (e != cudaSuccess) return fail("mark: %s", cudaGetErrorString(e));
+    mark_kernel<<<1, 32, 0, stream>>>();
+    return check_launch("mark");
+}

@@ -105,6 +105,12 @@ def embed_norm(table, weight, eps, tokens, out, status=None):
                                    _ptr(out), c_int(T), c_int(H), c_int(table.shape[0]), _ptr(status), _stream()), "embed_norm")
 
 
+def mark():
+    """What is launched on the current stream from here on starts when all that is in front of it has finished (see join_branch)."""
+    lib = build.load("elementwise")
+    _check(lib, lib.mhb_mark(_stream()), "mark")
+
+
 def norm_mix(x, weight, eps, *, delta=None, nsplit=1, split_stride=0, alpha=1.0, keep=0.0, copy=None):
     """x <- keep * x + rms(alpha * x + delta) * weight, row by row in float32, in place; ``copy`` (compute
     dtype, same shape) receives the new rows too.  alpha = 0 leaves x out of the norm (a normalised branch

@@ -616,7 +616,7 @@ class GQAttention(Mixer):
                     long_portions()
                     join.record(side)
                 short_segments()
-                join_branch(main, join, ws)
+                join_branch(main, join)
             else:
                 if n_small:
                     short_segments()

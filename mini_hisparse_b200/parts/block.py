@@ -158,7 +158,7 @@ class ParallelBlock(Block):
             f = self.feed_forward.forward(h, ctx)
             join.record(branch)
         a = self.mixer.forward(h, ctx, cache)
-        join_branch(main, join, ctx.ws)
+        join_branch(main, join)
         return Product(a.tensor, a.nsplit, also=f)
 
 

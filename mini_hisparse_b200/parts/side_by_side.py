@@ -99,5 +99,5 @@ class SideBySide(Mixer):
             b = self.right.forward_projected(proj, self.col, ctx, right_view, "mix_out_right")
             join.record(branch)
         a = self.left.forward_projected(proj, 0, ctx, left_view, "mix_out")
-        join_branch(main, join, ctx.ws)
+        join_branch(main, join)
         return Product(a.tensor, a.nsplit, also=b)

@@ -31,6 +31,8 @@ class SinkAttention(Mixer):
     Scores, softmax, norms and angles are float32; q, k and v are kept in the compute dtype.
     """
 
+    merges_in_clusters = True       # key splits of decoded tokens, where the kernel can
+
     def __init__(self, spec: PartSpec, rt=None):
         super().__init__(spec, rt)
         self.hidden = int(spec["hidden_size"])
@@ -83,7 +85,8 @@ class SinkAttention(Mixer):
     def planner(self, page_size: int, sm_count: int):
         family = self.kernel_family(page_size)
         shape = AttentionShape(self.nq, self.nkv, self.window, {"tc": 128, "mma": 64, "simt": ROW_TILE}[family])
-        return tma_planner(shape, sm_count, self.dk) if family == "tc" else AttentionPlanner(shape, sm_count)
+        clusters = family == "tc" and self.merges_in_clusters
+        return tma_planner(shape, sm_count, self.dk) if clusters else AttentionPlanner(shape, sm_count)
 
     def parameters(self):
         p = {"q": ParamSpec((self.qw, self.hidden)), "g": ParamSpec((self.ow, self.hidden)),
@@ -145,7 +148,8 @@ class SinkAttention(Mixer):
                                         page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                         sink=sink, slopes=slopes, **gate, tok_nsplit=meta["tok_nsplit"], counters=counters,
                                         status=ctx.status, fresh=SPLIT_MAX_TOKENS,
-                                        cluster=tma_cluster(meta, self.dk, self.nq // self.nkv))
+                                        cluster=(tma_cluster(meta, self.dk, self.nq // self.nkv)
+                                                 if self.merges_in_clusters else 0))
                 else:
                     K.attention_mma_ext(*args, meta["items"], n_small, 16, *tail, **common,
                                         tok_nsplit=meta["tok_nsplit"], counters=counters)
