@@ -385,7 +385,7 @@ class ModelRunner:
         self.stats = {"steps": 0, "tokens": 0, "graph_steps": 0, "graph_captures": 0, "two_stream_layers": 0,
                       "prepared_steps": 0, "graph_deferred": 0}
         self._ahead = None      # index arrays of the next decode step, packed while the GPU ran this one
-        build.build_all(model.kernel_modules())
+        build.build_all([m for m in model.kernel_modules() if not build.is_loaded(m)])
 
     def _cache_views(self, views) -> list[CacheView | None]:
         out = []

@@ -151,6 +151,12 @@ def load(module: str) -> ctypes.CDLL:
     return lib
 
 
+def is_loaded(module: str) -> bool:
+    """This process has the module's library already (its source needs no second look)."""
+    with _lock:
+        return module in _loaded
+
+
 def build_all(modules=MODULES, jobs: int | None = None) -> list[Path]:
     """Compile several modules in parallel (used before a model's first step and by build())."""
     modules = list(modules)
