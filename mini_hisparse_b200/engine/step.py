@@ -110,9 +110,9 @@ class _PlanSlot:
 
 class _DecodeBuffers:
     """A captured step's pinned host buffers, used in turn: what does not change from step to step (the order of the tokens,
-    the items' heads and splits) is written once per buffer.  An event per half of the ring says when its copies are done: it
-    is recorded when the ring moves on to the other half, so with eight buffers three steps of four pay for no event at all.
-    Beyond 64 KB they are two: pinned memory is not for keeping."""
+    the items' heads and splits) is written once per buffer.  A buffer is written again (``next``) when the event that was
+    recorded behind its copy (``sent``) has passed.  An event stands behind every half of a ring's worth of copies, so with
+    eight buffers three steps of four pay for none.  Beyond 64 KB they are two: pinned memory is not for keeping."""
 
     def __init__(self, layout: _Layout, device: torch.device):
         self.ring = 8 if layout.total <= 1 << 14 else 2
@@ -134,27 +134,46 @@ class _DecodeBuffers:
                 plans=[{name: a[at[name] : at[name] + n] for name, n in caps.items()} for at, caps in zip(layout.plans, layout.plan_caps)],
                 first=True))
         self.turn = 0
-        self.events = [None, None]
         self.device = device.index if device.index is not None or not self.cuda else torch.cuda.current_device()
-        self.stream = None          # the stream of the copies since the last event
+        self.guards = [None] * self.ring      # the event behind a buffer's last copy (None: nothing to wait for)
+        self.pending = []                     # buffers with a queued copy and no event behind it yet
+        self.spare = []                       # events that guard nothing
+        self.stream = None                    # the stream of the last copy
+        self.each = False                     # the steps have changed streams: from then on an event per copy
 
     def next(self) -> int:
+        """The buffer whose turn it is; nothing reads it any more."""
         i = self.turn
         self.turn = (i + 1) % self.ring
-        if self.cuda:
-            half = self.ring // 2
-            now = torch._C._cuda_getCurrentRawStream(self.device)
-            if self.stream is not None and now != self.stream:
-                torch.cuda.synchronize()        # the ring's copies lie on another stream than the next ones
-            self.stream = now
-            if i % half == 0:
-                before, mine = 1 - i // half, i // half
-                if self.events[before] is None:
-                    self.events[before] = torch.cuda.Event()
-                self.events[before].record()
-                if self.events[mine] is not None:
-                    self.events[mine].synchronize()
+        if i in self.pending:               # what was packed since its copy has been dropped
+            torch.cuda.synchronize(self.device)
+            self.pending.clear()
+        elif self.guards[i] is not None:
+            passed = self.guards[i]
+            passed.synchronize()
+            self.spare.append(passed)
+            self.guards = [None if e is passed else e for e in self.guards]
         return i
+
+    def sent(self, i: int) -> None:
+        """Buffer ``i``'s copy has just been queued on the current stream."""
+        if not self.cuda:
+            return
+        now = torch._C._cuda_getCurrentRawStream(self.device)
+        if now != self.stream:
+            if self.stream is not None:
+                self.each = True
+            if self.pending:                # their copies lie on the other stream
+                torch.cuda.synchronize(self.device)
+                self.pending.clear()
+            self.stream = now
+        self.pending.append(i)
+        if self.each or len(self.pending) >= self.ring // 2:
+            behind = self.spare.pop() if self.spare else torch.cuda.Event()
+            behind.record()
+            for p in self.pending:
+                self.guards[p] = behind
+            self.pending.clear()
 
 
 class _DecodeGraph:
@@ -529,6 +548,7 @@ class ModelRunner:
             elif facts != g.facts:
                 raise StepError(f"a decode plan changed after its graph was captured: {facts} vs {g.facts}")
         g.meta.copy_(g.buffers.rows[turn], non_blocking=True)
+        g.buffers.sent(turn)
         if device_tokens is not None:
             g.meta[layout.tokens : layout.tokens + B].copy_(device_tokens)
         if g.graph is None:

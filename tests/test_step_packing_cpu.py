@@ -271,3 +271,103 @@ def test_decode_arrays_written_again_into_a_graphs_buffers(fixed, window):
         assert ring.views[turn]["tables"][0].tolist() == cache.table_rows(0, [s.slot for s in segments], 32).tolist()
         for r in "abc":
             cache.advance(r, 1)
+
+
+class LazyGPU:
+    """Streams that run what is queued on them as late as they may: at a synchronise, and at the end.  A copy remembers what its
+    source held when it was queued, and looks again when it runs."""
+
+    def __init__(self):
+        self.queues, self.stream, self.stale, self.copies = {}, 1, 0, 0
+
+    def queue(self, what):
+        self.queues.setdefault(self.stream, []).append(what)
+
+    def run(self, stream, until=None):
+        queue = self.queues.get(stream, [])
+        while queue:
+            op = queue.pop(0)
+            if op is until:
+                return
+            if not isinstance(op, Recorded):
+                source, held = op
+                self.stale += not torch.equal(source, held)
+
+    def synchronize(self, device=None):
+        for s in list(self.queues):
+            self.run(s)
+
+    def copy_(self, source, non_blocking=False):
+        self.copies += 1
+        self.queue((source, source.clone()))
+
+
+class Recorded:
+    pass
+
+
+def lazy_gpu(monkeypatch):
+    gpu = LazyGPU()
+
+    class Event:
+        def record(self, stream=None):
+            self.at = (gpu.stream, Recorded())
+            gpu.queue(self.at[1])
+
+        def synchronize(self):
+            if self.at[1] in gpu.queues.get(self.at[0], []):
+                gpu.run(self.at[0], self.at[1])
+
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: True)
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch.cuda, "synchronize", gpu.synchronize)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: gpu.stream, raising=False)
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda t: t)
+    return gpu
+
+
+@pytest.mark.parametrize("width,ring", [(16, 8), (8192, 2)])
+@pytest.mark.parametrize("where", ["one stream", "packed elsewhere", "steps change streams", "dropped"])
+def test_no_host_buffer_is_written_while_its_copy_is_queued(monkeypatch, width, ring, where):
+    """A captured graph's steps queued without waiting for any of them: packed at the step or ahead of it, on the stream of the
+    step or on another, packed ahead and dropped, and steps that change streams.  Every copy finds what it was queued for."""
+    from mini_hisparse_b200.engine.step import ModelRunner, _Layout
+
+    gpu = lazy_gpu(monkeypatch)
+    part = attention(4, 2)
+    cache = CacheManager([part.cache_need()], CacheConfig(num_pages=8200, page_size=16, max_requests=3, dtype=torch.float32,
+                                                          device="cpu", allocate_storage=False))
+    runner = ModelRunner.__new__(ModelRunner)
+    runner.cache, runner.device, runner.use_graphs, runner.graph_after = cache, torch.device("cuda", 0), True, 1
+    runner.model = type("Model", (), {"spec": type("Spec", (), {"max_positions": None})})
+    runner.batch = BatchBuilder(cache, "cpu", sm_count=8)
+    runner.batch.add_user(0, part)
+    runner.stats, runner._ahead = {"prepared_steps": 0, "graph_steps": 0}, None
+    runner._table_width = lambda last: width
+    lengths = dict(a=1, b=9, c=40)
+    for name, n in lengths.items():
+        cache.open(name), cache.ensure(name, n), cache.advance(name, n)
+    key = runner._graph_key(runner.batch.segments([StepEntry(r, [0], [0]) for r in "abc"])[0], np.asarray([1, 9, 40]))
+    layout = _Layout(3, 3, 3, [width], [runner.batch.slots[0].planner.capacity(3, 3, key[2][0])])
+    graph = type("Graph", (), dict(layout=layout, fixed=list(key[2]), capturable=True, facts=None, meta=gpu, launches=0, logits=None,
+                                   buffers=None, graph=type("Exec", (), {"replay": lambda self: None})()))()
+    runner.graphs = {key: graph}
+    for step in range(4 * 8):
+        requests = ["abc", "bca", "cab"][step % 3]
+        if step and (where == "packed elsewhere" or where == "dropped" and step % 5 < 3):
+            gpu.stream = 1
+            for _ in range(1 if where == "packed elsewhere" else 3):
+                runner.prepare_decode_ahead(list(requests))
+            assert runner._ahead is not None
+        ahead, runner._ahead = runner._ahead, None
+        entries = [StepEntry(r, [step + i], [0]) for i, r in enumerate(requests[::-1] if where == "dropped" else requests)]
+        segments, _ = runner.batch.segments(entries)
+        for s in segments:
+            cache.ensure(s.request, s.start + 1)
+        gpu.stream = {"packed elsewhere": 2, "steps change streams": 1 + step // 3 % 2}.get(where, 1)
+        runner._step_graph(entries, segments, ahead)
+        for r in "abc":
+            cache.advance(r, 1)
+    assert graph.buffers.ring == ring and gpu.copies == 32 and runner.stats["prepared_steps"] == (31 if where == "packed elsewhere" else 0)
+    gpu.synchronize()
+    assert gpu.stale == 0
