@@ -302,8 +302,13 @@ class BatchBuilder:
         views["seg_slot"][:] = slots
         for g, table in zip(self.cache.page_groups, views["tables"]):
             np.take(g.table_np[:, : table.shape[1]], slots, axis=0, out=table)
-        first, views["first"] = views["first"], False
-        return [slot.planner.write_decode(starts, fixed[pi], views["plans"][pi], first) for pi, slot in enumerate(self.slots)]
+        first, views["first"] = views["first"], True         # a planner that raises leaves plans half written
+        try:
+            facts = [slot.planner.write_decode(starts, fixed[pi], views["plans"][pi], first) for pi, slot in enumerate(self.slots)]
+        except ValueError as e:
+            raise StepError(str(e)) from e
+        views["first"] = False
+        return facts
 
     def _views(self, meta: torch.Tensor, layout: _Layout, T: int, S: int, R: int, facts) -> dict:
         def v(off, n):

@@ -273,6 +273,36 @@ def test_decode_arrays_written_again_into_a_graphs_buffers(fixed, window):
             cache.advance(r, 1)
 
 
+def test_a_decode_buffer_whose_plan_could_not_be_written(monkeypatch):
+    """A plan of another size than the graph's layout is refused as a StepError, and what a planner that raised has left in the
+    buffer does not count as written: the next step in its turn writes every word."""
+    from mini_hisparse_b200.engine.step import _DecodeBuffers, _Layout
+
+    part = attention(4, 2)
+    cache = CacheManager([part.cache_need()], CacheConfig(num_pages=20, page_size=4, max_requests=2, dtype=torch.float32,
+                                                          device="cpu", allocate_storage=False))
+    batch = BatchBuilder(cache, "cpu", sm_count=8)
+    batch.add_user(0, part)
+    cache.open("a"), cache.ensure("a", 7), cache.advance("a", 6)
+    planner, entries = batch.slots[0].planner, [StepEntry("a", [1], [0])]
+    segments, _ = batch.segments(entries)
+    layout, starts = _Layout(1, 1, 1, [16], [planner.capacity(1, 1, (1, 1))]), np.asarray([6])
+    ring, fresh = (_DecodeBuffers(layout, torch.device("cpu")) for _ in range(2))
+    write = type(planner).plan_decode
+
+    def fails(self, starts, fixed):
+        raise KeyError("a planner's own trouble")
+
+    for plan, error in ((fails, KeyError), (lambda self, starts, fixed: write(self, starts, (2, 1)), StepError)):
+        monkeypatch.setattr(type(planner), "plan_decode", plan)
+        with pytest.raises(error):
+            batch._fill_decode(ring.views[0], entries, segments, [(1, 1)], starts)
+    monkeypatch.setattr(type(planner), "plan_decode", write)
+    for buffers in (ring, fresh):
+        batch._fill_decode(buffers.views[0], entries, segments, [(1, 1)], starts)
+    assert torch.equal(ring.rows[0], fresh.rows[0])
+
+
 class LazyGPU:
     """Streams that run what is queued on them as late as they may: at a synchronise, and at the end.  A copy remembers what its
     source held when it was queued, and looks again when it runs."""
