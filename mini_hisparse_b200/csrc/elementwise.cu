@@ -715,9 +715,34 @@ MHB_EXPORT int mhb_mark(cudaStream_t stream) {
         e = cudaGraphAddEmptyNode(&node, graph, deps, n);
         if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(stream, &node, 1, cudaStreamSetCaptureDependencies);
         if (e != cudaSuccess) return fail("mark: %s", cudaGetErrorString(e));
-        return 0;
+        return 1;
     }
     if (e != cudaSuccess) return fail("mark: %s", cudaGetErrorString(e));
     mark_kernel<<<1, 32, 0, stream>>>();
     return check_launch("mark");
+}
+
+// `branch` has just been made to wait for what is in front on `stream`.  In a capture, its next kernel gets ONE node in front
+// (see fork_branch in parts/base.py): with `alone` what is in front on `stream`, and no longer the branch's own last kernel
+// as well; else an empty node behind both.  Nothing outside a capture.
+MHB_EXPORT int mhb_fork(cudaStream_t branch, cudaStream_t stream, int alone) {
+    cudaStreamCaptureStatus status, other;
+    unsigned long long id = 0, other_id = 0;
+    cudaGraph_t graph = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t n = 0;
+    cudaError_t e = cudaStreamGetCaptureInfo_v2(stream, &status, &id);
+    if (e == cudaSuccess && status != cudaStreamCaptureStatusActive) return 0;
+    if (e == cudaSuccess) e = cudaStreamGetCaptureInfo_v2(branch, &other, &other_id);
+    if (e != cudaSuccess) return fail("fork: %s", cudaGetErrorString(e));
+    if (other != status || other_id != id) return fail("fork: the branch does not belong to the stream's capture");
+    e = cudaStreamGetCaptureInfo_v2(alone ? stream : branch, &status, &id, &graph, &deps, &n);
+    cudaGraphNode_t node;
+    if (e == cudaSuccess && !alone) {
+        e = cudaGraphAddEmptyNode(&node, graph, deps, n);
+        deps = &node;
+        n = 1;
+    }
+    if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(branch, const_cast<cudaGraphNode_t*>(deps), n, cudaStreamSetCaptureDependencies);
+    return e == cudaSuccess ? 0 : fail("fork: %s", cudaGetErrorString(e));
 }

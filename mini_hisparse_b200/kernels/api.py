@@ -108,7 +108,18 @@ def embed_norm(table, weight, eps, tokens, out, status=None):
 def mark():
     """What is launched on the current stream from here on starts when all that is in front of it has finished (see join_branch)."""
     lib = build.load("elementwise")
-    _check(lib, lib.mhb_mark(_stream()), "mark")
+    code = lib.mhb_mark(_stream())
+    if code == 1:
+        return              # a captured graph's empty node is no launch
+    _check(lib, code, "mark")
+
+
+def fork(branch, alone: bool):
+    """``branch`` has just been made to wait for the current stream: see fork_branch.  ``alone``: nothing that was launched on the
+    branch before is left for its next kernel to wait for."""
+    lib = build.load("elementwise")
+    if lib.mhb_fork(c_void_p(branch.cuda_stream), _stream(), c_int(1 if alone else 0)) != 0:
+        raise KernelError(f"fork: {lib.mhb_last_error().decode()}")
 
 
 def norm_mix(x, weight, eps, *, delta=None, nsplit=1, split_stride=0, alpha=1.0, keep=0.0, copy=None):

@@ -8,7 +8,7 @@ import numpy as np
 import torch
 
 from ..kernels import api as K
-from .base import CacheView, Mixer, Product, StepContext, StepPlanner, join_branch
+from .base import CacheView, Mixer, Product, StepContext, StepPlanner, fork_branch, join_branch
 from .registry import POSITIONS, register_mixer
 from .spec import PagedKVNeed, ParamSpec, PartSpec
 
@@ -608,15 +608,13 @@ class GQAttention(Mixer):
                 # the short segments (a mixed serving step has some dozens of decode tokens beside a
                 # prompt portion, and neither kernel fills the GPU for as long as the other runs).
                 ctx.extras["two_stream_layers"] = ctx.extras.get("two_stream_layers", 0) + 1
-                main = torch.cuda.current_stream()
                 fork, join = ctx.extras["side_events"]
-                fork.record(main)
-                side.wait_event(fork)
+                fork_branch(ctx, side, fork)
                 with torch.cuda.stream(side), K.stream_scope():
                     long_portions()
                     join.record(side)
                 short_segments()
-                join_branch(main, join)
+                join_branch(ctx, side, join)
             else:
                 if n_small:
                     short_segments()

@@ -119,15 +119,28 @@ class Workspace:
         return sum(b.numel() for b in self._buffers.values())
 
 
-def join_branch(main, done) -> None:
-    """The main stream waits for a second stream's event ``done``, and its next kernel starts only when BOTH streams have
-    finished.  Every kernel of a step may start before the one in front of it has finished (csrc/common.cuh); behind a join
-    there are two in front, one of each stream.  Should one of them be enough, the kernels behind the join could take every
-    SM's shared memory while they wait for a kernel of the other stream that still has CTAs to place.  So something that no
-    kernel starts early behind stands in between: an empty node in a captured graph (a layer of two branches takes about as
-    long as without it), an empty launch else."""
-    main.wait_event(done)
+def fork_branch(ctx: "StepContext", branch, event) -> None:
+    """The second stream goes on from where the current one is, and its next kernel has ONE node in front.  Every kernel of a
+    step may start before the one in front of it has finished (csrc/common.cuh).  In a captured graph an event's wait ADDS a
+    dependency: the branch's last kernel of the layer before would stay one too.  Should one of two such kernels be enough for
+    a kernel to start, the branch's could take every SM's shared memory while it waits for the main stream, whose kernels
+    then find no room.  What the branch did before lies behind a join on the main stream already, so the dependency on the
+    fork holds it too; where a fork lies inside another (what the branch did is not joined yet), an empty node stands behind
+    both.  (Outside a capture a kernel behind an event's wait starts when the event has passed.)"""
+    event.record()
+    branch.wait_event(event)
+    K.fork(branch, alone=branch not in ctx.open_branches)
+    ctx.open_branches.append(branch)
+
+
+def join_branch(ctx: "StepContext", branch, done) -> None:
+    """The current stream waits for the second stream's event ``done``, and its next kernel starts only when BOTH streams have
+    finished: with two kernels in front that it may start beside (one of each stream) it could start too early, as at a fork.
+    So something that no kernel starts early behind stands in between: an empty node in a captured graph (a layer of two
+    branches takes about as long as without it), an empty launch else."""
+    torch.cuda.current_stream().wait_event(done)
     K.mark()
+    ctx.open_branches.remove(branch)
 
 
 class Runtime:
@@ -243,6 +256,7 @@ class StepContext:
     status: torch.Tensor            # [1] int32 error bits set by kernels
     seg_offset: torch.Tensor | None = None   # [S + 1] int32: first token of each segment, and T
     extras: dict = field(default_factory=dict)
+    open_branches: list = field(default_factory=list)       # second streams that are forked off and not yet joined
 
     @property
     def longest(self) -> int:

@@ -4,7 +4,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .base import Block, CacheView, Product, StepContext, join_branch
+from .base import Block, CacheView, Product, StepContext, fork_branch, join_branch
 from .feed_forward import TokenSide
 from .norm import RMSNorm
 from .registry import FEED_FORWARDS, GATES, INPUT_CONVS, MIXERS, NORMS, register_block
@@ -150,15 +150,13 @@ class ParallelBlock(Block):
         # buffers of their own, so the feed-forward runs on a second stream beside the mixer (in a captured
         # graph: two branches of the graph) and the next norm waits for both.  Only for few tokens: their
         # products are the ones that need no scratch shared between launches.
-        main = torch.cuda.current_stream()
         fork, join = ctx.extras["branch_events"]
-        fork.record(main)
-        branch.wait_event(fork)
+        fork_branch(ctx, branch, fork)
         with torch.cuda.stream(branch), K.stream_scope():
             f = self.feed_forward.forward(h, ctx)
             join.record(branch)
         a = self.mixer.forward(h, ctx, cache)
-        join_branch(main, join)
+        join_branch(ctx, branch, join)
         return Product(a.tensor, a.nsplit, also=f)
 
 

@@ -4,7 +4,7 @@ from __future__ import annotations
 import torch
 
 from ..kernels import api as K
-from .base import CacheView, Mixer, Product, StepContext, join_branch
+from .base import CacheView, Mixer, Product, StepContext, fork_branch, join_branch
 from .multimap_attention import _pad_rows
 from .registry import MIXERS, register_mixer
 from .spec import PartSpec
@@ -91,13 +91,11 @@ class SideBySide(Mixer):
             return Product(a.tensor, a.nsplit, also=b)
         # few tokens: two chains of small kernels that read the same product and write buffers of their own; their
         # products need no scratch shared between launches
-        main = torch.cuda.current_stream()
         fork, join = ctx.extras["branch_events"]
-        fork.record(main)
-        branch.wait_event(fork)
+        fork_branch(ctx, branch, fork)
         with torch.cuda.stream(branch), K.stream_scope():
             b = self.right.forward_projected(proj, self.col, ctx, right_view, "mix_out_right")
             join.record(branch)
         a = self.left.forward_projected(proj, 0, ctx, left_view, "mix_out")
-        join_branch(main, join)
+        join_branch(ctx, branch, join)
         return Product(a.tensor, a.nsplit, also=b)

@@ -1,6 +1,7 @@
 """Each CUDA kernel alone against a plain PyTorch float32 reference of the same operation, at
 sizes other than the engine's test models (widths and vocabularies that are no power of two,
 head sizes in steps of 16, odd group counts)."""
+import contextlib
 import hashlib
 import math
 
@@ -1228,3 +1229,81 @@ def test_sample_temperature_equals_the_plain_draw():
     K().sample(logits[sel].contiguous(), temps[sel].contiguous(), seeds[sel].contiguous(),
                counters[sel].contiguous(), again)
     assert again.tolist() == [int(out[i]) for i in sel]
+
+
+def captured_edges(graph):
+    """{node: [(node in front, whether the launch allows an early start)]} of a captured graph that kept its nodes."""
+    import ctypes
+
+    cudart, n = ctypes.CDLL("libcudart.so.12"), ctypes.c_size_t(0)
+    raw = ctypes.c_void_p(graph.raw_cuda_graph())
+    assert cudart.cudaGraphGetEdges_v2(raw, None, None, None, ctypes.byref(n)) == 0
+    front, behind, data = (ctypes.c_void_p * n.value)(), (ctypes.c_void_p * n.value)(), (ctypes.c_uint8 * (8 * n.value))()
+    assert cudart.cudaGraphGetEdges_v2(raw, front, behind, data, ctypes.byref(n)) == 0
+    edges = {}
+    for i in range(n.value):
+        edges.setdefault(behind[i], []).append((front[i], data[8 * i + 2] == 1))
+    return edges
+
+
+@pytest.mark.parametrize("nested", [False, True])
+def test_kernels_behind_forks_and_joins_have_one_node_in_front(nested):
+    """Three layers of two branches (in each a fork inside the fork, too), captured: no kernel may start beside one of two nodes
+    in front, every branch is joined, and the replay gives what the launches one by one give."""
+    from types import SimpleNamespace
+
+    from mini_hisparse_b200.parts.base import fork_branch, join_branch
+
+    branch, events = torch.cuda.Stream(), [torch.cuda.Event() for _ in range(2)]
+    first = (torch.arange(8 * 256) % 7).float().view(8, 256)
+    x, want = torch.empty(6, 8, 256, device=DEV), torch.zeros(6, 8, 256)
+    want[1] = first
+
+    def layers(add, fork, join):
+        for _ in range(3):
+            add(0, 1)
+            with fork():
+                add(2, 0)
+                add(2, 0)
+            if nested:
+                add(3, 0)
+                with fork():
+                    add(4, 3)
+                add(5, 0)
+                join()
+                add(3, 4)
+                add(3, 5)
+            add(3, 0)
+            join()
+            add(1, 2)
+            add(1, 3)
+
+    def on_the_gpu():
+        ctx = SimpleNamespace(open_branches=[])
+
+        @contextlib.contextmanager
+        def fork():
+            fork_branch(ctx, branch, events[0])
+            with torch.cuda.stream(branch):
+                yield
+                events[1].record(branch)
+
+        layers(lambda into, what: K().residual_add(x[into], x[what]), fork, lambda: join_branch(ctx, branch, events[1]))
+        assert not ctx.open_branches
+
+    def check(run):
+        x.zero_()
+        x[1].copy_(first)
+        run()
+        torch.cuda.synchronize()
+        assert torch.equal(x.cpu(), want)
+
+    layers(lambda into, what: want[into].add_(want[what]), contextlib.nullcontext, lambda: None)
+    check(on_the_gpu)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        on_the_gpu()
+    edges = captured_edges(graph)
+    assert any(early for front in edges.values() for _, early in front) and any(len(front) == 2 for front in edges.values())
+    assert all(len(front) == 1 for front in edges.values() if any(early for _, early in front))
+    check(graph.replay)

@@ -11,6 +11,7 @@ used again; long decoding; sizes that are equal or 1; generation through Engine 
 bin/trace_run.
 """
 import copy
+import gc
 import json
 
 import pytest
@@ -742,3 +743,36 @@ def test_trace_run_picks_the_model_by_its_config(models, tmp_path):
             row += len(e["want"])
     assert run.close() == 0
     check_against_plain({k: torch.cat(v) for k, v in got.items()}, refs, "float32")
+
+
+@pytest.mark.parametrize("design", ["dotivik", "zetenex"])
+def test_no_kernel_of_a_captured_step_has_two_nodes_to_start_beside(models, tmp_path, monkeypatch, design):
+    """The decode graphs of the designs whose layers run on two streams: a kernel that may start early has one node in front."""
+    from test_dotivik_gpu import CFG_A as dotivik
+    from test_kernels_gpu import captured_edges
+
+    from mini_hisparse_b200 import CacheConfig, CacheManager, load_model, write_random_model
+    from mini_hisparse_b200.engine import ModelRunner, StepEntry
+
+    folder = models["A"][0]
+    if design == "dotivik":
+        write_random_model(dotivik, 3, folder := tmp_path, dtype=torch.bfloat16, matrix_std=0.15)
+    model = load_model(folder, dtype="bfloat16")
+    cache = CacheManager(model.cache_needs, CacheConfig(num_pages=32, page_size=16, max_requests=2, dtype=torch.bfloat16))
+    runner = ModelRunner(model, cache)
+    real = torch.cuda.CUDAGraph
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", lambda: real(keep_graph=True))
+    for r in "ab":
+        cache.open(r)
+    runner.step([StepEntry(r, [1, 2, 3, 4, 5], [4]) for r in "ab"])
+    for step in range(3):
+        logits = runner.step([StepEntry(r, [step], [0]) for r in "ab"])
+    runner.check_status()
+    assert bool(logits.isfinite().all())
+    (graph,) = runner.graphs.values()
+    edges = captured_edges(graph.graph)
+    assert any(len(front) == 2 for front in edges.values()), "no layer of two branches"
+    assert sum(early for front in edges.values() for _, early in front) > len(edges) // 2
+    assert all(len(front) == 1 for front in edges.values() if any(early for _, early in front))
+    del runner, graph, model
+    gc.collect()
