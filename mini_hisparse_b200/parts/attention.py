@@ -240,13 +240,16 @@ class AttentionPlanner(StepPlanner):
 
     def __init__(self, shape: AttentionShape, sm_count: int, clusters_of=None, max_cluster: int = 0,
                  min_share: int = MIN_KEYS_PER_SPLIT, max_groups: int = MAX_SPLITS, token_share: int = 0,
-                 max_ctas: int = 0):
+                 max_ctas: int = 0, memory_merge: bool = False):
         """``clusters_of(n)``: how many clusters of n CTAs the mixer's decode kernel can run at once, if
         it merges a token's key splits inside a cluster of up to ``max_cluster`` CTAs (None: it does not).
         ``min_share``: keys that a share of a cluster has at least; ``max_groups``: clusters per token and KV head;
-        ``max_ctas``: CTAs of a launch of clusters (0: as many as are resident); ``token_share``: a step of single tokens is cut into shares of that many keys, once there are four (0: as the
-        shape says)."""
+        ``max_ctas``: CTAs of a launch of clusters (0: as many as are resident); ``memory_merge``: the kernel merges
+        splits through global memory too, which a plan of n clusters of ONE share asks for (see _merged);
+        ``token_share``: a step of single tokens is cut into shares of that many keys, once there are four (0: as
+        the shape says)."""
         self.min_share, self.max_groups, self.token_share, self.max_ctas = min_share, max_groups, token_share, max_ctas
+        self.memory_merge = memory_merge
         self.shape, self.sm_count = shape, sm_count
         self.clusters_of, self.max_cluster = clusters_of, max_cluster
         self._uneven = {}        # decode_fixed_for's answers
@@ -349,8 +352,20 @@ class AttentionPlanner(StepPlanner):
                 for g in range(2, min(n // c, room(c) // ctas, self.max_groups) + 1):
                     if cost(c, g) < best_cost:
                         best, best_cost = (c, g), cost(c, g)
-        # no cluster fits: the shares go through the kernels that merge through global memory
-        return best if best is not None else (plain, 1)
+        return best if best is not None else self._merged(plain, ctas)
+
+    def _merged(self, n: int, ctas: int) -> tuple[int, int]:
+        """How ``n`` shares that were not counted as clusters meet: in clusters all the same, or, for a kernel that can, through
+        global memory (n clusters of one share).  A cluster's merge is some 3 us shorter, but its CTAs wait for one
+        another's SMs: memory is better where clusters need another round of the GPU.  16 heads over 4 KV heads, 2 clusters
+        of 3 and so on, us in a cluster and through memory: 37 requests of 700 keys cut in 2 (148 of 148 clusters)
+        12.2, 15.4; 20 of 1,500 in 3 (80 of 93) 13.7, 16.6; 24 of 1,500 in 3 (96 of 93, 288 CTAs) 22.4, 18.0; 18 of 1,500 in 4 (72 of
+        71) 19.4, 15.3; 40 requests, one of 4,000 keys and 39 of 200, in 4 (160 of 71, 640 CTAs) 28.1, 30.9."""
+        if n > 1 and self.memory_merge:
+            room = self.clusters_of(n) if n <= self.max_cluster and self.chunks == 1 else 0
+            if not room or -(-ctas // room) > -(-ctas * n // (2 * self.sm_count)):
+                return 1, n
+        return n, 1
 
     UNEVEN_CANDIDATES = (2, 3, 4, 6, 8, 12, 16)
 
@@ -382,8 +397,8 @@ class AttentionPlanner(StepPlanner):
                 best, best_time = n, t
         if len(self._uneven) > 512:
             self._uneven.clear()
-        self._uneven[key] = (best, 1)
-        return best, 1
+        self._uneven[key] = hit = self._merged(best, ctas)
+        return hit
 
     def _launch_time(self, tiles, n: int) -> float:
         """Key tiles of time until the last CTA of a decode launch with n key splits is done: CTAs start
@@ -426,13 +441,14 @@ def tma_planner(shape: AttentionShape, sm_count: int, d: int) -> AttentionPlanne
     8.3 us uncut, 7.2 in clusters of 4, 9.3 in clusters of 8, which wait for one another)."""
     groups = shape.q_heads // shape.kv_heads
     return AttentionPlanner(shape, sm_count, lambda n: K.attention_tma_max_clusters(d, groups, n), K.DECODE_MAX_SPLITS,
-                            min_share=KEY_TILE, max_groups=1, max_ctas=sm_count)
+                            min_share=KEY_TILE, max_groups=1, max_ctas=sm_count, memory_merge=True)
 
 
-def tma_cluster(meta: dict, d: int, groups: int) -> int:
-    """Splits that attention_tma_ext merges in a cluster in this step (0: it merges through the partial buffers)."""
+def tma_cluster(meta: dict) -> int:
+    """Splits that attention_tma_ext merges in a cluster in this step, as tma_planner has planned it (0: it merges through the
+    partial buffers)."""
     n = meta.get("decode_nsplit", 0)
-    return n if n > 1 and meta.get("decode_groups", 1) == 1 and K.attention_tma_max_clusters(d, groups, n) > 0 else 0
+    return n if n > 1 else 0
 
 
 @register_mixer("gq_attention")

@@ -158,7 +158,7 @@ class LatentAttention(Mixer):
                                         page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                         shared_kv=True, **opts, tok_nsplit=meta["tok_nsplit"], counters=counters,
                                         status=ctx.status, fresh=SPLIT_MAX_TOKENS,
-                                        cluster=tma_cluster(meta, self.width, self.heads))
+                                        cluster=tma_cluster(meta))
                 else:
                     K.attention_mma_ext(*args, meta["items"], n_small, 16, *tail, **common,
                                         tok_nsplit=meta["tok_nsplit"], counters=counters)

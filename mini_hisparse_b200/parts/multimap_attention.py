@@ -145,7 +145,7 @@ class DifferentialAttention(Mixer):
                                     page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                     softcap=self.softcap, tok_nsplit=meta["tok_nsplit"], counters=counters,
                                     status=ctx.status, fresh=SPLIT_MAX_TOKENS,
-                                    cluster=tma_cluster(meta, self.dv, self.nq // self.nkv))
+                                    cluster=tma_cluster(meta))
             if n_big:
                 K.attention_tc_ext(q, cache.storage, maps, big_items, n_big, ctx.positions, meta["block_table"],
                                    nq=self.nq, nkv=self.nkv, d=self.dv, page_size=cache.page_size,

@@ -148,8 +148,7 @@ class SinkAttention(Mixer):
                                         page_size=cache.page_size, window=self.window or 0, scale=self.scale,
                                         sink=sink, slopes=slopes, **gate, tok_nsplit=meta["tok_nsplit"], counters=counters,
                                         status=ctx.status, fresh=SPLIT_MAX_TOKENS,
-                                        cluster=(tma_cluster(meta, self.dk, self.nq // self.nkv)
-                                                 if self.merges_in_clusters else 0))
+                                        cluster=tma_cluster(meta) if self.merges_in_clusters else 0)
                 else:
                     K.attention_mma_ext(*args, meta["items"], n_small, 16, *tail, **common,
                                         tok_nsplit=meta["tok_nsplit"], counters=counters)

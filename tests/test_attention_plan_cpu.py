@@ -163,3 +163,41 @@ def test_cluster_sizes_of_a_decode_step():
     assert len(arrays["items"]) == cluster * groups * ITEM_INTS
     plain = AttentionPlanner(AttentionShape(28, 4, None, 128), 148)      # a kernel without clusters
     assert plain.decode_fixed(1, 32768) == (64, 1) and plain.decode_fixed(4, 4096) == (16, 1)
+
+
+def test_a_kernel_merges_in_clusters_only_what_was_planned_for_them(monkeypatch):
+    """tma_planner with the resident-cluster counts that the driver reports: what is cut reaches the kernel as clusters exactly
+    where these take no more rounds of the GPU than CTAs that meet through memory would, for even and uneven histories; the shares'
+    number and their items are the same either way."""
+    from mini_hisparse_b200.parts import attention as A
+
+    reported = {2: 148, 3: 93, 4: 71, 5: 56, 6: 45, 7: 37, 8: 33, 9: 30, 10: 26, 11: 21, 12: 21, 13: 17, 14: 14, 15: 14, 16: 14}
+
+    def built(d, groups, n):
+        return 0 if groups > 16 or (n + 1) * -(-groups // n) > 17 else reported[n]
+
+    monkeypatch.setattr(A.K, "attention_tma_max_clusters", built)
+    seen = set()
+    for heads, kv in ((16, 4), (32, 8), (16, 1), (40, 1)):
+        shape = A.AttentionShape(heads, kv, None, 128)
+        planner = A.tma_planner(shape, 148, 128)
+        for B in range(1, 101):
+            for keys in (200, 300, 700, 1500, 3000, 8000):
+                even = np.full(B, keys - 1)
+                long = np.asarray([keys - 1] + [150] * (B - 1))
+                for starts in (even, long):
+                    cluster, groups = fixed = planner.decode_fixed_for(starts, keys)
+                    n = cluster * groups
+                    arrays, facts = planner.plan_decode(starts, fixed)
+                    taken = A.tma_cluster(facts)
+                    plain = A.plan_decode(shape, starts, n)
+                    assert np.array_equal(arrays["items"], plain.items.reshape(-1)) and facts["part_rows_cap"] == plain.part_rows
+                    assert planner.capacity(B, B, fixed)["items"] == arrays["items"].size
+                    if n == 1 or planner.chunks > 1:
+                        assert taken == 0
+                        continue
+                    room, ctas = built(128, heads // kv, n) if n <= 16 else 0, B * kv
+                    fits = room > 0 and -(-ctas // room) <= -(-ctas * n // 296)
+                    assert taken == (n if fits else 0), (heads, kv, B, keys, fixed)
+                    seen.add((fits, starts is even))
+    assert seen == {(True, True), (True, False), (False, True), (False, False)}
