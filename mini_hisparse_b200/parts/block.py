@@ -151,11 +151,14 @@ class ParallelBlock(Block):
         # graph: two branches of the graph) and the next norm waits for both.  Only for few tokens: their
         # products are the ones that need no scratch shared between launches.
         fork, join = ctx.extras["branch_events"]
+        # The main stream's kernels come first: a captured graph runs on where the fork stands with the node that was added
+        # first, and only that one starts beside the kernel in front (16 steps of 1 to 8 requests, 4,096 wide: 15.9 to 20.6 ms,
+        # 17.2 to 21.8 with the feed-forward first, 17.4 to 22.0 on one stream).
         fork_branch(ctx, branch, fork)
+        a = self.mixer.forward(h, ctx, cache)
         with torch.cuda.stream(branch), K.stream_scope():
             f = self.feed_forward.forward(h, ctx)
             join.record(branch)
-        a = self.mixer.forward(h, ctx, cache)
         join_branch(ctx, branch, join)
         return Product(a.tensor, a.nsplit, also=f)
 

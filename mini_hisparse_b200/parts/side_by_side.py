@@ -93,9 +93,9 @@ class SideBySide(Mixer):
         # products need no scratch shared between launches
         fork, join = ctx.extras["branch_events"]
         fork_branch(ctx, branch, fork)
+        a = self.left.forward_projected(proj, 0, ctx, left_view, "mix_out")
         with torch.cuda.stream(branch), K.stream_scope():
             b = self.right.forward_projected(proj, self.col, ctx, right_view, "mix_out_right")
             join.record(branch)
-        a = self.left.forward_projected(proj, 0, ctx, left_view, "mix_out")
         join_branch(ctx, branch, join)
         return Product(a.tensor, a.nsplit, also=b)
