@@ -17,7 +17,7 @@ KEY_TILE = 64          # split boundaries are multiples of the kernels' key tile
 ITEM_INTS = 8
 MIN_KEYS_PER_SPLIT = 256
 MIN_KEYS_PER_SIMT_SPLIT = 128
-KEYS_PER_TOKEN_SPLIT = 512     # attention_tokens: one round of its sixteen warps; a merge is a launch
+KEYS_PER_TOKEN_SPLIT = 512     # attention_tokens: one round of its sixteen warps (see _most_splits)
 SPLIT_MAX_TOKENS = 16  # only short segments (decode tokens, tiny portions) are split along the keys
 MAX_SPLITS = 64
 MAX_BIG_SPLITS = 8       # key splits of a long portion's tile (tcgen05 kernel only)
@@ -246,11 +246,12 @@ class AttentionPlanner(StepPlanner):
         ``min_share``: keys that a share of a cluster has at least; ``max_groups``: clusters per token and KV head;
         ``max_ctas``: CTAs of a launch of clusters (0: as many as are resident); ``memory_merge``: the kernel merges
         splits through global memory too, which a plan of n clusters of ONE share asks for (see _merged);
-        ``token_share``: a step of single tokens is cut into shares of that many keys, once there are four (0: as
-        the shape says)."""
+        ``token_share``: the kernel is attention_tokens, one CTA of which fills an SM and walks that many keys in a round
+        (0: two CTAs an SM, splits as the shape says)."""
         self.min_share, self.max_groups, self.token_share, self.max_ctas = min_share, max_groups, token_share, max_ctas
         self.memory_merge = memory_merge
         self.shape, self.sm_count = shape, sm_count
+        self.resident = sm_count if token_share else 2 * sm_count        # CTAs that run at once
         self.clusters_of, self.max_cluster = clusters_of, max_cluster
         self._uneven = {}        # decode_fixed_for's answers
         self._fixed = {}         # decode_fixed's: they depend on two numbers
@@ -284,9 +285,15 @@ class AttentionPlanner(StepPlanner):
         every = None if fixed is None else fixed[0] * fixed[1]
         return self._out(plan_attention(self.shape, segments, T, self.sm_count, fixed_nsplit=every))
 
-    def _most_splits(self, keys: int) -> int:
+    def _most_splits(self, keys: int, fit: int = MAX_SPLITS) -> int:
+        """attention_tokens: as many shares as there are rounds of keys, and four for two or three rounds if all CTAs of
+        these fit.  A merge is a launch of 2 us that a second round in a lone CTA outlasts (steps of two layers over graphs for
+        1,024 keys, uncut / 2 / 4 / 8 shares: 28 heads over 4 of 128, 1 request 726 / 682 / 669 / 670 us, 8 requests 1,148 /
+        1,108 / 1,104 / 1,144; 3 heads of 32 over one, 4 requests 61.9 / 56.8 / 58.6 / 60.0, but 64 requests 144 / 153), a
+        first one does not (graphs for 512, 4 requests: 50.7 / 71.0 / 72.3)."""
         if self.token_share:
-            return keys // self.token_share if keys >= 4 * self.token_share else 1
+            rounds = keys // self.token_share
+            return rounds if rounds >= 4 else 4 if rounds >= 2 and fit >= 4 else 1
         return self.shape.max_splits(keys)
 
     # what a CTA costs beside its keys (the query and the merge) and what a launch of attention_combine
@@ -307,14 +314,15 @@ class AttentionPlanner(StepPlanner):
     def _decode_fixed(self, segments_count, max_positions):
         """Key shares per decoded token for a batch of B with at most ``max_positions`` cached keys, as
         (shares in a cluster, clusters per token and KV head): as many CTAs as are resident at once (two per
-        SM), never more, so that no CTA waits for a second wave, and no share shorter than
+        SM; attention_tokens: one, 8 requests of 4,000 keys over 4 KV heads in 4 shares 1,172 us, in 8 1,182), never more, so that no CTA waits for a second wave, and no share shorter than
         ``shape.max_splits`` allows.  Without a cluster kernel: (shares, 1)."""
         ctas = segments_count * self.shape.kv_heads * self.chunks
         if self.shape.window:            # a token never attends to more keys than its window holds
             max_positions = min(max_positions, self.shape.window)
-        plain = n = max(1, min(MAX_SPLITS, (2 * self.sm_count) // ctas, self._most_splits(max_positions)))
+        fit = min(MAX_SPLITS, self.resident // ctas)
+        plain = n = max(1, min(fit, self._most_splits(max_positions, fit)))
         if self.clusters_of is not None and self.chunks == 1:
-            n = max(n, min((2 * self.sm_count) // ctas, self.max_cluster, max_positions // self.min_share))
+            n = max(n, min(self.resident // ctas, self.max_cluster, max_positions // self.min_share))
         if self.clusters_of is None or self.chunks != 1 or n == 1:
             return n, 1
         # The shares of a cluster are merged in its shared memory, and a cluster is placed inside one
@@ -363,7 +371,7 @@ class AttentionPlanner(StepPlanner):
         71) 19.4, 15.3; 40 requests, one of 4,000 keys and 39 of 200, in 4 (160 of 71, 640 CTAs) 28.1, 30.9."""
         if n > 1 and self.memory_merge:
             room = self.clusters_of(n) if n <= self.max_cluster and self.chunks == 1 else 0
-            if not room or -(-ctas // room) > -(-ctas * n // (2 * self.sm_count)):
+            if not room or -(-ctas // room) > -(-ctas * n // self.resident):
                 return 1, n
         return n, 1
 
@@ -379,7 +387,8 @@ class AttentionPlanner(StepPlanner):
         fixed = self.decode_fixed(len(starts), max_positions)
         n0 = fixed[0] * fixed[1]
         B = len(starts)
-        limit = min(self._most_splits(max_positions), self.max_cluster or MAX_SPLITS)
+        fit = self.resident // (B * self.shape.kv_heads * self.chunks)
+        limit = min(self._most_splits(max_positions, fit), self.max_cluster or MAX_SPLITS)
         if n0 > 1 or B < 2 or limit < 2:       # fewer requests: their splits are sized for one round of CTAs
             return fixed
         tiles = (np.asarray(starts, np.int64) + KEY_TILE) // KEY_TILE
@@ -402,13 +411,13 @@ class AttentionPlanner(StepPlanner):
 
     def _launch_time(self, tiles, n: int) -> float:
         """Key tiles of time until the last CTA of a decode launch with n key splits is done: CTAs start
-        in launch order (splits of a token together, tokens in order, KV heads outermost) on two
-        slots per SM, and a slot takes the next CTA when its own is done."""
+        in launch order (splits of a token together, tokens in order, KV heads outermost) on the
+        resident slots, and a slot takes the next CTA when its own is done."""
         import heapq
 
         per_cta = np.repeat(-(-tiles // n) + self.CTA_FIXED_TILES, n)
         order = np.tile(per_cta, self.shape.kv_heads * self.chunks).tolist()
-        slots = 2 * self.sm_count
+        slots = self.resident
         if len(order) <= slots:
             return max(order)
         busy = order[:slots]

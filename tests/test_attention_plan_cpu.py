@@ -201,3 +201,24 @@ def test_a_kernel_merges_in_clusters_only_what_was_planned_for_them(monkeypatch)
                     assert taken == (n if fits else 0), (heads, kv, B, keys, fixed)
                     seen.add((fits, starts is even))
     assert seen == {(True, True), (True, False), (False, True), (False, False)}
+
+
+def test_shares_of_decoded_tokens_on_the_cuda_cores():
+    """Uncut within one round of attention_tokens' warps; from two rounds on cut in four if a CTA an SM holds them; as many shares
+    as rounds beyond, never more CTAs than SMs; a window's keys count, not the history's."""
+    from mini_hisparse_b200.parts import PartSpec
+    from mini_hisparse_b200.parts.attention import GQAttention
+
+    def shares(heads, kv, d, B, keys, window=None):
+        part = GQAttention(PartSpec.make("gq_attention", hidden_size=32, q_heads=heads, kv_heads=kv, head_dim=d, window=window,
+                                         position=PartSpec.make("none")))
+        planner = part.planner(16, 148)
+        cluster, groups = planner.decode_fixed(B, keys)
+        assert groups == 1 and (keys >= 2048 or planner.decode_fixed_for(np.full(B, keys - 1), keys) == (cluster, 1))
+        return cluster
+
+    assert [shares(28, 4, 128, 1, n) for n in (256, 512, 1023, 1024, 1600, 2048, 4096, 32768)] == [1, 1, 1, 4, 4, 4, 8, 37]
+    assert [shares(28, 4, 128, B, 1024) for B in (1, 8, 9, 10, 64)] == [4, 4, 4, 1, 1]
+    assert [shares(28, 4, 128, B, 8192) for B in (1, 2, 4, 8, 16, 37, 38, 100)] == [16, 16, 9, 4, 2, 1, 1, 1]
+    assert [shares(3, 1, 32, B, 1024) for B in (4, 37, 38, 64)] == [4, 4, 1, 1]
+    assert shares(28, 4, 128, 1, 32768, window=700) == 1 and shares(28, 4, 128, 1, 32768, window=1100) == 4
