@@ -1109,7 +1109,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 //
 // FEATURES: the roles of the operands change, a tile is 256 features x bn tokens.  A tile's 256 rows are all paid for,
 // its bn columns can be any multiple of 16: with 543 tokens (a portion of 512 beside 31 decoding requests) three tiles of
-// 256 tokens are 768 rows of work, three of 192 are 576.  (see choose_features_bn).
+// 256 tokens are 768 rows of work, three of 192 are 576 (see choose_pair_form).
 //
 // A stage of the ring holds one or two K blocks of 64 (`kbs`).  The thread that issues the MMAs pays some
 // 250 cycles for the barrier it looks at before a stage, whatever the stage holds: with tiles 256 wide
@@ -1490,32 +1490,61 @@ int choose_persistent_bn(int tiles_m, int N, int sms, int step) {
     return best;
 }
 
-// What a launch of the two-SM kernel takes, in rows of 64 operand elements that a pair loads: its rounds of tiles, each
-// (256 + bn) rows per K block and a fixed cost, or what reading the weights takes if that is longer.  Fitted to 2,048 and
-// 543 tokens at the 14B, 7B and 2,048-wide shapes (0.74 ns a row; 14B down of 2,048 tokens: 228 us measured, 228 counted; 7B
-// gate/up: 350, 371; 2,048-wide gate/up: 106, 99).  The epilogue that rotates and appends takes longer where rows are features.
-constexpr double PAIR_ROUND_ROWS = 2800.0, PAIR_HEADS_ROWS = 12000.0, PAIR_WEIGHT_BYTES = 4800.0;
-double pair_cost(long long tiles, int bn, int N, int K, int pairs, double fixed) {
-    const double rows = (double)((tiles + pairs - 1) / pairs) * ((256 + bn) * (double)((K + BK - 1) / BK) + fixed);
-    const double weights = (double)N * K * 2 / PAIR_WEIGHT_BYTES;
-    return rows > weights ? rows : weights;
+// How long a launch of the two-SM kernel takes, in us.  A pair loads 256 + bn rows a K block; the epilogue of a tile (by its
+// columns and kind) goes on beside the next tile's products, so a round takes the longer of the two, and the last one both.
+// Fitted to 617 products of 257 to 4,096 tokens by 1,024 to 55,296 features, K 1,024 to 27,648, in all widths of both forms.
+// With tiles of features the epilogue turns every chunk of 16 tokens through shared memory: 0.6 to 1.1 us each where
+// it has more to do than store (2,048-wide gate/up, K 2,048: 10.8 us of epilogue beside 11.2 of products a round), which a count
+// of operand rows alone did not see (7B q/k/v of 1,000 tokens: 36 us with tiles of tokens, 47 with the features it took).
+struct PairEpilogue { double fixed, chunk; };
+constexpr PairEpilogue pair_epilogue(int epi, bool features) {
+    return features ? PairEpilogue{0.2, epi == 2 ? 1.06 : is_glu(epi) ? 0.80 : epi ? 0.58 : 0.0}
+                    : PairEpilogue{1.75, epi == 2 ? 0.37 : is_glu(epi) ? 0.60 : epi ? 0.28 : 0.0};
 }
-long long features_tiles(int bn, int M, int N) { return (long long)((M + bn - 1) / bn) * ((N + 2 * BM - 1) / (2 * BM)); }
-// Tokens of a tile whose rows are features: the multiple of 16 that takes least.
-int choose_features_bn(int M, int N, int K, int pairs, double fixed) {
-    int best = P_BN_MAX;
-    double best_cost = 1e30;
-    for (int bn = P_BN_MAX; bn >= 96; bn -= 16) {
-        const double cost = pair_cost(features_tiles(bn, M, N), bn, N, K, pairs, fixed);
-        if (cost < best_cost * (1 - 1e-9)) { best_cost = cost; best = bn; }
+double pair_time(long long tiles, int bn, int N, int K, int pairs, int epi, bool features) {
+    const PairEpilogue e = pair_epilogue(epi, features);
+    const double product = ((K + BK - 1) / BK) * (0.18 + 0.0008 * bn), epilogue = e.fixed + e.chunk * bn / 16;
+    const double longer = product > epilogue ? product : epilogue, shorter = product > epilogue ? epilogue : product;
+    const double rounds = (double)((tiles + pairs - 1) / pairs) * longer + shorter;
+    const double weights = (double)N * K * 2e-6 / 5.0;        // bytes that come from memory, at 5 TB/s
+    return 4.0 + (rounds > weights ? rounds : weights);
+}
+
+struct PairForm {
+    bool features;
+    int bn, tiles_m;         // tiles along the tokens
+    long long tiles;
+};
+// Tiles of 256 features by the multiple of 16 tokens that takes least, where that is 5 % less than 256 tokens by the width that
+// fills the rounds of pairs.  At these 617 sizes the choice is 4.8 % faster than tiles of tokens alone on average (4.5 to 5 % for
+// one half's sizes by the other half's constants) and 3 % slower at two; a few us each way:
+// 14B, 543 tokens: gate/up 153 for 176, q/k/v 50 for 65, o 30 for 37, down 73 for 85; 7B, 257 tokens: gate/up 84 for 103; 2,079 tokens: q/k/v 66 for
+// 78; tiles of tokens kept: 2,048-wide gate/up of 2,079 tokens, 121 for 156 with 208 tokens a tile.
+PairForm choose_pair_form(int M, int N, int K, int pairs, int epi) {
+    PairForm f = {};
+    f.tiles_m = (M + 2 * BM - 1) / (2 * BM);
+    f.bn = N >= P_BN_MAX ? P_BN_MAX : (N + 31) / 32 * 32;
+    if (epi != 2 && N >= P_BN_MAX) f.bn = choose_persistent_bn(f.tiles_m, N, pairs, is_glu(epi) ? 32 : 16);
+    if (epi == 2 && N >= P_BN_MAX) {
+        // tiles begin and end on heads: 256 wide, or 128 where that fills the rounds of pairs better
+        const long long wide = ((long long)f.tiles_m * ((N + 255) / 256) + pairs - 1) / pairs * (256 + 24);
+        const long long narrow = ((long long)f.tiles_m * ((N + 127) / 128) + pairs - 1) / pairs * (128 + 24);
+        if (narrow < wide) f.bn = 128;
     }
-    return best;
+    f.tiles = (long long)f.tiles_m * ((N + f.bn - 1) / f.bn);
+    if (M <= 2 * BM) return f;          // up to 256 tokens fit one tile's rows
+    double best = 0.95 * pair_time(f.tiles, f.bn, N, K, pairs, epi, false);
+    for (int bn = P_BN_MAX; bn >= 96; bn -= 16) {
+        const int tiles_m = (M + bn - 1) / bn;
+        const long long tiles = (long long)tiles_m * ((N + 2 * BM - 1) / (2 * BM));
+        const double time = pair_time(tiles, bn, N, K, pairs, epi, true);
+        if (time < best * (1 - 1e-9)) {
+            best = time;
+            f.features = true; f.bn = bn; f.tiles_m = tiles_m; f.tiles = tiles;
+        }
+    }
+    return f;
 }
-// Tiles of features are taken when they are this much shorter by that count.  Measured beside tiles of tokens (us): 543
-// tokens, 14B: gate/up 134 instead of 154, q/k/v 52 for 68, down 70 for 77; 257 tokens, 14B gate/up 77 for 99, 2,048 wide 28 for
-// 43; 2,048 tokens, 14B q/k/v 129 for 168.  Between 0.9 and 1 either may win (2,048-wide gate/up of 2,079 tokens: 0.91 counted,
-// 156 for 130: with K short the epilogue's pace counts).
-constexpr double FEATURES_GAIN = 0.905;
 
 template <typename OT, int EPI, bool FEATURES>
 int launch_pair(const void* X, const void* W, void* C, int M, int N, int K, long long lda, long long ldw, long long ldc,
@@ -1605,25 +1634,10 @@ int launch_persistent(const void* X, const void* W, void* C, int M, int N, int K
     if (pair_enabled() && !share && M > BM) {
         // two SMs on one tile of 256 tokens: whole tiles only
         const int pairs = sms / 2;
-        int pbn = N >= P_BN_MAX ? P_BN_MAX : (N + 31) / 32 * 32;
-        const int tiles_m2 = (M + 2 * BM - 1) / (2 * BM);
-        if (EPI != 2 && N >= P_BN_MAX) pbn = choose_persistent_bn(tiles_m2, N, pairs, is_glu(EPI) ? 32 : 16);
-        if (EPI == 2 && qr && qr->d <= 128 && N >= P_BN_MAX) {
-            // tiles begin and end on heads: 256 wide, or 128 where that fills the rounds of pairs better
-            const long long wide = ((long long)tiles_m2 * ((N + 255) / 256) + pairs - 1) / pairs * (256 + 24);
-            const long long narrow = ((long long)tiles_m2 * ((N + 127) / 128) + pairs - 1) / pairs * (128 + 24);
-            if (narrow < wide) pbn = 128;
-        }
-        const long long pair_tiles = (long long)tiles_m2 * ((N + pbn - 1) / pbn);
-        if (M > 2 * BM) {       // up to 256 tokens fit one tile's rows
-            const double fixed = EPI == 2 ? PAIR_HEADS_ROWS : PAIR_ROUND_ROWS;
-            const int fbn = choose_features_bn(M, N, K, pairs, fixed);
-            const long long tiles = features_tiles(fbn, M, N);
-            if (pair_cost(tiles, fbn, N, K, pairs, fixed) < FEATURES_GAIN * pair_cost(pair_tiles, pbn, N, K, pairs, PAIR_ROUND_ROWS))
-                return launch_pair<OT, EPI, true>(X, W, C, M, N, K, lda, ldw, ldc, fbn, (M + fbn - 1) / fbn, tiles, pairs, status,
-                                                  stream, qr);
-        }
-        return launch_pair<OT, EPI, false>(X, W, C, M, N, K, lda, ldw, ldc, pbn, tiles_m2, pair_tiles, pairs, status, stream, qr);
+        const PairForm f = choose_pair_form(M, N, K, pairs, EPI);
+        if (f.features)
+            return launch_pair<OT, EPI, true>(X, W, C, M, N, K, lda, ldw, ldc, f.bn, f.tiles_m, f.tiles, pairs, status, stream, qr);
+        return launch_pair<OT, EPI, false>(X, W, C, M, N, K, lda, ldw, ldc, f.bn, f.tiles_m, f.tiles, pairs, status, stream, qr);
     }
     if (EPI != 2 && !share && N >= P_BN_MAX) {     // (epilogue 2 needs tiles that begin and end on heads)
         // whole tiles only: a narrower tile may fill the last round better
@@ -1656,6 +1670,13 @@ MHB_EXPORT unsigned mhb_gemm_tc_wait_limit(unsigned limit) {
     const unsigned before = g_wait_limit;
     g_wait_limit = limit ? limit : WAIT_LIMIT;
     return before;
+}
+
+// The tile that a product of more than 128 tokens on `pairs` pairs of SMs takes (see choose_pair_form; epilogue: 0 plain, 1 a
+// gate, 2 heads, 4 an activation): tokens of a tile of 256 features, or minus the features of a tile of 256 tokens.
+MHB_EXPORT int mhb_gemm_tc_pair_form(int M, int N, int K, int pairs, int epilogue) {
+    const PairForm f = choose_pair_form(M, N, K, pairs, epilogue);
+    return f.features ? f.bn : -f.bn;
 }
 
 // C[M, N] = X[M, K] * W[N, K]^T, bfloat16 in, float32 accumulation, C float32 or bfloat16.

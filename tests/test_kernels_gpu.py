@@ -437,6 +437,21 @@ def test_gemm_tiles_of_features(M, N, K_, epilogue):
         torch.testing.assert_close(out[:M].float(), y, atol=2.0 ** -8 * float(y.abs().max()), rtol=2.0 ** -8)
 
 
+@pytest.mark.parametrize("M,N,K_", [(543, 14001, 2056), (272, 13826, 2056), (543, 27650, 3080), (321, 27648, 3080)])
+@pytest.mark.parametrize("epilogue", ["float32", "bfloat16", "silu", "gelu_tanh", "gelu_act", "heads128", "heads64"])
+def test_gemm_tiles_of_features_where_they_are_taken(M, N, K_, epilogue):
+    """The same at sizes of which the choice (made for whole products' times) takes this form with every epilogue."""
+    from ctypes import c_int
+
+    from mini_hisparse_b200.kernels import build
+
+    kind, step = {"silu": (1, 32), "gelu_tanh": (3, 32), "gelu_act": (4, 1), "heads128": (2, 128), "heads64": (2, 64)}.get(epilogue, (0, 1))
+    pairs = torch.cuda.get_device_properties(0).multi_processor_count // 2
+    if pairs == 74:
+        assert build.load("gemm_tc").mhb_gemm_tc_pair_form(c_int(M), c_int(N // step * step), c_int(K_), c_int(pairs), c_int(kind)) > 0
+    test_gemm_tiles_of_features(M, N, K_, epilogue)
+
+
 @pytest.mark.parametrize("T,I,block,nsplit", [(1, 4, 4, 1), (3, 1020, 1020, 1), (5, 1028, 4, 3), (562, 304, 16, 1), (2, 176, 16, 9), (7, 102, 102, 2),
                                               (3, 30, 6, 1)])
 @pytest.mark.parametrize("dtype", DTYPES)
