@@ -62,6 +62,7 @@ struct AttnArgs {
     int out_f32;                // `out` is float32 (a sum of the outputs is still to be taken in 32 bits)
     int cluster;                // > 1: blockIdx.x = token * cluster + split, and a cluster of that many CTAs merges them
     int gate_vec;               // the gate's columns can be read four at a time
+    int out_vec, part_vec;      // the outputs and the partial buffers lie where four elements can be stored at a time
     const float* slopes;        // [nq] or null: slope_h * (query position - key position) is taken off the scaled score
 };
 
@@ -90,8 +91,17 @@ __device__ __forceinline__ float4 gate4_of(const AttnArgs& a, int t, int hq, int
     return z;
 }
 __device__ __forceinline__ void store4_out(const AttnArgs& a, size_t idx, float4 v) {
-    if (a.out_f32) *(float4*)((float*)a.out + idx) = v;
-    else *(uint2*)(a.out + idx) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    if (!a.out_vec) {
+        const float f[4] = {v.x, v.y, v.z, v.w};
+        for (int i = 0; i < 4; ++i) {
+            if (a.out_f32) ((float*)a.out)[idx + i] = f[i];
+            else a.out[idx + i] = __float2bfloat16_rn(f[i]);
+        }
+    } else if (a.out_f32) {
+        *(float4*)((float*)a.out + idx) = v;
+    } else {
+        *(uint2*)(a.out + idx) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    }
 }
 __device__ __forceinline__ float4 times(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 __device__ __forceinline__ float4 over(float4 acc, float lsum) {
@@ -446,17 +456,20 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
                 if (e == 0) asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(dst + D * 4), "f"(M), "f"(lsum) : "memory");
             } else if (split < 0) {
                 float4 res = over(acc, lsum);
-                if constexpr (EXT) {
-                    if (a.gate) res = times(res, vec4(gates + row * MS + e));
-                    store4_out(a, ((size_t)t * a.nq + hq) * D + e, res);
-                } else {
-                    *(uint2*)(a.out + ((size_t)t * a.nq + hq) * D + e) = make_uint2(pack_bf16(res.x, res.y), pack_bf16(res.z, res.w));
-                }
+                if (EXT && a.gate) res = times(res, vec4(gates + row * MS + e));
+                store4_out(a, ((size_t)t * a.nq + hq) * D + e, res);
             } else {
                 const size_t prow = (size_t)a.tok_part_row[t] + split;
-                *(float4*)(a.part_acc + (prow * a.nq + hq) * D + e) = acc;
-                if (e == 0)
-                    *(float2*)(a.part_ml + (prow * a.nq + hq) * 2) = make_float2(M == -INFINITY ? -INFINITY : M * a.scale, lsum);
+                float* part = a.part_acc + (prow * a.nq + hq) * D + e;
+                if (a.part_vec) {
+                    *(float4*)part = acc;
+                } else {
+                    part[0] = acc.x; part[1] = acc.y; part[2] = acc.z; part[3] = acc.w;
+                }
+                if (e == 0) {
+                    a.part_ml[(prow * a.nq + hq) * 2] = M == -INFINITY ? -INFINITY : M * a.scale;
+                    a.part_ml[(prow * a.nq + hq) * 2 + 1] = lsum;
+                }
             }
         }
         if constexpr (EXT) {
@@ -516,7 +529,8 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
                 for (int idx = tid; idx < nrows * ns; idx += CWARPS * 32) {     // all (maximum, sum) pairs at once
                     const int row = idx / ns, sp = idx - row * ns;
                     const int t = tok0 + row / nheads, hq = kvh * groups + head0 + row % nheads;
-                    ml_s[row][sp] = __ldcg((const float2*)(a.part_ml + (((size_t)a.tok_part_row[t] + sp) * a.nq + hq) * 2));
+                    const float* ml = a.part_ml + (((size_t)a.tok_part_row[t] + sp) * a.nq + hq) * 2;
+                    ml_s[row][sp] = a.part_vec ? __ldcg((const float2*)ml) : make_float2(__ldcg(ml), __ldcg(ml + 1));
                 }
                 compute_sync();
                 if (tid < nrows) {
@@ -539,7 +553,12 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
                     const float* src = a.part_acc + ((size_t)a.tok_part_row[t] * a.nq + hq) * D + e;
                     const size_t step = (size_t)a.nq * D;
                     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int s0 = 0; s0 < ns; s0 += 8) {
+#pragma unroll 1
+                    for (int sp = a.part_vec ? ns : 0; sp < ns; ++sp, src += step) {
+                        const float w = wgt_s[row][sp];
+                        acc.x += w * __ldcg(src); acc.y += w * __ldcg(src + 1); acc.z += w * __ldcg(src + 2); acc.w += w * __ldcg(src + 3);
+                    }
+                    for (int s0 = a.part_vec ? 0 : ns; s0 < ns; s0 += 8) {
                         float4 v[8];
 #pragma unroll
                         for (int q = 0; q < 8; ++q) v[q] = __ldcg((const float4*)(src + (size_t)min(s0 + q, ns - 1) * step));
@@ -555,16 +574,8 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
                     if constexpr (EXT) {
                         const float4 g = gate4_of(a, t, hq, D, e);
                         acc.x *= g.x; acc.y *= g.y; acc.z *= g.z; acc.w *= g.w;
-                        if (a.out_f32) {
-                            *(float4*)((float*)a.out + ((size_t)t * a.nq + hq) * D + e) =
-                                make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-                            continue;
-                        }
                     }
-                    uint2 packed;
-                    packed.x = pack_bf16(acc.x * inv, acc.y * inv);
-                    packed.y = pack_bf16(acc.z * inv, acc.w * inv);
-                    *(uint2*)(a.out + ((size_t)t * a.nq + hq) * D + e) = packed;
+                    store4_out(a, ((size_t)t * a.nq + hq) * D + e, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
                 }
             }
         }
@@ -615,6 +626,13 @@ int launch(const CUtensorMap& map, const AttnArgs& a, int launch_items, cudaStre
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, map, a);
     if (e != cudaSuccess) return fail("attention_tma: launch of clusters of %d: %s", a.cluster, cudaGetErrorString(e));
     return check_launch("attention_tma");
+}
+
+// What can be read and written four elements at a time, by the addresses.
+void set_widths(AttnArgs& a) {
+    a.out_vec = ((uintptr_t)a.out & (a.out_f32 ? 15 : 7)) == 0;
+    a.part_vec = ((uintptr_t)a.part_acc & 15) == 0 && ((uintptr_t)a.part_ml & 7) == 0;
+    a.gate_vec = a.gate && !a.gate_per_head && a.gate_ld % 4 == 0 && a.gate_split_stride % 4 == 0 && ((uintptr_t)a.gate & 15) == 0;
 }
 
 // How many clusters of n CTAs of the kernel with options the device holds at once.
@@ -678,6 +696,7 @@ MHB_EXPORT int mhb_attention_tma(const void* q, const void* cache, void* out, fl
     a.fresh = fresh;
     a.gate_per_head = 0; a.shared_kv = 0; a.softcap = 0.f; a.out_f32 = 0; a.slopes = nullptr; a.cluster = 0; a.gate_vec = 0;
     a.sink = nullptr; a.gate = nullptr; a.gate_nsplit = 1; a.gate_ld = 0; a.gate_split_stride = 0;
+    set_widths(a);
     if (rows == 16) return d == 128 ? launch<128, 16, false>(map, a, launch_items, stream) : launch<64, 16, false>(map, a, launch_items, stream);
     return fail("attention_tma: tile height %d", rows);
 }
@@ -722,7 +741,7 @@ MHB_EXPORT int mhb_attention_tma_ext(const void* q, const void* cache, void* out
                         (cluster + 1) * ((heads + cluster - 1) / cluster) > Layout<128, 16>::RECV_ROWS))
         return fail("attention_tma: clusters of %d for %d items of %d heads are not built", cluster, launch_items, heads);
     a.cluster = cluster;
-    a.gate_vec = gate && !gate_per_head && gate_ld % 4 == 0 && gate_split_stride % 4 == 0 && ((uintptr_t)gate & 15) == 0;
+    set_widths(a);
     if (rows == 16) return d == 128 ? launch<128, 16, true>(map, a, launch_items, stream) : launch<64, 16, true>(map, a, launch_items, stream);
     return fail("attention_tma: tile height %d", rows);
 }

@@ -1023,6 +1023,39 @@ def test_attention_tma_splits_merged_in_a_cluster(nq, nkv, d, P_, nsplit, shared
             torch.testing.assert_close(got, ref, atol=1e-4 if dtype == torch.float32 else 2.0 ** -8 * float(ref.abs().max()), rtol=2.0 ** -8 if dtype == bf else 0)
 
 
+@pytest.mark.parametrize("kind,dtype", [("plain", torch.bfloat16), ("ext", torch.bfloat16), ("ext", torch.float32)])
+@pytest.mark.parametrize("nsplit,merge", [(1, "none"), (3, "counters"), (3, "later"), (2, "cluster")])
+def test_attention_tma_buffers_off_their_vectors(kind, dtype, nsplit, merge):
+    """Outputs and partial buffers that start an element off 8 and 16 bytes get what aligned ones get, bit for bit."""
+    from mini_hisparse_b200.parts.attention import AttentionShape, plan_decode
+
+    if (kind, merge) == ("plain", "cluster"):
+        pytest.skip("the kernel without options merges in no cluster")
+    nq, nkv, d, P_, lengths = 6, 2, 64, 16, [1, 70, 260]
+    g, B = torch.Generator().manual_seed(nsplit), len(lengths)
+    table = torch.arange(B * 17, dtype=torch.int32, device=DEV).view(B, 17)
+    cache = torch.randn(B * 17, 2, nkv, P_, d, generator=g).bfloat16().to(DEV)
+    q = torch.randn(B, nq * d, generator=g).bfloat16().to(DEV)
+    plan = plan_decode(AttentionShape(nq, nkv, None, 128), np.asarray(lengths) - 1, nsplit)
+    items, pos = torch.from_numpy(plan.items).to(DEV).reshape(-1), torch.tensor(lengths, dtype=torch.int32, device=DEV) - 1
+    tpr, tns = (torch.from_numpy(y).to(DEV) for y in (plan.tok_part_row, plan.tok_nsplit))
+    rows, results = max(1, plan.part_rows), []
+    for off in (0, 1):
+        out = torch.full((B * nq * d + 8,), float("nan"), dtype=dtype, device=DEV)
+        acc, ml = torch.full((rows * nq * d + 8,), 3.0, device=DEV), torch.full((rows * nq * 2 + 8,), 3.0, device=DEV)
+        o = out[off: off + B * nq * d].view(B, nq * d)
+        pa, pm = acc[off: off + rows * nq * d].view(rows, nq, d), ml[off: off + rows * nq * 2].view(rows, nq, 2)
+        counters, status = torch.zeros(B * nkv, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        extra = dict(cluster=nsplit) if merge == "cluster" else dict(counters=counters) if merge == "counters" else {}
+        call = K().attention_tma_ext if kind == "ext" else K().attention_tma
+        call(q, cache, o, pa, pm, items, len(plan.items), 16, pos, table, tpr, nq=nq, nkv=nkv, d=d, page_size=P_, tok_nsplit=tns,
+             status=status, **extra)
+        assert int(status) == 0 and bool(out[off + B * nq * d:].isnan().all()) and bool((acc[off + rows * nq * d:] == 3.0).all())
+        results.append([pa.cpu(), pm.cpu()] if merge == "later" else [o.cpu()])
+    for x, y in zip(*results):      # an empty split's partials have a maximum of minus infinity
+        assert torch.equal(x, y) and not bool(x.isnan().any())
+
+
 @pytest.mark.parametrize("ext", [False, True])
 @pytest.mark.parametrize("n", [1, 2, 16])
 def test_attention_tma_early_keys_behind_the_append(ext, n):
