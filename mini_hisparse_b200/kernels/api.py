@@ -902,6 +902,12 @@ def attention_tokens_supports(nq: int, nkv: int, d: int) -> bool:
     return nkv >= 1 and nq % nkv == 0 and nq // nkv <= 8 and 4 <= d <= 128 and d % 4 == 0
 
 
+def attention_tokens_takes(cache, nq: int, nkv: int, d: int) -> bool:
+    """The pool is one that attention_tokens is built for: it counts the pool's rows of ``d`` in 32 bits and reads 16 bytes at
+    a time."""
+    return attention_tokens_supports(nq, nkv, d) and cache.numel() // d <= 0x7FFFFFFF and cache.data_ptr() % 16 == 0
+
+
 def attention_tokens(q, cache, out, part_acc, part_ml, items, num_items, block_table, tok_part_row, *, nq, nkv, d, page_size,
                      scale=None):
     """attention_simt for items of single tokens with all heads of their KV heads, without options: the keys of an item are

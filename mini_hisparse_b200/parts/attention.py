@@ -645,7 +645,7 @@ class GQAttention(Mixer):
                     short_segments()
                 if n_big:
                     long_portions()
-        elif nsplit and K.attention_tokens_supports(self.nq, self.nkv, self.d) and cache.storage.data_ptr() % 16 == 0:
+        elif nsplit and K.attention_tokens_takes(cache.storage, self.nq, self.nkv, self.d):
             K.attention_tokens(*args, meta["items"], n_small, meta["block_table"], meta["tok_part_row"], nq=self.nq, nkv=self.nkv,
                                d=self.d, page_size=cache.page_size, scale=self.scale)
         else:

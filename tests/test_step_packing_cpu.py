@@ -303,6 +303,28 @@ def test_a_decode_buffer_whose_plan_could_not_be_written(monkeypatch):
     assert torch.equal(ring.rows[0], fresh.rows[0])
 
 
+@pytest.mark.parametrize("pages,kernel", [(1 << 20, "attention_tokens"), ((1 << 29) - 1, "attention_tokens"), (1 << 29, "attention_simt")])
+def test_pools_beyond_32_bit_rows_go_to_the_kernel_that_takes_them(monkeypatch, pages, kernel):
+    """Decoded tokens over a pool of 2^31 rows and more: the kernel whose offsets are 64 bits wide, as before there was the other."""
+    from types import SimpleNamespace
+
+    from mini_hisparse_b200.kernels import api as K
+    from mini_hisparse_b200.parts.base import Product
+
+    part, ran = attention(2, 1), []
+    part.rt, part.qkv_weight, part.o_weight = SimpleNamespace(dtype=torch.float32), None, None
+    for name in ("attention_tokens", "attention_simt", "attention_rows", "attention_combine"):
+        monkeypatch.setattr(K, name, lambda *a, name=name, **k: ran.append(name))
+    rt = SimpleNamespace(dtype=torch.float32, linear=lambda *a, **k: Product(torch.zeros(1)), qkv_rope_append=lambda *a, **k: True)
+    ctx = SimpleNamespace(rt=rt, ws=SimpleNamespace(get=lambda name, shape, dtype: torch.zeros(shape, dtype=dtype)), positions=None,
+                          status=None, extras={})
+    _, facts = part.planner(2, 148).plan_decode(np.asarray([5]), (1, 1))
+    view = SimpleNamespace(meta=dict(facts, block_table=None, items=None, tok_part_row=None), page_size=2, writable=True,
+                           storage=torch.empty(pages, 2, 1, 2, 16, device="meta"))
+    part.forward(torch.zeros(1, 32), ctx, view)
+    assert ran == [kernel]
+
+
 class LazyGPU:
     """Streams that run what is queued on them as late as they may: at a synchronise, and at the end.  A copy remembers what its
     source held when it was queued, and looks again when it runs."""
