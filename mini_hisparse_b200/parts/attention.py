@@ -428,7 +428,7 @@ class AttentionPlanner(StepPlanner):
 
     def write_decode(self, starts, fixed, regions, first):
         B, nsplit = len(starts), fixed[0] * fixed[1]
-        if first or nsplit > 1 or self.shape.window:
+        if first or nsplit > 1 or self.shape.window or type(self).plan_decode is not AttentionPlanner.plan_decode:
             return super().write_decode(starts, fixed, regions, first)
         # whole histories: nothing but the ends of the key ranges moves
         regions["items"].reshape(B, self.chunks, ITEM_INTS)[:, :, 6] = (starts + 1)[:, None]

@@ -303,6 +303,22 @@ def test_a_decode_buffer_whose_plan_could_not_be_written(monkeypatch):
     assert torch.equal(ring.rows[0], fresh.rows[0])
 
 
+def test_a_planner_derived_from_attentions_writes_its_own_plan_every_step():
+    """The short cut that moves only the ends of the key ranges is for AttentionPlanner's own plans."""
+    from mini_hisparse_b200.parts.attention import AttentionPlanner, AttentionShape
+
+    class Backwards(AttentionPlanner):
+        def plan_decode(self, starts, fixed):
+            arrays, facts = super().plan_decode(starts, fixed)
+            return dict(arrays, tok_part_row=(1000 + starts).astype(np.int32)), facts
+
+    planner = Backwards(AttentionShape(4, 2), 8)
+    regions = {name: np.zeros(n, np.int32) for name, n in planner.capacity(2, 2, (1, 1)).items()}
+    for step in range(3):
+        planner.write_decode(np.asarray([step, 9]), (1, 1), regions, step == 0)
+        assert regions["tok_part_row"].tolist() == [1000 + step, 1009]
+
+
 @pytest.mark.parametrize("pages,kernel", [(1 << 20, "attention_tokens"), ((1 << 29) - 1, "attention_tokens"), (1 << 29, "attention_simt")])
 def test_pools_beyond_32_bit_rows_go_to_the_kernel_that_takes_them(monkeypatch, pages, kernel):
     """Decoded tokens over a pool of 2^31 rows and more: the kernel whose offsets are 64 bits wide, as before there was the other."""
