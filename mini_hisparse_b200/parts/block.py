@@ -102,7 +102,9 @@ class PostNormBlock(Block):
             h = last.forward_post(x, ctx, out, alpha=self.alpha, keep=self.keep)
             last, out = self.ff_norm, self.feed_forward.forward(h, ctx)
         h = None
-        if self.side is not None and isinstance(last, RMSNorm) and isinstance(self.side, TokenSide):
+        # in one kernel where both steps are the ones that it knows (a part derived from them may bring its own)
+        if (isinstance(last, RMSNorm) and type(last).forward_post is RMSNorm.forward_post
+                and isinstance(self.side, TokenSide) and type(self.side).forward_into is TokenSide.forward_into):
             h = self.side.forward_behind(last, x, out, ctx, self.alpha, self.keep)
         if h is None:
             h = last.forward_post(x, ctx, out, alpha=self.alpha, keep=self.keep)

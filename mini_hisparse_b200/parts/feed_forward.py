@@ -149,8 +149,9 @@ class TokenSide(FeedForward):
         Returns the new rows in the compute dtype, or None where the kernel is not built for the step (more than 32 or 64
         tokens, float32, odd widths): then nothing has been done."""
         rt = ctx.rt
-        if (rt.dtype != torch.bfloat16 or delta is None or delta.also is not None or delta.tensor.dtype != torch.float32
-                or not delta.tensor.is_contiguous() or (delta.nsplit > 1 and delta.split_stride % 4)
+        if (rt.dtype != torch.bfloat16 or delta is None or delta.also is not None
+                or any(t.dtype != torch.float32 or not t.is_contiguous() for t in (x, delta.tensor))
+                or delta.tensor.data_ptr() % 16 or (delta.nsplit > 1 and delta.split_stride % 4)
                 or any(w.dtype != torch.float32 or w.data_ptr() % 16 for w in (norm.weight, self.norm))
                 or not K.side_branch_takes(x, self.gate, self.proj, self.table.weight)):
             return None

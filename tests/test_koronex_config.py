@@ -4,6 +4,7 @@ import copy
 
 import numpy as np
 import pytest
+import torch
 
 from mini_hisparse_b200.config.koronex import KoronexConfig
 from mini_hisparse_b200.config.qwen2 import ConfigError
@@ -67,3 +68,71 @@ def test_chunk_planner_cuts_long_segments_only():
     assert caps["chunks"] >= arrays["chunks"].size and caps["seg_chunks"] >= arrays["seg_chunks"].size
     arrays, facts = planner.plan_decode(np.asarray([3, 4]), planner.decode_fixed(2, 64))
     assert facts == {"num_chunks": 0, "num_long": 0} and arrays["chunks"].size == 0
+
+
+def post_norm_block(norm_class, side_class, ran):
+    """A post-norm block of hand-made parts without a feed-forward: what runs behind its mixer is written down in ``ran``."""
+    from types import SimpleNamespace
+
+    from mini_hisparse_b200.parts.block import PostNormBlock
+
+    block = PostNormBlock.__new__(PostNormBlock)
+    block.alpha, block.keep, block.feed_forward = 1.0, 0.0, None
+    block.mixer = SimpleNamespace(forward=lambda h, ctx, cache: "product")
+    block.mixer_norm, block.side = norm_class.__new__(norm_class), side_class.__new__(side_class)
+    x = torch.zeros(2, 1024)
+    ctx = SimpleNamespace(extras={"x_copy": x}, rt=SimpleNamespace(dtype=torch.bfloat16))
+    block.forward(x, None, ctx, None)
+    return ran
+
+
+def test_parts_derived_from_the_norm_or_the_token_input_keep_their_own_steps(monkeypatch):
+    """One kernel stands for RMSNorm and TokenSide; a part derived from one of them whose step is its own is asked for it."""
+    from mini_hisparse_b200.parts.feed_forward import TokenSide
+    from mini_hisparse_b200.parts.norm import RMSNorm
+
+    ran = []
+    monkeypatch.setattr(TokenSide, "forward_behind", lambda self, *a: ran.append("behind") or "rows")
+    monkeypatch.setattr(RMSNorm, "forward_post", lambda self, *a, **k: ran.append("norm") or "rows")
+    monkeypatch.setattr(TokenSide, "forward_into", lambda self, *a: ran.append("into") or "rows")
+
+    class Norm(RMSNorm):
+        def forward_post(self, x, ctx, delta, alpha=1.0, keep=0.0, name="x_copy"):
+            ran.append("own norm")
+            return "rows"
+
+    class Side(TokenSide):
+        def forward_into(self, x, h, ctx, keep_copy=True):
+            ran.append("own input")
+            return "rows"
+
+    for norm, side, want in ((RMSNorm, TokenSide, ["behind"]), (Norm, TokenSide, ["own norm", "into"]), (RMSNorm, Side, ["norm", "own input"])):
+        ran.clear()
+        assert post_norm_block(norm, side, ran) == want
+
+
+@pytest.mark.parametrize("off", ["nothing", "the product", "the stream's dtype", "the stream's order"])
+def test_the_one_kernel_of_norm_and_token_input_is_asked_only_for_what_it_takes(monkeypatch, off):
+    """A product off 16 bytes or another stream go to the kernels that take them."""
+    from types import SimpleNamespace
+
+    from mini_hisparse_b200.kernels import api as K
+    from mini_hisparse_b200.parts.base import Product
+    from mini_hisparse_b200.parts.feed_forward import TokenSide
+
+    ran = []
+    monkeypatch.setattr(K, "side_branch", lambda *a, **k: ran.append(k))
+    W, D, T = 1024, 16, 2
+    side, bf = TokenSide.__new__(TokenSide), torch.bfloat16
+    side.gate, side.proj, side.norm = torch.zeros(D, W, dtype=bf), torch.zeros(W, D, dtype=bf), torch.ones(W)
+    side.table, side.column0, side.eps = SimpleNamespace(weight=torch.zeros(10, D, dtype=bf)), 0, 1e-5
+    x, room = torch.zeros(T, W), torch.zeros(T * W + 4)
+    if off == "the stream's dtype":
+        x = x.to(bf)
+    if off == "the stream's order":
+        x = torch.zeros(W, T).T
+    delta = Product(room[1 if off == "the product" else 0:][: T * W].view(T, W))
+    ctx = SimpleNamespace(rt=SimpleNamespace(dtype=bf), ws=SimpleNamespace(get=lambda n, shape, dtype: torch.zeros(shape, dtype=dtype)),
+                          tokens=None, status=None)
+    got = side.forward_behind(SimpleNamespace(weight=torch.ones(W), eps=1e-5), x, delta, ctx, 1.0, 0.0)
+    assert (got is None) == (off != "nothing") and len(ran) == (off == "nothing")
