@@ -4,9 +4,7 @@
 // The math, the work items and the tile shape are those of attention_mma.cu
 // (mini_hisparse/model.py:173-179, mini_hisparse/attention.py:26-35): 16 query rows per CTA, the
 // keys of a tile split over the four compute warps, key splits across CTAs merged by the last CTA
-// of a token.  (The 64-row shape of the template is kept for reference but not instantiated: the
-// tcgen05 kernel serves every size this one takes.)  What differs is how keys and
-// values reach shared memory: a fifth warp walks the block table and issues one
+// of a token.  What differs is how keys and values reach shared memory: a fifth warp walks the block table and issues one
 // cp.async.bulk.tensor (TMA) per page, plane and 64-column half, with the 128-byte swizzle, into a
 // ring of stages guarded by full/empty mbarriers.  The compute warps never issue a load, so the
 // ring stays full while they work, which is what a decode step needs: it is bound by how many
@@ -29,6 +27,7 @@ MHB_EXPORT const char* mhb_last_error() { return error_buffer(); }
 
 namespace {
 constexpr int KT = 64;
+constexpr int ROWS = 16;                     // query rows of a tile: two blocks of 8
 constexpr int CWARPS = 4;                    // compute warps
 constexpr int THREADS = (CWARPS + 1) * 32;   // + the TMA warp
 constexpr int ITEM_INTS = 8;
@@ -115,7 +114,7 @@ __device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-template <int D, int ROWS>
+template <int D>
 struct Layout {
     static constexpr int HALVES = D / 64;
     static constexpr int STAGES = 3;
@@ -141,13 +140,12 @@ __device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, %0;" 
 // EXT: the options.  The sink starts ONE thread's running (max, sum) of a row at (sink / scale, 1), in the
 // unsplit item or in split 0 only; the softmax's weights enter the value product as two bfloat16 numbers (the
 // weight and what rounding it lost: 16 bits instead of 8); the output is multiplied by sigmoid(gate).
-template <int D, int ROWS, bool EXT>
+template <int D, bool EXT>
 __global__ void __launch_bounds__(THREADS, 2)
 attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs a) {
-    using L = Layout<D, ROWS>;
+    using L = Layout<D>;
     constexpr int STAGES = L::STAGES;
     constexpr int KSTEPS = D / 16;
-    static_assert(ROWS == 16, "two blocks of 8 query rows");
     extern __shared__ uint8_t smem_raw[];
     __shared__ int row_pos[ROWS];
     __shared__ int cta_failed;      // a bounded wait ran out somewhere in this CTA: it merges and stores nothing
@@ -582,10 +580,10 @@ attention_tma_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnArgs 
     }
 }
 
-template <int D, int ROWS, bool EXT>
+template <int D, bool EXT>
 int configure() {
-    auto kern = attention_tma_kernel<D, ROWS, EXT>;
-    constexpr int smem = Layout<D, ROWS>::TOTAL;
+    auto kern = attention_tma_kernel<D, EXT>;
+    constexpr int smem = Layout<D>::TOTAL;
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -599,11 +597,11 @@ int configure() {
     return 0;
 }
 
-template <int D, int ROWS, bool EXT>
+template <int D, bool EXT>
 int launch(const CUtensorMap& map, const AttnArgs& a, int launch_items, cudaStream_t stream) {
-    auto kern = attention_tma_kernel<D, ROWS, EXT>;
-    constexpr int smem = Layout<D, ROWS>::TOTAL;
-    int rc = configure<D, ROWS, EXT>();
+    auto kern = attention_tma_kernel<D, EXT>;
+    constexpr int smem = Layout<D>::TOTAL;
+    int rc = configure<D, EXT>();
     if (rc) return rc;
     if (a.cluster <= 1) {
         launch_kernel(kern, dim3(launch_items, a.nkv), dim3(THREADS), smem, stream, map, a);
@@ -638,12 +636,12 @@ void set_widths(AttnArgs& a) {
 // How many clusters of n CTAs of the kernel with options the device holds at once.
 template <int D>
 int max_clusters(int n) {
-    int rc = configure<D, 16, true>();
+    int rc = configure<D, true>();
     if (rc) return rc;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n, 1);
     cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = Layout<D, 16>::TOTAL;
+    cfg.dynamicSmemBytes = Layout<D>::TOTAL;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = n;
@@ -652,7 +650,7 @@ int max_clusters(int n) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int k = 0;
-    cudaError_t e = cudaOccupancyMaxActiveClusters(&k, attention_tma_kernel<D, 16, true>, &cfg);
+    cudaError_t e = cudaOccupancyMaxActiveClusters(&k, attention_tma_kernel<D, true>, &cfg);
     if (e != cudaSuccess) return fail("attention_tma: clusters of %d: %s", n, cudaGetErrorString(e));
     return k;
 }
@@ -697,7 +695,7 @@ MHB_EXPORT int mhb_attention_tma(const void* q, const void* cache, void* out, fl
     a.gate_per_head = 0; a.shared_kv = 0; a.softcap = 0.f; a.out_f32 = 0; a.slopes = nullptr; a.cluster = 0; a.gate_vec = 0;
     a.sink = nullptr; a.gate = nullptr; a.gate_nsplit = 1; a.gate_ld = 0; a.gate_split_stride = 0;
     set_widths(a);
-    if (rows == 16) return d == 128 ? launch<128, 16, false>(map, a, launch_items, stream) : launch<64, 16, false>(map, a, launch_items, stream);
+    if (rows == 16) return d == 128 ? launch<128, false>(map, a, launch_items, stream) : launch<64, false>(map, a, launch_items, stream);
     return fail("attention_tma: tile height %d", rows);
 }
 
@@ -738,10 +736,10 @@ MHB_EXPORT int mhb_attention_tma_ext(const void* q, const void* cache, void* out
     a.slopes = slopes;
     const int heads = nq / nkv;
     if (cluster > 1 && (cluster > 16 || heads > 16 || launch_items % cluster || launch_items != num_items ||
-                        (cluster + 1) * ((heads + cluster - 1) / cluster) > Layout<128, 16>::RECV_ROWS))
+                        (cluster + 1) * ((heads + cluster - 1) / cluster) > Layout<128>::RECV_ROWS))
         return fail("attention_tma: clusters of %d for %d items of %d heads are not built", cluster, launch_items, heads);
     a.cluster = cluster;
     set_widths(a);
-    if (rows == 16) return d == 128 ? launch<128, 16, true>(map, a, launch_items, stream) : launch<64, 16, true>(map, a, launch_items, stream);
+    if (rows == 16) return d == 128 ? launch<128, true>(map, a, launch_items, stream) : launch<64, true>(map, a, launch_items, stream);
     return fail("attention_tma: tile height %d", rows);
 }

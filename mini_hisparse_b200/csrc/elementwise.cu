@@ -662,9 +662,8 @@ __global__ void swiglu_kernel(const IT* __restrict__ gu, int nsplit, size_t spli
     out[idx] = from_float<OT>(s * u);
 }
 
-// The same four elements a thread (I and block in steps of 4, rows on 16 bytes), a row of CTAs per token: no 64-bit divisions, wide
-// loads.  562 rows of 18,944 float32: 23.4 us,
-// 54.8 with an element a thread.
+// The same four elements a thread (I and block in steps of 4, rows on 16 bytes), a row of CTAs per token: no 64-bit divisions,
+// wide loads.  562 rows of 18,944 float32: 23.4 us, 54.8 with an element a thread.
 template <typename IT, typename OT>
 __global__ void swiglu_vec_kernel(const IT* __restrict__ gu, int nsplit, size_t split_stride, OT* __restrict__ out, int I, int block) {
     pdl_launch_dependents();

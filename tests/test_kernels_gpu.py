@@ -787,13 +787,13 @@ def test_attention_tokens_scores_beyond_float32():
 @pytest.mark.parametrize("window", [None, 70])
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_tokens(nq, nkv, d, P_, nsplit, window, dtype):
-    """Decoded tokens on the CUDA cores with the keys dealt to warps: histories around a warp's run of 32 keys and a round of
-    256, odd pages, splits (empty ones too), a window, against 64 bits."""
+    """Decoded tokens on the CUDA cores with the keys dealt to warps: histories around a warp's run of 32 keys, half a round and
+    one and two rounds of 512 (the second fetches its rows ahead), odd pages, splits (empty ones too), a window, against 64 bits."""
     from mini_hisparse_b200.parts.attention import AttentionShape, plan_decode
 
     assert K().attention_tokens_supports(nq, nkv, d)
     g = torch.Generator().manual_seed(nq * d + nsplit)
-    lengths = [1, 31, 32, 33, 255, 256, 257, 600]
+    lengths = [1, 31, 32, 33, 255, 256, 257, 511, 512, 513, 600, 1025]
     B, need = len(lengths), [-(-n // P_) for n in lengths]
     order = torch.randperm(sum(need), generator=g).tolist()
     table = torch.full((B, max(need) + 1), -1, dtype=torch.int32)
