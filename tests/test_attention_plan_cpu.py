@@ -222,3 +222,14 @@ def test_shares_of_decoded_tokens_on_the_cuda_cores():
     assert [shares(28, 4, 128, B, 8192) for B in (1, 2, 4, 8, 16, 37, 38, 100)] == [16, 16, 9, 4, 2, 1, 1, 1]
     assert [shares(3, 1, 32, B, 1024) for B in (4, 37, 38, 64)] == [4, 4, 1, 1]
     assert shares(28, 4, 128, 1, 32768, window=700) == 1 and shares(28, 4, 128, 1, 32768, window=1100) == 4
+
+
+def test_shares_beyond_four_and_eight_are_longer():
+    """The fused decode kernel's planner: shares of 128 keys; beyond four of them (eight of a lone request) of 192, unless
+    several requests have sixteen."""
+    from mini_hisparse_b200.parts.attention import KEY_TILE, AttentionPlanner
+
+    planner = AttentionPlanner(AttentionShape(28, 4, None, 128), 148, lambda n: 148, 16, min_share=2 * KEY_TILE, wide_share=3 * KEY_TILE)
+    sizes = (100, 256, 512, 768, 1024, 2048, 4096)
+    assert [planner.decode_fixed(1, n) for n in sizes] == [(n, 1) for n in (1, 2, 4, 6, 8, 10, 16)]
+    assert [planner.decode_fixed(2, n) for n in sizes] == [(n, 1) for n in (1, 2, 4, 4, 5, 16, 16)]
