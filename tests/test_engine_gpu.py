@@ -335,3 +335,46 @@ def test_command_line_generate(folders, tmp_path):
     assert report["outputs"]["0"] == P.generate(pc, w, prompt, 6)
     assert report["requests"]["0"] == {"prefill_count": 1, "decode_count": 5, "generated_tokens": 6}
     assert json.loads(res.stdout)["outputs"] == report["outputs"]
+
+
+@pytest.mark.parametrize("width", [16, 8192])
+@pytest.mark.parametrize("way", ["at the step", "ahead", "streams"])
+def test_decode_steps_queued_behind_a_busy_gpu(folders, width, way):
+    """More steps of one captured graph than it has host buffers (eight, or two of a large layout), queued while the GPU is busy
+    with something else: each gives what the same step gives launch by launch, waited for.  Packed at the step, ahead of it (for
+    another order of the requests every third time, which is dropped), and on two streams in turn."""
+    from mini_hisparse_b200 import CacheConfig, CacheManager
+    from mini_hisparse_b200.engine import ModelRunner, StepEntry
+
+    model = load(folders["B"], "float32")
+    vocab, got = TINY["B"][0]["vocab_size"], {}
+    for graphs in (False, True):
+        cache = CacheManager(model.cache_needs, CacheConfig(num_pages=8200, page_size=4, max_requests=3, dtype=torch.float32))
+        runner = ModelRunner(model, cache, use_graphs=graphs)
+        runner._table_width = lambda last: width
+        for i, r in enumerate("abc"):
+            cache.open(r)
+            runner.step([StepEntry(r, random_tokens(vocab, 3 + 7 * i, i), [])])
+        tokens = random_tokens(vocab, 3 * 22, 9)
+        side, out = torch.cuda.Stream(), got.setdefault(graphs, [])
+        for step in range(22):
+            order = ["abc", "cab"][step // 3 % 2]
+            if graphs and step == 1:
+                torch.cuda.synchronize()
+                torch.cuda._sleep(100_000_000)         # some 50 ms of the GPU's time; the steps wait behind it
+            entries = [StepEntry(r, [t], [0]) for r, t in zip(order, tokens[3 * step:])]
+            stream = side if graphs and way == "streams" and step // 5 % 2 else torch.cuda.current_stream()
+            stream.wait_stream(torch.cuda.current_stream() if stream is side else side)
+            with torch.cuda.stream(stream):
+                out.append(runner.step(entries).clone())
+            if way == "ahead":
+                runner.prepare_decode_ahead(list("abc" if step % 3 else "bca"))
+            if not graphs:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        runner.check_status()
+        if graphs:
+            (graph,) = runner.graphs.values()
+            assert graph.buffers.ring == (8 if width == 16 else 2) and runner.stats["graph_steps"] == 22
+    for step, (a, b) in enumerate(zip(got[True], got[False])):
+        torch.testing.assert_close(a, b, atol=1e-5, rtol=1e-5, msg=lambda m: f"step {step}: {m}")
