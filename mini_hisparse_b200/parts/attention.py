@@ -240,17 +240,17 @@ class AttentionPlanner(StepPlanner):
 
     def __init__(self, shape: AttentionShape, sm_count: int, clusters_of=None, max_cluster: int = 0,
                  min_share: int = MIN_KEYS_PER_SPLIT, max_groups: int = MAX_SPLITS, token_share: int = 0,
-                 max_ctas: int = 0, memory_merge: bool = False, wide_share: int = 0):
+                 max_ctas: int = 0, memory_merge: bool = False, wide_shares: tuple[int, int] = ()):
         """``clusters_of(n)``: how many clusters of n CTAs the mixer's decode kernel can run at once, if
         it merges a token's key splits inside a cluster of up to ``max_cluster`` CTAs (None: it does not).
-        ``min_share``: keys that a share of a cluster has at least (``wide_share``: beyond four shares, or eight of a
-        lone request; see GQAttention.planner); ``max_groups``: clusters per token and KV head;
+        ``min_share``: keys that a share of a cluster has at least (``wide_shares``: beyond eight shares of a lone request,
+        and beyond four of several; see GQAttention.planner); ``max_groups``: clusters per token and KV head;
         ``max_ctas``: CTAs of a launch of clusters (0: as many as are resident); ``memory_merge``: the kernel merges
         splits through global memory too, which a plan of n clusters of ONE share asks for (see _merged);
         ``token_share``: the kernel is attention_tokens, one CTA of which fills an SM and walks that many keys in a round
         (0: two CTAs an SM, splits as the shape says)."""
         self.min_share, self.max_groups, self.token_share, self.max_ctas = min_share, max_groups, token_share, max_ctas
-        self.memory_merge, self.wide_share = memory_merge, wide_share
+        self.memory_merge, self.wide_shares = memory_merge, wide_shares
         self.shape, self.sm_count = shape, sm_count
         self.resident = sm_count if token_share else 2 * sm_count        # CTAs that run at once
         self.clusters_of, self.max_cluster = clusters_of, max_cluster
@@ -323,9 +323,10 @@ class AttentionPlanner(StepPlanner):
         fit = min(MAX_SPLITS, self.resident // ctas)
         plain = n = max(1, min(fit, self._most_splits(max_positions, fit)))
         if self.clusters_of is not None and self.chunks == 1:
-            most, few = max_positions // self.min_share, 4 if segments_count > 1 else 8
-            if self.wide_share and most > few and (segments_count == 1 or most < self.max_cluster):
-                most = max(few, max_positions // self.wide_share)
+            most, several = max_positions // self.min_share, segments_count > 1
+            few = 4 if several else 8
+            if self.wide_shares and most > few and not (several and most >= self.max_cluster):
+                most = max(few, max_positions // self.wide_shares[several])
             n = max(n, min(self.resident // ctas, self.max_cluster, most))
         if self.clusters_of is None or self.chunks != 1 or n == 1:
             return n, 1
@@ -531,13 +532,14 @@ class GQAttention(Mixer):
         shape = AttentionShape(self.nq, self.nkv, self.window, self.big_tile_rows(page_size),
                                cuda_cores=self.kernel_family(page_size) == "simt")
         if self.kernel_family(page_size) == "tc" and self.nq // self.nkv <= ROW_TILE:
-            # Inside a step of several requests a cluster of five does as well as one of eight or better, one of sixteen as
-            # well as one of ten or better; a lone request's clusters of eight do better than either (four layers of the 7B
-            # shape over graphs for 1,024 keys, shares of 4 / 5 / 8: 1 request of 900 keys 522.5 / 519.5 / 513.7 us, 2 of 600
-            # 522.0 / 517.5 / 521.0, 8 545.9 / 544.7 / 548.3; 16 heads of 64 over 4: 2 of 600 127.5 / 125.9 / 132.8, 2 of 2,000 in
-            # 10 / 16 140.5 / 137.4, 1 of 2,000 in 8 / 16 131.0 / 137.4).
+            # Inside a step of several requests a cluster of six does as well as one of eight or better, one of sixteen as
+            # well as one of ten or better; a lone request's clusters of eight do better than smaller and larger ones (four
+            # layers over graphs for 1,024 keys, shares of 4 / 5 / 6 / 8, us: 7B shape, 2 requests of 560 keys 525.8 / 523.0 / 522.5 /
+            # 525.5, 8 of 1,000 550.0 / 550.4 / 544.6 / 548.3; 16 heads of 64 over 4, 2 of 1,000 131.2 / 131.6 / 128.7 / 136.3, 1 of
+            # 900 129.5 / 127.5 / 126.0 / 124.8; over graphs for 2,048 keys 2 of 2,000 in 10 / 16 140.5 / 137.4, 1 in 10 / 16
+            # 131.6 / 135.7).
             return AttentionPlanner(shape, sm_count, lambda n: K.attention_decode_max_clusters(self.d, n),
-                                    K.DECODE_MAX_SPLITS, min_share=2 * KEY_TILE, wide_share=3 * KEY_TILE)
+                                    K.DECODE_MAX_SPLITS, min_share=2 * KEY_TILE, wide_shares=(3 * KEY_TILE, 5 * KEY_TILE // 2))
         if self.kernel_family(page_size) == "simt" and K.attention_tokens_supports(self.nq, self.nkv, self.d):
             return AttentionPlanner(shape, sm_count, token_share=KEYS_PER_TOKEN_SPLIT)
         return AttentionPlanner(shape, sm_count)

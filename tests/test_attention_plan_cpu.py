@@ -225,11 +225,12 @@ def test_shares_of_decoded_tokens_on_the_cuda_cores():
 
 
 def test_shares_beyond_four_and_eight_are_longer():
-    """The fused decode kernel's planner: shares of 128 keys; beyond four of them (eight of a lone request) of 192, unless
-    several requests have sixteen."""
+    """The fused decode kernel's planner: shares of 128 keys; beyond eight of them of 192 for a lone request, beyond four of 160
+    for several, unless these have sixteen."""
     from mini_hisparse_b200.parts.attention import KEY_TILE, AttentionPlanner
 
-    planner = AttentionPlanner(AttentionShape(28, 4, None, 128), 148, lambda n: 148, 16, min_share=2 * KEY_TILE, wide_share=3 * KEY_TILE)
+    planner = AttentionPlanner(AttentionShape(28, 4, None, 128), 148, lambda n: 148, 16, min_share=2 * KEY_TILE,
+                               wide_shares=(3 * KEY_TILE, 5 * KEY_TILE // 2))
     sizes = (100, 256, 512, 768, 1024, 2048, 4096)
     assert [planner.decode_fixed(1, n) for n in sizes] == [(n, 1) for n in (1, 2, 4, 6, 8, 10, 16)]
-    assert [planner.decode_fixed(2, n) for n in sizes] == [(n, 1) for n in (1, 2, 4, 4, 5, 16, 16)]
+    assert [planner.decode_fixed(2, n) for n in sizes] == [(n, 1) for n in (1, 2, 4, 4, 6, 16, 16)]
